@@ -1,0 +1,78 @@
+"""The leaf searches that give each block N lanes of a warp, where such a split can go wrong: job counts
+around a warp's and a CTA's blocks, rejected jobs among good ones, displayed windows that cut a block at
+every remainder of the weighted SSE's tiles, levels of every size class (empty blocks, above 63, Golomb
+tails), no trellis, a tight tx-search bound.  Bit for bit against the oracle."""
+import os
+
+import numpy as np
+import pytest
+
+from maroontree_b200 import abi, synth
+
+W, H = 208, 144
+
+
+def _case(kind, seed):
+    """Source, reconstruction of a content kind."""
+    rng = np.random.default_rng(seed)
+    if kind == "flat":  # every block predicted exactly somewhere, small residuals elsewhere
+        src = np.full((H, W), 90, np.uint16)
+        src[:, W // 2:] += rng.integers(0, 3, (H, W - W // 2)).astype(np.uint16)
+    elif kind == "hard":  # full-scale noise: long runs of large levels
+        src = np.where(rng.random((H, W)) < 0.5, 0, 255).astype(np.uint16)
+    else:
+        src = synth.rgb_to_luma(synth.generate_rgb(W, H, seed))
+    return src, synth.synthetic_recon(src, seed + 5)
+
+
+def _jobs(family, seed):
+    modes, deltas = range(13), (-2, 0, 3)
+    if family == "quad32" or family == "grid16":
+        return synth.leaf64_jobs(W, H, modes, deltas, seed=seed, grid=family == "grid16")
+    return synth.leaf8_jobs(W, H, modes, deltas, seed=seed, n=32 if family == "leaf32" else 16)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("family", ["leaf16", "refine16", "leaf32", "quad32", "grid16"])
+@pytest.mark.parametrize("n,kind,qidx,vis,wsse,lam0", [
+    (1, "photo", 70, None, 0.0, 0.05),        # one block: idle lanes in its warp
+    (2, "hard", 1, (203, 139), 1.0, 0.05),    # the finest steps: Golomb levels
+    (7, "flat", 200, (197, 133), 0.5, 0.3),   # empty blocks
+    (9, "hard", 40, (190, 100), 1.0, 0.0),    # no trellis; blocks past the displayed frame
+    (41, "photo", 1, (201, 130), 0.0, 0.9),
+    (83, "photo", 140, (199, 141), 1.0, 0.2),
+])
+def test_lane_leaves_match_oracle(mt_lib, oracle_lib, cuda, family, n, kind, qidx, vis, wsse, lam0):
+    src, rec = _case(kind, qidx + n)
+    size = 32 if family in ("leaf32", "quad32") else 16
+    qm_level = 15 if qidx == 1 else 4 + qidx % 9
+    q = oracle_lib.quant_new(qidx, 8, qm_level)
+    qm = oracle_lib.qm_row(qm_level, 0, size) if qm_level < 15 else None
+    c = oracle_lib.default_cdfs(oracle_lib.qcat(qidx), size)
+    rng = np.random.default_rng(n)
+    jobs = _jobs(family, n)
+    jobs = jobs[rng.permutation(len(jobs))[:n]]  # mixed modes in a warp
+    for i in range(2, n, 5):  # rejected: outside the frame, or no such mode
+        if i % 2:
+            jobs["mode"][i] = 13
+        else:
+            jobs["px"][i] = W - 8
+    prm = mt_lib.split16_params(W, H, trellis_lambda0=lam0, rd_lambda=0.02 if kind == "hard" else 0.5 * qidx + 1.0,
+                                band_tilt=1.9 if n % 2 else 0.0, wsse_scale=wsse, tx_guard_shift=2, vis=vis,
+                                skip_bits=[(2.5 + k, 0.4) for k in range(13)] if n % 3 else None)
+    costs, threads = mt_lib.coef_costs(c), os.cpu_count() or 1
+    args, oargs = (src, rec, prm, q, qm, costs, jobs), (src, rec, prm, q, qm, c, jobs)
+    if family == "quad32":
+        got, want = [mt_lib.quad32_luma(*args)], [oracle_lib.quad32_luma(*oargs, threads=threads)]
+    elif family == "grid16":
+        got = mt_lib.grid16_luma(*args, want_cf=True)
+        want = oracle_lib.grid16_luma(*oargs, threads=threads, want_cf=True)
+    elif family == "leaf32":
+        got = mt_lib.leaf32(*args, want_cf=True, want_rec=True)
+        want = oracle_lib.leaf32(*oargs, threads=threads)
+    else:
+        refine = family == "refine16"
+        got = mt_lib.leaf16(*args, refine=refine, want_cf=True, want_rec=True)
+        want = oracle_lib.leaf16(*oargs, refine=refine, threads=threads)
+    for a, b in zip(got, want):
+        assert np.asarray(a).tobytes() == np.asarray(b).tobytes()
