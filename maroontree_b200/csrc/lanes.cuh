@@ -290,9 +290,11 @@ __device__ __forceinline__ void lane_predict(const R& rd, int fw, int fh, int ox
 }
 
 // Forward transform + quantisation (+ the QM of the 2-D types) of src - pred
-// into w.cf / w.tf: fwd8x8 / fwd16x16 / fwd32x32 and apply_qm.  qs: the
-// forward scale of each QM weight value.  8x8 and 32x32 take the 2-D types
-// only (32x32: DCT_DCT).  Returns the sum of the residual.
+// into w.cf / w.tf: fwd8x8 / fwd16x16 and apply_qm; at 32x32 the residual gets
+// 6 bits of headroom and each output the 64-bit rounding (x * 16384 + 2^21) >>
+// 22 of dct32x32_quant_t_direct (src/dct.rs:705-736).  qs: the forward scale of
+// each QM weight value.  8x8 and 32x32 take the 2-D types only (32x32:
+// DCT_DCT).  Returns the sum of the residual.
 template <int N, typename W>
 __device__ __forceinline__ int32_t lane_fwd(const uint16_t* __restrict__ src, int stride, int tx, const mt_quant& q,
                                             const uint8_t* qm, const float* qs, W& w, const Lanes<N>& g) {
@@ -796,8 +798,8 @@ __device__ __forceinline__ int lane_trellis_plain(W& w, float dc_q, float ac_q, 
   return keep - 1;
 }
 
-// Dequantisation and inverse transform of w.cf (inv8x8 / inv16x16 / inv32x32),
-// the reconstruction clamp(pred + inverse) into w.rec() and the error against
+// Dequantisation and inverse transform of w.cf (inv8x8 / inv16x16; TX_32X32
+// halves the masked product, src/idct.rs:2281-2320), the reconstruction clamp(pred + inverse) into w.rec() and the error against
 // the displayed part (vw x vh) of the source, 0 past it, into w.tf (int32,
 // row-major).
 template <int N, typename W>

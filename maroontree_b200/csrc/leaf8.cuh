@@ -30,10 +30,6 @@ __device__ __forceinline__ float hi_cost(const mt_coef_costs& T, uint32_t m, int
 }
 
 __constant__ uint16_t kScan32[1024] = {MT_SCAN_32X32_LIST};
-// The 32x32 default scan as trellis_sq's accessor.
-struct Scan32 {
-  __device__ __forceinline__ int operator()(int i) const { return kScan32[i]; }
-};
 
 // Default scan of a W x W block (scan index -> rc = x*W + y).
 template <int W>
@@ -510,22 +506,6 @@ __host__ bool arena_launch_shape(K kernel, int n, int stride, int cap, int* thre
 // and left coefficient-context bytes.
 __constant__ uint8_t kSkipCtxTbl[5][5] = {
     {1, 2, 2, 2, 3}, {2, 4, 4, 4, 5}, {2, 4, 4, 4, 5}, {2, 4, 4, 4, 5}, {3, 5, 5, 5, 6}};
-
-// coef_res_ctx of a W x W transform (levels column-major, the default scan).
-template <int W, typename C>
-__device__ __forceinline__ uint8_t coef_res_ctx_w(const C* __restrict__ cf) {
-  int eob = -1;
-  for (int i = W * W - 1; i >= 0; i--)
-    if (cf[scan_rc<W>(i)] != 0) {
-      eob = i;
-      break;
-    }
-  if (eob < 0) return 0x40;
-  uint32_t cul = 0;
-  for (int i = 0; i <= eob && cul < 63u; i++) cul += uabs(cf[scan_rc<W>(i)]);
-  const uint32_t dcb = cf[0] == 0 ? 0x40u : (cf[0] < 0 ? 0u : 0x80u);
-  return (uint8_t)(min(cul, 63u) | dcb);
-}
 
 // coef_res_ctx: min(cumulative level, 63) | the dc-sign marker (0x40 zero,
 // 0x00 negative, 0x80 positive), or 0x40 for an all-zero block.

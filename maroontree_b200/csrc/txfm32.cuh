@@ -1,9 +1,7 @@
-// Device 32x32 DCT_DCT of the luma leaf (the only TX_32X32 intra type): the
-// forward transform with quantisation -- the reference's integer butterflies,
-// dct1d_32_i32 built on the 16-point one (src/dct.rs:589-631), on a residual
-// with 6 bits of headroom and the 64-bit rounding of
-// dct32x32_quant_t_direct (src/dct.rs:705-736) -- and the dav1d inverse with
-// the TX_32X32 dequantisation (src/idct.rs:2130-2320).
+// The 1-D passes of the 32x32 DCT_DCT (the only TX_32X32 intra type): the
+// reference's integer butterflies, dct1d_32_i32 built on the 16-point one
+// (src/dct.rs:589-631), and the dav1d inverse (src/idct.rs:2130-2279).
+// lanes.cuh runs them over a block's rows and columns.
 #pragma once
 #include <stdint.h>
 
@@ -36,39 +34,6 @@ __device__ __forceinline__ void fdct32(int32_t* v) {
   for (int i = 0; i < 16; i++) {
     v[2 * i] = t[i];
     v[2 * i + 1] = t[16 + i];
-  }
-}
-
-// Forward 32x32 DCT + quantisation of a row-major residual into column-major
-// levels and f32 targets: columns (x 64 headroom), rows, each output
-// (x * 16384 + 2^21) >> 22 in 64 bits, quantised with the Q16 multipliers.
-// The QM step is applied by the caller.  t: 1024 words.
-template <typename I, typename C>
-__device__ void fwd32x32(const I* __restrict__ in, const mt_quant& q, C* __restrict__ cf, float* __restrict__ tf,
-                         int32_t* __restrict__ t) {
-#pragma unroll 1
-  for (int x = 0; x < 32; x++) {
-    int32_t v[32];
-#pragma unroll
-    for (int r = 0; r < 32; r++) v[r] = (int32_t)in[r * 32 + x] * 64;
-    fdct32(v);
-#pragma unroll
-    for (int r = 0; r < 32; r++) t[r * 32 + x] = v[r];
-  }
-#pragma unroll 1
-  for (int r = 0; r < 32; r++) {
-    int32_t v[32];
-#pragma unroll
-    for (int u = 0; u < 32; u++) v[u] = t[r * 32 + u];
-    fdct32(v);
-#pragma unroll
-    for (int u = 0; u < 32; u++) {
-      const int idx = u * 32 + r;
-      const int32_t m = idx == 0 ? q.q_mult_dc : q.q_mult_ac;
-      const int32_t c = (int32_t)(((long long)v[u] * 16384 + (1ll << 21)) >> 22);
-      cf[idx] = (C)quant_q16(c, m);
-      tf[idx] = __fmul_rn(__fmul_rn((float)c, (float)m), 1.0f / 65536.0f);
-    }
   }
 }
 
@@ -132,32 +97,6 @@ __device__ __forceinline__ void idct32s(int32_t* c, int s, int32_t mn, int32_t m
     c[k * s] = cl(e[k] + o[k]);
     c[(31 - k) * s] = cl(e[k] - o[k]);
   }
-}
-
-// Dequantisation of TX_32X32 (src/idct.rs:2281-2320: the product masked to
-// 24 bits, then halved, clamped to cf_max) and the 2-D inverse:
-// tmp[y*32+x] = coeff[y + x*32]; rows (row clip), (t+2)>>2 with the column
-// clip, columns, (t+8)>>4.  qm: the dequantisation weights (NULL: flat).
-template <typename C, typename O>
-__device__ void inv32x32(const C* __restrict__ cf, const mt_quant& q, const uint8_t* __restrict__ qm,
-                         O* __restrict__ out, int32_t* __restrict__ t) {
-#pragma unroll 4
-  for (int rc = 0; rc < 1024; rc++) {
-    const int32_t l = cf[rc];
-    const int32_t base = rc == 0 ? q.dc_q : q.ac_q;
-    const int32_t step = qm ? ((base * (int32_t)qm[rc] + 16) >> 5) : base;
-    int32_t mag = (int32_t)(((uabs(l) * (uint32_t)step) & 0xffffffu) >> 1);
-    mag = min(mag, q.cf_max + (l < 0 ? 1 : 0));
-    t[(rc & 31) * 32 + (rc >> 5)] = l == 0 ? 0 : (l < 0 ? -mag : mag);
-  }
-#pragma unroll 1
-  for (int y = 0; y < 32; y++) idct32s(t + y * 32, 1, q.rmin, q.rmax);
-#pragma unroll 4
-  for (int i = 0; i < 1024; i++) t[i] = clampi((t[i] + 2) >> 2, q.cmin, q.cmax);
-#pragma unroll 1
-  for (int x = 0; x < 32; x++) idct32s(t + x, 32, q.cmin, q.cmax);
-#pragma unroll 4
-  for (int i = 0; i < 1024; i++) out[i] = (O)((t[i] + 8) >> 4);
 }
 
 }  // namespace mtd

@@ -1,25 +1,17 @@
-// The 16x16 leaf's 4:2:0 chroma search (pick_uv16_420,
-// src/coder/block16.rs:980-1381) with the shipped tuning (uv16_joint on,
-// uv8_joint_k 4, cfl_alpha_rd_steps 0), batched over leaves, one thread per
-// leaf.  The 8x8 chroma block of each leaf runs the DC path, the CfL path
-// (the AC of the 16x16 luma reconstruction, the closed-form alphas) and the
-// joint (mode, delta) SATD shortlist, whose first joint_k entries are priced
-// in full; every priced candidate goes through the same per-plane chain:
-// prediction, the transform (DCT_DCT, or the uv mode's type for the
-// shortlist) with the QM, the chroma trellis (trellis_optimize_ctx against
-// the chroma TX_8X8 costs), preserve_dc where the reference applies it, the
-// inverse, sse_recon and chroma_bits.  The candidate and the winner live in
-// the two slots of UvWork; a candidate that wins swaps them.
+// The leaves' chroma searches, batched over leaves: pick_uv16_420
+// (src/coder/block16.rs:980-1381), pick_uv16_444 (:437-978), pick_uv32_420
+// (src/coder/block32.rs:2797-3120) and pick_uv32_444 (:2264-2720) with the
+// shipped tuning (uv16_joint on, uv8_joint_k 4, cfl_alpha_rd_steps 0).  Each
+// leaf runs the DC path, the CfL path (the AC of the leaf's luma
+// reconstruction, the closed-form alphas) and the SATD-ranked directional
+// stage; every priced candidate goes through the same per-plane chain
+// (plane_chain).  A leaf is a CTA, a plane of a candidate N lanes of it.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <type_traits>
-
 #include "../../include/maroontree_b200.h"
 #include "common.cuh"
-#include "leaf8.cuh"
-#include "txfm32.cuh"
-#include "wsse.cuh"
+#include "lanes.cuh"
 
 namespace mth {
 float scaled_trellis_lambda_host(float dc_q, float lambda0);
@@ -29,7 +21,6 @@ namespace {
 
 using namespace mtd;
 
-constexpr int kUvThreads = 32;  // one warp per CTA: 8,040 leaves at 1080p reach every SM
 constexpr int kJointModes = 12;
 constexpr int kMaxJoint = 12;
 
@@ -39,22 +30,6 @@ struct UvArgs {
   mt_quant q;           // the chroma quantiser
   float lambda;         // scaled_trellis_lambda of the chroma trellis (0: off)
   int has_qm;
-};
-
-// Both planes of one candidate: predictions, levels and inverses.
-struct UvSlot {
-  int16_t pred[2][64];
-  int16_t cf[2][64];
-  int16_t rr[2][64];
-};
-
-struct UvWork {
-  UvSlot s[2];     // the candidate and the winner
-  int32_t u[128];  // prediction edges, then the targets [0, 64) and the transform temporary [64, 128)
-  int16_t resid[64];
-  int16_t ac[64];  // CfL AC of the leaf's luma
-  TrellisCtxScratch tr;
-  alignas(16) uint8_t lv[160];  // the rate walk stores it as 32-bit words
 };
 
 // The shortlist's modes in the reference's order (block16.rs:1143-1156).
@@ -92,8 +67,8 @@ __device__ float uv_mode_bits(const mt_uv_mode_costs& C, int y_mode, int uv, boo
   return bits;
 }
 
-// Per-plane constants of a job: source / reconstruction origins, displayed
-// extent, coefficient contexts.
+// One plane of a leaf: source / reconstruction origins, displayed extent,
+// coefficient contexts.
 struct UvPlane {
   const uint16_t* src;  // block origin
   const uint16_t* rec;  // plane base
@@ -102,450 +77,262 @@ struct UvPlane {
   float skip1, skip0;
 };
 
-// One plane of a candidate after its prediction: residual, transform with
-// the QM, trellis, preserve_dc (src/rd_sse.rs:759-765) when `keep_dc`,
-// inverse, sse_recon and the rate.  Returns the plane's rd_cost_i64.
-__device__ float plane_chain(const UvArgs& a, const UvPlane& P, const mt_coef_costs& T, const uint8_t* qm,
-                             const float* sQs, int tx, bool keep_dc, int16_t* pred, int16_t* cf, int16_t* rr,
-                             UvWork& w) {
-  const mt_split16_params& p = a.p;
-  const mt_quant& q = a.q;
-  int32_t sum = 0;
-#pragma unroll 8
-  for (int i = 0; i < 64; i++) {
-    const int32_t r = (int32_t)P.src[(size_t)(i >> 3) * p.stride + (i & 7)] - pred[i];
-    w.resid[i] = (int16_t)r;
-    sum += r;
-  }
-  float* tf = reinterpret_cast<float*>(w.u);
-  int32_t* tmp = w.u + 64;
-  fwd8x8(w.resid, tx, q, cf, tf, tmp);
-  if (qm) apply_qm(cf, tf, sQs, 64);
-  if (a.lambda > 0.0f)
-    trellis_ctx8(cf, tf, (float)q.dc_q, (float)q.ac_q, a.lambda, T, P.ds, qm, q.qm_level >= 5, p.band_tilt, w.tr);
-  if (keep_dc) {
-    const int32_t mean = sum / 64;  // truncating, as the reference's i32 division
-    if (cf[0] == 0 && abs(mean) >= 8) cf[0] = (int16_t)(mean > 0 ? 1 : -1);
-  }
-  inv8x8(cf, tx, q, qm, rr, tmp);
-  ErrBlock<int16_t, int16_t> eb;
-  eb.src = P.src;
-  eb.stride = p.stride;
-  eb.pred = pred;
-  eb.resid = rr;
-  eb.w = 8;
-  eb.vw = P.vw;
-  eb.vh = P.vh;
-  eb.maxv = (1 << p.bd) - 1;
-  const long long sse = sse_recon_block(eb, p.wsse_scale);
-  const float bits = rate_bounded<8>(cf, T, P.sk, P.ds, 0, -1, p.use_skip_bits != 0, P.skip1, P.skip0,
-                                     __int_as_float(0x7f800000), w.lv);
-  return rd_cost_i64(sse, p.rd_lambda, bits);
-}
-
-// cfl_best_alpha (src/intrapred.rs:1211-1258) over the displayed part: the
-// closed-form alpha, then the first minimum of the prediction's SSE over
-// alpha - 3 .. alpha + 3 within +-16.
-__device__ int cfl_alpha(const int16_t* ac, const UvPlane& P, int stride, int32_t dc, int32_t maxv) {
-  long long num = 0, den = 0;
-  for (int y = 0; y < P.vh; y++)
-    for (int x = 0; x < P.vw; x++) {
-      const long long v = ac[y * 8 + x];
-      num += (long long)((int32_t)P.src[(size_t)y * stride + x] - dc) * v;
-      den += v * v;
-    }
-  if (den == 0) return 0;
-  const long long sg = num > 0 ? 1 : (num < 0 ? -1 : 0);
-  long long a0 = (64 * num + (den >> 1) * sg) / den;
-  a0 = a0 < -16 ? -16 : (a0 > 16 ? 16 : a0);
-  long long best_e = 0x7fffffffffffffffLL;
-  int best_a = 0;
-  for (int c = (int)a0 - 3; c <= (int)a0 + 3; c++) {
-    if (c < -16 || c > 16) continue;
-    long long e = 0;
-    for (int y = 0; y < P.vh; y++)
-      for (int x = 0; x < P.vw; x++) {
-        const long long d = (int32_t)P.src[(size_t)y * stride + x] - cfl_pred_pixel(dc, ac[y * 8 + x], c, maxv);
-        e += d * d;
-      }
-    if (e < best_e) {
-      best_e = e;
-      best_a = c;
-    }
-  }
-  return best_a;
-}
-
-__global__ void __launch_bounds__(kUvThreads) uv16_420_kernel(
-    const uint16_t* __restrict__ src_u, const uint16_t* __restrict__ src_v, const uint16_t* __restrict__ rec_u,
-    const uint16_t* __restrict__ rec_v, const uint16_t* __restrict__ luma, UvArgs a,
-    const uint8_t* __restrict__ qm_row, const mt_coef_costs* __restrict__ costs,
-    const mt_uv_mode_costs* __restrict__ mode_costs, const mt_uv16_job* __restrict__ jobs, int n,
-    mt_uv16_result* __restrict__ res, int32_t* __restrict__ cf_out, uint16_t* __restrict__ rec_out, int arena) {
-  __shared__ mt_coef_costs sT;
-  __shared__ mt_uv_mode_costs sM;
-  __shared__ uint8_t sQm[64];
-  __shared__ float sQs[64];
-  {
-    const float* g = reinterpret_cast<const float*>(costs);
-    float* s = reinterpret_cast<float*>(&sT);
-    for (int i = threadIdx.x; i < (int)(sizeof(mt_coef_costs) / 4); i += blockDim.x) s[i] = g[i];
-    const float* gm = reinterpret_cast<const float*>(mode_costs);
-    float* sm = reinterpret_cast<float*>(&sM);
-    for (int i = threadIdx.x; i < (int)(sizeof(mt_uv_mode_costs) / 4); i += blockDim.x) sm[i] = gm[i];
-    for (int i = threadIdx.x; i < 64; i += blockDim.x) {
-      const int wq = a.has_qm ? qm_row[i] : 32;
-      sQm[i] = (uint8_t)wq;
-      sQs[i] = fwd_qm_scale(wq);
-    }
-    __syncthreads();
-  }
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const mt_split16_params& p = a.p;
-  const mt_uv16_job jb = jobs[j];
-  mt_uv16_result& r = res[j];
-  const int cx = jb.px >> 1, cy = jb.py >> 1;
-  const float kInf = __int_as_float(0x7f800000);
-  const bool ok = (jb.px & 15) == 0 && (jb.py & 15) == 0 && cx + 8 <= p.frame_w && cy + 8 <= p.frame_h &&
-                  jb.y_mode <= MT_PAETH_PRED;
-  if (!ok) {
-    r.total = r.dc_total = r.cfl_total = kInf;
-    r.uv_mode = 255;
-    r.angle_delta = 0;
-    r.cfl_alpha[0] = r.cfl_alpha[1] = 0;
-    if (cf_out)
-      for (int i = 0; i < 128; i++) cf_out[(size_t)j * 128 + i] = 0;
-    if (rec_out)
-      for (int i = 0; i < 128; i++) rec_out[(size_t)j * 128 + i] = 0;
-    return;
-  }
-  const mt_coef_costs& T = sT;
-  const mt_uv_mode_costs& M = sM;
-  const uint8_t* qm = a.has_qm ? sQm : nullptr;
-  const int32_t maxv = (1 << p.bd) - 1;
-  const float mlam = p.rd_lambda;
-  const bool have_tr = jb.flags & MT_CAND_HAVE_TR, have_bl = jb.flags & MT_CAND_HAVE_BL;
-  const bool ft = jb.flags & MT_CAND_FILTER_TYPE;
-  const int vis_w = p.vis_w > 0 ? p.vis_w : p.frame_w, vis_h = p.vis_h > 0 ? p.vis_h : p.frame_h;
-  UvPlane P[2];
-  for (int pl = 0; pl < 2; pl++) {
-    UvPlane& q = P[pl];
-    q.src = (pl ? src_v : src_u) + (size_t)cy * p.stride + cx;
-    q.rec = pl ? rec_v : rec_u;
-    q.vw = min(max(vis_w - cx, 0), 8);
-    q.vh = min(max(vis_h - cy, 0), 8);
-    const uint32_t a0 = jb.a_coef[pl][0], a1 = jb.a_coef[pl][1], l0 = jb.l_coef[pl][0], l1 = jb.l_coef[pl][1];
-    q.sk = 7 + (a0 != 0x40 || a1 != 0x40) + (l0 != 0x40 || l1 != 0x40);
-    const int s = (int)(a0 >> 6) + (int)(a1 >> 6) + (int)(l0 >> 6) + (int)(l1 >> 6) - 4;
-    q.ds = (s != 0) + (s > 0);
-    q.skip1 = p.use_skip_bits ? p.skip_bits[q.sk][0] : 0.0f;
-    q.skip0 = p.use_skip_bits ? p.skip_bits[q.sk][1] : 0.0f;
-  }
-  UvWork& w = smem_arena<UvWork>(arena);
-  int best = 0;
-  // 1. DC on both planes (block16.rs:999-1046): no mode bits in its total
-  int32_t dc[2];
-  float dc_total = 0.0f;
-  for (int pl = 0; pl < 2; pl++) {
-    predict_sq<8>(P[pl].rec, p.stride, p.frame_w, p.frame_h, cx, cy, MT_DC_PRED, 0, have_tr, have_bl, ft, p.bd,
-                  w.s[0].pred[pl], w.u);
-    dc[pl] = w.s[0].pred[pl][0];
-    dc_total = __fadd_rn(dc_total, plane_chain(a, P[pl], T, qm, sQs, MT_TX_DCT_DCT, true, w.s[0].pred[pl],
-                                               w.s[0].cf[pl], w.s[0].rr[pl], w));
-  }
-  float best_total = dc_total;
-  int mode = MT_DC_PRED, delta = 0;
-  // 2. CfL (:1058-1128): the AC of the 16x16 luma reconstruction, the
-  // closed-form alphas, each plane's prediction through the DCT chain
-  {
-    const int ls = a.u.luma_stride;
-    const uint16_t* l = luma + (size_t)jb.py * ls + jb.px;
-    int32_t sum = 32;
-    for (int i = 0; i < 64; i++) {
-      const int y = i >> 3, x = i & 7;
-      const uint16_t* q = l + (size_t)(2 * y) * ls + 2 * x;
-      const int32_t v = ((int32_t)q[0] + q[1] + q[ls] + q[ls + 1]) << 1;
-      w.ac[i] = (int16_t)v;
-      sum += v;
-    }
-    const int32_t mean = sum >> 6;
-    for (int i = 0; i < 64; i++) w.ac[i] = (int16_t)(w.ac[i] - mean);
-  }
-  int alpha[2];
-  for (int pl = 0; pl < 2; pl++) alpha[pl] = cfl_alpha(w.ac, P[pl], p.stride, dc[pl], maxv);
-  {
-    UvSlot& c = w.s[1 - best];
-    float body = 0.0f;
-    for (int pl = 0; pl < 2; pl++) {
-      for (int i = 0; i < 64; i++) c.pred[pl][i] = (int16_t)cfl_pred_pixel(dc[pl], w.ac[i], alpha[pl], maxv);
-      body = __fadd_rn(body, plane_chain(a, P[pl], T, qm, sQs, MT_TX_DCT_DCT, false, c.pred[pl], c.cf[pl],
-                                         c.rr[pl], w));
-    }
-    const float cfl_total =
-        __fsub_rn(__fadd_rn(body, __fmul_rn(mlam, uv_mode_bits(M, jb.y_mode, MT_UV_CFL_PRED, true, alpha[0], alpha[1]))),
-                  __fmul_rn(mlam, uv_mode_bits(M, jb.y_mode, MT_DC_PRED, false, 0, 0)));
-    r.cfl_total = cfl_total;
-    if ((alpha[0] != 0 || alpha[1] != 0) && cfl_total < best_total) {
-      best_total = cfl_total;
-      mode = MT_UV_CFL_PRED;
-      best = 1 - best;
-    }
-  }
-  // 3. the joint (mode, delta) shortlist (:1157-1240): the two planes'
-  // satd_sad_proxy per candidate, the first joint_k by (score, mode, delta)
-  const int k = min(max(a.u.joint_k, 1), kMaxJoint);
-  unsigned long long ks[kMaxJoint];
-  uint8_t km[kMaxJoint];
-  int8_t kd[kMaxJoint];
-  int nk = 0;
-  int16_t* sp = w.s[1 - best].pred[0];  // scratch prediction
-  for (int ci = 0; ci < kJointModes; ci++) {
-    const int m = kJointList[ci];
-    const bool dir = directional(m) && a.u.angle_deltas;
-    for (int d = dir ? -3 : 0; d <= (dir ? 3 : 0); d++) {
-      unsigned long long sc = 0;
-      for (int pl = 0; pl < 2; pl++) {
-        predict_sq<8>(P[pl].rec, p.stride, p.frame_w, p.frame_h, cx, cy, m, d, have_tr, have_bl, ft, p.bd, sp, w.u);
-        sc += satd_sad_proxy<8>(pl ? src_v : src_u, p.stride, cx, cy, sp, P[pl].vw, P[pl].vh);
-      }
-      // insert (sc, m, d) into the ascending list of at most k entries
-      auto less = [&](int e) {
-        return sc < ks[e] || (sc == ks[e] && (m < km[e] || (m == km[e] && d < kd[e])));
-      };
-      if (nk == k && !less(nk - 1)) continue;
-      int e = nk < k ? nk++ : nk - 1;
-      while (e > 0 && less(e - 1)) {
-        ks[e] = ks[e - 1];
-        km[e] = km[e - 1];
-        kd[e] = kd[e - 1];
-        e--;
-      }
-      ks[e] = sc;
-      km[e] = (uint8_t)m;
-      kd[e] = (int8_t)d;
-    }
-  }
-  for (int e = 0; e < nk; e++) {
-    const int m = km[e], d = kd[e], tx = chroma_tx(m);
-    float ad_bits = 0.0f;
-    if (directional(m)) ad_bits = __fsub_rn(M.angle_delta[m - MT_V_PRED][d + 3], M.angle_delta[m - MT_V_PRED][3]);
-    float total = __fmul_rn(mlam, __fadd_rn(uv_mode_bits(M, jb.y_mode, m, false, 0, 0), ad_bits));
-    UvSlot& c = w.s[1 - best];
-    for (int pl = 0; pl < 2; pl++) {
-      predict_sq<8>(P[pl].rec, p.stride, p.frame_w, p.frame_h, cx, cy, m, d, have_tr, have_bl, ft, p.bd, c.pred[pl],
-                    w.u);
-      total = __fadd_rn(total, plane_chain(a, P[pl], T, qm, sQs, tx, true, c.pred[pl], c.cf[pl], c.rr[pl], w));
-      if (pl == 0 && total >= best_total) break;  // cannot win: the second plane is skipped
-    }
-    if (total < best_total) {
-      best_total = total;
-      mode = m;
-      delta = d;
-      best = 1 - best;
-    }
-  }
-  r.total = best_total;
-  r.dc_total = dc_total;
-  r.uv_mode = (uint8_t)mode;
-  r.angle_delta = (int8_t)delta;
-  r.cfl_alpha[0] = (int8_t)alpha[0];
-  r.cfl_alpha[1] = (int8_t)alpha[1];
-  const UvSlot& b = w.s[best];
-  if (cf_out)
-    for (int pl = 0; pl < 2; pl++)
-      for (int i = 0; i < 64; i++) cf_out[(size_t)j * 128 + pl * 64 + i] = b.cf[pl][i];
-  if (rec_out)
-    for (int pl = 0; pl < 2; pl++)
-      for (int i = 0; i < 64; i++)
-        rec_out[(size_t)j * 128 + pl * 64 + i] = (uint16_t)clampi((int32_t)b.pred[pl][i] + b.rr[pl][i], 0, maxv);
-}
-
-// ---- 4:4:4: pick_uv16_444 and pick_uv32_444 ----
-
-// Both planes of one N x N candidate: predictions, levels (32-bit at 32x32,
-// where a full-scale DC passes 16 bits) and inverses.
-template <int N>
-struct UvBigSlot {
-  using Coef = std::conditional_t<N == 32, int32_t, int16_t>;
-  int16_t pred[2][N * N];
-  Coef cf[2][N * N];
-  int16_t rr[2][N * N];
-};
-
-template <int N>
-struct UvBigWork {
-  UvBigSlot<N> s[2];   // the current choice and the candidate
-  int32_t u[2 * N * N];  // prediction edges, then the targets [0, N*N) and the transform temporary [N*N, 2N*N)
-  int16_t resid[N * N];
-  int16_t ac[N * N];
-  float suf[N * N + 1];  // trellis_sq scratch
-  std::conditional_t<N == 16, TrellisCtxScratchW<16>, char> trc;  // trellis_ctx<16> scratch (4:2:0 at 16x16)
-  alignas(16) uint8_t lv[(N + 2) * N];  // the rate walk stores it as 32-bit words
-};
-using Uv444Slot = UvBigSlot<16>;
-using Uv444Work = UvBigWork<16>;
-
 struct PlaneCost {
   long long sse;
   float bits;
 };
 
-// One N x N plane of a candidate after its prediction: the transform with
-// the QM (DCT_DCT only at 32x32), the plain trellis_optimize (the 4:4:4
-// chroma_rect_trellis) or, CTX, trellis_optimize_ctx against the chroma
-// costs in the plane's dc_sign context (4:2:0), preserve_dc when `keep_dc`,
-// the inverse, sse_recon and chroma_bits.
-template <int N, bool CTX = false>
-__device__ PlaneCost plane_chain(const UvArgs& a, const UvPlane& P, const mt_coef_costs& T, const uint8_t* qm,
-                                 const float* sQs, const float* lut, int tx, bool keep_dc, int16_t* pred,
-                                 typename UvBigSlot<N>::Coef* cf, int16_t* rr, UvBigWork<N>& w) {
-  static_assert(N == 16 || N == 32, "16x16 and 32x32 chroma blocks");
-  static_assert(!CTX || N == 16, "the context trellis runs at 16x16 here");
-  constexpr int NN = N * N, L = log2w<N>();
+// The four searches.
+enum class UvForm { k16_420, k32_420, k16_444, k32_444 };
+
+// Shape of a search: N the chroma block's side, CTX the context trellis (4:2:0)
+// or the plain one (4:4:4), Slots the blocks a CTA evaluates at a time, each on
+// N lanes: consecutive slots are U and V of one candidate.
+// A leaf is a CTA and its candidates go Slots / 2 at a time: DC and CfL
+// together, the ranking's predictions, the ranked modes, the deltas.  Six slots
+// of 16x16 (3 warps, 27 KB, 6 CTAs per SM) take the three ranked modes in one
+// step and the six deltas in two; at 32x32 six would leave one CTA per SM, four
+// (4 warps, 79 KB) leave two.  Eight of 8x8 (2 warps) take the default
+// shortlist of four at once.
+template <UvForm F>
+struct UvShape {
+  static constexpr int N = F == UvForm::k16_420 ? 8 : (F == UvForm::k32_444 ? 32 : 16);
+  static constexpr bool k420 = F == UvForm::k16_420 || F == UvForm::k32_420;
+  static constexpr bool kCtx = k420;
+  static constexpr int kSlots = N == 8 ? 8 : (N == 16 ? 6 : 4);
+  static constexpr int kThreads = kSlots * N;
+};
+
+// One N x N plane of a candidate after its prediction (w.pred): the transform
+// with the QM (DCT_DCT only at 32x32), trellis_optimize_ctx against the chroma
+// costs in the plane's dc_sign context (CTX) or the plain trellis_optimize (the
+// 4:4:4 chroma_rect_trellis), preserve_dc (src/rd_sse.rs:759-765) when
+// `keep_dc`, the inverse, sse_recon and chroma_bits.
+// Called, not inlined, as is the predictor: a search prices candidates in three
+// places, and one copy of the chain in the instruction cache beats three
+// (1080p: pick_uv16_444 3.45 -> 2.27 ms, pick_uv32_420 1.11 -> 0.78 ms).
+template <int N, bool CTX>
+__device__ __noinline__ PlaneCost plane_chain(const UvArgs& a, const UvPlane& P, const LaneTables<N * N>& S,
+                                                 const float* lut, int tx, bool keep_dc, LaneBuf<N>& w,
+                                                 const Lanes<N>& g) {
   const mt_split16_params& p = a.p;
   const mt_quant& q = a.q;
-  int32_t sum = 0;
-#pragma unroll 8
-  for (int i = 0; i < NN; i++) {
-    const int32_t r = (int32_t)P.src[(size_t)(i >> L) * p.stride + (i & (N - 1))] - pred[i];
-    w.resid[i] = (int16_t)r;
-    sum += r;
-  }
-  float* tf = reinterpret_cast<float*>(w.u);
-  int32_t* tmp = w.u + NN;
-  if constexpr (N == 16) fwd16x16(w.resid, tx, q, cf, tf, tmp);
-  else fwd32x32(w.resid, q, cf, tf, tmp);
-  if (qm) apply_qm(cf, tf, sQs, NN);
+  const uint8_t* qm = a.has_qm ? S.qm : nullptr;
+  const int32_t sum = lane_fwd<N>(P.src, p.stride, tx, q, qm, S.qs, w, g);
+  int eob;
   if (a.lambda > 0.0f) {
     if constexpr (CTX)
-      trellis_ctx<16>(cf, tf, (float)q.dc_q, (float)q.ac_q, a.lambda, T, P.ds, qm, q.qm_level >= 5, p.band_tilt,
-                      w.trc);
-    else if constexpr (N == 16)
-      trellis_sq<NN>(cf, tf, w.suf, (float)q.dc_q, (float)q.ac_q, a.lambda, lut, Scan16{});
+      eob = lane_trellis_ctx<N>(w, (float)q.dc_q, (float)q.ac_q, a.lambda, S.T, P.ds, qm, q.qm_level >= 5, p.band_tilt,
+                                g);
     else
-      trellis_sq<NN>(cf, tf, w.suf, (float)q.dc_q, (float)q.ac_q, a.lambda, lut, Scan32{});
+      eob = lane_trellis_plain<N>(w, (float)q.dc_q, (float)q.ac_q, a.lambda, lut, g);
+  } else {
+    eob = lane_eob<N>(w, g);
   }
-  if (keep_dc) {
-    const int32_t mean = sum / NN;
-    if (cf[0] == 0 && abs(mean) >= 8) cf[0] = mean > 0 ? 1 : -1;
+  const int32_t mean = sum / (N * N);  // truncating, as the reference's i32 division
+  const bool keep = keep_dc && w.cf[0] == 0 && abs(mean) >= 8;
+  g.sync();
+  if (keep) {
+    if (g.j == 0) w.cf[0] = mean > 0 ? 1 : -1;
+    eob = max(eob, 0);
   }
-  if constexpr (N == 16) inv16x16(cf, tx, q, qm, rr, tmp);
-  else inv32x32(cf, q, qm, rr, tmp);
-  ErrBlock<int16_t, int16_t> eb;
-  eb.src = P.src;
-  eb.stride = p.stride;
-  eb.pred = pred;
-  eb.resid = rr;
-  eb.w = N;
-  eb.vw = P.vw;
-  eb.vh = P.vh;
-  eb.maxv = (1 << p.bd) - 1;
+  g.sync();
+  lane_inv_err<N>(P.src, p.stride, tx, q, qm, P.vw, P.vh, (1 << p.bd) - 1, w, g);
   PlaneCost c;
-  c.sse = sse_recon_block(eb, p.wsse_scale);
-  c.bits = rate_bounded<N>(cf, T, P.sk, P.ds, 0, -1, p.use_skip_bits != 0, P.skip1, P.skip0,
-                           __int_as_float(0x7f800000), w.lv);
+  c.sse = lane_sse<N>(w, P.vw, P.vh, p.wsse_scale, g);
+  c.bits = lane_rate<N, false>(w, eob, S.T, P.sk, P.ds, 0, -1, p.use_skip_bits != 0, P.skip1, P.skip0,
+                               __int_as_float(0x7f800000), g);
   return c;
 }
 
-// cfl_best_alpha over an N x N block's displayed part (as cfl_alpha).
-template <int N>
-__device__ int cfl_alpha_n(const int16_t* ac, const UvPlane& P, int stride, int32_t dc, int32_t maxv) {
+// The CfL prediction of a plane into w.pred: the AC of the leaf's luma
+// reconstruction at l (4:2:0: the 2x2 sums << 1, cfl_ac_sub; 4:4:4: << 3), less
+// its rounded mean, and cfl_best_alpha (src/intrapred.rs:1211-1258) over the
+// displayed part: the closed-form alpha, then the first minimum of the
+// prediction's SSE over alpha - 3 .. alpha + 3 within +-16.  Returns the alpha.
+template <int N, bool SUB>
+__device__ __forceinline__ int lane_cfl(const uint16_t* __restrict__ l, int ls, const UvPlane& P, int stride, int32_t dc,
+                                        int32_t maxv, LaneBuf<N>& w, const Lanes<N>& g) {
+  constexpr int L = log2w<N>();
+  const int x = g.j;
+  int16_t ac[N];
+  int32_t sum = 0;
+#pragma unroll
+  for (int y = 0; y < N; y++) {
+    int32_t v;
+    if constexpr (SUB) {
+      const uint16_t* q = l + (size_t)(2 * y) * ls + 2 * x;
+      v = ((int32_t)q[0] + q[1] + q[ls] + q[ls + 1]) << 1;
+    } else {
+      v = (int32_t)l[(size_t)y * ls + x] << 3;
+    }
+    ac[y] = (int16_t)v;
+    sum += v;
+  }
+  const int32_t mean = (g.sum(sum) + N * N / 2) >> (2 * L);
+  const bool vis_x = x < P.vw;
   long long num = 0, den = 0;
-  for (int y = 0; y < P.vh; y++)
-    for (int x = 0; x < P.vw; x++) {
-      const long long v = ac[y * N + x];
+#pragma unroll
+  for (int y = 0; y < N; y++) {
+    ac[y] = (int16_t)(ac[y] - mean);
+    if (vis_x && y < P.vh) {
+      const long long v = ac[y];
       num += (long long)((int32_t)P.src[(size_t)y * stride + x] - dc) * v;
       den += v * v;
     }
-  if (den == 0) return 0;
+  }
+  num = g.sum(num);
+  den = g.sum(den);
+  int alpha = 0;
   const long long sg = num > 0 ? 1 : (num < 0 ? -1 : 0);
-  long long a0 = (64 * num + (den >> 1) * sg) / den;
+  long long a0 = den == 0 ? 0 : (64 * num + (den >> 1) * sg) / den;
   a0 = a0 < -16 ? -16 : (a0 > 16 ? 16 : a0);
-  long long best_e = 0x7fffffffffffffffLL;
-  int best_a = 0;
-  for (int c = (int)a0 - 3; c <= (int)a0 + 3; c++) {
-    if (c < -16 || c > 16) continue;
-    long long e = 0;
-    for (int y = 0; y < P.vh; y++)
-      for (int x = 0; x < P.vw; x++) {
-        const long long d = (int32_t)P.src[(size_t)y * stride + x] - cfl_pred_pixel(dc, ac[y * N + x], c, maxv);
-        e += d * d;
+  long long e[7];
+#pragma unroll
+  for (int k = 0; k < 7; k++) e[k] = 0;
+#pragma unroll
+  for (int y = 0; y < N; y++) {
+    if (vis_x && y < P.vh) {
+      const int32_t s = P.src[(size_t)y * stride + x];
+#pragma unroll
+      for (int k = 0; k < 7; k++) {
+        const long long d = s - cfl_pred_pixel(dc, ac[y], (int)a0 - 3 + k, maxv);
+        e[k] += d * d;
       }
-    if (e < best_e) {
-      best_e = e;
-      best_a = c;
     }
   }
-  return best_a;
+  long long best_e = 0x7fffffffffffffffLL;
+#pragma unroll
+  for (int k = 0; k < 7; k++) {
+    const long long ek = g.sum(e[k]);
+    const int c = (int)a0 - 3 + k;
+    if (c >= -16 && c <= 16 && ek < best_e) {
+      best_e = ek;
+      alpha = c;
+    }
+  }
+  if (den == 0) alpha = 0;
+#pragma unroll
+  for (int y = 0; y < N; y++) w.pred[y * N + x] = (int16_t)cfl_pred_pixel(dc, ac[y], alpha, maxv);
+  g.sync();
+  return alpha;
 }
 
-// The 4:4:4 leaf searches: N = 16 is pick_uv16_444 (block16.rs:437-978), N =
-// 32 pick_uv32_444 (block32.rs:2264-2720).  J: the job (four or eight
-// context bytes per plane and side).
-template <int N, typename J>
-__global__ void __launch_bounds__(kUvThreads) uv444_kernel(
+// satd_sad_proxy of w.pred over the block's lanes, a 4x4 tile at a time each.
+template <int N>
+__device__ __forceinline__ unsigned long long lane_satd_sad(const UvPlane& P, int stride, const LaneBuf<N>& w,
+                                                            const Lanes<N>& g) {
+  uint32_t sad = 0, satd = 0;
+  for (int tile = g.j; tile < (N / 4) * (N / 4); tile += N) {
+    const int ty = (tile / (N / 4)) * 4, tx = (tile % (N / 4)) * 4;
+    int32_t r[4][4];
+#pragma unroll
+    for (int y = 0; y < 4; y++) {
+      int32_t d[4];
+#pragma unroll
+      for (int x = 0; x < 4; x++) {
+        const bool vis = tx + x < P.vw && ty + y < P.vh;
+        d[x] = vis ? (int32_t)P.src[(size_t)(ty + y) * stride + tx + x] - w.pred[(ty + y) * N + tx + x] : 0;
+        sad += uabs(d[x]);
+      }
+      const int32_t e = d[0] + d[2], f = d[0] - d[2], gg = d[1] + d[3], h = d[1] - d[3];
+      r[y][0] = e + gg;
+      r[y][1] = f + h;
+      r[y][2] = f - h;
+      r[y][3] = e - gg;
+    }
+#pragma unroll
+    for (int x = 0; x < 4; x++) {
+      const int32_t e = r[0][x] + r[2][x], f = r[0][x] - r[2][x], gg = r[1][x] + r[3][x], h = r[1][x] - r[3][x];
+      satd += uabs(e + gg) + uabs(f + h) + uabs(f - h) + uabs(e - gg);
+    }
+  }
+  return (unsigned long long)g.sum((unsigned long long)sad) + (g.sum((unsigned long long)satd) >> 2);
+}
+
+// The prediction of (mode, delta) into w.pred.
+template <int N>
+__device__ __noinline__ void plane_predict(const uint16_t* __restrict__ rec, int stride, int fw, int fh, int cx, int cy,
+                                              int mode, int delta, bool tr, bool bl, bool ft, int bd, LaneBuf<N>& w,
+                                              const Lanes<N>& g) {
+  lane_predict<N>(PlaneRead{rec, stride}, fw, fh, cx, cy, mode, delta, tr, bl, ft, bd, w.pred,
+                  reinterpret_cast<int32_t*>(&w), g);
+}
+
+// A leaf's chroma search.  Every thread follows the decisions on the costs that
+// the slots leave in shared memory; a candidate that wins is written out at
+// once, over the winner before it.
+// k16_444 is pick_uv16_444 (block16.rs:437-978), k32_444 pick_uv32_444
+// (block32.rs:2264-2720): DC, CfL against DC on the chroma lambda (the 16x16
+// search on the summed SSE and bits, the 32x32 one on the planes' costs), the
+// 12 modes ranked by SATD into a top-3 priced in list order on dir_lambda, the
+// zone-2 deltas of a directional winner.  k32_420 is pick_uv32_420
+// (block32.rs:2797-3120): the same on the one chroma lambda with the context
+// trellis, DC's total without mode bits, no deltas after CfL.  k16_420 is
+// pick_uv16_420 (block16.rs:980-1381): the joint (mode, delta) shortlist of the
+// SATD ranking in place of the top-3 and the deltas.
+// Bound by issue and the chains' latency, HBM is idle.  Measured at 1080p against
+// a thread per leaf with its working set in shared memory (3, 10 or 50 KB, so
+// 55, 21 or 4 leaves per SM): k16_420 2.83 -> 1.09 ms, k16_444 25.2 -> 2.27 ms,
+// k32_420 24.2 -> 0.78 ms, k32_444 56 -> 2.15 ms.
+template <UvForm F, typename J>
+__global__ void __launch_bounds__(UvShape<F>::kThreads) uv_kernel(
     const uint16_t* __restrict__ src_u, const uint16_t* __restrict__ src_v, const uint16_t* __restrict__ rec_u,
-    const uint16_t* __restrict__ rec_v, const uint16_t* __restrict__ luma, UvArgs a,
+    const uint16_t* __restrict__ rec_v, const uint16_t* __restrict__ luma, const __grid_constant__ UvArgs a,
     const uint8_t* __restrict__ qm_row, const mt_coef_costs* __restrict__ costs,
     const mt_uv_mode_costs* __restrict__ mode_costs, const J* __restrict__ jobs, int n,
-    mt_uv16_result* __restrict__ res, int32_t* __restrict__ cf_out, uint16_t* __restrict__ rec_out, int arena) {
-  constexpr int NN = N * N, U = N / 4, L = log2w<N>();
-  __shared__ mt_coef_costs sT;
-  __shared__ mt_uv_mode_costs sM;
-  __shared__ uint8_t sQm[NN];
-  __shared__ float sQs[NN];
-  __shared__ float sLut[64];
-  {
-    const float* g = reinterpret_cast<const float*>(costs);
-    float* s = reinterpret_cast<float*>(&sT);
-    for (int i = threadIdx.x; i < (int)(sizeof(mt_coef_costs) / 4); i += blockDim.x) s[i] = g[i];
-    const float* gm = reinterpret_cast<const float*>(mode_costs);
-    float* sm = reinterpret_cast<float*>(&sM);
-    for (int i = threadIdx.x; i < (int)(sizeof(mt_uv_mode_costs) / 4); i += blockDim.x) sm[i] = gm[i];
-    for (int i = threadIdx.x; i < NN; i += blockDim.x) {
-      const int wq = a.has_qm ? qm_row[i] : 32;
-      sQm[i] = (uint8_t)wq;
-      sQs[i] = fwd_qm_scale(wq);
-    }
-    for (int i = threadIdx.x; i < 64; i += blockDim.x) sLut[i] = kCoefRateLut[i];
-    __syncthreads();
-  }
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
+    mt_uv16_result* __restrict__ res, int32_t* __restrict__ cf_out, uint16_t* __restrict__ rec_out) {
+  constexpr int N = UvShape<F>::N, NN = N * N, U = N / 4, kSlots = UvShape<F>::kSlots, kCands = kSlots / 2;
+  constexpr bool kCtx = UvShape<F>::kCtx, k420 = UvShape<F>::k420, kJoint = F == UvForm::k16_420;
+  __shared__ LaneTables<NN> S;
+  __shared__ mt_uv_mode_costs M;
+  __shared__ float lut[64];
+  __shared__ PlaneCost cost[kCands][2];
+  __shared__ int salpha[2];
+  __shared__ unsigned long long score[kJoint ? 60 : 12][2];
+  __shared__ uint8_t list[kMaxJoint];  // the joint shortlist, as indexes of the ranking
+  extern __shared__ __align__(128) unsigned char lane_smem[];
+  const int job = blockIdx.x;
   const mt_split16_params& p = a.p;
-  const J jb = jobs[j];
-  mt_uv16_result& r = res[j];
-  const int cx = jb.px, cy = jb.py;
-  const float kInf = __int_as_float(0x7f800000);
-  const bool ok = (cx & (N - 1)) == 0 && (cy & (N - 1)) == 0 && cx + N <= p.frame_w && cy + N <= p.frame_h &&
-                  jb.y_mode <= MT_PAETH_PRED;
+  const J jb = jobs[job];
+  constexpr int kLeaf = k420 ? 2 * N : N;
+  const int cx = k420 ? jb.px >> 1 : jb.px, cy = k420 ? jb.py >> 1 : jb.py;
+  const bool ok = (jb.px & (kLeaf - 1)) == 0 && (jb.py & (kLeaf - 1)) == 0 && cx + N <= p.frame_w &&
+                  cy + N <= p.frame_h && jb.y_mode <= MT_PAETH_PRED;
   if (!ok) {
-    r.total = r.dc_total = r.cfl_total = kInf;
-    r.uv_mode = 255;
-    r.angle_delta = 0;
-    r.cfl_alpha[0] = r.cfl_alpha[1] = 0;
-    if (cf_out)
-      for (int i = 0; i < 2 * NN; i++) cf_out[(size_t)j * 2 * NN + i] = 0;
-    if (rec_out)
-      for (int i = 0; i < 2 * NN; i++) rec_out[(size_t)j * 2 * NN + i] = 0;
+    if (threadIdx.x == 0) {
+      mt_uv16_result r = {};
+      r.total = r.dc_total = r.cfl_total = __int_as_float(0x7f800000);
+      r.uv_mode = 255;
+      res[job] = r;
+    }
+    for (int i = threadIdx.x; i < 2 * NN; i += blockDim.x) {
+      if (cf_out) cf_out[(size_t)job * 2 * NN + i] = 0;
+      if (rec_out) rec_out[(size_t)job * 2 * NN + i] = 0;
+    }
     return;
   }
-  const mt_coef_costs& T = sT;
-  const mt_uv_mode_costs& M = sM;
-  const uint8_t* qm = a.has_qm ? sQm : nullptr;
+  {
+    const float* gm = reinterpret_cast<const float*>(mode_costs);
+    float* sm = reinterpret_cast<float*>(&M);
+    for (int i = threadIdx.x; i < (int)(sizeof(mt_uv_mode_costs) / 4); i += blockDim.x) sm[i] = gm[i];
+    for (int i = threadIdx.x; i < 64; i += blockDim.x) lut[i] = kCoefRateLut[i];
+  }
+  S.load(costs, qm_row, a.has_qm);
+  const Lanes<N> g;
+  const int slot = threadIdx.x / N, pl = slot & 1;
+  LaneBuf<N>& w = reinterpret_cast<LaneBuf<N>*>(lane_smem)[slot];
   const int32_t maxv = (1 << p.bd) - 1;
-  const float mlam = p.rd_lambda, dlam = a.u.dir_lambda;
+  const float mlam = p.rd_lambda, dlam = k420 ? p.rd_lambda : a.u.dir_lambda;
   const bool have_tr = jb.flags & MT_CAND_HAVE_TR, have_bl = jb.flags & MT_CAND_HAVE_BL;
   const bool ft = jb.flags & MT_CAND_FILTER_TYPE;
   const int vis_w = p.vis_w > 0 ? p.vis_w : p.frame_w, vis_h = p.vis_h > 0 ? p.vis_h : p.frame_h;
-  UvPlane P[2];
-  for (int pl = 0; pl < 2; pl++) {
-    UvPlane& q = P[pl];
-    q.src = (pl ? src_v : src_u) + (size_t)cy * p.stride + cx;
-    q.rec = pl ? rec_v : rec_u;
-    q.vw = min(max(vis_w - cx, 0), N);
-    q.vh = min(max(vis_h - cy, 0), N);
+  UvPlane P;  // this slot's plane
+  P.src = (pl ? src_v : src_u) + (size_t)cy * p.stride + cx;
+  P.rec = pl ? rec_v : rec_u;
+  P.vw = min(max(vis_w - cx, 0), N);
+  P.vh = min(max(vis_h - cy, 0), N);
+  {
     bool anz = false, lnz = false;
     int s = -2 * U;
     for (int k = 0; k < U; k++) {
@@ -553,360 +340,256 @@ __global__ void __launch_bounds__(kUvThreads) uv444_kernel(
       lnz |= jb.l_coef[pl][k] != 0x40;
       s += (jb.a_coef[pl][k] >> 6) + (jb.l_coef[pl][k] >> 6);
     }
-    q.sk = 7 + anz + lnz;       // the chroma txb_skip context over the block's units
-    q.ds = (s != 0) + (s > 0);  // dc_sign_ctx_span over U + U units
-    q.skip1 = p.use_skip_bits ? p.skip_bits[q.sk][0] : 0.0f;
-    q.skip0 = p.use_skip_bits ? p.skip_bits[q.sk][1] : 0.0f;
+    P.sk = 7 + anz + lnz;       // the chroma txb_skip context over the block's units
+    P.ds = (s != 0) + (s > 0);  // dc_sign_ctx_span over U + U units
+    P.skip1 = p.use_skip_bits ? p.skip_bits[P.sk][0] : 0.0f;
+    P.skip0 = p.use_skip_bits ? p.skip_bits[P.sk][1] : 0.0f;
   }
-  UvBigWork<N>& w = smem_arena<UvBigWork<N>>(arena);
-  // DC, slot 0
-  int32_t dc[2];
-  PlaneCost dcc[2], cfc[2];
-  for (int pl = 0; pl < 2; pl++) {
-    predict_sq<N>(P[pl].rec, p.stride, p.frame_w, p.frame_h, cx, cy, MT_DC_PRED, 0, have_tr, have_bl, ft, p.bd,
-                  w.s[0].pred[pl], w.u);
-    dc[pl] = w.s[0].pred[pl][0];
-    dcc[pl] = plane_chain<N>(a, P[pl], T, qm, sQs, sLut, MT_TX_DCT_DCT, true, w.s[0].pred[pl], w.s[0].cf[pl],
-                             w.s[0].rr[pl], w);
-  }
-  // CfL against DC, slot 1: cfl_ac_444 (each luma sample << 3, less the rounded mean)
-  {
-    const int ls = a.u.luma_stride;
-    const uint16_t* l = luma + (size_t)cy * ls + cx;
-    int32_t sum = NN / 2;
-    for (int i = 0; i < NN; i++) {
-      const int32_t v = (int32_t)l[(size_t)(i >> L) * ls + (i & (N - 1))] << 3;
-      w.ac[i] = (int16_t)v;
-      sum += v;
-    }
-    const int32_t mean = sum >> (2 * L);
-    for (int i = 0; i < NN; i++) w.ac[i] = (int16_t)(w.ac[i] - mean);
-  }
-  int alpha[2];
-  for (int pl = 0; pl < 2; pl++) alpha[pl] = cfl_alpha_n<N>(w.ac, P[pl], p.stride, dc[pl], maxv);
-  for (int pl = 0; pl < 2; pl++) {
-    for (int i = 0; i < NN; i++) w.s[1].pred[pl][i] = (int16_t)cfl_pred_pixel(dc[pl], w.ac[i], alpha[pl], maxv);
-    cfc[pl] = plane_chain<N>(a, P[pl], T, qm, sQs, sLut, MT_TX_DCT_DCT, false, w.s[1].pred[pl], w.s[1].cf[pl],
-                             w.s[1].rr[pl], w);
-  }
-  const float sig = uv_mode_bits(M, jb.y_mode, MT_UV_CFL_PRED, true, alpha[0], alpha[1]);
-  const float dc_bits = uv_mode_bits(M, jb.y_mode, MT_DC_PRED, false, 0, 0);
-  float dc_total, cfl_total;
-  if constexpr (N == 16) {
-    // rd_cost_i64 of the summed SSE and bits (block16.rs:587-597)
-    dc_total = rd_cost_i64(dcc[0].sse + dcc[1].sse, mlam, __fadd_rn(__fadd_rn(dcc[0].bits, dcc[1].bits), dc_bits));
-    cfl_total = rd_cost_i64(cfc[0].sse + cfc[1].sse, mlam, __fadd_rn(__fadd_rn(cfc[0].bits, cfc[1].bits), sig));
-  } else {
-    // the planes' rd_cost_i64 summed, then the mode bits (block32.rs:2399-2404)
-    dc_total = __fadd_rn(__fadd_rn(rd_cost_i64(dcc[0].sse, mlam, dcc[0].bits), rd_cost_i64(dcc[1].sse, mlam, dcc[1].bits)),
-                         __fmul_rn(mlam, dc_bits));
-    cfl_total = __fadd_rn(__fadd_rn(rd_cost_i64(cfc[0].sse, mlam, cfc[0].bits), rd_cost_i64(cfc[1].sse, mlam, cfc[1].bits)),
-                          __fmul_rn(mlam, sig));
-  }
-  const bool use_cfl = cfl_total < dc_total && (alpha[0] != 0 || alpha[1] != 0);
-  int best = use_cfl ? 1 : 0;
-  const PlaneCost* cur = use_cfl ? cfc : dcc;
-  // the directional stage on dir_lambda: the current choice's total, then the ranked modes
-  float best_total = __fmul_rn(dlam, use_cfl ? sig : dc_bits);
-  for (int pl = 0; pl < 2; pl++) best_total = __fadd_rn(best_total, rd_cost_i64(cur[pl].sse, dlam, cur[pl].bits));
-  int mode = MT_DC_PRED, delta = 0;
-  // rank_chroma_modes (superblock.rs:469-513) into DirectionalTopK (coder.rs:326-365), K = 3
-  unsigned long long tc[3];
-  int tm[3], tn = 0;
-  int16_t* sp = w.s[1 - best].pred[0];
-  for (int ci = 0; ci < kJointModes; ci++) {
-    const int m = kJointList[ci];
-    unsigned long long sc = 0;
-    for (int pl = 0; pl < 2; pl++) {
-      predict_sq<N>(P[pl].rec, p.stride, p.frame_w, p.frame_h, cx, cy, m, 0, have_tr, have_bl, ft, p.bd, sp, w.u);
-      sc += satd_sad_proxy<N>(pl ? src_v : src_u, p.stride, cx, cy, sp, P[pl].vw, P[pl].vh);
-    }
-    int pos = tn < 3 ? tn : 2;
-    if (tn == 3 && sc >= tc[pos]) continue;
-    if (tn < 3) pos = tn++;
-    while (pos > 0 && sc < tc[pos - 1]) {
-      tc[pos] = tc[pos - 1];
-      tm[pos] = tm[pos - 1];
-      pos--;
-    }
-    tc[pos] = sc;
-    tm[pos] = m;
-  }
-  for (int ci = 0; ci < kJointModes; ci++) {
-    const int m = kJointList[ci];
-    bool in = false;
-    for (int e = 0; e < tn; e++) in |= tm[e] == m;
-    if (!in) continue;
-    const int tx = N == 32 ? MT_TX_DCT_DCT : chroma_tx(m);  // forced DCT_DCT at TX_32X32
-    float total = __fmul_rn(dlam, uv_mode_bits(M, jb.y_mode, m, false, 0, 0));
-    UvBigSlot<N>& c = w.s[1 - best];
-    for (int pl = 0; pl < 2; pl++) {
-      predict_sq<N>(P[pl].rec, p.stride, p.frame_w, p.frame_h, cx, cy, m, 0, have_tr, have_bl, ft, p.bd,
-                    c.pred[pl], w.u);
-      const PlaneCost pc = plane_chain<N>(a, P[pl], T, qm, sQs, sLut, tx, true, c.pred[pl], c.cf[pl], c.rr[pl], w);
-      total = __fadd_rn(total, rd_cost_i64(pc.sse, dlam, pc.bits));
-    }
-    if (total < best_total) {
-      best_total = total;
-      mode = m;
-      best = 1 - best;
-    }
-  }
-  // the zone-2 angle deltas of a directional winner (uv_ad; uv_ad32 at 32x32)
-  if (a.u.angle_deltas && directional(mode)) {
-    const int m = mode, tx = N == 32 ? MT_TX_DCT_DCT : chroma_tx(m);
-    int lo = 0, hi = -1;
-    if (m == MT_V_PRED) lo = 1, hi = 3;
-    else if (m == MT_H_PRED) lo = -3, hi = -1;
-    else if (m == MT_D113_PRED || m == MT_D135_PRED || m == MT_D157_PRED) lo = -3, hi = 3;
-    const float base_sig = __fsub_rn(uv_mode_bits(M, jb.y_mode, m, false, 0, 0), M.angle_delta[m - MT_V_PRED][3]);
-    for (int d = lo; d <= hi; d++) {
-      if (d == 0) continue;
-      float total = __fmul_rn(dlam, __fadd_rn(base_sig, M.angle_delta[m - MT_V_PRED][d + 3]));
-      UvBigSlot<N>& c = w.s[1 - best];
-      for (int pl = 0; pl < 2; pl++) {
-        predict_sq<N>(P[pl].rec, p.stride, p.frame_w, p.frame_h, cx, cy, m, d, false, false, ft, p.bd, c.pred[pl],
-                      w.u);
-        const PlaneCost pc = plane_chain<N>(a, P[pl], T, qm, sQs, sLut, tx, true, c.pred[pl], c.cf[pl], c.rr[pl], w);
-        total = __fadd_rn(total, rd_cost_i64(pc.sse, dlam, pc.bits));
-      }
-      if (total < best_total) {
-        best_total = total;
-        delta = d;
-        best = 1 - best;
-      }
-    }
-  }
-  r.total = best_total;
-  r.dc_total = dc_total;
-  r.cfl_total = cfl_total;
-  r.uv_mode = (uint8_t)(mode != MT_DC_PRED ? mode : (use_cfl ? MT_UV_CFL_PRED : MT_DC_PRED));
-  r.angle_delta = (int8_t)delta;
-  r.cfl_alpha[0] = (int8_t)alpha[0];
-  r.cfl_alpha[1] = (int8_t)alpha[1];
-  const UvBigSlot<N>& b = w.s[best];
-  if (cf_out)
-    for (int pl = 0; pl < 2; pl++)
-      for (int i = 0; i < NN; i++) cf_out[(size_t)j * 2 * NN + pl * NN + i] = b.cf[pl][i];
-  if (rec_out)
-    for (int pl = 0; pl < 2; pl++)
-      for (int i = 0; i < NN; i++)
-        rec_out[(size_t)j * 2 * NN + pl * NN + i] = (uint16_t)clampi((int32_t)b.pred[pl][i] + b.rr[pl][i], 0, maxv);
-}
-
-// ---- the 32x32 leaf at 4:2:0: pick_uv32_420 ----
-
-// pick_uv32_420 (src/coder/block32.rs:2797-3120) with the shipped tuning on
-// the 32x32 leaf's 16x16 chroma blocks: DC (the 4:2:0 context trellis,
-// preserve_dc), CfL from the AC of the 32x32 luma reconstruction against
-// DC, the 12 modes ranked by SATD into a top-3 priced in list order, then a
-// directional winner's zone-2 deltas (uv_ad, uv_ad32; not after CfL); every
-// total on the one chroma lambda.
-__global__ void __launch_bounds__(kUvThreads) uv32_420_kernel(
-    const uint16_t* __restrict__ src_u, const uint16_t* __restrict__ src_v, const uint16_t* __restrict__ rec_u,
-    const uint16_t* __restrict__ rec_v, const uint16_t* __restrict__ luma, UvArgs a,
-    const uint8_t* __restrict__ qm_row, const mt_coef_costs* __restrict__ costs,
-    const mt_uv_mode_costs* __restrict__ mode_costs, const mt_uv16_444_job* __restrict__ jobs, int n,
-    mt_uv16_result* __restrict__ res, int32_t* __restrict__ cf_out, uint16_t* __restrict__ rec_out, int arena) {
-  __shared__ mt_coef_costs sT;
-  __shared__ mt_uv_mode_costs sM;
-  __shared__ uint8_t sQm[256];
-  __shared__ float sQs[256];
-  {
-    const float* g = reinterpret_cast<const float*>(costs);
-    float* s = reinterpret_cast<float*>(&sT);
-    for (int i = threadIdx.x; i < (int)(sizeof(mt_coef_costs) / 4); i += blockDim.x) s[i] = g[i];
-    const float* gm = reinterpret_cast<const float*>(mode_costs);
-    float* sm = reinterpret_cast<float*>(&sM);
-    for (int i = threadIdx.x; i < (int)(sizeof(mt_uv_mode_costs) / 4); i += blockDim.x) sm[i] = gm[i];
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-      const int wq = a.has_qm ? qm_row[i] : 32;
-      sQm[i] = (uint8_t)wq;
-      sQs[i] = fwd_qm_scale(wq);
+  auto predict = [&](int m, int d, bool tr, bool bl) {
+    plane_predict<N>(P.rec, p.stride, p.frame_w, p.frame_h, cx, cy, m, d, tr, bl, ft, p.bd, w, g);
+  };
+  // candidate c of the last step becomes the leaf's output
+  auto put = [&](int c) {
+    if (slot >> 1 != c) return;
+    const size_t o = (size_t)job * 2 * NN + pl * NN;
+    if (cf_out)
+      for (int i = g.j; i < NN; i += N) cf_out[o + i] = w.cf[i];
+    if (rec_out)
+      for (int i = g.j; i < NN; i += N) rec_out[o + i] = (uint16_t)w.pred[i];
+  };
+  auto plane_rd = [&](const PlaneCost& c, float lam) { return rd_cost_i64(c.sse, lam, c.bits); };
+  // Evaluates one candidate per pair of slots: f(c) predicts candidate c.
+  // `step` counts the candidates of this step; the spare slots of a warp that
+  // holds a candidate repeat one.
+  auto evaluate = [&](int step, auto f) {
+    const int c0 = (int)(threadIdx.x & ~31u) / N >> 1;  // the warp's first candidate
+    if (c0 < step) {
+      const int c = min(slot >> 1, step - 1);
+      int tx = MT_TX_DCT_DCT;
+      const bool keep_dc = f(c, &tx);
+      const PlaneCost pc = plane_chain<N, kCtx>(a, P, S, lut, tx, keep_dc, w, g);
+      if (slot >> 1 < step && g.j == 0) cost[slot >> 1][pl] = pc;
     }
     __syncthreads();
-  }
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const mt_split16_params& p = a.p;
-  const mt_uv16_444_job jb = jobs[j];
-  mt_uv16_result& r = res[j];
-  const int cx = jb.px >> 1, cy = jb.py >> 1;
-  const float kInf = __int_as_float(0x7f800000);
-  const bool ok = (jb.px & 31) == 0 && (jb.py & 31) == 0 && cx + 16 <= p.frame_w && cy + 16 <= p.frame_h &&
-                  jb.y_mode <= MT_PAETH_PRED;
-  if (!ok) {
-    r.total = r.dc_total = r.cfl_total = kInf;
-    r.uv_mode = 255;
-    r.angle_delta = 0;
-    r.cfl_alpha[0] = r.cfl_alpha[1] = 0;
-    if (cf_out)
-      for (int i = 0; i < 512; i++) cf_out[(size_t)j * 512 + i] = 0;
-    if (rec_out)
-      for (int i = 0; i < 512; i++) rec_out[(size_t)j * 512 + i] = 0;
-    return;
-  }
-  const mt_coef_costs& T = sT;
-  const mt_uv_mode_costs& M = sM;
-  const uint8_t* qm = a.has_qm ? sQm : nullptr;
-  const int32_t maxv = (1 << p.bd) - 1;
-  const float mlam = p.rd_lambda;
-  const bool have_tr = jb.flags & MT_CAND_HAVE_TR, have_bl = jb.flags & MT_CAND_HAVE_BL;
-  const bool ft = jb.flags & MT_CAND_FILTER_TYPE;
-  const int vis_w = p.vis_w > 0 ? p.vis_w : p.frame_w, vis_h = p.vis_h > 0 ? p.vis_h : p.frame_h;
-  UvPlane P[2];
-  for (int pl = 0; pl < 2; pl++) {
-    UvPlane& q = P[pl];
-    q.src = (pl ? src_v : src_u) + (size_t)cy * p.stride + cx;
-    q.rec = pl ? rec_v : rec_u;
-    q.vw = min(max(vis_w - cx, 0), 16);
-    q.vh = min(max(vis_h - cy, 0), 16);
-    bool anz = false, lnz = false;
-    int s = -8;
-    for (int k = 0; k < 4; k++) {
-      anz |= jb.a_coef[pl][k] != 0x40;
-      lnz |= jb.l_coef[pl][k] != 0x40;
-      s += (jb.a_coef[pl][k] >> 6) + (jb.l_coef[pl][k] >> 6);
+  };
+
+  // DC (slots 0, 1) and CfL (slots 2, 3)
+  evaluate(2, [&](int c, int*) {
+    predict(MT_DC_PRED, 0, have_tr, have_bl);
+    const int32_t dc = w.pred[0];
+    g.sync();
+    if (__any_sync(kFull, c == 1)) {
+      // a warp that holds both candidates runs both and keeps DC's prediction
+      int16_t flat[N];
+#pragma unroll
+      for (int y = 0; y < N; y++) flat[y] = (int16_t)dc;
+      const int al = lane_cfl<N, k420>(luma + (size_t)jb.py * a.u.luma_stride + jb.px, a.u.luma_stride, P, p.stride, dc,
+                                       maxv, w, g);
+      if (c == 1) {
+        if (g.j == 0 && slot >> 1 == 1) salpha[pl] = al;
+      } else {
+#pragma unroll
+        for (int y = 0; y < N; y++) w.pred[y * N + g.j] = flat[y];
+      }
+      g.sync();
     }
-    q.sk = 7 + anz + lnz;
-    q.ds = (s != 0) + (s > 0);
-    q.skip1 = p.use_skip_bits ? p.skip_bits[q.sk][0] : 0.0f;
-    q.skip0 = p.use_skip_bits ? p.skip_bits[q.sk][1] : 0.0f;
+    return c == 0;  // preserve_dc
+  });
+  const int au = salpha[0], av = salpha[1];
+  const float sig = uv_mode_bits(M, jb.y_mode, MT_UV_CFL_PRED, true, au, av);
+  const float dc_bits = uv_mode_bits(M, jb.y_mode, MT_DC_PRED, false, 0, 0);
+  float dc_total, cfl_total, best_total;
+  bool use_cfl;
+  if constexpr (F == UvForm::k16_444) {
+    // rd_cost_i64 of the summed SSE and bits (block16.rs:587-597)
+    dc_total = rd_cost_i64(cost[0][0].sse + cost[0][1].sse, mlam,
+                           __fadd_rn(__fadd_rn(cost[0][0].bits, cost[0][1].bits), dc_bits));
+    cfl_total = rd_cost_i64(cost[1][0].sse + cost[1][1].sse, mlam,
+                            __fadd_rn(__fadd_rn(cost[1][0].bits, cost[1][1].bits), sig));
+    use_cfl = cfl_total < dc_total && (au != 0 || av != 0);
+  } else if constexpr (F == UvForm::k32_444) {
+    // the planes' rd_cost_i64 summed, then the mode bits (block32.rs:2399-2404)
+    dc_total = __fadd_rn(__fadd_rn(plane_rd(cost[0][0], mlam), plane_rd(cost[0][1], mlam)), __fmul_rn(mlam, dc_bits));
+    cfl_total = __fadd_rn(__fadd_rn(plane_rd(cost[1][0], mlam), plane_rd(cost[1][1], mlam)), __fmul_rn(mlam, sig));
+    use_cfl = cfl_total < dc_total && (au != 0 || av != 0);
+  } else {
+    // no mode bits in DC's total (block16.rs:999-1046)
+    dc_total = __fadd_rn(__fadd_rn(0.0f, plane_rd(cost[0][0], mlam)), plane_rd(cost[0][1], mlam));
+    const float body = __fadd_rn(__fadd_rn(0.0f, plane_rd(cost[1][0], mlam)), plane_rd(cost[1][1], mlam));
+    cfl_total = __fsub_rn(__fadd_rn(body, __fmul_rn(mlam, sig)), __fmul_rn(mlam, dc_bits));
+    use_cfl = (au != 0 || av != 0) && cfl_total < dc_total;
   }
-  Uv444Work& w = smem_arena<Uv444Work>(arena);
-  int best = 0;
-  int32_t dc[2];
-  float dc_total = 0.0f;
-  for (int pl = 0; pl < 2; pl++) {
-    predict_sq<16>(P[pl].rec, p.stride, p.frame_w, p.frame_h, cx, cy, MT_DC_PRED, 0, have_tr, have_bl, ft, p.bd,
-                   w.s[0].pred[pl], w.u);
-    dc[pl] = w.s[0].pred[pl][0];
-    const PlaneCost c = plane_chain<16, true>(a, P[pl], T, qm, sQs, nullptr, MT_TX_DCT_DCT, true, w.s[0].pred[pl],
-                                           w.s[0].cf[pl], w.s[0].rr[pl], w);
-    dc_total = __fadd_rn(dc_total, rd_cost_i64(c.sse, mlam, c.bits));
+  if constexpr (k420) {
+    best_total = use_cfl ? cfl_total : dc_total;
+  } else {
+    // the directional stage on dir_lambda: the current choice's total, then the ranked modes
+    const PlaneCost* cur = cost[use_cfl ? 1 : 0];
+    best_total = __fmul_rn(dlam, use_cfl ? sig : dc_bits);
+    for (int k = 0; k < 2; k++) best_total = __fadd_rn(best_total, plane_rd(cur[k], dlam));
   }
-  float best_total = dc_total;
+  put(use_cfl ? 1 : 0);
   int mode = MT_DC_PRED, delta = 0;
-  bool use_cfl = false;
-  // CfL: cfl_ac_sub of the 32x32 luma into 16x16
-  {
-    const int ls = a.u.luma_stride;
-    const uint16_t* l = luma + (size_t)jb.py * ls + jb.px;
-    int32_t sum = 128;
-    for (int i = 0; i < 256; i++) {
-      const int y = i >> 4, x = i & 15;
-      const uint16_t* q = l + (size_t)(2 * y) * ls + 2 * x;
-      const int32_t v = ((int32_t)q[0] + q[1] + q[ls] + q[ls + 1]) << 1;
-      w.ac[i] = (int16_t)v;
-      sum += v;
+  __syncthreads();  // the choice is written and the costs are read
+
+  // the SATD ranking: the 12 modes, or (joint) the directional ones at 7 deltas
+  const bool deltas = a.u.angle_deltas;
+  const int nrank = kJoint && deltas ? 60 : 12;
+  auto ranked = [&](int i, int* m, int* d) {  // entry i of the ranking
+    if (nrank == 12) {
+      *m = kJointList[i];
+      *d = 0;
+    } else if (i < 4) {  // the list's first four have no angle
+      *m = kJointList[i];
+      *d = 0;
+    } else {
+      *m = kJointList[4 + (i - 4) / 7];
+      *d = (i - 4) % 7 - 3;
     }
-    const int32_t mean = sum >> 8;
-    for (int i = 0; i < 256; i++) w.ac[i] = (int16_t)(w.ac[i] - mean);
+  };
+  for (int b = 0; b < nrank; b += kCands) {
+    const int i = min(b + (slot >> 1), nrank - 1);
+    int m, d;
+    ranked(i, &m, &d);
+    predict(m, d, have_tr, have_bl);
+    const unsigned long long sc = lane_satd_sad<N>(P, p.stride, w, g);
+    if (b + (slot >> 1) < nrank && g.j == 0) score[i][pl] = sc;
+    g.sync();  // the prediction is read
   }
-  int alpha[2];
-  for (int pl = 0; pl < 2; pl++) alpha[pl] = cfl_alpha_n<16>(w.ac, P[pl], p.stride, dc[pl], maxv);
-  {
-    Uv444Slot& c = w.s[1 - best];
-    float body = 0.0f;
-    for (int pl = 0; pl < 2; pl++) {
-      for (int i = 0; i < 256; i++) c.pred[pl][i] = (int16_t)cfl_pred_pixel(dc[pl], w.ac[i], alpha[pl], maxv);
-      const PlaneCost pc = plane_chain<16, true>(a, P[pl], T, qm, sQs, nullptr, MT_TX_DCT_DCT, false, c.pred[pl],
-                                               c.cf[pl], c.rr[pl], w);
-      body = __fadd_rn(body, rd_cost_i64(pc.sse, mlam, pc.bits));
+  __syncthreads();
+  if constexpr (kJoint) {
+    // the first joint_k entries by (score, mode, delta), each priced in full
+    const int nk = min(min(max(a.u.joint_k, 1), kMaxJoint), nrank);
+    for (int i = threadIdx.x; i < nrank; i += blockDim.x) {
+      int m, d;
+      ranked(i, &m, &d);
+      const unsigned long long sc = score[i][0] + score[i][1];
+      int before = 0;
+      for (int k = 0; k < nrank; k++) {
+        int mk, dk;
+        ranked(k, &mk, &dk);
+        const unsigned long long sk = score[k][0] + score[k][1];
+        before += sk < sc || (sk == sc && (mk < m || (mk == m && dk < d)));
+      }
+      if (before < nk) list[before] = (uint8_t)i;
     }
-    const float cfl_total =
-        __fsub_rn(__fadd_rn(body, __fmul_rn(mlam, uv_mode_bits(M, jb.y_mode, MT_UV_CFL_PRED, true, alpha[0], alpha[1]))),
-                  __fmul_rn(mlam, uv_mode_bits(M, jb.y_mode, MT_DC_PRED, false, 0, 0)));
+    __syncthreads();
+    for (int b = 0; b < nk; b += kCands) {
+      const int step = min(kCands, nk - b);
+      evaluate(step, [&](int c, int* tx) {
+        int m, d;
+        ranked(list[b + c], &m, &d);
+        *tx = chroma_tx(m);
+        predict(m, d, have_tr, have_bl);
+        return true;
+      });
+      int win = -1;
+      for (int c = 0; c < step; c++) {
+        int m, d;
+        ranked(list[b + c], &m, &d);
+        float ad_bits = 0.0f;
+        if (directional(m)) ad_bits = __fsub_rn(M.angle_delta[m - MT_V_PRED][d + 3], M.angle_delta[m - MT_V_PRED][3]);
+        float total = __fmul_rn(mlam, __fadd_rn(uv_mode_bits(M, jb.y_mode, m, false, 0, 0), ad_bits));
+        total = __fadd_rn(total, plane_rd(cost[c][0], mlam));
+        // once U's total reaches the best, V is not looked at
+        if (!(total >= best_total)) total = __fadd_rn(total, plane_rd(cost[c][1], mlam));
+        if (total < best_total) {
+          best_total = total;
+          mode = m;
+          delta = d;
+          use_cfl = false;
+          win = c;
+        }
+      }
+      if (win >= 0) put(win);
+      __syncthreads();
+    }
+  } else {
+    // rank_chroma_modes (superblock.rs:469-513) into DirectionalTopK
+    // (coder.rs:326-365), K = 3: earlier list entries win ties; priced in list order
+    uint32_t top = 0;
+    {
+      unsigned long long tc[3];
+      int ti[3], tn = 0;
+      for (int i = 0; i < 12; i++) {
+        const unsigned long long sc = score[i][0] + score[i][1];
+        if (tn == 3 && sc >= tc[2]) continue;
+        int pos = tn < 3 ? tn++ : 2;
+        for (; pos > 0 && sc < tc[pos - 1]; pos--) {
+          tc[pos] = tc[pos - 1];
+          ti[pos] = ti[pos - 1];
+        }
+        tc[pos] = sc;
+        ti[pos] = i;
+      }
+      for (int k = 0; k < tn; k++) top |= 1u << ti[k];
+    }
+    auto top_mode = [&](int c) { return (int)kJointList[__fns(top, 0, c + 1)]; };
+    for (int b = 0; b < 3; b += kCands) {
+      const int step = min(kCands, 3 - b);
+      evaluate(step, [&](int c, int* tx) {
+        const int m = top_mode(b + c);
+        *tx = N == 32 ? MT_TX_DCT_DCT : chroma_tx(m);  // forced DCT_DCT at TX_32X32
+        predict(m, 0, have_tr, have_bl);
+        return true;
+      });
+      int win = -1;
+      for (int c = 0; c < step; c++) {
+        const int m = top_mode(b + c);
+        float total = __fmul_rn(dlam, uv_mode_bits(M, jb.y_mode, m, false, 0, 0));
+        for (int k = 0; k < 2; k++) total = __fadd_rn(total, plane_rd(cost[c][k], dlam));
+        if (total < best_total) {
+          best_total = total;
+          mode = m;
+          if (k420) use_cfl = false;
+          win = c;
+        }
+      }
+      if (win >= 0) put(win);
+      __syncthreads();
+    }
+    // the zone-2 angle deltas of a directional winner (uv_ad; uv_ad32 at 32x32)
+    if (!(k420 && use_cfl) && deltas && directional(mode)) {
+      const int m = mode, tx0 = N == 32 ? MT_TX_DCT_DCT : chroma_tx(m);
+      int lo = 0, nd = 0;  // deltas lo, lo + 1, ... without 0
+      if (m == MT_V_PRED) lo = 1, nd = 3;
+      else if (m == MT_H_PRED) lo = -3, nd = 3;
+      else if (m == MT_D113_PRED || m == MT_D135_PRED || m == MT_D157_PRED) lo = -3, nd = 6;
+      auto nth = [&](int i) { return lo + i + (lo < 0 && lo + i >= 0); };
+      const float base_sig = __fsub_rn(uv_mode_bits(M, jb.y_mode, m, false, 0, 0), M.angle_delta[m - MT_V_PRED][3]);
+      for (int b = 0; b < nd; b += kCands) {
+        const int step = min(kCands, nd - b);
+        evaluate(step, [&](int c, int* tx) {
+          *tx = tx0;
+          predict(m, nth(b + c), false, false);
+          return true;
+        });
+        int win = -1;
+        for (int c = 0; c < step; c++) {
+          const int d = nth(b + c);
+          float total = __fmul_rn(dlam, __fadd_rn(base_sig, M.angle_delta[m - MT_V_PRED][d + 3]));
+          for (int k = 0; k < 2; k++) total = __fadd_rn(total, plane_rd(cost[c][k], dlam));
+          if (total < best_total) {
+            best_total = total;
+            delta = d;
+            win = c;
+          }
+        }
+        if (win >= 0) put(win);
+        __syncthreads();
+      }
+    }
+  }
+  if (threadIdx.x == 0) {
+    mt_uv16_result r;
+    r.total = best_total;
+    r.dc_total = dc_total;
     r.cfl_total = cfl_total;
-    if ((alpha[0] != 0 || alpha[1] != 0) && cfl_total < best_total) {
-      best_total = cfl_total;
-      use_cfl = true;
-      best = 1 - best;
-    }
+    r.uv_mode = (uint8_t)(mode != MT_DC_PRED ? mode : (use_cfl ? MT_UV_CFL_PRED : MT_DC_PRED));
+    r.angle_delta = (int8_t)delta;
+    r.cfl_alpha[0] = (int8_t)au;
+    r.cfl_alpha[1] = (int8_t)av;
+    res[job] = r;
   }
-  // rank_chroma_modes into DirectionalTopK (K = 3), then the ranked modes in list order
-  unsigned long long tc[3];
-  int tm[3], tn = 0;
-  int16_t* sp = w.s[1 - best].pred[0];
-  for (int ci = 0; ci < kJointModes; ci++) {
-    const int m = kJointList[ci];
-    unsigned long long sc = 0;
-    for (int pl = 0; pl < 2; pl++) {
-      predict_sq<16>(P[pl].rec, p.stride, p.frame_w, p.frame_h, cx, cy, m, 0, have_tr, have_bl, ft, p.bd, sp, w.u);
-      sc += satd_sad_proxy<16>(pl ? src_v : src_u, p.stride, cx, cy, sp, P[pl].vw, P[pl].vh);
-    }
-    int pos = tn < 3 ? tn : 2;
-    if (tn == 3 && sc >= tc[pos]) continue;
-    if (tn < 3) pos = tn++;
-    while (pos > 0 && sc < tc[pos - 1]) {
-      tc[pos] = tc[pos - 1];
-      tm[pos] = tm[pos - 1];
-      pos--;
-    }
-    tc[pos] = sc;
-    tm[pos] = m;
-  }
-  for (int ci = 0; ci < kJointModes; ci++) {
-    const int m = kJointList[ci];
-    bool in = false;
-    for (int e = 0; e < tn; e++) in |= tm[e] == m;
-    if (!in) continue;
-    const int tx = chroma_tx(m);
-    float total = __fmul_rn(mlam, uv_mode_bits(M, jb.y_mode, m, false, 0, 0));
-    Uv444Slot& c = w.s[1 - best];
-    for (int pl = 0; pl < 2; pl++) {
-      predict_sq<16>(P[pl].rec, p.stride, p.frame_w, p.frame_h, cx, cy, m, 0, have_tr, have_bl, ft, p.bd,
-                     c.pred[pl], w.u);
-      const PlaneCost pc =
-          plane_chain<16, true>(a, P[pl], T, qm, sQs, nullptr, tx, true, c.pred[pl], c.cf[pl], c.rr[pl], w);
-      total = __fadd_rn(total, rd_cost_i64(pc.sse, mlam, pc.bits));
-    }
-    if (total < best_total) {
-      best_total = total;
-      mode = m;
-      use_cfl = false;
-      best = 1 - best;
-    }
-  }
-  if (!use_cfl && a.u.angle_deltas && directional(mode)) {
-    const int m = mode, tx = chroma_tx(m);
-    int lo = 0, hi = -1;
-    if (m == MT_V_PRED) lo = 1, hi = 3;
-    else if (m == MT_H_PRED) lo = -3, hi = -1;
-    else if (m == MT_D113_PRED || m == MT_D135_PRED || m == MT_D157_PRED) lo = -3, hi = 3;
-    const float base_sig = __fsub_rn(uv_mode_bits(M, jb.y_mode, m, false, 0, 0), M.angle_delta[m - MT_V_PRED][3]);
-    for (int d = lo; d <= hi; d++) {
-      if (d == 0) continue;
-      float total = __fmul_rn(mlam, __fadd_rn(base_sig, M.angle_delta[m - MT_V_PRED][d + 3]));
-      Uv444Slot& c = w.s[1 - best];
-      for (int pl = 0; pl < 2; pl++) {
-        predict_sq<16>(P[pl].rec, p.stride, p.frame_w, p.frame_h, cx, cy, m, d, false, false, ft, p.bd, c.pred[pl],
-                       w.u);
-        const PlaneCost pc =
-            plane_chain<16, true>(a, P[pl], T, qm, sQs, nullptr, tx, true, c.pred[pl], c.cf[pl], c.rr[pl], w);
-        total = __fadd_rn(total, rd_cost_i64(pc.sse, mlam, pc.bits));
-      }
-      if (total < best_total) {
-        best_total = total;
-        delta = d;
-        best = 1 - best;
-      }
-    }
-  }
-  r.total = best_total;
-  r.dc_total = dc_total;
-  r.uv_mode = (uint8_t)(use_cfl ? MT_UV_CFL_PRED : mode);
-  r.angle_delta = (int8_t)delta;
-  r.cfl_alpha[0] = (int8_t)alpha[0];
-  r.cfl_alpha[1] = (int8_t)alpha[1];
-  const Uv444Slot& b = w.s[best];
-  if (cf_out)
-    for (int pl = 0; pl < 2; pl++)
-      for (int i = 0; i < 256; i++) cf_out[(size_t)j * 512 + pl * 256 + i] = b.cf[pl][i];
-  if (rec_out)
-    for (int pl = 0; pl < 2; pl++)
-      for (int i = 0; i < 256; i++)
-        rec_out[(size_t)j * 512 + pl * 256 + i] = (uint16_t)clampi((int32_t)b.pred[pl][i] + b.rr[pl][i], 0, maxv);
 }
 
 int uv_check(const mt_split16_params* p, const mt_uv16_params* u, const mt_quant* q, int32_t n) {
@@ -933,16 +616,18 @@ int uv_check_444(const mt_split16_params* p, const mt_uv16_params* u, const mt_q
 
 size_t up256(size_t v) { return (v + 255) & ~(size_t)255; }
 
-template <int N, typename J>
-int uv444_device(const uint16_t* su, const uint16_t* sv, const uint16_t* ru, const uint16_t* rv, const uint16_t* luma,
-                 const mt_split16_params* prm, const mt_uv16_params* uvp, const mt_quant* quant, const uint8_t* d_qm,
-                 const mt_coef_costs* d_costs, const mt_uv_mode_costs* d_mc, const J* d_jobs, int32_t n,
-                 mt_uv16_result* d_res, int32_t* d_cf, uint16_t* d_rec, void* stream) {
-  const int rc = uv_check_444(prm, uvp, quant, n);
+template <UvForm F, typename J>
+int uv_device(const uint16_t* su, const uint16_t* sv, const uint16_t* ru, const uint16_t* rv, const uint16_t* luma,
+              const mt_split16_params* prm, const mt_uv16_params* uvp, const mt_quant* quant, const uint8_t* d_qm,
+              const mt_coef_costs* d_costs, const mt_uv_mode_costs* d_mc, const J* d_jobs, int32_t n,
+              mt_uv16_result* d_res, int32_t* d_cf, uint16_t* d_rec, void* stream) {
+  using Shape = UvShape<F>;
+  const int rc = Shape::k420 ? uv_check(prm, uvp, quant, n) : uv_check_444(prm, uvp, quant, n);
   if (rc != MT_OK) return rc;
   if (n == 0) return MT_OK;
   if (!su || !sv || !ru || !rv || !luma || !d_costs || !d_mc || !d_jobs || !d_res) return MT_ERR_INVALID_INPUT;
-  if (!(uvp->dir_lambda > 0.0f) || prm->frame_w < N || prm->frame_h < N) return MT_ERR_INVALID_INPUT;
+  if (!Shape::k420 && (!(uvp->dir_lambda > 0.0f) || prm->frame_w < Shape::N || prm->frame_h < Shape::N))
+    return MT_ERR_INVALID_INPUT;
   UvArgs a;
   a.p = *prm;
   a.u = *uvp;
@@ -950,61 +635,12 @@ int uv444_device(const uint16_t* su, const uint16_t* sv, const uint16_t* ru, con
   a.lambda = prm->trellis_lambda0 > 0.0f ? mth::scaled_trellis_lambda_host((float)quant->dc_q, prm->trellis_lambda0)
                                          : 0.0f;
   a.has_qm = quant->qm_level < 15 && d_qm != nullptr;
-  const int stride = arena_stride(sizeof(UvBigWork<N>));
-  auto* kern = uv444_kernel<N, J>;
-  int threads = 0;
-  size_t dyn = 0;
-  if (!arena_launch_shape(kern, n, stride, kUvThreads, &threads, &dyn)) return MT_ERR_DEVICE;
-  kern<<<(unsigned)((n + threads - 1) / threads), threads, dyn, reinterpret_cast<cudaStream_t>(stream)>>>(
-      su, sv, ru, rv, luma, a, d_qm, d_costs, d_mc, d_jobs, n, d_res, d_cf, d_rec, stride);
-  return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_DEVICE;
-}
-
-int uv32_device(const uint16_t* su, const uint16_t* sv, const uint16_t* ru, const uint16_t* rv, const uint16_t* luma,
-                const mt_split16_params* prm, const mt_uv16_params* uvp, const mt_quant* quant, const uint8_t* d_qm,
-                const mt_coef_costs* d_costs, const mt_uv_mode_costs* d_mc, const mt_uv16_444_job* d_jobs, int32_t n,
-                mt_uv16_result* d_res, int32_t* d_cf, uint16_t* d_rec, void* stream) {
-  const int rc = uv_check(prm, uvp, quant, n);
-  if (rc != MT_OK) return rc;
-  if (n == 0) return MT_OK;
-  if (!su || !sv || !ru || !rv || !luma || !d_costs || !d_mc || !d_jobs || !d_res) return MT_ERR_INVALID_INPUT;
-  UvArgs a;
-  a.p = *prm;
-  a.u = *uvp;
-  a.q = *quant;
-  a.lambda = prm->trellis_lambda0 > 0.0f ? mth::scaled_trellis_lambda_host((float)quant->dc_q, prm->trellis_lambda0)
-                                         : 0.0f;
-  a.has_qm = quant->qm_level < 15 && d_qm != nullptr;
-  const int stride = arena_stride(sizeof(Uv444Work));
-  int threads = 0;
-  size_t dyn = 0;
-  if (!arena_launch_shape(uv32_420_kernel, n, stride, kUvThreads, &threads, &dyn)) return MT_ERR_DEVICE;
-  uv32_420_kernel<<<(unsigned)((n + threads - 1) / threads), threads, dyn, reinterpret_cast<cudaStream_t>(stream)>>>(
-      su, sv, ru, rv, luma, a, d_qm, d_costs, d_mc, d_jobs, n, d_res, d_cf, d_rec, stride);
-  return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_DEVICE;
-}
-
-int uv16_device(const uint16_t* su, const uint16_t* sv, const uint16_t* ru, const uint16_t* rv, const uint16_t* luma,
-                const mt_split16_params* prm, const mt_uv16_params* uvp, const mt_quant* quant, const uint8_t* d_qm,
-                const mt_coef_costs* d_costs, const mt_uv_mode_costs* d_mc, const mt_uv16_job* d_jobs, int32_t n,
-                mt_uv16_result* d_res, int32_t* d_cf, uint16_t* d_rec, void* stream) {
-  const int rc = uv_check(prm, uvp, quant, n);
-  if (rc != MT_OK) return rc;
-  if (n == 0) return MT_OK;
-  if (!su || !sv || !ru || !rv || !luma || !d_costs || !d_mc || !d_jobs || !d_res) return MT_ERR_INVALID_INPUT;
-  UvArgs a;
-  a.p = *prm;
-  a.u = *uvp;
-  a.q = *quant;
-  a.lambda = prm->trellis_lambda0 > 0.0f ? mth::scaled_trellis_lambda_host((float)quant->dc_q, prm->trellis_lambda0)
-                                         : 0.0f;
-  a.has_qm = quant->qm_level < 15 && d_qm != nullptr;
-  const int stride = arena_stride(sizeof(UvWork));
-  int threads = 0;
-  size_t dyn = 0;
-  if (!arena_launch_shape(uv16_420_kernel, n, stride, kUvThreads, &threads, &dyn)) return MT_ERR_DEVICE;
-  uv16_420_kernel<<<(unsigned)((n + threads - 1) / threads), threads, dyn, reinterpret_cast<cudaStream_t>(stream)>>>(
-      su, sv, ru, rv, luma, a, d_qm, d_costs, d_mc, d_jobs, n, d_res, d_cf, d_rec, stride);
+  auto* kern = uv_kernel<F, J>;
+  constexpr size_t dyn = sizeof(LaneBuf<Shape::N>) * Shape::kSlots;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn) != cudaSuccess)
+    return MT_ERR_DEVICE;
+  kern<<<(unsigned)n, Shape::kThreads, dyn, reinterpret_cast<cudaStream_t>(stream)>>>(
+      su, sv, ru, rv, luma, a, d_qm, d_costs, d_mc, d_jobs, n, d_res, d_cf, d_rec);
   return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_DEVICE;
 }
 
@@ -1073,7 +709,7 @@ int mt_pick_uv16_420_device(const uint16_t* d_src_u, const uint16_t* d_src_v, co
                             const mt_coef_costs* d_costs, const mt_uv_mode_costs* d_mode_costs,
                             const mt_uv16_job* d_jobs, int32_t n, mt_uv16_result* d_results, int32_t* d_cf,
                             uint16_t* d_rec, void* stream) {
-  return uv16_device(d_src_u, d_src_v, d_rec_u, d_rec_v, d_luma, prm, uvp, quant, d_qm_row, d_costs, d_mode_costs,
+  return uv_device<UvForm::k16_420>(d_src_u, d_src_v, d_rec_u, d_rec_v, d_luma, prm, uvp, quant, d_qm_row, d_costs, d_mode_costs,
                      d_jobs, n, d_results, d_cf, d_rec, stream);
 }
 
@@ -1089,7 +725,7 @@ int mt_pick_uv16_420(const uint16_t* src_u, const uint16_t* src_v, const uint16_
                  [&](const uint16_t* su, const uint16_t* sv, const uint16_t* ru, const uint16_t* rv, const uint16_t* l,
                      const uint8_t* qm, const mt_coef_costs* c, const mt_uv_mode_costs* mc, const mt_uv16_job* j,
                      mt_uv16_result* r, int32_t* cf, uint16_t* rec) {
-                   return uv16_device(su, sv, ru, rv, l, prm, uvp, quant, qm, c, mc, j, n, r, cf, rec, nullptr);
+                   return uv_device<UvForm::k16_420>(su, sv, ru, rv, l, prm, uvp, quant, qm, c, mc, j, n, r, cf, rec, nullptr);
                  });
 }
 
@@ -1099,7 +735,7 @@ int mt_pick_uv32_444_device(const uint16_t* d_src_u, const uint16_t* d_src_v, co
                             const mt_coef_costs* d_costs, const mt_uv_mode_costs* d_mode_costs,
                             const mt_uv32_444_job* d_jobs, int32_t n, mt_uv16_result* d_results, int32_t* d_cf,
                             uint16_t* d_rec, void* stream) {
-  return uv444_device<32>(d_src_u, d_src_v, d_rec_u, d_rec_v, d_luma, prm, uvp, quant, d_qm_row, d_costs,
+  return uv_device<UvForm::k32_444>(d_src_u, d_src_v, d_rec_u, d_rec_v, d_luma, prm, uvp, quant, d_qm_row, d_costs,
                           d_mode_costs, d_jobs, n, d_results, d_cf, d_rec, stream);
 }
 
@@ -1116,7 +752,7 @@ int mt_pick_uv32_444(const uint16_t* src_u, const uint16_t* src_v, const uint16_
                  [&](const uint16_t* su, const uint16_t* sv, const uint16_t* ru, const uint16_t* rv, const uint16_t* l,
                      const uint8_t* qm, const mt_coef_costs* c, const mt_uv_mode_costs* mc,
                      const mt_uv32_444_job* j, mt_uv16_result* r, int32_t* cf, uint16_t* rec) {
-                   return uv444_device<32>(su, sv, ru, rv, l, prm, uvp, quant, qm, c, mc, j, n, r, cf, rec, nullptr);
+                   return uv_device<UvForm::k32_444>(su, sv, ru, rv, l, prm, uvp, quant, qm, c, mc, j, n, r, cf, rec, nullptr);
                  });
 }
 
@@ -1126,7 +762,7 @@ int mt_pick_uv32_420_device(const uint16_t* d_src_u, const uint16_t* d_src_v, co
                             const mt_coef_costs* d_costs, const mt_uv_mode_costs* d_mode_costs,
                             const mt_uv32_420_job* d_jobs, int32_t n, mt_uv16_result* d_results, int32_t* d_cf,
                             uint16_t* d_rec, void* stream) {
-  return uv32_device(d_src_u, d_src_v, d_rec_u, d_rec_v, d_luma, prm, uvp, quant, d_qm_row, d_costs, d_mode_costs,
+  return uv_device<UvForm::k32_420>(d_src_u, d_src_v, d_rec_u, d_rec_v, d_luma, prm, uvp, quant, d_qm_row, d_costs, d_mode_costs,
                      d_jobs, n, d_results, d_cf, d_rec, stream);
 }
 
@@ -1142,7 +778,7 @@ int mt_pick_uv32_420(const uint16_t* src_u, const uint16_t* src_v, const uint16_
                  [&](const uint16_t* su, const uint16_t* sv, const uint16_t* ru, const uint16_t* rv, const uint16_t* l,
                      const uint8_t* qm, const mt_coef_costs* c, const mt_uv_mode_costs* mc,
                      const mt_uv32_420_job* j, mt_uv16_result* r, int32_t* cf, uint16_t* rec) {
-                   return uv32_device(su, sv, ru, rv, l, prm, uvp, quant, qm, c, mc, j, n, r, cf, rec, nullptr);
+                   return uv_device<UvForm::k32_420>(su, sv, ru, rv, l, prm, uvp, quant, qm, c, mc, j, n, r, cf, rec, nullptr);
                  });
 }
 
@@ -1152,7 +788,7 @@ int mt_pick_uv16_444_device(const uint16_t* d_src_u, const uint16_t* d_src_v, co
                             const mt_coef_costs* d_costs, const mt_uv_mode_costs* d_mode_costs,
                             const mt_uv16_444_job* d_jobs, int32_t n, mt_uv16_result* d_results, int32_t* d_cf,
                             uint16_t* d_rec, void* stream) {
-  return uv444_device<16>(d_src_u, d_src_v, d_rec_u, d_rec_v, d_luma, prm, uvp, quant, d_qm_row, d_costs,
+  return uv_device<UvForm::k16_444>(d_src_u, d_src_v, d_rec_u, d_rec_v, d_luma, prm, uvp, quant, d_qm_row, d_costs,
                           d_mode_costs, d_jobs, n, d_results, d_cf, d_rec, stream);
 }
 
@@ -1169,7 +805,7 @@ int mt_pick_uv16_444(const uint16_t* src_u, const uint16_t* src_v, const uint16_
                  [&](const uint16_t* su, const uint16_t* sv, const uint16_t* ru, const uint16_t* rv, const uint16_t* l,
                      const uint8_t* qm, const mt_coef_costs* c, const mt_uv_mode_costs* mc,
                      const mt_uv16_444_job* j, mt_uv16_result* r, int32_t* cf, uint16_t* rec) {
-                   return uv444_device<16>(su, sv, ru, rv, l, prm, uvp, quant, qm, c, mc, j, n, r, cf, rec, nullptr);
+                   return uv_device<UvForm::k16_444>(su, sv, ru, rv, l, prm, uvp, quant, qm, c, mc, j, n, r, cf, rec, nullptr);
                  });
 }
 

@@ -76,3 +76,46 @@ def test_lane_leaves_match_oracle(mt_lib, oracle_lib, cuda, family, n, kind, qid
         want = oracle_lib.leaf16(*oargs, refine=refine, threads=threads)
     for a, b in zip(got, want):
         assert np.asarray(a).tobytes() == np.asarray(b).tobytes()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["16_420", "32_420", "16_444", "32_444"])
+@pytest.mark.parametrize("kind,qidx,cut,wsse,lam0,joint_k,ad", [
+    ("photo", 70, (0, 0), 0.0, 0.05, 1, True),
+    ("hard", 1, (5, 3), 1.0, 0.05, 12, True),    # the finest steps; shortlists past one step's candidates
+    ("flat", 200, (9, 50), 0.5, 0.3, 5, True),   # empty blocks, leaves past the displayed frame
+    ("hard", 40, (17, 6), 1.0, 0.0, 4, False),   # no trellis, no deltas
+    ("photo", 130, (2, 1), 1.0, 0.6, 7, True),
+])
+def test_lane_chroma_matches_oracle(mt_lib, oracle_lib, cuda, form, kind, qidx, cut, wsse, lam0, joint_k, ad):
+    leaf, sub = int(form[:2]), form.endswith("420")
+    n = leaf // 2 if sub else leaf
+    y, yr = _case(kind, qidx)
+    (u, ur), (v, vr) = _case(kind, qidx + 1), _case("photo", qidx + 2)
+    if sub:
+        u, ur, v, vr = [np.ascontiguousarray(a[::2, ::2]) for a in (u, ur, v, vr)]
+    qm_level = 15 if qidx == 1 else 3 + qidx % 9
+    q = oracle_lib.quant_new_chroma(qidx, 0, 0, 8, qm_level)
+    qm = oracle_lib.qm_row(qm_level, 1, n) if qm_level < 15 else None
+    ch, cw = u.shape
+    prm = mt_lib.split16_params(cw, ch, trellis_lambda0=lam0, rd_lambda=0.03 if kind == "hard" else 0.4 * qidx + 1.0,
+                                band_tilt=0.7, wsse_scale=wsse, vis=(cw - cut[0], ch - cut[1]),
+                                skip_bits=[(2.0 + 0.3 * k, 0.5) for k in range(13)] if qidx > 100 else None)
+    uvp = mt_lib.uv16_params(W, joint_k=joint_k, angle_deltas=ad, dir_lambda=0.3 * qidx + 0.5)
+    if form == "16_420":
+        jobs = synth.uv16_jobs(W, H, qidx)
+    elif form == "32_444":
+        jobs = synth.uv32_444_jobs(W, H, qidx)
+    else:
+        jobs = synth.uv16_444_jobs(W, H, qidx, leaf=leaf)
+    jobs["px"][1] = W - leaf + 4  # off the leaf grid: rejected
+    jobs["y_mode"][2] = 13
+    qctx = oracle_lib.qcat(qidx)
+    got = getattr(mt_lib, "pick_uv" + form)(
+        u, v, ur, vr, yr, prm, uvp, q, qm, mt_lib.coef_costs(mt_lib.coef_cdfs_default(qctx, n, n, 1)),
+        mt_lib.uv_mode_costs(mt_lib.uv_mode_cdfs_default()), jobs, want_cf=True, want_rec=True)
+    want = getattr(oracle_lib, "pick_uv" + form)(
+        u, v, ur, vr, yr, prm, uvp, q, qm, oracle_lib.default_cdfs(qctx, n, plane=1), oracle_lib.uv_mode_cdfs(), jobs,
+        threads=os.cpu_count() or 1, want_cf=True, want_rec=True)
+    for a, b in zip(got, want):
+        assert np.asarray(a).tobytes() == np.asarray(b).tobytes()
