@@ -20,9 +20,9 @@
 // blocks from a ticket counter in dependency-level order (a block after its
 // left, top, top-left and, where its edges use them, top-right and
 // bottom-left neighbours inside its tile) and waits on those neighbours'
-// done counts with bounded polls.  The 91 luma candidates of a block are
-// split over the cluster's CTAs, each evaluated by eight lanes; the cluster
-// minimum picks the winner.  Frames code in the spec-minimum uniform tiling
+// done counts with bounded polls.  The 13 modes of a block are split over the
+// cluster's CTAs and the seven transform types over a CTA's warps, each (mode,
+// type) candidate on eight lanes; the cluster minimum picks the winner.  Frames code in the spec-minimum uniform tiling
 // (one tile up to 64 superblocks wide and 2304 in area), tiles independent.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -38,8 +38,6 @@
 
 #include "../../include/maroontree_b200.h"
 #include "av1_tables.h"
-#include "chain4.cuh"
-#include "chain8.cuh"
 #include "coop8.cuh"
 #include "pack.h"
 
@@ -50,10 +48,6 @@ float scaled_trellis_lambda_host(float dc_q, float lambda0);
 namespace {
 
 namespace cg = cooperative_groups;
-
-constexpr int kCands = 13 * 7;
-__constant__ uint8_t kEncTypes[7] = {MT_TX_IDTX,      MT_TX_DCT_DCT,   MT_TX_V_DCT,  MT_TX_H_DCT,
-                                     MT_TX_ADST_ADST, MT_TX_ADST_DCT, MT_TX_DCT_ADST};
 
 struct EncArgs {
   const uint16_t* src[3];
@@ -78,7 +72,6 @@ struct EncArgs {
 struct JobDesc {
   EncArgs a;
   const mt_coef_costs* cy;
-  const mt_coef_costs* cc;
   const uint8_t* qmy;
   const uint8_t* qmc;
   uint32_t* done;
@@ -118,52 +111,49 @@ __host__ __device__ inline void zorder(int k, int* bx, int* by, bool* thr, bool*
 
 __device__ __forceinline__ bool is_smooth(int m) { return m == MT_SMOOTH_PRED || m == MT_SMOOTH_V_PRED || m == MT_SMOOTH_H_PRED; }
 
-// The 91 candidates of a block are split over a cluster of kClusterCtas CTAs
-// (on as many SMs): CTA r takes candidate indices [23r, 23r + 23) (index =
-// mode * 7 + type, the order ties are broken in) and runs them type by type,
-// so the four octets of a warp mostly share a transform path.
+// A block is a cluster of kClusterCtas CTAs (on as many SMs).  CTA r takes the
+// modes [kModeLo[r], kModeLo[r + 1]), and its warp t the transform type t of
+// them, an octet of lanes per mode: a warp runs one transform path, a CTA
+// predicts each mode once for the seven types.  The last warp codes a chroma
+// plane in CTAs 2 and 3 and fetches the cluster's next block in CTA 0.
+// Candidate index = mode * 7 + type, the order ties are broken in.
 constexpr int kClusterCtas = 4;
 // CTAs of the decision kernel resident per SM (its register budget follows).
 #ifndef MT_ENC_CTAS_PER_SM
 #define MT_ENC_CTAS_PER_SM 2
 #endif
-constexpr int kCandPerCta = 23;
-constexpr int kLumaThreads = 192;  // 23 octets, rounded up to whole warps
+constexpr int kTypes = 7;  // MT_TX_IDTX .. MT_TX_DCT_ADST
+constexpr int kLumaThreads = kTypes * 32;
 constexpr int kStepThreads = kLumaThreads + 32;
+constexpr int kOctBufs = kTypes * 4 + 8;  // an octet each, and eight groups of four lanes for chroma
+__device__ __forceinline__ int mode_lo(int rank) { return rank ? 3 * rank + 1 : 0; }  // 0, 4, 7, 10
+__device__ __forceinline__ int mode_rank(int m) { return m < 4 ? 0 : (m - 1) / 3; }
 
-struct CandOrder {
-  int8_t t[kClusterCtas][kLumaThreads / 8];  // candidate index per octet, -1 none
+// The next block of a cluster: its ticket (kNoTicket past an abort) and its
+// list entry.
+constexpr uint32_t kNoTicket = 0xffffffffu;
+struct NextBlock {
+  uint32_t ticket, entry, image, pad;
 };
-constexpr CandOrder make_order() {
-  CandOrder o{};
-  for (int r = 0; r < kClusterCtas; ++r) {
-    const int lo = r * kCandPerCta, hi = lo + kCandPerCta < kCands ? lo + kCandPerCta : kCands;
-    int k = 0;
-    for (int ti = 0; ti < 7; ++ti)
-      for (int m = 0; m < 13; ++m)
-        if (m * 7 + ti >= lo && m * 7 + ti < hi) o.t[r][k++] = (int8_t)(m * 7 + ti);
-    for (; k < kLumaThreads / 8; ++k) o.t[r][k] = -1;
-  }
-  return o;
-}
-__constant__ CandOrder kOrder = make_order();
 
-// Everything one CTA keeps in shared memory.
+// Everything one CTA keeps in shared memory beside the octets' buffers.
 struct StepShared {
-  mt_coef_costs cy, cc;
-  float qsY[64], qsC[64], lut[64];
-  uint8_t qmY[64], qmC[64];
-  mtd::CoopTabs tabs;
-  int16_t pred[4][64];              // the predictions of this CTA's four modes (angle delta 0)
-  int16_t cpred[64];                // the chroma DC prediction (4:4:4)
-  uint16_t src[64], csrc[64];       // the block's luma and chroma source samples
-  int16_t above[2][17], left[2][16];  // the block's luma / chroma neighbours (mtd::EdgeRead)
-  mtd::Edge8 edge[5];                 // the edges of the four luma predictions and the chroma one
-  unsigned long long best;
-  uint32_t ticket, abort;
-  int cur;                            // the image whose tables are staged (-1: none)
-  JobDesc job;                        // its descriptor
-  mtd::Oct8 oct[kLumaThreads / 8 + 1];  // one per candidate octet, then the chroma plane's
+  alignas(16) int16_t pcol[4][64];  // the predictions of this CTA's modes, by columns
+  alignas(16) int16_t rcol[4][64];  // their residuals by columns
+  alignas(16) int16_t rrow[4][64];  // and by rows
+  alignas(16) int16_t ccol[64];     // the chroma residual by columns (4:4:4)
+  alignas(16) int16_t src[64], csrc[64];  // the block's luma and chroma source samples, by columns
+  mtd::CoopEdges edge;
+  mtd::CoopPredBuf pb[4];
+  mtd::CoopPlane py, pc;
+  mtd::CoopScan scan;
+  mt_coef_costs cy;
+  unsigned long long key[kTypes];            // the warps' minima
+  unsigned long long ckey[2][kClusterCtas];  // the CTAs' minima, by block parity
+  alignas(16) NextBlock next[2];             // by block parity
+  uint8_t nb_mode[2];                        // modes of the blocks above and to the left
+  int cur;                                   // the image whose tables are staged (-1: none)
+  JobDesc job;                               // its descriptor
 };
 
 __device__ __forceinline__ void luma_bar() { asm volatile("bar.sync 1, %0;" ::"n"(kLumaThreads) : "memory"); }
@@ -173,122 +163,150 @@ __device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-
-// Writes of a winning 8x8 chain: levels, and prediction + inverse residual
-// into the reconstruction plane (lane j: row j, and levels [8j, 8j+8)).
-__device__ __forceinline__ void put8(const mtd::Oct8& o, const int16_t* pred, int32_t* lv, uint16_t* rec, int stride,
-                                     int px, int py, int j) {
-#pragma unroll
-  for (int i = 0; i < 8; ++i) lv[j * 8 + i] = o.cf[j * 8 + i];
-#pragma unroll
-  for (int x = 0; x < 8; ++x)
-    rec[(size_t)(py + j) * stride + px + x] = (uint16_t)min(max((int)pred[j * 8 + x] + o.rr[j * 8 + x], 0), 255);
-}
-
-// A block's neighbours (above run of 17 from (ox - 1, oy - 1), left run of 16
-// from (ox - 1, oy)) into shared memory for lanes k in [0, 33), read past L1
-// (they were written by other SMs); only the sides inside the block's tile are
-// read, and positions outside the plane are clamped (never read by the
-// predictor).
-__device__ __forceinline__ void stage_edges(const uint16_t* rec, int stride, int fw, int fh, int ox, int oy, bool top,
-                                            bool lft, int16_t* above, int16_t* left, int k) {
-  if (k < 17) {
-    if (top) above[k] = (int16_t)__ldcg(rec + (size_t)(oy - 1) * stride + min(max(ox - 1 + k, 0), fw - 1));
-  } else if (k < 33) {
-    if (lft) left[k - 17] = (int16_t)__ldcg(rec + (size_t)min(oy + k - 17, fh - 1) * stride + ox - 1);
-  }
+__device__ __forceinline__ void add_release(uint32_t* p) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
 }
 
 constexpr uint32_t kDonePerBlock = kClusterCtas;  // each CTA of the coding cluster publishes once
 constexpr int kMaxPolls = 1 << 20;               // a dependency wait gives up after this many polls
 
+// One chroma plane of a block on the last warp: UV_DC_PRED and DCT_DCT, 8x8 in
+// 4:4:4 and 4x4 in 4:2:0.  Only the levels and the reconstruction are wanted,
+// so the chain stops after the inverse.  Every group of lanes computes the
+// block; the first one writes it.
+__device__ __forceinline__ void code_chroma(StepShared& S, mtd::OctBuf* bufs, const EncArgs& a, int pl, int b, int px,
+                                            int py, bool has_t, bool has_l) {
+  const int lane = threadIdx.x & 31;
+  const int n = a.sub ? 4 : 8, ln = a.sub ? 2 : 3;
+  const int cx = a.sub ? px / 2 : px, cy = a.sub ? py / 2 : py, stride = a.pc.stride;
+  uint16_t* rec = a.rec[1 + pl] + (size_t)cy * stride + cx;
+  int32_t* lv = (pl == 0 ? a.lv_u : a.lv_v) + (size_t)b * n * n;
+  int32_t s = 0;  // dc_pred_sq_at; the neighbours are read past L1 (other SMs wrote them)
+  if (lane < n) {
+    if (has_t) s = __ldcg(rec - stride + lane);
+  } else if (lane < 2 * n) {
+    if (has_l) s = __ldcg(rec + (size_t)(lane - n) * stride - 1);
+  }
+  s = __reduce_add_sync(0xffffffffu, s);
+  const int32_t dc = (has_t && has_l) ? (n + s) >> (ln + 1) : ((has_t || has_l) ? ((n >> 1) + s) >> ln : 128);
+  int32_t c[8], v[8];
+  float at[8];
+  int e[8];
+  if (n == 8) {
+    const mtd::Coop<8> g;
+    mtd::OctBuf& o = bufs[lane >> 3];
+    for (int i = lane; i < 64; i += 32) S.ccol[i] = (int16_t)(S.csrc[i] - dc);
+    __syncwarp();
+#pragma unroll
+    for (int x = 0; x < 8; x++) e[x] = S.scan.row8[g.j][x];
+    mtd::coop8_fwd(MT_TX_DCT_DCT, S.ccol, nullptr, S.pc, c, at, o, g);
+    mtd::coop_trellis<8>(c, at, e, S.pc, o, g);
+    mtd::coop8_inv(MT_TX_DCT_DCT, c, S.pc, v, o, g);
+    if (lane < 8) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        lv[k * 8 + g.j] = c[k];
+        rec[(size_t)k * stride + g.j] = (uint16_t)min(max(dc + v[k], 0), 255);
+      }
+    }
+  } else {
+    const mtd::Coop<4> g;
+    mtd::OctBuf& o = bufs[lane >> 2];
+#pragma unroll
+    for (int x = 0; x < 4; x++) {
+      e[x] = S.scan.row4[g.j][x];
+      v[x] = S.csrc[g.j * 4 + x] - dc;
+    }
+    mtd::coop4_fwd(v, S.pc, c, at, o, g);
+    mtd::coop_trellis<4>(c, at, e, S.pc, o, g);
+    mtd::coop4_inv(c, S.pc, v, o, g);
+    if (lane < 4) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        lv[k * 4 + g.j] = c[k];
+        rec[(size_t)k * stride + g.j] = (uint16_t)min(max(dc + v[k], 0), 255);
+      }
+    }
+  }
+}
+
 // The 8x8 blocks of the frame in dependency order, coded by persistent
-// clusters (one block per cluster at a time).  A cluster takes the next block
-// from the ticket counter, waits until the block's left, top, top-left and,
-// where its intra edges use them, top-right and bottom-left neighbours are
-// published (done[] == kDonePerBlock), stages the neighbours and the source
-// block in shared memory, and evaluates the block: in each CTA the luma warps
-// run its share of the 91 candidates (the first four octets also build the
-// four predictions the share needs), the last warp codes a chroma plane in
-// CTAs 2 (U) and 3 (V).  The cluster's winner is the minimum of the CTAs'
-// keys (cost, candidate index), read through distributed shared memory; the
-// CTA holding it writes it out; then every CTA publishes.  Tickets follow the
-// dependency levels, so a block waits only on blocks that running clusters
-// took earlier.  A wait that runs out of polls sets *err; once *err is set
-// the remaining waits stop and every cluster leaves at its next ticket.
+// clusters (one block per cluster at a time).  A cluster takes blocks from the
+// ticket counter (CTA 0 fetches the next one while the current block is
+// evaluated, and writes it to every CTA before the cluster meets), waits until
+// the block's left, top, top-left and, where its intra edges use them,
+// top-right and bottom-left neighbours are published (done[] ==
+// kDonePerBlock), builds the intra edges once, predicts its modes (a warp each)
+// and evaluates its candidates.  The CTAs exchange their minimum keys (cost,
+// candidate index) through distributed shared memory before the one cluster
+// barrier of the block; then the octet that holds the cluster's minimum writes
+// the block out and every CTA publishes.  Keys and next blocks alternate
+// between two slots, so nothing is overwritten before all have read it.
+// Tickets follow the dependency levels, so the lowest unfinished ticket's
+// cluster has nothing left to wait for: a cluster holds a later ticket only
+// while it works on an earlier one.  A wait that runs out of polls sets *err;
+// once *err is set the remaining waits stop and every cluster leaves at its
+// next ticket.
 // list[i] = block index | have-top-right (bit 30) | left-has-bottom (bit 31).
+//
+// Bound by the dependency chain: a level's latency is the wait for the
+// neighbours, the edges, the prediction, one candidate chain and the exchange.
 __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThreads, MT_ENC_CTAS_PER_SM)
     encode_blocks_kernel(const JobDesc* __restrict__ jobs, const uint2* __restrict__ list, int nlist,
                          uint32_t* ticket_ctr, uint32_t* err) {
   __shared__ StepShared S;
+  extern __shared__ __align__(16) unsigned char oct_smem[];
+  mtd::OctBuf* bufs = reinterpret_cast<mtd::OctBuf*>(oct_smem);
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
-  const int t = threadIdx.x;
-  if (t < 64) {
-    S.lut[t] = mtd::kCoefRateLut[t];
-    S.tabs.load(t, 64);
-  } else if (t == 64) {
-    S.best = ~0ull;
-    S.cur = -1;
-  }
-  __syncthreads();
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  if (t < 64) S.scan.stage(t);
+  if (t == 64) S.cur = -1;
+  auto fetch = [&](int slot) {  // one thread of CTA 0
+    const uint32_t tk = atomicAdd(ticket_ctr, 1u);
+    const uint32_t ab = *(volatile uint32_t*)err;
+    uint2 ent = make_uint2(0, 0);
+    if (tk < (uint32_t)nlist) ent = list[tk];
+    const uint4 v = make_uint4(ab ? kNoTicket : tk, ent.x, ent.y, 0);
+    for (int q = 0; q < kClusterCtas; ++q) *reinterpret_cast<uint4*>(cluster.map_shared_rank(&S.next[slot], q)) = v;
+  };
+  cluster.sync();  // every CTA of the cluster has started
+  if (rank == 0 && t == kLumaThreads) fetch(0);
+  cluster.sync();
   const EncArgs& a = S.job.a;
-  const int mlo = rank * kCandPerCta / 7;  // first mode of this CTA's share
-  const int c = t - kLumaThreads;          // lane of the chroma warp
-  const int pl = rank - 2;                 // its plane (CTAs 2 and 3)
-  for (;;) {
-    if (rank == 0 && t == 0) {
-      S.ticket = atomicAdd(ticket_ctr, 1u);
-      S.abort = *(volatile uint32_t*)err;
-    }
-    cluster.sync();
-    const uint32_t tk = *cluster.map_shared_rank(&S.ticket, 0);
-    const uint32_t ab = *cluster.map_shared_rank(&S.abort, 0);
-    if (ab || tk >= (uint32_t)nlist) break;  // the same for every CTA of the cluster
-    const uint2 ent = list[tk];
-    const int img = (int)ent.y;
-    if (img != S.cur) {  // another image: its descriptor, then its cost and QM tables
+  const int mlo = mode_lo(rank), nm = mode_lo(rank + 1) - mlo;  // this CTA's modes
+  for (int par = 0;; par ^= 1) {
+    const NextBlock nx = S.next[par];
+    if (nx.ticket >= (uint32_t)nlist) break;  // the same for every CTA of the cluster
+    const int img = (int)nx.image;
+    if (img != S.cur) {  // another image: its descriptor, then its tables
+      __syncthreads();
       const int* gj = reinterpret_cast<const int*>(jobs + img);
       int* sj = reinterpret_cast<int*>(&S.job);
       for (int i = t; i < (int)(sizeof(JobDesc) / 4); i += blockDim.x) sj[i] = gj[i];
       __syncthreads();
       const float* gy = reinterpret_cast<const float*>(S.job.cy);
-      const float* gc = reinterpret_cast<const float*>(S.job.cc);
       float* sy = reinterpret_cast<float*>(&S.cy);
-      float* sc = reinterpret_cast<float*>(&S.cc);
-      for (int i = t; i < (int)(sizeof(mt_coef_costs) / 4); i += blockDim.x) {
-        sy[i] = gy[i];
-        sc[i] = gc[i];
-      }
-      if (t < 64) {
-        const int w = a.has_qm_y ? S.job.qmy[t] : 32;
-        S.qmY[t] = (uint8_t)w;
-        S.qsY[t] = mtd::fwd_qm_scale(w);
-      } else if (t < 128) {
-        const int i = t - 64;
-        const int w = (a.has_qm_c && i < (a.sub ? 16 : 64)) ? S.job.qmc[i] : 32;
-        S.qmC[i] = (uint8_t)w;
-        S.qsC[i] = mtd::fwd_qm_scale(w);
-      }
+      for (int i = t; i < (int)(sizeof(mt_coef_costs) / 4); i += blockDim.x) sy[i] = gy[i];
+      if (t < 64) S.py.stage(t, a.qy, a.tly, a.has_qm_y ? S.job.qmy : nullptr, 64);
+      else if (t < 128) S.pc.stage(t - 64, a.qc, a.tlc, a.has_qm_c ? S.job.qmc : nullptr, a.sub ? 16 : 64);
       __syncthreads();
       if (t == 0) S.cur = img;
     }
     uint32_t* const done = S.job.done;
     const int nbx = a.w8 / 8;
-    const uint32_t e = ent.x;
+    const uint32_t e = nx.entry;
     const int b = (int)(e & 0x3fffffffu);
     const int bx = b % nbx, by = b / nbx;
     const int px = bx * 8, py = by * 8;
     const bool thr = (e >> 30) & 1, lhb = (e >> 31) & 1;
     // the block's tile: neighbours outside it are unavailable (AV1 intra edges
-    // and contexts stop at tile edges); the predictor works in tile coordinates
+    // and contexts stop at tile edges)
     const int tx0 = bx - bx % a.tile_w8, ty0 = by - by % a.tile_h8;
     const int tx1 = min(tx0 + a.tile_w8, nbx), ty1 = min(ty0 + a.tile_h8, a.h8 / 8);
     const bool has_l = bx > tx0, has_t = by > ty0;
     const bool have_tr = thr && has_t && bx + 1 < tx1;
     const bool have_bl = lhb && has_l && by + 1 < ty1;
-    const uint8_t flags = (have_tr ? 1 : 0) | (have_bl ? 2 : 0);
-    const int rx = px - tx0 * 8, ry = py - ty0 * 8;  // tile-relative position
     if (t < 5) {  // one thread per dependency
       int dep = -1;
       if (t == 0 && has_l) dep = b - 1;
@@ -297,124 +315,122 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThre
       if (t == 3 && have_tr) dep = b - nbx + 1;
       if (t == 4 && have_bl) dep = b + nbx - 1;
       if (dep >= 0) {
-        int it = 0;
-        while (ld_acquire(done + dep) < kDonePerBlock) {
-          if (*(volatile uint32_t*)err) break;
-          if (++it > kMaxPolls) {
+        for (int it = 1; ld_acquire(done + dep) < kDonePerBlock; ++it) {
+          if ((it & 15) == 0 && *(volatile uint32_t*)err) break;
+          if (it > kMaxPolls) {
             atomicExch(err, 1u);
             break;
           }
-          __nanosleep(64);
         }
       }
+    } else if (t >= 64 && t < 128) {  // the source block, which waits for nothing
+      const int i = t - 64, y = i >> 3, x = i & 7;
+      S.src[x * 8 + y] = (int16_t)a.src[0][(size_t)(py + y) * a.py.stride + px + x];
+    } else if (rank >= 2 && warp == kTypes) {
+      const int n = a.sub ? 4 : 8, sh = a.sub ? 2 : 3, cx = a.sub ? px / 2 : px, cy = a.sub ? py / 2 : py;
+      for (int i = lane; i < n * n; i += 32) {
+        const int y = i >> sh, x = i & (n - 1);
+        S.csrc[x * n + y] = (int16_t)a.src[rank - 1][(size_t)(cy + y) * a.pc.stride + cx + x];
+      }
     }
     __syncthreads();
-    // the block's neighbours and source samples
-    if (t < 33) {
-      stage_edges(a.rec[0], a.py.stride, a.w8, a.h8, px, py, has_t, has_l, S.above[0], S.left[0], t);
-    } else if (t >= 64 && t < 128) {
-      const int i = t - 64;
-      S.src[i] = a.src[0][(size_t)(py + (i >> 3)) * a.py.stride + px + (i & 7)];
-    } else if (rank >= 2 && c >= 0) {
-      const int cx = a.sub ? px / 2 : px, cy = a.sub ? py / 2 : py, n = a.sub ? 4 : 8;
-      stage_edges(a.rec[1 + pl], a.pc.stride, a.pc.frame_w, a.pc.frame_h, cx, cy, has_t, has_l, S.above[1],
-                  S.left[1], c);
-      if (c == 0)
-        stage_edges(a.rec[1 + pl], a.pc.stride, a.pc.frame_w, a.pc.frame_h, cx, cy, has_t, has_l, S.above[1],
-                    S.left[1], 32);
-      if (n == 8)
-        for (int i = c; i < 64; i += 32) S.csrc[i] = a.src[1 + pl][(size_t)(cy + i / 8) * a.pc.stride + cx + (i % 8)];
-    }
-    __syncthreads();
-    if (t < kLumaThreads) {
-      const mtd::Octet g;
-      const int o = t >> 3;
-      const bool ft = (has_t && is_smooth(__ldcg(a.mode + b - nbx))) || (has_l && is_smooth(__ldcg(a.mode + b - 1)));
-      mt_candidate cd = {};
-      cd.px = (uint16_t)rx;
-      cd.py = (uint16_t)ry;
-      cd.flags = flags | (ft ? 4 : 0);
-      const mtd::EdgeRead rd{S.above[0], S.left[0], rx, ry};
-      if (o < 4 && mlo + o < 13) {
-        cd.mode = (uint8_t)(mlo + o);
-        mtd::coop8_predict(rd, a.py, cd, S.pred[o], S.edge[o], g);
+    int32_t c[8], rv[8];  // an octet's levels (row j) and reconstruction (column j)
+    if (warp == kTypes) {
+      if (rank >= 2) code_chroma(S, bufs + kTypes * 4, a, rank - 2, b, px, py, has_t, has_l);
+      else if (rank == 0 && lane == 0) fetch(par ^ 1);
+    } else {
+      // the intra edges with their fills (predict_sq_at), read past L1 (other
+      // SMs wrote them); an available far side lies inside the frame
+      if (t < 35) {
+        const uint16_t* r = a.rec[0] + (size_t)py * a.py.stride + px;
+        const int stride = a.py.stride;
+        auto px_at = [&](int x, int y) { return (int16_t)__ldcg(r + (ptrdiff_t)y * stride + x); };
+        if (t < 16) {
+          S.edge.a[2 + t] = has_t ? px_at(have_tr ? t : min(t, 7), -1) : (has_l ? px_at(-1, 0) : (int16_t)127);
+        } else if (t < 32) {
+          const int k = t - 16;
+          S.edge.l[2 + k] = has_l ? px_at(-1, have_bl ? k : min(k, 7)) : (has_t ? px_at(0, -1) : (int16_t)129);
+        } else if (t == 32) {
+          const int16_t cn = has_l ? px_at(-1, has_t ? -1 : 0) : (has_t ? px_at(0, -1) : (int16_t)128);
+          S.edge.a[1] = S.edge.l[1] = cn;
+        } else {  // the neighbours' modes: the filter type
+          const bool have = t == 33 ? has_t : has_l;
+          S.nb_mode[t - 33] = have ? __ldcg(a.mode + (t == 33 ? b - nbx : b - 1)) : (uint8_t)MT_DC_PRED;
+        }
       }
       luma_bar();
-      const int ci = kOrder.t[rank][o];
-      if (ci >= 0) {
-        cd.mode = (uint8_t)(ci / 7);
-        cd.tx_type = kEncTypes[ci % 7];
-        mt_candidate_result r;
-        mtd::coop8_tx(S.src, 8, 0, 0, a.py, a.qy, a.tly, a.has_qm_y ? S.qmY : nullptr, S.qsY, S.lut, S.cy, cd,
-                      S.pred[cd.mode - mlo], r, S.oct[o], S.tabs, g);
-        if (g.j == 0) atomicMin(&S.best, ((unsigned long long)__float_as_uint(r.cost) << 32) | (unsigned)ci);
+      if (warp < nm)
+        mtd::coop8_predict(mlo + warp, S.edge, has_t, has_l, is_smooth(S.nb_mode[0]) || is_smooth(S.nb_mode[1]), S.src,
+                           S.pcol[warp], S.rcol[warp], S.rrow[warp], S.pb[warp]);
+      luma_bar();
+      const mtd::Coop<8> g;
+      const int oct = lane >> 3, ms = min(oct, nm - 1), mode = mlo + ms, TX = warp;
+      mtd::OctBuf& o = bufs[warp * 4 + oct];
+      int sc[8];
+      {
+        const uint2 w = *reinterpret_cast<const uint2*>(S.scan.row8[g.j]);
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+          sc[x] = (w.x >> (8 * x)) & 255;
+          sc[x + 4] = (w.y >> (8 * x)) & 255;
+        }
       }
-    } else if (rank >= 2) {  // chroma: UV_DC_PRED with DCT_DCT, U in CTA 2, V in CTA 3
-      int32_t* lvc = pl == 0 ? a.lv_u : a.lv_v;
-      if (a.sub == 0 && c < 8) {
-        const mtd::Octet g;
-        mt_candidate cc = {};
-        cc.px = (uint16_t)rx;
-        cc.py = (uint16_t)ry;
-        cc.flags = flags;
-        cc.mode = MT_DC_PRED;
-        cc.tx_type = MT_TX_DCT_DCT;
-        mtd::coop8_predict(mtd::EdgeRead{S.above[1], S.left[1], rx, ry}, a.pc, cc, S.cpred, S.edge[4], g);
-        g.sync();
-        mt_candidate_result r;
-        mtd::Oct8& oc = S.oct[kLumaThreads / 8];
-        mtd::coop8_tx(S.csrc, 8, 0, 0, a.pc, a.qc, a.tlc, a.has_qm_c ? S.qmC : nullptr, S.qsC, S.lut, S.cc, cc,
-                      S.cpred, r, oc, S.tabs, g);
-        put8(oc, S.cpred, lvc + (size_t)b * 64, a.rec[1 + pl], a.pc.stride, px, py, g.j);
-      } else if (a.sub != 0 && c == 0) {
-        mt_candidate cc = {};
-        cc.mode = MT_DC_PRED;
-        cc.tx_type = MT_TX_DCT_DCT;
-        cc.px = (uint16_t)(rx / 2);
-        cc.py = (uint16_t)(ry / 2);
-        mt_candidate_result r;
-        int32_t st4[mtd::kWork4Words];
-        mtd::Work4 w4{st4};
-        // the source plane from the tile's origin, so that tile coordinates address it
-        const uint16_t* tsrc = a.src[1 + pl] + (size_t)(ty0 * 4) * a.pc.stride + tx0 * 4;
-        mtd::chain4_one_rd<false>(tsrc, mtd::EdgeRead{S.above[1], S.left[1], cc.px, cc.py}, a.pc, a.qc, a.tlc,
-                                  a.has_qm_c ? S.qmC : nullptr, S.qsC, S.lut, S.cc, cc, r, w4);
-        const int16_t* cf = w4.cf();
-        const int16_t* pr = w4.pred();
-        const int16_t* rr = w4.rr();
-        int32_t* lv = lvc + (size_t)b * 16;
-        for (int i = 0; i < 16; ++i) lv[i] = cf[i];
-        for (int y = 0; y < 4; ++y)
-          for (int x = 0; x < 4; ++x)
-            a.rec[1 + pl][(size_t)(py / 2 + y) * a.pc.stride + px / 2 + x] =
-                (uint16_t)min(max((int)pr[y * 4 + x] + rr[y * 4 + x], 0), 255);
+      float at[8];
+      mtd::coop8_fwd(TX, S.rcol[ms], S.rrow[ms], S.py, c, at, o, g);
+      const int eob = mtd::coop_trellis<8>(c, at, sc, S.py, o, g);
+      mtd::coop8_inv(TX, c, S.py, rv, o, g);
+      int32_t d[8], pr[8], sr[8];
+      mtd::load8(S.pcol[ms] + g.j * 8, pr);
+      mtd::load8(S.src + g.j * 8, sr);
+#pragma unroll
+      for (int y = 0; y < 8; y++) {
+        rv[y] = min(max(pr[y] + rv[y], 0), 255);
+        d[y] = sr[y] - rv[y];
       }
+      const uint32_t satd = mtd::coop8_satd(d, g);
+      float price = __fmul_rn(__fmul_rn(__fmul_rn((float)satd, fmaxf((float)S.py.q.ac_q, 1.0f)), 0.25f), a.py.satd_scale);
+      if (a.py.satd_bridge != 0.0f) price = __fmul_rn(price, a.py.satd_bridge);
+      const float bits = mtd::coop8_rate(c, sc, eob, S.cy, mode, TX, o, g);
+      const float cost = __fadd_rn(price, __fmul_rn(a.py.mode_lambda, bits));
+      unsigned long long k = ~0ull;
+      if (g.j == 0 && oct < nm)
+        k = ((unsigned long long)__float_as_uint(cost) << 32) | (unsigned)(mode * kTypes + TX);
+#pragma unroll
+      for (int s = 8; s < 32; s <<= 1) {
+        const unsigned long long ok = __shfl_xor_sync(0xffffffffu, k, s);
+        k = ok < k ? ok : k;
+      }
+      if (lane == 0) S.key[warp] = k;
     }
-    cluster.sync();  // every CTA's key is final
-    unsigned long long w = ~0ull;
-    for (int q = 0; q < kClusterCtas; ++q) {
-      const unsigned long long k = *cluster.map_shared_rank(&S.best, q);
-      w = k < w ? k : w;
+    __syncthreads();
+    if (t < kClusterCtas) {  // this CTA's minimum to CTA t
+      unsigned long long k = S.key[0];
+#pragma unroll
+      for (int i = 1; i < kTypes; ++i) k = S.key[i] < k ? S.key[i] : k;
+      *cluster.map_shared_rank(&S.ckey[par][rank], t) = k;
     }
-    const int wi = (int)(w & 0xffffffffu);
-    if (t < kLumaThreads && rank == wi / kCandPerCta && kOrder.t[rank][t >> 3] == wi) {
-      const int j = t & 7;
-      put8(S.oct[t >> 3], S.pred[wi / 7 - mlo], a.lv_y + (size_t)b * 64, a.rec[0], a.py.stride, px, py, j);
+    cluster.sync();  // the keys and the next block are everywhere
+    unsigned long long w = S.ckey[par][0];
+#pragma unroll
+    for (int q = 1; q < kClusterCtas; ++q) w = S.ckey[par][q] < w ? S.ckey[par][q] : w;
+    const int wi = (int)(w & 0xffffffffu), wm = wi / kTypes;
+    if (rank == mode_rank(wm) && warp == wi % kTypes && lane >> 3 == wm - mlo) {
+      const int j = lane & 7;
+      int32_t* lv = a.lv_y + (size_t)b * 64 + j;
+      uint16_t* r = a.rec[0] + (size_t)py * a.py.stride + px + j;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) r[(size_t)k * a.py.stride] = (uint16_t)rv[k];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) lv[k * 8] = c[k];
       if (j == 0) {
-        a.mode[b] = (uint8_t)(wi / 7);
-        a.tx[b] = kEncTypes[wi % 7];
+        a.mode[b] = (uint8_t)wm;
+        a.tx[b] = (uint8_t)warp;
       }
     }
     __syncthreads();  // this CTA's writes of the block are issued
-    if (t == 0) {
-      __threadfence();
-      atomicAdd(done + b, 1u);
-    }
-    cluster.sync();  // every CTA has read the keys
-    if (t == 0) S.best = ~0ull;
+    if (t == 0) add_release(done + b);
   }
-  // The last ticket was read from CTA 0's shared memory by the other CTAs:
-  // none may leave while such a read can still be in flight.
+  // None may leave while another CTA can still write to its shared memory.
   cluster.sync();
 }
 
@@ -773,17 +789,15 @@ int job_setup(Job& j, Buffers& buf, int i) {
   j.tile_sb_w = (sb_cols + (1 << j.tcl) - 1) >> j.tcl;
   j.tile_sb_h = (sb_rows + (1 << j.trl) - 1) >> j.trl;
   const int cl = j.cl = sub ? 16 : 64;  // chroma levels per block
-  // quantisers, QM rows, default CDF slices and their bit costs, lambdas
+  // quantisers, QM rows, the default luma CDF slice and its bit costs, lambdas
   mt_quant qy, qc;
   if (mt_quant_init(j.plan.base_q_idx, 8, j.plan.qm_y, &qy) != MT_OK) return MT_ERR_INVALID_INPUT;
   if (mt_quant_init_chroma(j.plan.base_q_idx, 0, 0, 8, j.plan.qm_u, &qc) != MT_OK) return MT_ERR_INVALID_INPUT;
-  mt_coef_cdfs cdy, cdc;
-  mt_coef_costs cy, cc;
+  mt_coef_cdfs cdy;
+  mt_coef_costs cy;
   const int qctx = mt_qcat(j.plan.base_q_idx);
   mt_coef_cdfs_default(qctx, 8, 8, 0, &cdy);
-  mt_coef_cdfs_default(qctx, sub ? 4 : 8, sub ? 4 : 8, 1, &cdc);
   mt_coef_costs_build(&cdy, &cy);
-  mt_coef_costs_build(&cdc, &cc);
   mt_rd_lambdas lam;
   if (mt_rd_lambdas_init(j.plan.base_q_idx, qy.dc_q, sub, 8, &lam) != MT_OK) return MT_ERR_INVALID_INPUT;
   const uint8_t* qmy = mt_qm_row(j.plan.qm_y, 0, 8, 8);
@@ -794,7 +808,7 @@ int job_setup(Job& j, Buffers& buf, int i) {
                                 : (size_t)width * height + 2 * (size_t)((width + sx) >> sx) * ((height + sx) >> sx);
   uint8_t* d_rgbbuf = buf.get<uint8_t>(i, kRgb, j.rgb_on_device ? 1 : in_bytes);
   uint16_t* d_planes = buf.get<uint16_t>(i, kPlanes, (ny + 2 * nc) * 2 * 2);
-  uint8_t* d_tabs = buf.get<uint8_t>(i, kTables, 2 * sizeof(mt_coef_costs) + 128);
+  uint8_t* d_tabs = buf.get<uint8_t>(i, kTables, sizeof(mt_coef_costs) + 128);
   uint8_t* d_decs = buf.get<uint8_t>(i, kDecisions, (size_t)nb * 2);
   int32_t* d_levels = buf.get<int32_t>(i, kLevels, (size_t)nb * (64 + 2 * cl) * 4);
   j.d_res = buf.get<uint8_t>(i, kRes, (size_t)nb * 3);
@@ -807,8 +821,7 @@ int job_setup(Job& j, Buffers& buf, int i) {
     j.rec[p] = d_planes + ny + 2 * nc + (p == 0 ? 0 : ny + (size_t)(p - 1) * nc);
   }
   mt_coef_costs* d_cy = reinterpret_cast<mt_coef_costs*>(d_tabs);
-  mt_coef_costs* d_cc = d_cy + 1;
-  uint8_t* d_qmy = reinterpret_cast<uint8_t*>(d_cc + 1);
+  uint8_t* d_qmy = reinterpret_cast<uint8_t*>(d_cy + 1);
   uint8_t* d_qmc = d_qmy + 64;
   j.cs.reset(new CallStats(j.stats));
   CallStats& cs = *j.cs;
@@ -836,12 +849,11 @@ int job_setup(Job& j, Buffers& buf, int i) {
     cs.h2d(n0 + 2 * n1);
     cs.launches(3);
   }
-  cudaMemsetAsync(d_tabs, 32, 2 * sizeof(mt_coef_costs) + 128, st);  // flat QM weights past a 4x4 row
+  cudaMemsetAsync(d_tabs, 32, sizeof(mt_coef_costs) + 128, st);  // flat QM weights past a 4x4 row
   cudaMemcpyAsync(d_cy, &cy, sizeof(cy), cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(d_cc, &cc, sizeof(cc), cudaMemcpyHostToDevice, st);
   if (qmy) cudaMemcpyAsync(d_qmy, qmy, 64, cudaMemcpyHostToDevice, st);
   if (qmc) cudaMemcpyAsync(d_qmc, qmc, sub ? 16 : 64, cudaMemcpyHostToDevice, st);
-  cs.h2d(2 * sizeof(mt_coef_costs) + (qmy ? 64 : 0) + (qmc ? (sub ? 16 : 64) : 0));
+  cs.h2d(sizeof(mt_coef_costs) + (qmy ? 64 : 0) + (qmc ? (sub ? 16 : 64) : 0));
   EncArgs& a = j.a;
   a = EncArgs{};
   for (int p = 0; p < 3; ++p) {
@@ -882,7 +894,6 @@ int job_setup(Job& j, Buffers& buf, int i) {
   a.lv_v = a.lv_u + (size_t)nb * cl;
   j.desc.a = a;
   j.desc.cy = d_cy;
-  j.desc.cc = d_cc;
   j.desc.qmy = d_qmy;
   j.desc.qmc = d_qmc;
   j.desc.done = d_done;
@@ -1000,8 +1011,11 @@ int decide_all(std::vector<Job>& jobs, Buffers& buf) {
     jobs[(size_t)d].cs->h2d(jobs[(size_t)d].sched.size() * 8 + sizeof(JobDesc));
     jobs[(size_t)d].cs->mark(1, ks);
   }
-  encode_blocks_kernel<<<nclusters * kClusterCtas, kStepThreads, 0, ks>>>(d_jobs, d_list, (int)list.size(), d_ctl,
-                                                                          d_ctl + 1);
+  constexpr int dyn = kOctBufs * (int)sizeof(mtd::OctBuf);
+  if (cudaFuncSetAttribute(encode_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess)
+    return MT_ERR_DEVICE;
+  encode_blocks_kernel<<<nclusters * kClusterCtas, kStepThreads, dyn, ks>>>(d_jobs, d_list, (int)list.size(), d_ctl,
+                                                                            d_ctl + 1);
   for (int d : slot) {
     jobs[(size_t)d].cs->mark(2, ks);
     jobs[(size_t)d].cs->launches(1);

@@ -174,8 +174,8 @@ __device__ __forceinline__ void lane_predict(const R& rd, int fw, int fh, int ox
 #pragma unroll
     for (int i = 0; i < 2; i++) {
       const int o = j + i * N;
-      fa[i] = sa && o < na - 1 ? edge_tap(A - 1, o, na, sa) : 0;
-      fl[i] = sl && o < nl - 1 ? edge_tap(Lf - 1, o, nl, sl) : 0;
+      fa[i] = sa && o < na - 1 ? edge_tap(A, o, na, sa) : 0;
+      fl[i] = sl && o < nl - 1 ? edge_tap(Lf, o, nl, sl) : 0;
     }
     g.sync();
 #pragma unroll
@@ -950,27 +950,6 @@ __device__ __forceinline__ long long lane_sse(const W& w, int vw, int vh, float 
   const float s2 = __fadd_rn(sum, __shfl_xor_sync(kFull, sum, 2));
   const float d = __fadd_rn(s2, __shfl_xor_sync(kFull, s2, 1));
   return vw <= 0 || vh <= 0 ? 0 : __float2ll_rz(roundf(__fmul_rn(d, scale)));
-}
-
-// b + 1 + 1 + ... (n times, one rounding each): inside a binade of [1, 2^23)
-// the sums are exact, so each binade takes one addition and one for the step
-// across its end.
-__device__ __forceinline__ float add_ones(float b, int n) {
-  while (n > 0) {
-    int s = 0;
-    if (b >= 1.0f && b < 8388608.0f) {
-      const float top = __int_as_float((__float_as_int(b) & 0x7f800000) + 0x00800000);
-      s = ::min((int)ceilf(__fsub_rn(top, b)) - 1, n);
-    }
-    if (s > 0) {
-      b = __fadd_rn(b, (float)s);
-      n -= s;
-    } else {
-      b = __fadd_rn(b, 1.0f);
-      n--;
-    }
-  }
-  return b;
 }
 
 // rate_bounded<N> over the block's lanes: the terms of the reverse walk are
