@@ -1,13 +1,16 @@
-// The encoder's 8x8 candidate chain (chain8.cuh) with EIGHT lanes per candidate
-// (an octet), for a launch whose latency, not its throughput, bounds the run:
-// the wavefront of the encoder, where a few dozen blocks per dependency level
-// are all the work there is.
+// The encoder's 8x8 candidate chain (chain8.cuh) with EIGHT lanes per candidate,
+// for a launch whose latency, not its throughput, bounds the run: the wavefront
+// of the encoder, where a few dozen blocks per dependency level are all the work
+// there is.
 //
-// The four octets of a warp run one transform type, so the warp never splits:
-// every sync is the whole warp's and every loop has a warp-wide bound.  Lane j
-// of an octet holds a row or a column of the block in registers from the
-// residual to the cost; shared memory carries the two transposes, the terms of
-// the ordered float sums, and tables.
+// The four groups of a warp run one transform type, so the warp never splits:
+// every sync is the whole warp's.  Lane j of a group holds row j of the block in
+// registers from the quantisation to the cost (column j after the inverse).
+// Shared memory carries the two transposes, the terms of the ordered float sums,
+// and tables.  Sixteen lanes per candidate (half rows) were slower (512x512 4:4:4
+// 8.8 against 8.4 us a dependency level, 1080p 9.9 against 8.8): both halves
+// have to run the row and column passes, and a block's warps share the issue
+// slots of the SMs it runs on.
 //
 // Same arithmetic, same order, same results as the one-thread chain (bit for
 // bit):
@@ -18,7 +21,9 @@
 //     zeroing distortion, its running prefix cost, the rate walk's sum) keep
 //     it: their terms are computed by all lanes and added by one lane in the
 //     reference's order, positions outside a chain's range adding an exact +0;
-//     integer sums (SATD, counts) are reduced across lanes in any order.
+//     integer sums (SATD, counts) are reduced across lanes in any order;
+//   * levels become floats, and targets levels, by adding and subtracting 2^23
+//     (exact for them), which spares the conversion unit.
 #pragma once
 #include <stdint.h>
 
@@ -27,19 +32,20 @@
 
 namespace mtd {
 
-// Shared-memory working set of one octet.  t: transposes (stride 9, or 5 at
+// Shared-memory working set of one group.  t: transposes (stride 9, or 5 at
 // 4x4).  Trellis: sr[4 + k] = the suffix sum from scan index 63 - k (sr[3] = 0
-// is the empty sum), b / r the prefix terms.  Rate: b, r and t hold the walk's
-// three terms, at 63 - scan index.  296 words: the octets of a warp start 8
-// banks apart.
-struct OctBuf {
+// is the empty sum), b[e] and r[e] the prefix terms.  Rate: the walk's terms at
+// 63 - scan index, the first of each position in b, or where some level has two
+// the pairs over b and r; the third ones in t.  296 words: the groups of a warp
+// start 8 banks apart.
+struct GroupBuf {
   int32_t t[72];
   float sr[68];
   float b[64];
   float r[64];
   float pad[28];
 };
-static_assert(sizeof(OctBuf) / 4 % 32 == 8 && sizeof(OctBuf) % 16 == 0, "octet bank offset");
+static_assert(sizeof(GroupBuf) / 4 % 32 == 8 && sizeof(GroupBuf) % 16 == 0, "bank offset of a group");
 
 // What one plane of an image needs beside its quantiser: per coefficient the
 // forward QM scale and the dequantisation step (rc = 8 x + y, or 4 x + y), per
@@ -52,9 +58,11 @@ struct CoopPlane {
   float lsig[64];   // lambda * (0.9 bin + extra + 2) of an end of block at scan index e
   float lambda;     // 0: no trellis
   float dq2, aq2;
+  float mdc, mac;    // the multipliers / 65536 (exact, so scaling by them rounds once, as the reference's two steps do)
   uint32_t idiv[2];  // 2^32 / dc_q, 2^32 / ac_q, rounded up
   int has_qm;
   mt_quant q;
+  alignas(16) float zero[64];  // the suffix chain's empty second terms
 
   // Thread t of 64: qm the plane's inverse QM row (NULL: flat), n its samples.
   __device__ __forceinline__ void stage(int t, const mt_quant& quant, float lam, const uint8_t* qm, int n) {
@@ -62,6 +70,7 @@ struct CoopPlane {
     qs[t] = fwd_qm_scale(w);
     const int32_t base = t == 0 ? quant.dc_q : quant.ac_q;
     step[t] = qm ? (base * w + 16) >> 5 : base;
+    zero[t] = 0.0f;
     lrate[t] = __fmul_rn(lam, kCoefRateLut[t]);
     const int bin = t < 2 ? t : 32 - __clz(t), extra = bin > 1 ? bin - 2 : 0;
     lsig[t] = __fmul_rn(lam, __fadd_rn(__fmul_rn((float)bin, 0.9f), __fadd_rn((float)extra, 2.0f)));
@@ -69,6 +78,8 @@ struct CoopPlane {
       lambda = lam;
       dq2 = __fmul_rn((float)quant.dc_q, (float)quant.dc_q);
       aq2 = __fmul_rn((float)quant.ac_q, (float)quant.ac_q);
+      mdc = (float)quant.q_mult_dc / 65536.0f;
+      mac = (float)quant.q_mult_ac / 65536.0f;
       idiv[0] = 0xffffffffu / (uint32_t)quant.dc_q + 1u;
       idiv[1] = 0xffffffffu / (uint32_t)quant.ac_q + 1u;
       has_qm = qm != nullptr;
@@ -90,19 +101,29 @@ struct CoopScan {
   }
 };
 
-// A group of W lanes of a warp (W = 8 an octet; 4 for the 4x4 chroma block).
+// Lane j of a group of W lanes (8 for an 8x8 block, 4 for a 4x4 one).
 template <int W>
 struct Coop {
   int j;
   __device__ __forceinline__ Coop() : j(threadIdx.x & (W - 1)) {}
-  __device__ __forceinline__ int max(int v) const {
+  __device__ __forceinline__ uint32_t max(uint32_t v) const {
 #pragma unroll
     for (int s = W / 2; s; s >>= 1) v = ::max(v, __shfl_xor_sync(0xffffffffu, v, s));
+    return v;
+  }
+  __device__ __forceinline__ uint32_t min(uint32_t v) const {
+#pragma unroll
+    for (int s = W / 2; s; s >>= 1) v = ::min(v, __shfl_xor_sync(0xffffffffu, v, s));
     return v;
   }
   __device__ __forceinline__ uint32_t sum(uint32_t v) const {
 #pragma unroll
     for (int s = W / 2; s; s >>= 1) v += __shfl_xor_sync(0xffffffffu, v, s);
+    return v;
+  }
+  __device__ __forceinline__ uint32_t any_of(uint32_t v) const {
+#pragma unroll
+    for (int s = W / 2; s; s >>= 1) v |= __shfl_xor_sync(0xffffffffu, v, s);
     return v;
   }
 };
@@ -130,35 +151,62 @@ __device__ __forceinline__ void coop_transpose(int32_t* v, int32_t* t, int j) {
   __syncwarp();
 }
 
-// Quantisation of 8-bit residuals' coefficients: every |coefficient| is below
-// 2^15 and every multiplier at most 65536 / 4, so the products stay in 32 bits.
-__device__ __forceinline__ int32_t quant_half32(int32_t d, int32_t m) {
-  const int32_t p = d * m, l = (abs(p) + 32768) >> 16;
-  return p < 0 ? -l : l;
+// float(v) of |v| < 2^22, and floor(x) of 0 <= x < 2^22 as an integer and as a
+// float.
+__device__ __forceinline__ float small_float(int32_t v) {
+  return __fsub_rn(__int_as_float(0x4b400000 + v), 12582912.0f);
+}
+__device__ __forceinline__ int32_t small_floor(float x, float* f) {
+  const float y = __fadd_rz(x, 8388608.0f);
+  *f = __fsub_rn(y, 8388608.0f);
+  return __float_as_int(y) - 0x4b000000;
+}
+
+// Quantisation (+ QM) of row j of 2-D coefficients v, |v| < 2^16 (8-bit
+// residuals) and multipliers of at most 2^15, so that the products stay in 32
+// bits: levels c and target magnitudes at.  scale: 1, or 2 at 4x4
+// (src/dct.rs:3076-3100).
+template <int W>
+__device__ __forceinline__ void coop_quant(const int32_t* v, const CoopPlane& P, int scale, int32_t* c, float* at,
+                                           const Coop<W>& g) {
+#pragma unroll
+  for (int k = 0; k < W; k++) {
+    const bool dc = k == 0 && g.j == 0;
+    const float tf = __fmul_rn(small_float(v[k]), (dc ? P.mdc : P.mac) * (float)scale);
+    if (P.has_qm) {  // apply_qm: round half away from zero by the fraction
+      at[k] = fabsf(__fmul_rn(tf, P.qs[k * W + g.j]));
+      float tr;
+      int32_t l = small_floor(at[k], &tr);
+      l += __fsub_rn(at[k], tr) >= 0.5f;
+      c[k] = v[k] < 0 ? -l : l;
+    } else {
+      const int32_t p = v[k] * ((dc ? P.q.q_mult_dc : P.q.q_mult_ac) * scale), l = (abs(p) + 32768) >> 16;
+      at[k] = fabsf(tf);
+      c[k] = p < 0 ? -l : l;
+    }
+  }
 }
 
 // Forward transform and quantisation of type TX from the residual (col / row:
-// columns and rows of eight int16): lane j gets row j of the levels (c) and of
-// the targets' magnitudes (at).
+// columns and rows of eight int16).
 __device__ __forceinline__ void coop8_fwd(int TX, const int16_t* col, const int16_t* row, const CoopPlane& P, int32_t* c,
-                                          float* at, OctBuf& o, const Coop<8>& g) {
+                                          float* at, GroupBuf& o, const Coop<8>& g) {
   const int j = g.j;
   int32_t v[8];
   if (TX == MT_TX_IDTX) {
     load8(row + j * 8, v);
 #pragma unroll
-    for (int x = 0; x < 8; x++) {
-      const bool dc = x == 0 && j == 0;
-      const int32_t qd = dc ? P.q.dc_q : P.q.ac_q, num = v[x] * 8;
-      at[x] = fabsf(__fdiv_rn((float)num, (float)qd));
+    for (int k = 0; k < 8; k++) {
+      const bool dc = k == 0 && j == 0;
+      const int32_t qd = dc ? P.q.dc_q : P.q.ac_q, num = v[k] * 8;
+      at[k] = fabsf(__fdiv_rn((float)num, (float)qd));
       const uint32_t am = (uint32_t)abs(num);
       // (am + qd / 2) / qd: exact for am + qd / 2 < 2^16 and qd < 2^12
       const int32_t level = (int32_t)__umulhi(am + (uint32_t)(qd >> 1), dc ? P.idiv[0] : P.idiv[1]);
-      c[x] = (int32_t)am < qd ? 0 : (num < 0 ? -level : level);
+      c[k] = (int32_t)am < qd ? 0 : (num < 0 ? -level : level);
     }
     return;
   }
-  const bool one_d = TX == MT_TX_V_DCT || TX == MT_TX_H_DCT;
   if (TX == MT_TX_H_DCT) {
     load8(row + j * 8, v);
   } else {
@@ -168,118 +216,100 @@ __device__ __forceinline__ void coop8_fwd(int TX, const int16_t* col, const int1
   }
   if (TX == MT_TX_ADST_ADST || TX == MT_TX_DCT_ADST) fadst8(v);
   else if (TX != MT_TX_V_DCT) fdct8(v);
+  if (TX == MT_TX_V_DCT || TX == MT_TX_H_DCT) {  // quant_fullstep
 #pragma unroll
-  for (int x = 0; x < 8; x++) {
-    const int32_t m = x == 0 && j == 0 ? P.q.q_mult_dc : P.q.q_mult_ac;
-    if (one_d) {
-      const int32_t p = v[x] * 2 * m, l = (abs(p) + 32768) >> 16;
-      at[x] = fabsf(__fmul_rn((float)p, 1.0f / 65536.0f));
-      c[x] = abs(p) < 65536 ? 0 : (p < 0 ? -l : l);
-    } else {
-      float tf = __fmul_rn(__fmul_rn((float)v[x], (float)m), 1.0f / 65536.0f);
-      if (P.has_qm) {  // apply_qm
-        tf = __fmul_rn(tf, P.qs[x * 8 + j]);
-        const float tr = truncf(tf);
-        const float st = fabsf(__fsub_rn(tf, tr)) >= 0.5f ? copysignf(1.0f, tf) : 0.0f;
-        c[x] = (int32_t)__fadd_rn(tr, st);
-      } else {
-        c[x] = quant_half32(v[x], m);
-      }
-      at[x] = fabsf(tf);
+    for (int k = 0; k < 8; k++) {
+      const int32_t p = v[k] * 2 * (k == 0 && j == 0 ? P.q.q_mult_dc : P.q.q_mult_ac), l = (abs(p) + 32768) >> 16;
+      at[k] = fabsf(__fmul_rn((float)p, 1.0f / 65536.0f));
+      c[k] = abs(p) < 65536 ? 0 : (p < 0 ? -l : l);
     }
+  } else {
+    coop_quant<8>(v, P, 1, c, at, g);
   }
 }
 
-// The 4x4 DCT_DCT of the same form (multipliers doubled, src/dct.rs:3076-3100).
-__device__ __forceinline__ void coop4_fwd(int32_t* v, const CoopPlane& P, int32_t* c, float* at, OctBuf& o,
+// The 4x4 DCT_DCT of the same form from column j (v).
+__device__ __forceinline__ void coop4_fwd(int32_t* v, const CoopPlane& P, int32_t* c, float* at, GroupBuf& o,
                                           const Coop<4>& g) {
-  const int j = g.j;
   fdct4v(v);
-  coop_transpose<4>(v, o.t, j);
+  coop_transpose<4>(v, o.t, g.j);
   fdct4v(v);
-#pragma unroll
-  for (int x = 0; x < 4; x++) {
-    const int32_t m = 2 * (x == 0 && j == 0 ? P.q.q_mult_dc : P.q.q_mult_ac);
-    float tf = __fmul_rn(__fmul_rn((float)v[x], (float)m), 1.0f / 65536.0f);
-    if (P.has_qm) {
-      tf = __fmul_rn(tf, P.qs[x * 4 + j]);
-      const float tr = truncf(tf);
-      const float st = fabsf(__fsub_rn(tf, tr)) >= 0.5f ? copysignf(1.0f, tf) : 0.0f;
-      c[x] = (int32_t)__fadd_rn(tr, st);
-    } else {
-      c[x] = quant_half32(v[x], m);
-    }
-    at[x] = fabsf(tf);
-  }
+  coop_quant<4>(v, P, 2, c, at, g);
 }
 
-// trellis_optimize (trellis8 / trellis4) over row-wise levels c and target
-// magnitudes at, e the scan indexes.  Returns the final end of block (-1: all
+// trellis_optimize (trellis8 / trellis4) over row j's levels c and target
+// magnitudes at, e their scan indexes.  Returns the final end of block (-1: all
 // zero).
 template <int W>
-__device__ __forceinline__ int coop_trellis(int32_t* c, const float* at, const int* e, const CoopPlane& P, OctBuf& o,
+__device__ __forceinline__ int coop_trellis(int32_t* c, const float* at, const int* e, const CoopPlane& P, GroupBuf& o,
                                             const Coop<W>& g) {
   constexpr unsigned kAll = 0xffffffffu;
-  const int j = g.j;
   int e1 = 0;
+  bool big = false;
 #pragma unroll
-  for (int x = 0; x < W; x++)
-    if (c[x] != 0) e1 = ::max(e1, e[x] + 1);
-  const int m = g.max(e1);
-  if (!(P.lambda > 0.0f)) return m - 1;
-  const int M8 = ((int)__reduce_max_sync(kAll, (unsigned)m) + 7) & ~7;
-  if (M8 == 0) return -1;
+  for (int k = 0; k < W; k++) {
+    if (c[k] != 0) e1 = ::max(e1, e[k] + 1);
+    big |= abs(c[k]) > 63;
+  }
+  const int m = (int)g.max((unsigned)e1);
+  if (!(P.lambda > 0.0f) || !__any_sync(kAll, m != 0)) return m - 1;
   const int full8 = m & ~7, chunked = full8 + ((m - full8) >= 4 ? 4 : 0);
   // step A.  The reference decides each position of a chunk (of eight, then one
   // of four) from the chunk's starting values, in the AVX2 FMA form unless the
   // chunk holds a level above 63; then, and in the scalar tail, the plain form.
+  const bool any_big = __any_sync(kAll, big);
   unsigned bigb = 0;  // bit k: chunk k holds one
+  if (any_big) {
 #pragma unroll
-  for (int x = 0; x < W; x++)
-    if (abs(c[x]) > 63 && e[x] < chunked) bigb |= 1u << (e[x] >> 3);
-  if (__any_sync(kAll, bigb != 0)) {
-#pragma unroll
-    for (int s = W / 2; s; s >>= 1) bigb |= __shfl_xor_sync(kAll, bigb, s);
+    for (int k = 0; k < W; k++)
+      if (abs(c[k]) > 63 && e[k] < chunked) bigb |= 1u << (e[k] >> 3);
+    bigb = g.any_of(bigb);
   }
 #pragma unroll
-  for (int x = 0; x < W; x++) {
-    const float q2 = x == 0 && j == 0 ? P.dq2 : P.aq2;
-    const int32_t l = abs(c[x]), ld = ::max(l - 1, 0);
-    const float el = __fsub_rn(at[x], (float)l), ed = __fsub_rn(at[x], (float)ld);
-    const float rl = l < 64 ? P.lrate[l] : __fmul_rn(P.lambda, coef_rate_bits((uint32_t)l));
-    const float rd = ld < 64 ? P.lrate[ld] : __fmul_rn(P.lambda, coef_rate_bits((uint32_t)ld));
-    const bool fma_form = e[x] < chunked && !((bigb >> (e[x] >> 3)) & 1u);
+  for (int k = 0; k < W; k++) {
+    const float q2 = k == 0 && g.j == 0 ? P.dq2 : P.aq2;
+    const int32_t l = abs(c[k]), ld = ::max(l - 1, 0);
+    const float fl = small_float(l), fd = fmaxf(__fsub_rn(fl, 1.0f), 0.0f);
+    const float el = __fsub_rn(at[k], fl), ed = __fsub_rn(at[k], fd);
+    float rl, rd;
+    bool fma_form = e[k] < chunked;
+    if (!any_big) {
+      rl = P.lrate[l];
+      rd = P.lrate[ld];
+    } else {
+      rl = l < 64 ? P.lrate[l] : __fmul_rn(P.lambda, coef_rate_bits((uint32_t)l));
+      rd = ld < 64 ? P.lrate[ld] : __fmul_rn(P.lambda, coef_rate_bits((uint32_t)ld));
+      fma_form = fma_form && !((bigb >> (e[k] >> 3)) & 1u);
+    }
     const float l2 = __fmul_rn(el, el), d2 = __fmul_rn(ed, ed);
-    const float cl = fma_form ? __fmaf_rn(q2, l2, rl) : __fadd_rn(__fmul_rn(q2, l2), rl);
-    const float cd = fma_form ? __fmaf_rn(q2, d2, rd) : __fadd_rn(__fmul_rn(q2, d2), rd);
-    if (l != 0 && cd < cl) c[x] = c[x] < 0 ? c[x] + 1 : c[x] - 1;
-    // the terms of the ordered sums, +0 past the end of block: S = q2 at^2 (the
-    // zeroing distortion), B = q2 (at - l)^2, R = lambda rate(l)
-    const int32_t l1 = abs(c[x]);
-    const float ec = __fsub_rn(at[x], (float)l1);
-    const bool in = e[x] < m;
-    o.sr[67 - e[x]] = in ? __fmul_rn(q2, __fmul_rn(at[x], at[x])) : 0.0f;
-    o.b[e[x]] = in ? __fmul_rn(q2, __fmul_rn(ec, ec)) : 0.0f;
-    o.r[e[x]] = in ? (l1 < 64 ? P.lrate[l1] : __fmul_rn(P.lambda, coef_rate_bits((uint32_t)l1))) : 0.0f;
+    const float ql = __fmul_rn(q2, l2), qd = __fmul_rn(q2, d2);
+    const float cl = fma_form ? __fmaf_rn(q2, l2, rl) : __fadd_rn(ql, rl);
+    const float cd = fma_form ? __fmaf_rn(q2, d2, rd) : __fadd_rn(qd, rd);
+    const bool dn = l != 0 && cd < cl;
+    if (dn) c[k] = c[k] < 0 ? c[k] + 1 : c[k] - 1;
+    // the terms of the ordered sums: S = q2 at^2 (the zeroing distortion, +0
+    // past the end of block), B = q2 (at - l)^2, R = lambda rate(l)
+    o.sr[67 - e[k]] = e[k] < m ? __fmul_rn(q2, __fmul_rn(at[k], at[k])) : 0.0f;
+    o.b[e[k]] = dn ? qd : ql;
+    o.r[e[k]] = dn ? rd : rl;
   }
-  if (j == 0) o.sr[3] = 0.0f;
-  if (W == 4 && j == 0) o.sr[67 - 16] = 0.0f;  // S(16): the scan ends there
+  if (g.j == 0) o.sr[W == 4 ? 67 - 16 : 3] = 0.0f;  // the empty sum past the whole scan
   __syncwarp();
   // Lane 0: the suffix sums right to left (acc += S; S = acc).  Lane 1: the
   // prefix cost left to right (b = pre + B; B = b; pre = b + R).
-  if (j < 2) {
-    float* arr = j == 0 ? o.sr + 4 + (64 - M8) : o.b;
+  if (g.j < 2) {
+    const int m8 = (m + 7) & ~7;
+    float* arr = g.j == 0 ? o.sr + 4 + (64 - m8) : o.b;
+    const float* add = g.j == 0 ? P.zero : o.r;
     float acc = 0.0f;
 #pragma unroll 1
-    for (int s = 0; s < M8; s += 8) {
+    for (int s = 0; s < m8; s += 8) {
       float v[8], r[8];
 #pragma unroll
       for (int u = 0; u < 8; u += 4) {
-        const float4 a = *reinterpret_cast<const float4*>(arr + s + u);
-        float4 q = *reinterpret_cast<const float4*>(o.r + s + u);
-        if (j == 0) q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        v[u] = a.x, v[u + 1] = a.y, v[u + 2] = a.z, v[u + 3] = a.w;
-        r[u] = q.x, r[u + 1] = q.y, r[u + 2] = q.z, r[u + 3] = q.w;
+        const float4 x = *reinterpret_cast<const float4*>(arr + s + u), y = *reinterpret_cast<const float4*>(add + s + u);
+        v[u] = x.x, v[u + 1] = x.y, v[u + 2] = x.z, v[u + 3] = x.w;
+        r[u] = y.x, r[u + 1] = y.y, r[u + 2] = y.z, r[u + 3] = y.w;
       }
 #pragma unroll
       for (int u = 0; u < 8; u++) {
@@ -292,53 +322,47 @@ __device__ __forceinline__ int coop_trellis(int32_t* c, const float* at, const i
     }
   }
   __syncwarp();
-  // candidate ends: the lowest cost, the first position on ties
-  float best = __int_as_float(0x7f800000);
-  int best_e = 64;
+  // candidate ends: the lowest cost (costs are not negative, so their bits order
+  // like their values), the first position on ties
+  uint32_t cost[W], low = 0x7f800000u;
 #pragma unroll
-  for (int x = 0; x < W; x++) {
-    if (c[x] != 0) {
-      const float cst = __fadd_rn(__fadd_rn(o.b[e[x]], P.lsig[e[x]]), o.sr[66 - e[x]]);
-      if (cst < best || (cst == best && e[x] < best_e)) {
-        best = cst;
-        best_e = e[x];
-      }
-    }
+  for (int k = 0; k < W; k++) {
+    cost[k] = 0x7f800000u;
+    if (c[k] != 0) cost[k] = __float_as_uint(__fadd_rn(__fadd_rn(o.b[e[k]], P.lsig[e[k]]), o.sr[66 - e[k]]));
+    low = ::min(low, cost[k]);
   }
+  low = g.min(low);
+  uint32_t first = 64;
 #pragma unroll
-  for (int s = W / 2; s; s >>= 1) {
-    const float ob = __shfl_xor_sync(kAll, best, s);
-    const int oe = __shfl_xor_sync(kAll, best_e, s);
-    if (ob < best || (ob == best && oe < best_e)) {
-      best = ob;
-      best_e = oe;
-    }
-  }
+  for (int k = 0; k < W; k++)
+    if (cost[k] == low && c[k] != 0) first = ::min(first, (uint32_t)e[k]);
+  const int best_e = (int)g.min(first);
+  const float best = __uint_as_float(low);
   const float skip = __fadd_rn(o.sr[67], P.lambda);
   const int keep = (best_e == 64 || skip < best) ? 0 : best_e + 1;
 #pragma unroll
-  for (int x = 0; x < W; x++)
-    if (e[x] >= keep) c[x] = 0;
+  for (int k = 0; k < W; k++)
+    if (e[k] >= keep) c[k] = 0;
   __syncwarp();
   return keep - 1;
 }
 
-// Dequantised row j of c (step: per coefficient, or the flat step).
+// Dequantised row j of c (flat: without the QM).
 template <int W>
 __device__ __forceinline__ void coop_dequant(const int32_t* c, bool flat, const CoopPlane& P, int32_t* v, int j) {
 #pragma unroll
-  for (int x = 0; x < W; x++) {
-    const int32_t l = c[x];
-    const int32_t step = flat ? (x == 0 && j == 0 ? P.q.dc_q : P.q.ac_q) : P.step[x * W + j];
+  for (int k = 0; k < W; k++) {
+    const int32_t l = c[k];
+    const int32_t step = flat ? (k == 0 && j == 0 ? P.q.dc_q : P.q.ac_q) : P.step[k * W + j];
     int32_t mag = (int32_t)(((uint32_t)abs(l) * (uint32_t)step) & 0xffffffu);
     mag = ::min(mag, P.q.cf_max + (l < 0 ? 1 : 0));
-    v[x] = l < 0 ? -mag : mag;
+    v[k] = l < 0 ? -mag : mag;
   }
 }
 
 // Dequantisation + inverse transform of type TX: lane j gets column j of the
 // inverse residual.
-__device__ __forceinline__ void coop8_inv(int TX, const int32_t* c, const CoopPlane& P, int32_t* v, OctBuf& o,
+__device__ __forceinline__ void coop8_inv(int TX, const int32_t* c, const CoopPlane& P, int32_t* v, GroupBuf& o,
                                           const Coop<8>& g) {
   const mt_quant& q = P.q;
   coop_dequant<8>(c, TX == MT_TX_IDTX || TX == MT_TX_V_DCT || TX == MT_TX_H_DCT, P, v, g.j);
@@ -364,7 +388,7 @@ __device__ __forceinline__ void coop8_inv(int TX, const int32_t* c, const CoopPl
 #pragma unroll
   for (int y = 0; y < 8; y++) v[y] = (v[y] + 8) >> 4;
 }
-__device__ __forceinline__ void coop4_inv(const int32_t* c, const CoopPlane& P, int32_t* v, OctBuf& o,
+__device__ __forceinline__ void coop4_inv(const int32_t* c, const CoopPlane& P, int32_t* v, GroupBuf& o,
                                           const Coop<4>& g) {
   const mt_quant& q = P.q;
   coop_dequant<4>(c, false, P, v, g.j);
@@ -421,125 +445,128 @@ __device__ __forceinline__ float add_ones(float b, int n) {
   return b;
 }
 
-// rate8 (txb_skip and dc_sign context 0, no skip price) over the octet, lane j
-// holding row j of the levels.  The reference's reverse walk has entered
-// exactly the later scan positions when it reads a context, and the five
-// neighbours of a position inside the block are later ones (past a column's
-// end its map holds nothing yet), so contexts come from the final levels: own
-// columns from registers, rows j + 1 and j + 2 by shuffles of packed level
-// bytes.  Lane 0 returns the bits.
-__device__ __forceinline__ float coop8_rate(const int32_t* c, const int* e, int eob, const mt_coef_costs& T, int mode,
-                                            int tx, OctBuf& o, const Coop<8>& g) {
+// The first terms of a coded block's rate, in the walk's order: txb_skip, the
+// tx-type symbol, the end-of-block position (rate8, contexts 0, no skip price).
+__device__ __forceinline__ float coop8_rate_head(const mt_coef_costs& T, int mode, int tx, int eob) {
+  float bits = __fadd_rn(T.txb_skip[0][0], T.txtp[mode][tx]);
+  const int bin = eob < 2 ? eob : 32 - __clz(eob);
+  bits = __fadd_rn(bits, T.eob_bin[bin]);
+  if (bin > 1) {
+    const int nb = bin - 2;
+    bits = __fadd_rn(bits, T.eob_hi[bin][(eob >> nb) & 1]);
+    bits = __fadd_rn(bits, (float)nb);
+  }
+  return bits;
+}
+
+// rate8 (txb_skip and dc_sign context 0, no skip price) over the group; head:
+// coop8_rate_head of the candidate's (mode, type) by end of block.  The
+// reference's reverse walk has entered exactly the later scan positions when it
+// reads a context, and the five neighbours of a position inside the block are
+// later ones (past a column's end its map holds nothing yet), so contexts come
+// from the final levels: the row's from registers, rows j + 1 and j + 2 by
+// shuffles of packed level bytes, summed two to a register.  Every position up
+// to the end of block puts its terms (the base token; of a level of 3 or more
+// the br cost; of one of 15 or more the golomb cost, which the end of block and
+// DC add to the br cost first) in shared memory in the walk's order, an absent
+// one as +0, and lane 0 adds them, DC's sign and the sign bits behind them, and
+// returns the bits.
+__device__ __forceinline__ float coop8_rate(const int32_t* c, const int* e, int eob, const mt_coef_costs& T,
+                                            const float* head, GroupBuf& o, const Coop<8>& g) {
   constexpr unsigned kAll = 0xffffffffu;
   const int j = g.j;
-  const int E = (int)__reduce_max_sync(kAll, (unsigned)(eob + 1));  // the longest walk of the warp, + 1
-  uint32_t lo = 0, hi = 0;  // level bytes of columns 0..3 and 4..7
+  uint32_t m[8], w[2] = {0, 0}, nz = 0, top = 0;
 #pragma unroll
-  for (int x = 0; x < 4; x++) {
-    lo |= level_byte((uint32_t)abs(c[x])) << (8 * x);
-    hi |= level_byte((uint32_t)abs(c[x + 4])) << (8 * x);
+  for (int k = 0; k < 8; k++) {
+    m[k] = (uint32_t)abs(c[k]);
+    const uint32_t t = ::min(m[k], 15u);
+    w[k >> 2] |= (t >= 3 ? t + 0xc0u : t * 0x41u) << (8 * (k & 3));  // level_byte
+    nz += m[k] != 0;
+    top = ::max(top, m[k]);
   }
-  uint32_t lo1 = __shfl_down_sync(kAll, lo, 1, 8), hi1 = __shfl_down_sync(kAll, hi, 1, 8);
-  uint32_t lo2 = __shfl_down_sync(kAll, lo, 2, 8), hi2 = __shfl_down_sync(kAll, hi, 2, 8);
-  if (j == 7) lo1 = hi1 = 0;
-  if (j >= 6) lo2 = hi2 = 0;
-  auto at = [](uint32_t l, uint32_t h, int x) -> uint32_t {
-    return x > 7 ? 0u : (x < 4 ? (l >> (8 * (x & 3))) & 255u : (h >> (8 * (x & 3))) & 255u);
-  };
-  const uint32_t dcmag = (at(lo1, hi1, 0) + at(lo, hi, 1) + at(lo1, hi1, 1)) & 63;  // lane 0's: (0,1), (1,0), (1,1)
-  float* T1 = o.b;
-  float* T2 = o.r;
+  uint32_t a[2], b[2];  // rows j + 1 and j + 2
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    a[i] = __shfl_down_sync(kAll, w[i], 1, 8);
+    b[i] = __shfl_down_sync(kAll, w[i], 2, 8);
+    if (j == 7) a[i] = 0;
+    if (j >= 6) b[i] = 0;
+  }
+  nz = g.sum(nz);  // DC, the end of block and the interior
+  const bool any3 = __any_sync(kAll, top >= 3), any15 = __any_sync(kAll, top >= 15);
+  auto even = [](uint32_t v) { return __byte_perm(v, 0, 0x4140); };  // bytes 0, 1 as halves
+  auto odd = [](uint32_t v) { return __byte_perm(v, 0, 0x4342); };   // bytes 2, 3
+  const uint32_t w1[2] = {__funnelshift_r(w[0], w[1], 8), w[1] >> 8}, w2[2] = {__funnelshift_r(w[0], w[1], 16), w[1] >> 16};
+  const uint32_t a1[2] = {__funnelshift_r(a[0], a[1], 8), a[1] >> 8};
+  uint32_t hm2[4], mg2[4];
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    hm2[2 * i] = even(a[i]) + even(w1[i]) + even(a1[i]);
+    hm2[2 * i + 1] = odd(a[i]) + odd(w1[i]) + odd(a1[i]);
+    mg2[2 * i] = hm2[2 * i] + even(b[i]) + even(w2[i]);
+    mg2[2 * i + 1] = hm2[2 * i + 1] + odd(b[i]) + odd(w2[i]);
+  }
+  // the end of block's base row (one column on), and its br context: 0 at DC, 7
+  // inside the first 2 x 2, else 14
+  const int eob_row = eob <= 0 ? 0 : 1 + (eob > 8) + (eob > 16);
+  const int eob_bc = eob <= 0 ? 0 : (eob == 1 || eob == 2 || eob == 4 ? 7 : 14);
   float* T3 = reinterpret_cast<float*>(o.t);
-  bool any3 = false;
-  uint32_t nz = 0, me = 0;
-  if (E > 1) {
 #pragma unroll
-    for (int x = 0; x < 8; x++) {
-      const uint32_t m = (uint32_t)abs(c[x]);
-      const bool in = e[x] >= 1 && e[x] < eob;
-      any3 |= in && m >= 3;
-      nz += in && m != 0;
-      me |= e[x] == eob ? m : 0u;
-    }
-    any3 = __any_sync(kAll, any3);
-    nz = g.sum(nz);
-    me = g.sum(me);
-#pragma unroll
-    for (int x = 0; x < 8; x++) {
-      const uint32_t m = (uint32_t)abs(c[x]);
-      const bool in = e[x] >= 1 && e[x] < eob;
-      const uint32_t hm = at(lo1, hi1, x) + at(lo, hi, x + 1) + at(lo1, hi1, x + 1);
-      const uint32_t mag = hm + at(lo2, hi2, x) + at(lo, hi, x + 2);
-      const int d = x + j;
-      const int ctx = (d < 2 ? d : (d < 4 ? 6 : 21)) + ::min((int)((mag + 64) >> 7), 4);
-      const float t1 = T.base_tok[ctx][::min(m, 3u)];
-      T1[63 - e[x]] = in ? t1 : 0.0f;
-      if (any3) {
-        float t2 = 0.0f, t3 = 0.0f;
-        if (in && m >= 3) {
-          const uint32_t hmag = hm & 63;
-          t2 = T.br_cum[((j | x) > 1 ? 14 : 7) + (hmag > 12 ? 6 : (int)((hmag + 1) >> 1))][::min((int32_t)m - 3, 12)];
-          if (m >= 15) t3 = golomb_cost(m - 15);
+  for (int k = 0; k < 8; k++) {
+    const bool in = e[k] <= eob, end = e[k] == eob, dc = k == 0 && j == 0;
+    const uint32_t hm = (hm2[k >> 1] >> (16 * (k & 1))) & 0xffffu, mag = (mg2[k >> 1] >> (16 * (k & 1))) & 0xffffu;
+    const int d = k + j;
+    const int ctx = dc ? 0 : (d < 2 ? d : (d < 4 ? 6 : 21)) + ::min((int)((mag + 64) >> 7), 4);
+    const int tok = (int)::min(m[k], 3u);
+    const float* t1p = end ? &T.eob_base[eob_row][::max(tok - 1, 0)] : &T.base_tok[ctx][tok];
+    const float t1 = in ? *t1p : 0.0f;
+    if (!any3) {
+      o.b[63 - e[k]] = t1;
+    } else {
+      float t2 = 0.0f, t3 = 0.0f;
+      if (m[k] >= 3) {
+        const int mg = (int)(hm & 63);
+        const int bc = end ? eob_bc : (dc ? 0 : (d > 1 && !(d == 2 && j == 1) ? 14 : 7)) + ::min((mg + 1) >> 1, 6);
+        t2 = T.br_cum[bc][::min((int32_t)m[k] - 3, 12)];
+        if (m[k] >= 15) {
+          t3 = golomb_cost(m[k] - 15);
+          if (end || dc) {
+            t2 = __fadd_rn(t2, t3);
+            t3 = 0.0f;
+          }
         }
-        T2[63 - e[x]] = t2;
-        T3[63 - e[x]] = t3;
       }
+      *reinterpret_cast<float2*>(o.b + 2 * (63 - e[k])) = make_float2(t1, t2);
+      if (any15) T3[63 - e[k]] = t3;
     }
   }
   __syncwarp();
   float bits = 0.0f;
   if (j == 0) {
-    if (eob < 0) {
-      bits = T.txb_skip[0][1];
-    } else {
-      bits = __fadd_rn(T.txb_skip[0][0], T.txtp[mode][tx]);
-      const uint32_t dm = (uint32_t)abs(c[0]);
-      const float sign = T.dc_sign[0][c[0] < 0];
-      auto hi_tok = [&](uint32_t m, int bc) -> float {
-        float h = T.br_cum[bc][::min((int32_t)m - 3, 12)];
-        if (m >= 15) h = __fadd_rn(h, golomb_cost(m - 15));
-        return h;
-      };
-      if (eob == 0) {
-        bits = __fadd_rn(bits, T.eob_bin[0]);
-        bits = __fadd_rn(bits, T.eob_base[0][::min(dm, 3u) - 1]);
-        if (dm >= 3) bits = __fadd_rn(bits, hi_tok(dm, 0));
-        bits = __fadd_rn(bits, sign);
+    bits = eob < 0 ? T.txb_skip[0][1] : head[eob];
+    if (eob >= 0) {
+      const int first = (63 - eob) & ~3;
+      if (!any3) {
+#pragma unroll 2
+        for (int k = first; k < 64; k += 4) {
+          const float4 x = *reinterpret_cast<const float4*>(o.b + k);
+          bits = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(bits, x.x), x.y), x.z), x.w);
+        }
+      } else if (!any15) {
+#pragma unroll 2
+        for (int k = first; k < 64; k += 4) {
+          const float4 x = *reinterpret_cast<const float4*>(o.b + 2 * k);
+          const float4 y = *reinterpret_cast<const float4*>(o.b + 2 * k + 4);
+          bits = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(bits, x.x), x.y), x.z), x.w);
+          bits = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(bits, y.x), y.y), y.z), y.w);
+        }
       } else {
-        const int eob_bin = eob < 2 ? eob : 32 - __clz(eob);
-        bits = __fadd_rn(bits, T.eob_bin[eob_bin]);
-        if (eob_bin > 1) {
-          const int nb = eob_bin - 2;
-          bits = __fadd_rn(bits, T.eob_hi[eob_bin][(eob >> nb) & 1]);
-          bits = __fadd_rn(bits, (float)nb);
-        }
-        bits = __fadd_rn(bits, T.eob_base[1 + (eob > 8) + (eob > 16)][::min(me, 3u) - 1]);
-        // the end of block's br context: 7 inside the first 2 x 2, else 14
-        if (me >= 3) bits = __fadd_rn(bits, hi_tok(me, eob == 1 || eob == 2 || eob == 4 ? 7 : 14));
-        const int first = 64 - ((E + 7) & ~7);
-        if (!any3) {
-#pragma unroll 2
-          for (int k = first; k < 64; k += 4) {
-            const float4 a = *reinterpret_cast<const float4*>(T1 + k);
-            bits = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(bits, a.x), a.y), a.z), a.w);
-          }
-        } else {
-#pragma unroll 2
-          for (int k = first; k < 64; k += 4) {
-            const float4 a = *reinterpret_cast<const float4*>(T1 + k);
-            const float4 b = *reinterpret_cast<const float4*>(T2 + k);
-            const float4 d = *reinterpret_cast<const float4*>(T3 + k);
-            bits = __fadd_rn(__fadd_rn(__fadd_rn(bits, a.x), b.x), d.x);
-            bits = __fadd_rn(__fadd_rn(__fadd_rn(bits, a.y), b.y), d.y);
-            bits = __fadd_rn(__fadd_rn(__fadd_rn(bits, a.z), b.z), d.z);
-            bits = __fadd_rn(__fadd_rn(__fadd_rn(bits, a.w), b.w), d.w);
-          }
-        }
-        bits = __fadd_rn(bits, T.base_tok[0][::min(dm, 3u)]);
-        if (dm >= 3) bits = __fadd_rn(bits, hi_tok(dm, dcmag > 12 ? 6 : (int)((dcmag + 1) >> 1)));
-        if (dm != 0) bits = __fadd_rn(bits, sign);
-        bits = add_ones(bits, 1 + (int)nz);
+#pragma unroll 1
+        for (int k = first; k < 64; k++)
+          bits = __fadd_rn(__fadd_rn(__fadd_rn(bits, o.b[2 * k]), o.b[2 * k + 1]), T3[k]);
       }
+      if (c[0] != 0) bits = __fadd_rn(bits, T.dc_sign[0][c[0] < 0]);
+      if (eob > 0) bits = add_ones(bits, (int)nz - (c[0] != 0));
     }
   }
   __syncwarp();

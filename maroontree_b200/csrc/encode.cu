@@ -112,10 +112,10 @@ __host__ __device__ inline void zorder(int k, int* bx, int* by, bool* thr, bool*
 __device__ __forceinline__ bool is_smooth(int m) { return m == MT_SMOOTH_PRED || m == MT_SMOOTH_V_PRED || m == MT_SMOOTH_H_PRED; }
 
 // A block is a cluster of kClusterCtas CTAs (on as many SMs).  CTA r takes the
-// modes [kModeLo[r], kModeLo[r + 1]), and its warp t the transform type t of
-// them, an octet of lanes per mode: a warp runs one transform path, a CTA
-// predicts each mode once for the seven types.  The last warp codes a chroma
-// plane in CTAs 2 and 3 and fetches the cluster's next block in CTA 0.
+// modes [mode_lo(r), mode_lo(r + 1)), a warp each transform type of them, eight
+// lanes per mode: a warp runs one transform path, a CTA predicts each mode once
+// for the seven types.  One more warp codes a chroma plane in CTAs 2 and 3 and
+// fetches the cluster's next block in CTA 0.
 // Candidate index = mode * 7 + type, the order ties are broken in.
 constexpr int kClusterCtas = 4;
 // CTAs of the decision kernel resident per SM (its register budget follows).
@@ -123,9 +123,10 @@ constexpr int kClusterCtas = 4;
 #define MT_ENC_CTAS_PER_SM 2
 #endif
 constexpr int kTypes = 7;  // MT_TX_IDTX .. MT_TX_DCT_ADST
+constexpr int kSideWarp = kTypes;  // the chroma / next-block warp, behind one per type
 constexpr int kLumaThreads = kTypes * 32;
 constexpr int kStepThreads = kLumaThreads + 32;
-constexpr int kOctBufs = kTypes * 4 + 8;  // an octet each, and eight groups of four lanes for chroma
+constexpr int kGroupBufs = 4 * kTypes + 8;  // one per candidate, and eight groups of four lanes for chroma
 __device__ __forceinline__ int mode_lo(int rank) { return rank ? 3 * rank + 1 : 0; }  // 0, 4, 7, 10
 __device__ __forceinline__ int mode_rank(int m) { return m < 4 ? 0 : (m - 1) / 3; }
 
@@ -136,7 +137,7 @@ struct NextBlock {
   uint32_t ticket, entry, image, pad;
 };
 
-// Everything one CTA keeps in shared memory beside the octets' buffers.
+// Everything one CTA keeps in shared memory beside the groups' buffers.
 struct StepShared {
   alignas(16) int16_t pcol[4][64];  // the predictions of this CTA's modes, by columns
   alignas(16) int16_t rcol[4][64];  // their residuals by columns
@@ -148,6 +149,7 @@ struct StepShared {
   mtd::CoopPlane py, pc;
   mtd::CoopScan scan;
   mt_coef_costs cy;
+  float head[4][kTypes][64];                 // coop8_rate_head of this CTA's modes, by type and end of block
   unsigned long long key[kTypes];            // the warps' minima
   unsigned long long ckey[2][kClusterCtas];  // the CTAs' minima, by block parity
   alignas(16) NextBlock next[2];             // by block parity
@@ -174,7 +176,7 @@ constexpr int kMaxPolls = 1 << 20;               // a dependency wait gives up a
 // 4:4:4 and 4x4 in 4:2:0.  Only the levels and the reconstruction are wanted,
 // so the chain stops after the inverse.  Every group of lanes computes the
 // block; the first one writes it.
-__device__ __forceinline__ void code_chroma(StepShared& S, mtd::OctBuf* bufs, const EncArgs& a, int pl, int b, int px,
+__device__ __forceinline__ void code_chroma(StepShared& S, mtd::GroupBuf* bufs, const EncArgs& a, int pl, int b, int px,
                                             int py, bool has_t, bool has_l) {
   const int lane = threadIdx.x & 31;
   const int n = a.sub ? 4 : 8, ln = a.sub ? 2 : 3;
@@ -194,11 +196,11 @@ __device__ __forceinline__ void code_chroma(StepShared& S, mtd::OctBuf* bufs, co
   int e[8];
   if (n == 8) {
     const mtd::Coop<8> g;
-    mtd::OctBuf& o = bufs[lane >> 3];
+    mtd::GroupBuf& o = bufs[lane >> 3];
     for (int i = lane; i < 64; i += 32) S.ccol[i] = (int16_t)(S.csrc[i] - dc);
     __syncwarp();
 #pragma unroll
-    for (int x = 0; x < 8; x++) e[x] = S.scan.row8[g.j][x];
+    for (int k = 0; k < 8; k++) e[k] = S.scan.row8[g.j][k];
     mtd::coop8_fwd(MT_TX_DCT_DCT, S.ccol, nullptr, S.pc, c, at, o, g);
     mtd::coop_trellis<8>(c, at, e, S.pc, o, g);
     mtd::coop8_inv(MT_TX_DCT_DCT, c, S.pc, v, o, g);
@@ -211,7 +213,7 @@ __device__ __forceinline__ void code_chroma(StepShared& S, mtd::OctBuf* bufs, co
     }
   } else {
     const mtd::Coop<4> g;
-    mtd::OctBuf& o = bufs[lane >> 2];
+    mtd::GroupBuf& o = bufs[lane >> 2];
 #pragma unroll
     for (int x = 0; x < 4; x++) {
       e[x] = S.scan.row4[g.j][x];
@@ -239,7 +241,7 @@ __device__ __forceinline__ void code_chroma(StepShared& S, mtd::OctBuf* bufs, co
 // kDonePerBlock), builds the intra edges once, predicts its modes (a warp each)
 // and evaluates its candidates.  The CTAs exchange their minimum keys (cost,
 // candidate index) through distributed shared memory before the one cluster
-// barrier of the block; then the octet that holds the cluster's minimum writes
+// barrier of the block; then the lanes that hold the cluster's minimum write
 // the block out and every CTA publishes.  Keys and next blocks alternate
 // between two slots, so nothing is overwritten before all have read it.
 // Tickets follow the dependency levels, so the lowest unfinished ticket's
@@ -251,12 +253,16 @@ __device__ __forceinline__ void code_chroma(StepShared& S, mtd::OctBuf* bufs, co
 //
 // Bound by the dependency chain: a level's latency is the wait for the
 // neighbours, the edges, the prediction, one candidate chain and the exchange.
+// Measured against octets that mixed the types of a warp and three cluster
+// barriers a block: 512x512 4:4:4 (402 levels) 7.4 -> 3.4 ms, 1080p 4:2:0 (1,148
+// levels) 24.7 -> 10.1 ms, 4096x4096 4:4:4 (2,354 levels, 111 blocks each)
+// 136.9 -> 41.3 ms.
 __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThreads, MT_ENC_CTAS_PER_SM)
     encode_blocks_kernel(const JobDesc* __restrict__ jobs, const uint2* __restrict__ list, int nlist,
                          uint32_t* ticket_ctr, uint32_t* err) {
   __shared__ StepShared S;
-  extern __shared__ __align__(16) unsigned char oct_smem[];
-  mtd::OctBuf* bufs = reinterpret_cast<mtd::OctBuf*>(oct_smem);
+  extern __shared__ __align__(16) unsigned char group_smem[];
+  mtd::GroupBuf* bufs = reinterpret_cast<mtd::GroupBuf*>(group_smem);
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -271,7 +277,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThre
     for (int q = 0; q < kClusterCtas; ++q) *reinterpret_cast<uint4*>(cluster.map_shared_rank(&S.next[slot], q)) = v;
   };
   cluster.sync();  // every CTA of the cluster has started
-  if (rank == 0 && t == kLumaThreads) fetch(0);
+  if (rank == 0 && t == 0) fetch(0);
   cluster.sync();
   const EncArgs& a = S.job.a;
   const int mlo = mode_lo(rank), nm = mode_lo(rank + 1) - mlo;  // this CTA's modes
@@ -290,6 +296,11 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThre
       for (int i = t; i < (int)(sizeof(mt_coef_costs) / 4); i += blockDim.x) sy[i] = gy[i];
       if (t < 64) S.py.stage(t, a.qy, a.tly, a.has_qm_y ? S.job.qmy : nullptr, 64);
       else if (t < 128) S.pc.stage(t - 64, a.qc, a.tlc, a.has_qm_c ? S.job.qmc : nullptr, a.sub ? 16 : 64);
+      __syncthreads();
+      for (int i = t; i < nm * kTypes * 64; i += blockDim.x) {
+        const int m = i / (kTypes * 64), x = i / 64 % kTypes;
+        S.head[m][x][i & 63] = mtd::coop8_rate_head(S.cy, mlo + m, x, i & 63);
+      }
       __syncthreads();
       if (t == 0) S.cur = img;
     }
@@ -326,7 +337,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThre
     } else if (t >= 64 && t < 128) {  // the source block, which waits for nothing
       const int i = t - 64, y = i >> 3, x = i & 7;
       S.src[x * 8 + y] = (int16_t)a.src[0][(size_t)(py + y) * a.py.stride + px + x];
-    } else if (rank >= 2 && warp == kTypes) {
+    } else if (rank >= 2 && warp == kSideWarp) {
       const int n = a.sub ? 4 : 8, sh = a.sub ? 2 : 3, cx = a.sub ? px / 2 : px, cy = a.sub ? py / 2 : py;
       for (int i = lane; i < n * n; i += 32) {
         const int y = i >> sh, x = i & (n - 1);
@@ -334,9 +345,9 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThre
       }
     }
     __syncthreads();
-    int32_t c[8], rv[8];  // an octet's levels (row j) and reconstruction (column j)
-    if (warp == kTypes) {
-      if (rank >= 2) code_chroma(S, bufs + kTypes * 4, a, rank - 2, b, px, py, has_t, has_l);
+    int32_t c[8], rv[8];  // a lane's levels (row j) and reconstruction (column j)
+    if (warp == kSideWarp) {
+      if (rank >= 2) code_chroma(S, bufs + 4 * kTypes, a, rank - 2, b, px, py, has_t, has_l);
       else if (rank == 0 && lane == 0) fetch(par ^ 1);
     } else {
       // the intra edges with their fills (predict_sq_at), read past L1 (other
@@ -364,37 +375,37 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThre
                            S.pcol[warp], S.rcol[warp], S.rrow[warp], S.pb[warp]);
       luma_bar();
       const mtd::Coop<8> g;
-      const int oct = lane >> 3, ms = min(oct, nm - 1), mode = mlo + ms, TX = warp;
-      mtd::OctBuf& o = bufs[warp * 4 + oct];
-      int sc[8];
+      const int slot = lane >> 3, ms = min(slot, nm - 1), TX = warp;
+      mtd::GroupBuf& o = bufs[4 * TX + slot];
+      int e[8];
       {
         const uint2 w = *reinterpret_cast<const uint2*>(S.scan.row8[g.j]);
 #pragma unroll
-        for (int x = 0; x < 4; x++) {
-          sc[x] = (w.x >> (8 * x)) & 255;
-          sc[x + 4] = (w.y >> (8 * x)) & 255;
+        for (int k = 0; k < 4; k++) {
+          e[k] = (w.x >> (8 * k)) & 255;
+          e[k + 4] = (w.y >> (8 * k)) & 255;
         }
       }
       float at[8];
       mtd::coop8_fwd(TX, S.rcol[ms], S.rrow[ms], S.py, c, at, o, g);
-      const int eob = mtd::coop_trellis<8>(c, at, sc, S.py, o, g);
+      const int eob = mtd::coop_trellis<8>(c, at, e, S.py, o, g);
       mtd::coop8_inv(TX, c, S.py, rv, o, g);
-      int32_t d[8], pr[8], sr[8];
+      int32_t d[8], pr[8];
       mtd::load8(S.pcol[ms] + g.j * 8, pr);
-      mtd::load8(S.src + g.j * 8, sr);
+      mtd::load8(S.src + g.j * 8, d);
 #pragma unroll
-      for (int y = 0; y < 8; y++) {
-        rv[y] = min(max(pr[y] + rv[y], 0), 255);
-        d[y] = sr[y] - rv[y];
+      for (int k = 0; k < 8; k++) {
+        rv[k] = min(max(pr[k] + rv[k], 0), 255);
+        d[k] -= rv[k];
       }
       const uint32_t satd = mtd::coop8_satd(d, g);
       float price = __fmul_rn(__fmul_rn(__fmul_rn((float)satd, fmaxf((float)S.py.q.ac_q, 1.0f)), 0.25f), a.py.satd_scale);
       if (a.py.satd_bridge != 0.0f) price = __fmul_rn(price, a.py.satd_bridge);
-      const float bits = mtd::coop8_rate(c, sc, eob, S.cy, mode, TX, o, g);
+      const float bits = mtd::coop8_rate(c, e, eob, S.cy, S.head[ms][TX], o, g);
       const float cost = __fadd_rn(price, __fmul_rn(a.py.mode_lambda, bits));
       unsigned long long k = ~0ull;
-      if (g.j == 0 && oct < nm)
-        k = ((unsigned long long)__float_as_uint(cost) << 32) | (unsigned)(mode * kTypes + TX);
+      if (g.j == 0 && slot < nm)
+        k = ((unsigned long long)__float_as_uint(cost) << 32) | (unsigned)((mlo + ms) * kTypes + TX);
 #pragma unroll
       for (int s = 8; s < 32; s <<= 1) {
         const unsigned long long ok = __shfl_xor_sync(0xffffffffu, k, s);
@@ -1011,7 +1022,7 @@ int decide_all(std::vector<Job>& jobs, Buffers& buf) {
     jobs[(size_t)d].cs->h2d(jobs[(size_t)d].sched.size() * 8 + sizeof(JobDesc));
     jobs[(size_t)d].cs->mark(1, ks);
   }
-  constexpr int dyn = kOctBufs * (int)sizeof(mtd::OctBuf);
+  constexpr int dyn = kGroupBufs * (int)sizeof(mtd::GroupBuf);
   if (cudaFuncSetAttribute(encode_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess)
     return MT_ERR_DEVICE;
   encode_blocks_kernel<<<nclusters * kClusterCtas, kStepThreads, dyn, ks>>>(d_jobs, d_list, (int)list.size(), d_ctl,

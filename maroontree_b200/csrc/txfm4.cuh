@@ -12,15 +12,16 @@ namespace mtd {
 // reference accumulates in i64, and for residuals of 8-bit samples no partial
 // sum of either pass leaves +-2^31 (row sums of |A| <= 15487, first-pass
 // outputs <= ~1.5k), so i32 accumulation gives the same value.
-__constant__ int16_t kAdst4Fwd[16] = {1868, 3510, 4730, 5379, 4730, 4730,  0,    -4730,
-                                      5379, -1868, -4730, 3510, 3510, -5379, 4730, -1868};
 __device__ __forceinline__ void fadst4(int32_t* v) {
+  // a local constant, so that the unrolled products take immediates
+  constexpr int16_t A[16] = {1868, 3510, 4730, 5379, 4730, 4730,  0,    -4730,
+                             5379, -1868, -4730, 3510, 3510, -5379, 4730, -1868};
   int32_t o[4];
 #pragma unroll
   for (int i = 0; i < 4; i++) {
     int32_t acc = 2048;
 #pragma unroll
-    for (int j = 0; j < 4; j++) acc += (int32_t)kAdst4Fwd[i * 4 + j] * v[j];
+    for (int j = 0; j < 4; j++) acc += (int32_t)A[i * 4 + j] * v[j];
     o[i] = acc >> 12;
   }
 #pragma unroll

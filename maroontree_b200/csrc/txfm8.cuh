@@ -70,23 +70,23 @@ __device__ __forceinline__ void fdct8(int32_t* v) {
   v[1] = o0; v[3] = o1; v[5] = o2; v[7] = o3;
 }
 // 8-point forward ADST as a Q12 matrix product (src/dct.rs:304-326).
-__constant__ int16_t kAdst8Fwd[64] = {
-    567,  1682,  2730, 3675,  4477,  5109,  5544,  5766,  1682, 4480,  5766,  5109,  2732,
-    -569, -3675, -5545, 2732, 5766,  3675,  -1682, -5544, -4479, 569,   5109,  3675,  5108,
-    -1681, -5764, -569, 5542,  2732,  -4479, 4479,  2732,  -5542, -569,  5764,  -1681, -5108,
-    3675,  5109,  -569, -4479, 5544,  -1682, -3675, 5766,  -2732, 5545,  -3675, 569,   2732,
-    -5109, 5766,  -4480, 1682, 5766,  -5544, 5109,  -4477, 3675,  -2730, 1682,  -567};
 // The reference accumulates in i64.  For residuals of 8-bit samples
 // (|r| <= 255) no partial sum of either pass leaves +-2^31 (row sums of |A|
 // are <= 29550, column outputs <= ~6.2k), so the i32 accumulation here is the
 // same value.
 __device__ __forceinline__ void fadst8(int32_t* v) {
+  // a local constant, so that the unrolled products take immediates
+  constexpr int16_t A[64] = {
+      567, 1682, 2730, 3675, 4477, 5109, 5544, 5766, 1682, 4480, 5766, 5109, 2732, -569, -3675, -5545,
+      2732, 5766, 3675, -1682, -5544, -4479, 569, 5109, 3675, 5108, -1681, -5764, -569, 5542, 2732, -4479,
+      4479, 2732, -5542, -569, 5764, -1681, -5108, 3675, 5109, -569, -4479, 5544, -1682, -3675, 5766, -2732,
+      5545, -3675, 569, 2732, -5109, 5766, -4480, 1682, 5766, -5544, 5109, -4477, 3675, -2730, 1682, -567};
   int32_t o[8];
 #pragma unroll
   for (int i = 0; i < 8; i++) {
     int32_t acc = 2048;
 #pragma unroll
-    for (int j = 0; j < 8; j++) acc += (int32_t)kAdst8Fwd[i * 8 + j] * v[j];
+    for (int j = 0; j < 8; j++) acc += (int32_t)A[i * 8 + j] * v[j];
     o[i] = acc >> 12;
   }
 #pragma unroll
