@@ -1093,16 +1093,21 @@ size_t mt_cdef_scratch_bytes(const mt_cdef_params* prm) {
   return make_layout(make_geo(prm), prm->mono != 0).total;
 }
 
-int mt_cdef_frame_device(uint16_t* d_y, uint16_t* d_u, uint16_t* d_v, const uint16_t* d_src_y,
-                         const uint16_t* d_src_u, const uint16_t* d_src_v, const uint8_t* d_skip8,
-                         const mt_cdef_params* prm, void* d_scratch, mt_cdef_decision* out, uint8_t* grid,
-                         void* stream) {
+}  // extern "C"
+
+namespace mth {
+
+// mt_cdef_frame_device up to the filtered planes, on the stream and without a
+// wait: `decided` (when given) is recorded once the strength search's decision
+// is on the device (*d_bits, and *d_grid per 64x64 unit), ahead of the filter.
+int cdef_frame_enqueue(uint16_t* d_y, uint16_t* d_u, uint16_t* d_v, const uint16_t* d_src_y, const uint16_t* d_src_u,
+                       const uint16_t* d_src_v, const uint8_t* d_skip8, const mt_cdef_params* prm, void* d_scratch,
+                       cudaEvent_t decided, const int32_t** d_bits, const uint8_t** d_grid, cudaStream_t st) {
   int rc = check_params(prm);
   if (rc != MT_OK) return rc;
   const bool mono = prm->mono != 0;
-  if (!d_y || !d_src_y || !d_skip8 || !d_scratch || !out) return MT_ERR_INVALID_INPUT;
+  if (!d_y || !d_src_y || !d_skip8 || !d_scratch) return MT_ERR_INVALID_INPUT;
   if (!mono && (!d_u || !d_v || !d_src_u || !d_src_v)) return MT_ERR_INVALID_INPUT;
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const Geo g = make_geo(prm);
   const Layout L = make_layout(g, mono);
   uint8_t* s = static_cast<uint8_t*>(d_scratch);
@@ -1140,6 +1145,9 @@ int mt_cdef_frame_device(uint16_t* d_y, uint16_t* d_u, uint16_t* d_v, const uint
   sa.ustr = s + L.ustr;
   if ((rc = launch_search(sa, st)) != MT_OK) return rc;
   mth::cdef_last_launches += kSearchLaunches;
+  if (d_bits) *d_bits = &sa.S->bits;
+  if (d_grid) *d_grid = sa.grid;
+  if (decided && cudaEventRecord(decided, st) != cudaSuccess) return MT_ERR_DEVICE;
   // the filter from a pre-CDEF snapshot, with each unit's strengths (all zero:
   // the planes stay as they are)
   ApplyArgs aa;
@@ -1157,10 +1165,20 @@ int mt_cdef_frame_device(uint16_t* d_y, uint16_t* d_u, uint16_t* d_v, const uint
   }
   cdef_apply_kernel<<<dim3(g.nbx, g.nby, mono ? 1 : 3), 64, 0, st>>>(aa, g, d_skip8, dirs, vars, s + L.ustr);
   mth::cdef_last_launches += 1;
-  // the decision back to the host, once, at the end
+  return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_DEVICE;
+}
+
+// The decision of the last cdef_frame_enqueue over d_scratch, read back; waits
+// for the stream.
+int cdef_frame_decision(const mt_cdef_params* prm, void* d_scratch, mt_cdef_decision* out, uint8_t* grid,
+                        cudaStream_t st) {
+  const Geo g = make_geo(prm);
+  const Layout L = make_layout(g, prm->mono != 0);
+  uint8_t* s = static_cast<uint8_t*>(d_scratch);
   SearchState hs;
   if (cudaMemcpyAsync(&hs, s + L.state, sizeof(hs), cudaMemcpyDeviceToHost, st) != cudaSuccess) return MT_ERR_DEVICE;
-  if (grid && cudaMemcpyAsync(grid, s + L.grid, nu, cudaMemcpyDeviceToHost, st) != cudaSuccess) return MT_ERR_DEVICE;
+  if (grid && cudaMemcpyAsync(grid, s + L.grid, (size_t)g.uc * g.ur, cudaMemcpyDeviceToHost, st) != cudaSuccess)
+    return MT_ERR_DEVICE;
   if (cudaStreamSynchronize(st) != cudaSuccess) return MT_ERR_DEVICE;
   out->bits = hs.bits;
   out->damping = 3 + std::min(prm->base_q_idx / 64, 3);
@@ -1169,6 +1187,24 @@ int mt_cdef_frame_device(uint16_t* d_y, uint16_t* d_u, uint16_t* d_v, const uint
   out->unit_rows = g.ur;
   memcpy(out->strengths, hs.strengths, sizeof(out->strengths));
   return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_DEVICE;
+}
+
+}  // namespace mth
+
+extern "C" {
+
+int mt_cdef_frame_device(uint16_t* d_y, uint16_t* d_u, uint16_t* d_v, const uint16_t* d_src_y,
+                         const uint16_t* d_src_u, const uint16_t* d_src_v, const uint8_t* d_skip8,
+                         const mt_cdef_params* prm, void* d_scratch, mt_cdef_decision* out, uint8_t* grid,
+                         void* stream) {
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (!out) {
+    const int rc = check_params(prm);
+    return rc != MT_OK ? rc : MT_ERR_INVALID_INPUT;
+  }
+  const int rc = mth::cdef_frame_enqueue(d_y, d_u, d_v, d_src_y, d_src_u, d_src_v, d_skip8, prm, d_scratch, nullptr,
+                                         nullptr, nullptr, st);
+  return rc != MT_OK ? rc : mth::cdef_frame_decision(prm, d_scratch, out, grid, st);
 }
 
 int mt_cdef_frame(uint16_t* y, uint16_t* u, uint16_t* v, const uint16_t* src_y, const uint16_t* src_u,

@@ -39,7 +39,7 @@
 #include "../../include/maroontree_b200.h"
 #include "av1_tables.h"
 #include "coop8.cuh"
-#include "pack.h"
+#include "stream.h"
 
 namespace mth {
 float scaled_trellis_lambda_host(float dc_q, float lambda0);
@@ -454,38 +454,6 @@ __global__ void pad_plane_kernel(const uint8_t* __restrict__ in, int w, int h, u
   out[(size_t)y * pw + x] = in[(size_t)min(y, h - 1) * w + min(x, w - 1)];
 }
 
-// The coefficient context byte each transform block leaves for its
-// neighbours (src/coeffs.rs eob_and_cul): min(sum of |levels| up to the end
-// of block, 63) | the DC sign bits, 0x40 when all levels are zero; the sum
-// runs in the block's coding order (the 2-D scan, or the 1-D classes' row /
-// column order).  res[3 b + p] for 8x8 block b and plane p.
-__global__ void res_ctx_kernel(const int32_t* __restrict__ lv_y, const int32_t* __restrict__ lv_u,
-                               const int32_t* __restrict__ lv_v, const uint8_t* __restrict__ tx, int nb, int sub,
-                               uint8_t* __restrict__ res) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 3 * nb) return;
-  const int b = i / 3, p = i % 3;
-  const int n = (p == 0 || sub == 0) ? 8 : 4, cl = sub ? 16 : 64;
-  const int32_t* cf = p == 0 ? lv_y + (size_t)b * 64 : (p == 1 ? lv_u : lv_v) + (size_t)b * cl;
-  const int cls = p == 0 ? (tx[b] == MT_TX_V_DCT ? 1 : (tx[b] == MT_TX_H_DCT ? 2 : 0)) : 0;
-  auto at = [&](int k) -> int {
-    if (cls == 1) return ((k & (n - 1)) * n) + k / n;  // vertical class order
-    if (cls == 2) return k;
-    return n == 4 ? mtd::kScan4[k] : mtd::kScan8[k];
-  };
-  int eob = -1;
-  for (int k = 0; k < n * n; ++k)
-    if (cf[at(k)]) eob = k;
-  if (eob < 0) {
-    res[i] = 0x40;
-    return;
-  }
-  uint32_t cul = 0;
-  for (int k = 0; k <= eob; ++k) cul += (uint32_t)abs(cf[at(k)]);
-  const uint8_t dcb = cf[0] == 0 ? 0x40 : (cf[0] < 0 ? 0 : 0x80);
-  res[i] = (uint8_t)((cul < 63 ? cul : 63) | dcb);
-}
-
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -493,152 +461,18 @@ __global__ void res_ctx_kernel(const int32_t* __restrict__ lv_y, const int32_t* 
 
 namespace {
 
-const int kIntraModeCtx[13] = {0, 1, 2, 3, 4, 4, 4, 4, 3, 0, 1, 2, 0};  // src/intrapred.rs:1088
-
-struct BlockSyntax {
-  const mt_cdf_slot_layout& L;
-  int w8, h8, sub, nbx;
-  const uint8_t* mode;
-  const uint8_t* tx;
-  std::vector<uint8_t> a_part, l_part, a_skip, l_skip, a_mode, l_mode;
-  std::vector<int8_t> a_tx, l_tx;
-  std::vector<uint8_t> a_coef[3], l_coef[3];
-  const uint8_t* res_ctx;  // per coefficient block, in coding order: (Y, U, V) per 8x8 block
-  std::vector<mt_coef_block>* blocks;
-  std::vector<std::vector<uint32_t>> sbs;  // tokens with coefficient placeholders
-  std::vector<int32_t> cdef_points;
-
-  static constexpr uint32_t kCoef = 0xFFFFFFFFu;  // placeholder: next coefficient block's tokens
-  std::vector<uint32_t>* out;
-
-  void tok(int32_t slot, uint32_t s) { out->push_back(((uint32_t)slot << 8) | s); }
-  int part_ctx(int bl, int x8, int y8) const {
-    const int sh = 4 - bl;
-    return ((a_part[x8] >> sh) & 1) + (((l_part[y8] >> sh) & 1) << 1);
-  }
-
-  void block8(int x8, int y8, int* cdef_point) {
-    const int px = x8 * 8, py = y8 * 8, bx4 = px / 4, by4 = py / 4;
-    const int b = y8 * nbx + x8;
-    const int m = mode[b], t = tx[b];
-    tok(L.skip + a_skip[bx4] + l_skip[by4], 0);
-    if (*cdef_point < 0) *cdef_point = (int)out->size();  // read_cdef() follows the SB's first coded skip flag
-    a_skip[bx4] = a_skip[bx4 + 1] = 0;
-    l_skip[by4] = l_skip[by4 + 1] = 0;
-    tok(L.kf_y + kIntraModeCtx[a_mode[bx4]] * 5 + kIntraModeCtx[l_mode[by4]], (uint32_t)m);
-    if (m >= MT_V_PRED && m <= MT_D67_PRED) tok(L.angle_delta + m - MT_V_PRED, 3);  // delta 0
-    tok(L.uv_mode + 13 + m, MT_DC_PRED);  // CfL allowed at 8x8
-    if (m == MT_DC_PRED) tok(L.palette_y_mode + 0, 0);
-    tok(L.palette_uv_mode + 0, 0);
-    if (m == MT_DC_PRED) tok(L.filter_intra + 3, 0);  // BLOCK_8X8
-    tok(L.txsz + 0 * 3 + (l_tx[by4] >= 1) + (a_tx[bx4] >= 1), 0);
-    a_tx[bx4] = a_tx[bx4 + 1] = 1;
-    l_tx[by4] = l_tx[by4 + 1] = 1;
-    // residual: Y (TX_8X8), then U and V (TX_8X8 in 4:4:4, TX_4X4 in 4:2:0)
-    for (int p = 0; p < 3; ++p) {
-      const int u = (p == 0 || sub == 0) ? 2 : 1;  // 4x4 units the transform spans
-      const int cx = (p == 0 || sub == 0) ? bx4 : bx4 / 2, cy = (p == 0 || sub == 0) ? by4 : by4 / 2;
-      std::vector<uint8_t>& A = a_coef[p];
-      std::vector<uint8_t>& Ll = l_coef[p];
-      int s = -2 * u, anz = 0, lnz = 0;
-      for (int k = 0; k < u; ++k) {
-        s += (A[cx + k] >> 6) + (Ll[cy + k] >> 6);
-        anz |= A[cx + k] != 0x40;
-        lnz |= Ll[cy + k] != 0x40;
-      }
-      mt_coef_block cb = {};
-      cb.log2n = u == 2 ? 3 : 2;
-      cb.plane = p ? 1 : 0;
-      cb.skip_ctx = (uint8_t)(p == 0 ? 0 : 7 + anz + lnz);
-      cb.dcs_ctx = (uint8_t)((s != 0) + (s > 0));
-      cb.y_mode = (uint8_t)m;
-      cb.txtp = (uint8_t)(p == 0 ? t : MT_TX_DCT_DCT);
-      cb.code_txtp = p == 0;
-      cb.tx_class = (uint8_t)(p == 0 && t == MT_TX_V_DCT ? 1 : (p == 0 && t == MT_TX_H_DCT ? 2 : 0));
-      blocks->push_back(cb);
-      out->push_back(kCoef);
-    }
-    a_mode[bx4] = a_mode[bx4 + 1] = (uint8_t)m;
-    l_mode[by4] = l_mode[by4 + 1] = (uint8_t)m;
-  }
-
-  // clear_above_context at a tile's start for its 8x8 columns [x0, x1), and
-  // clear_left_context at each superblock row of a tile for rows [y0, y1):
-  // the values of an unavailable neighbour.
-  void clear_above(int x0, int x1) {
-    for (int x = x0; x < x1; ++x) a_part[x] = 0;
-    for (int x = 2 * x0; x < 2 * x1; ++x) {
-      a_skip[x] = a_mode[x] = 0;
-      a_tx[x] = -1;
-    }
-    for (int p = 0; p < 3; ++p) {
-      const int k = (p == 0 || sub == 0) ? 2 : 1;
-      for (int x = k * x0; x < k * x1; ++x) a_coef[p][x] = 0x40;
-    }
-  }
-  void clear_left(int y0, int y1) {
-    for (int y = y0; y < y1; ++y) l_part[y] = 0;
-    for (int y = 2 * y0; y < 2 * y1; ++y) {
-      l_skip[y] = l_mode[y] = 0;
-      l_tx[y] = -1;
-    }
-    for (int p = 0; p < 3; ++p) {
-      const int k = (p == 0 || sub == 0) ? 2 : 1;
-      for (int y = k * y0; y < k * y1; ++y) l_coef[p][y] = 0x40;
-    }
-  }
-
-  // After a block's coefficient contexts are known: its res_ctx bytes.
-  void commit_res(int x8, int y8, const uint8_t r[3]) {
-    const int bx4 = x8 * 2, by4 = y8 * 2;
-    for (int p = 0; p < 3; ++p) {
-      const int u = (p == 0 || sub == 0) ? 2 : 1;
-      const int cx = (p == 0 || sub == 0) ? bx4 : bx4 / 2, cy = (p == 0 || sub == 0) ? by4 : by4 / 2;
-      for (int k = 0; k < u; ++k) {
-        a_coef[p][cx + k] = r[p];
-        l_coef[p][cy + k] = r[p];
-      }
-    }
-  }
-
-  // code_split (src/coder/superblock.rs:950-990) always taking SPLIT, down to
-  // 8x8 PARTITION_NONE leaves.
-  template <class F>
-  void node(int bl, int x8, int y8, int sz8, int* cdef_point, F&& leaf) {
-    if (sz8 == 1) {
-      tok(L.part_bl8 + part_ctx(4, x8, y8), 0);
-      leaf(x8, y8);
-      a_part[x8] = 0x1E;
-      l_part[y8] = 0x1E;
-      return;
-    }
-    const int hh = sz8 / 2;
-    const bool have_h = (x8 + hh) * 8 < w8, have_v = (y8 + hh) * 8 < h8;
-    const int32_t slot = L.part_split + (bl - 1) * 4 + part_ctx(bl, x8, y8);
-    if (have_h && have_v)
-      tok(slot, 3);
-    else if (have_h)
-      out->push_back((2u << 30) | ((uint32_t)slot << 2) | (1u << 1) | 1u);  // gathered: split, top
-    else if (have_v)
-      out->push_back((2u << 30) | ((uint32_t)slot << 2) | (1u << 1) | 0u);  // gathered: split, left
-    const int cx[4] = {x8, x8 + hh, x8, x8 + hh}, cy[4] = {y8, y8, y8 + hh, y8 + hh};
-    for (int c = 0; c < 4; ++c)
-      if (cx[c] * 8 < w8 && cy[c] * 8 < h8) node(bl + 1, cx[c], cy[c], hh, cdef_point, leaf);
-  }
-};
-
 // The device buffers of the images of an encode call.  Each device keeps
 // sets of them -- one per image of the largest batch seen, each grown to the
-// largest frame it carried, each with a stream -- until
+// largest frame it carried, each with two streams -- until
 // mt_encode_release_buffers or exit.  A call uses them when no other call on
 // that device holds them; otherwise it allocates its own for the call.
 constexpr int kSlots = 16;
-enum Slot { kRgb, kPlanes, kTables, kDecisions, kLevels, kSched, kEmit, kTokens, kMaps, kDeblock, kFiltered, kSkip8,
-            kCdef, kRes, kList, kJobs };
+enum Slot { kRgb, kPlanes, kTables, kDecisions, kLevels, kSched, kPlan, kTokens, kMaps, kDeblock, kFiltered, kSkip8,
+            kCdef, kDigits, kList, kJobs };
 struct BufSet {
   void* p[kSlots] = {};
   size_t cap[kSlots] = {};
-  cudaStream_t st = nullptr;
+  cudaStream_t st[2] = {nullptr, nullptr};
 };
 struct Arena {
   std::mutex mu;
@@ -659,7 +493,8 @@ class Buffers {
     if (ar_) ar_->mu.unlock();
     for (BufSet& b : own_) {
       for (void* q : b.p) cudaFree(q);
-      if (b.st) cudaStreamDestroy(b.st);
+      for (cudaStream_t s : b.st)
+        if (s) cudaStreamDestroy(s);
     }
   }
   template <class T>
@@ -675,10 +510,10 @@ class Buffers {
     }
     return reinterpret_cast<T*>(b.p[s]);
   }
-  cudaStream_t stream(int i) {
+  cudaStream_t stream(int i, int k) {  // 0: the image's own, 1: its entropy coding beside the filters
     BufSet& b = set(i);
-    if (!b.st && cudaStreamCreateWithFlags(&b.st, cudaStreamNonBlocking) != cudaSuccess) b.st = nullptr;
-    return b.st;
+    if (!b.st[k] && cudaStreamCreateWithFlags(&b.st[k], cudaStreamNonBlocking) != cudaSuccess) b.st[k] = nullptr;
+    return b.st[k];
   }
 
  private:
@@ -745,10 +580,13 @@ struct Job {
   JobDesc desc = {};
   uint16_t* src[3] = {};
   uint16_t* rec[3] = {};
-  uint8_t* d_res = nullptr;
+  mth::StreamGeom sg = {};
+  mth::StreamInput si = {};
+  void* d_plan = nullptr;
+  uint8_t* d_cdfs = nullptr;
   std::vector<uint32_t> sched;  // blocks in dependency-level order
   std::vector<int> lstart;      // first entry of each level
-  cudaStream_t st = nullptr;
+  cudaStream_t st = nullptr, st_code = nullptr;
   std::unique_ptr<CallStats> cs;
   int rc = MT_OK;
 };
@@ -756,6 +594,11 @@ struct Job {
 }  // namespace
 
 namespace mth {
+int cdef_frame_enqueue(uint16_t* d_y, uint16_t* d_u, uint16_t* d_v, const uint16_t* d_src_y, const uint16_t* d_src_u,
+                       const uint16_t* d_src_v, const uint8_t* d_skip8, const mt_cdef_params* prm, void* d_scratch,
+                       cudaEvent_t decided, const int32_t** d_bits, const uint8_t** d_grid, cudaStream_t st);
+int cdef_frame_decision(const mt_cdef_params* prm, void* d_scratch, mt_cdef_decision* out, uint8_t* grid,
+                        cudaStream_t st);
 void cdef_frame_transfer_bytes(const mt_cdef_params* p, size_t* d2h, size_t* h2d);
 extern thread_local int cdef_last_launches;
 extern thread_local int deblock_last_launches;
@@ -764,8 +607,6 @@ extern thread_local int deblock_last_launches;
 extern "C" {
 int mt_coef_costs_build(const mt_coef_cdfs* cdfs, mt_coef_costs* out);
 const uint8_t* mt_qm_row(int32_t qm_level, int32_t chroma, int32_t w, int32_t h);
-int mt_emit_coeffs_device(const int32_t* d_levels, const mt_coef_block* d_blocks, int32_t n, uint32_t* d_counts,
-                          uint32_t* d_offsets, uint32_t* d_tokens, uint8_t* d_res_ctx, void* stream);
 }
 
 namespace {
@@ -819,13 +660,29 @@ int job_setup(Job& j, Buffers& buf, int i) {
                                 : (size_t)width * height + 2 * (size_t)((width + sx) >> sx) * ((height + sx) >> sx);
   uint8_t* d_rgbbuf = buf.get<uint8_t>(i, kRgb, j.rgb_on_device ? 1 : in_bytes);
   uint16_t* d_planes = buf.get<uint16_t>(i, kPlanes, (ny + 2 * nc) * 2 * 2);
-  uint8_t* d_tabs = buf.get<uint8_t>(i, kTables, sizeof(mt_coef_costs) + 128);
+  constexpr size_t cost_bytes = (sizeof(mt_coef_costs) + 128 + 15) & ~(size_t)15;
+  const size_t cdf_bytes = mth::stream_cdf_bytes();
+  uint8_t* d_tabs = buf.get<uint8_t>(i, kTables, cost_bytes + cdf_bytes);
   uint8_t* d_decs = buf.get<uint8_t>(i, kDecisions, (size_t)nb * 2);
   int32_t* d_levels = buf.get<int32_t>(i, kLevels, (size_t)nb * (64 + 2 * cl) * 4);
-  j.d_res = buf.get<uint8_t>(i, kRes, (size_t)nb * 3);
+  mth::StreamGeom& sg = j.sg;
+  sg.w8 = pw;
+  sg.h8 = ph;
+  sg.nbx = nbx;
+  sg.nby = nby;
+  sg.sub = sub;
+  sg.sb_cols = sb_cols;
+  sg.sb_rows = sb_rows;
+  sg.tile_w8 = j.tile_sb_w * 8;
+  sg.tile_h8 = j.tile_sb_h * 8;
+  sg.tcols = (sb_cols + j.tile_sb_w - 1) / j.tile_sb_w;
+  sg.trows = (sb_rows + j.tile_sb_h - 1) / j.tile_sb_h;
+  j.d_plan = buf.get<void>(i, kPlan, mth::stream_plan_bytes(sg));
   uint32_t* d_done = buf.get<uint32_t>(i, kSched, (size_t)nb * 4);
-  const cudaStream_t st = j.st = buf.stream(i);
-  if (!d_rgbbuf || !d_planes || !d_tabs || !d_decs || !d_levels || !j.d_res || !d_done || !st) return MT_ERR_DEVICE;
+  const cudaStream_t st = j.st = buf.stream(i, 0);
+  j.st_code = buf.stream(i, 1);
+  if (!d_rgbbuf || !d_planes || !d_tabs || !d_decs || !d_levels || !j.d_plan || !d_done || !st || !j.st_code)
+    return MT_ERR_DEVICE;
   uint16_t* const* src = j.src;
   for (int p = 0; p < 3; ++p) {
     j.src[p] = d_planes + (p == 0 ? 0 : ny + (size_t)(p - 1) * nc);
@@ -864,7 +721,9 @@ int job_setup(Job& j, Buffers& buf, int i) {
   cudaMemcpyAsync(d_cy, &cy, sizeof(cy), cudaMemcpyHostToDevice, st);
   if (qmy) cudaMemcpyAsync(d_qmy, qmy, 64, cudaMemcpyHostToDevice, st);
   if (qmc) cudaMemcpyAsync(d_qmc, qmc, sub ? 16 : 64, cudaMemcpyHostToDevice, st);
-  cs.h2d(sizeof(mt_coef_costs) + (qmy ? 64 : 0) + (qmc ? (sub ? 16 : 64) : 0));
+  j.d_cdfs = d_tabs + cost_bytes;
+  cudaMemcpyAsync(j.d_cdfs, mth::stream_cdf_table(qctx, sub), cdf_bytes, cudaMemcpyHostToDevice, st);
+  cs.h2d(sizeof(mt_coef_costs) + cdf_bytes + (qmy ? 64 : 0) + (qmc ? (sub ? 16 : 64) : 0));
   EncArgs& a = j.a;
   a = EncArgs{};
   for (int p = 0; p < 3; ++p) {
@@ -903,6 +762,11 @@ int job_setup(Job& j, Buffers& buf, int i) {
   a.lv_y = d_levels;
   a.lv_u = a.lv_y + (size_t)nb * 64;
   a.lv_v = a.lv_u + (size_t)nb * cl;
+  j.si.mode = a.mode;
+  j.si.tx = a.tx;
+  j.si.lv[0] = a.lv_y;
+  j.si.lv[1] = a.lv_u;
+  j.si.lv[2] = a.lv_v;
   j.desc.a = a;
   j.desc.cy = d_cy;
   j.desc.qmy = d_qmy;
@@ -1046,9 +910,6 @@ int decide_all(std::vector<Job>& jobs, Buffers& buf) {
   return MT_OK;
 }
 
-// Everything after the decisions for image i: the context bytes, the block
-// syntax walk, the coefficient tokens, the filters, range coding, headers
-// and container.
 // A CUDA event destroyed with its scope.
 struct EventGuard {
   cudaEvent_t e = nullptr;
@@ -1057,128 +918,49 @@ struct EventGuard {
   }
 };
 
-// Host threads joined when their scope ends, on every return path.
-struct ThreadGroup {
-  std::vector<std::thread> v;
-  ~ThreadGroup() { join(); }
-  void join() {
-    for (std::thread& w : v)
-      if (w.joinable()) w.join();
-    v.clear();
-  }
+// A stream waited for when its scope ends, on every return path: the buffers
+// its work uses are the next call's.
+struct StreamGuard {
+  cudaStream_t s;
+  ~StreamGuard() { cudaStreamSynchronize(s); }
 };
 
+// Everything after the decisions for image i: the filters, with the entropy
+// coding beside them on the image's second stream, headers and container.
 int job_finish(Job& j, Buffers& buf, int i) {
   int rc = MT_OK;
   const cudaStream_t st = j.st;
   CallStats& cs = *j.cs;
   const mt_encode_config* cfg = j.cfg;
   const uint32_t width = j.width, height = j.height;
-  const int sub = j.sub, sx = j.sx, nbx = j.nbx, nby = j.nby, nb = j.nb, sb_cols = j.sb_cols, sb_rows = j.sb_rows,
-            cl = j.cl;
+  const int sub = j.sub, sx = j.sx, nb = j.nb;
   const int32_t pw = j.pw, ph = j.ph;
   const size_t ny = j.ny, nc = j.nc;
-  const EncArgs& a = j.a;
   uint16_t* const* src = j.src;
   uint16_t* const* rec = j.rec;
-  std::vector<uint8_t> mode(nb), tx(nb);
-  // The coefficient contexts of a block depend on its neighbours' context
-  // bytes, which depend on their levels only: computed on the device for
-  // every transform block, read back as three bytes per 8x8 block.
-  res_ctx_kernel<<<(unsigned)((3 * (size_t)nb + 255) / 256), 256, 0, st>>>(a.lv_y, a.lv_u, a.lv_v, a.tx, nb, sub,
-                                                                           j.d_res);
-  cs.launches(1);
-  std::vector<uint8_t> resb((size_t)nb * 3);
-  if (cudaMemcpyAsync(mode.data(), a.mode, nb, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaMemcpyAsync(tx.data(), a.tx, nb, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaMemcpyAsync(resb.data(), j.d_res, resb.size(), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess)
+  const cudaStream_t sc = j.st_code;
+  StreamGuard code_guard{sc};
+  // every token's place; its total sizes the buffers of the entropy coding
+  int nl = 0;
+  if ((rc = mth::stream_count(j.sg, j.si, j.d_plan, st, &nl)) != MT_OK) return rc;
+  mth::StreamTotals tot = {};
+  const int ntiles = j.sg.tcols * j.sg.trows;
+  std::vector<mth::StreamTile> tile((size_t)ntiles);
+  EventGuard counted, decided;
+  for (EventGuard* e : {&counted, &decided})
+    if (cudaEventCreateWithFlags(&e->e, cudaEventDisableTiming) != cudaSuccess) return MT_ERR_DEVICE;
+  if (cudaMemcpyAsync(&tot, mth::stream_totals(j.sg, j.d_plan), sizeof(tot), cudaMemcpyDeviceToHost, st) !=
+          cudaSuccess ||
+      cudaEventRecord(counted.e, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess ||
+      cudaStreamWaitEvent(sc, counted.e, 0) != cudaSuccess)
     return MT_ERR_DEVICE;
-  cs.d2h(2 * (size_t)nb + resb.size());
-  // block syntax in coding order, with the coefficient blocks it carries
-  mt_cdf_slot_layout L;
-  mt_cdf_layout(&L);
-  std::vector<mt_coef_block> blocks;
-  blocks.reserve((size_t)nb * 3);
-  BlockSyntax bs{L, pw, ph, sub, nbx, mode.data(), tx.data()};
-  bs.a_part.assign(nbx, 0);
-  bs.l_part.assign(nby, 0);
-  bs.a_skip.assign(nbx * 2, 0);
-  bs.l_skip.assign(nby * 2, 0);
-  bs.a_mode.assign(nbx * 2, 0);
-  bs.l_mode.assign(nby * 2, 0);
-  bs.a_tx.assign(nbx * 2, -1);
-  bs.l_tx.assign(nby * 2, -1);
-  for (int p = 0; p < 3; ++p) {
-    bs.a_coef[p].assign(nbx * 2, 0x40);
-    bs.l_coef[p].assign(nby * 2, 0x40);
-  }
-  bs.blocks = &blocks;
-  // tiles in raster order, superblocks in raster order inside each tile
-  // (decode_tile: the above context cleared per tile, the left per SB row)
-  std::vector<int> tile_first;  // first coded superblock of each tile
-  std::vector<int> sb_unit;     // frame-raster 64x64 unit of each coded superblock
-  std::vector<size_t> sb_coef_first;  // first coefficient block of each coded superblock
-  for (int r0 = 0; r0 < sb_rows; r0 += j.tile_sb_h)
-    for (int c0 = 0; c0 < sb_cols; c0 += j.tile_sb_w) {
-      const int r1 = std::min(r0 + j.tile_sb_h, sb_rows), c1 = std::min(c0 + j.tile_sb_w, sb_cols);
-      tile_first.push_back((int)bs.sbs.size());
-      bs.clear_above(c0 * 8, std::min(c1 * 8, nbx));
-      for (int sr = r0; sr < r1; ++sr) {
-        bs.clear_left(sr * 8, std::min(sr * 8 + 8, nby));
-        for (int sc = c0; sc < c1; ++sc) {
-          bs.sbs.emplace_back();
-          bs.out = &bs.sbs.back();
-          sb_coef_first.push_back(blocks.size());
-          sb_unit.push_back(sr * sb_cols + sc);
-          int cp = -1;
-          bs.node(1, sc * 8, sr * 8, 8, &cp, [&](int x8, int y8) {
-            const size_t first = blocks.size();
-            bs.block8(x8, y8, &cp);
-            const int b = y8 * nbx + x8;
-            const uint32_t off[3] = {(uint32_t)((size_t)b * 64), (uint32_t)((size_t)nb * 64 + (size_t)b * cl),
-                                     (uint32_t)((size_t)nb * (64 + cl) + (size_t)b * cl)};
-            for (int p = 0; p < 3; ++p) blocks[first + p].cf_offset = off[p];
-            bs.commit_res(x8, y8, &resb[(size_t)b * 3]);
-          });
-          bs.cdef_points.push_back(cp);
-        }
-      }
-    }
-  tile_first.push_back((int)bs.sbs.size());
-  sb_coef_first.push_back(blocks.size());
-  // coefficient tokens of every block in one launch
-  const int ncb = (int)blocks.size();
-  mt_coef_block* d_blocks = buf.get<mt_coef_block>(i, kEmit, (size_t)ncb * (sizeof(mt_coef_block) + 8) + 8);
-  if (!d_blocks) return MT_ERR_DEVICE;
-  uint32_t* d_cnt = reinterpret_cast<uint32_t*>(d_blocks + ncb);
-  uint32_t* d_off = d_cnt + ncb;
-  if (cudaMemcpyAsync(d_blocks, blocks.data(), (size_t)ncb * sizeof(mt_coef_block), cudaMemcpyHostToDevice, st) !=
-      cudaSuccess)
-    return MT_ERR_DEVICE;
-  if ((rc = mt_emit_coeffs_device(a.lv_y, d_blocks, ncb, d_cnt, d_off, nullptr, nullptr, st)) != MT_OK) return rc;
-  cs.h2d((size_t)ncb * sizeof(mt_coef_block));
-  cs.launches(2);
-  uint32_t total = 0;
-  if (cudaMemcpyAsync(&total, d_off + ncb, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess)
-    return MT_ERR_DEVICE;
-  uint32_t* d_tok = buf.get<uint32_t>(i, kTokens, (size_t)total * 4);
+  cs.d2h(sizeof(tot));
+  void* d_tok = buf.get<void>(i, kTokens, mth::stream_token_bytes(j.sg, tot.tokens));
   if (!d_tok) return MT_ERR_DEVICE;
-  if ((rc = mt_emit_coeffs_device(a.lv_y, d_blocks, ncb, d_cnt, d_off, d_tok, nullptr, st)) != MT_OK) return rc;
-  cs.launches(1);
-  std::vector<uint32_t> toks(total), offs((size_t)ncb + 1);
-  if (cudaMemcpyAsync(toks.data(), d_tok, (size_t)total * 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaMemcpyAsync(offs.data(), d_off, offs.size() * 4, cudaMemcpyDeviceToHost, st) != cudaSuccess)
-    return MT_ERR_DEVICE;
-  // the tokens are on the host once this event has passed; the filters
-  // carry on behind it on the stream
-  EventGuard tok_ev;
-  if (cudaEventCreateWithFlags(&tok_ev.e, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventRecord(tok_ev.e, st) != cudaSuccess)
-    return MT_ERR_DEVICE;
-  // deblocking (uniform 8x8 blocks and transforms) and the CDEF decision,
-  // enqueued before the host splices the tokens
+  if ((rc = mth::stream_trace(j.sg, j.si, j.d_plan, d_tok, tot.tokens, j.d_cdfs, cfg->updating_cdf != 0, sc, &nl)) !=
+      MT_OK)
+    return rc;
+  // deblocking (uniform 8x8 blocks and transforms) and the CDEF decision
   int32_t ly, luv, sharp;
   mt_loop_filter_levels(j.plan.base_q_idx, sx, sx, &ly, &luv, &sharp);
   const int n4 = (pw / 4) * (ph / 4);
@@ -1217,35 +999,6 @@ int job_finish(Job& j, Buffers& buf, int i) {
                                        m0 + 5 * (size_t)n4, &g, ly, luv, luv, d_db, st)) != MT_OK)
     return rc;
   cs.launches(mth::deblock_last_launches);
-  // phase 1 of the range coding (each token's store, with the CDF
-  // adaptation), one host thread per tile, reading the superblocks' syntax
-  // tokens and the coefficient blocks in place while the filters run
-  if (cudaEventSynchronize(tok_ev.e) != cudaSuccess) return MT_ERR_DEVICE;
-  cs.d2h(4 + (size_t)total * 4 + offs.size() * 4);
-  const int ntiles = (int)tile_first.size() - 1;
-  std::vector<std::unique_ptr<mth::TileStores>> stores((size_t)ntiles);
-  size_t nstores = 0;
-  for (int t = 0; t < ntiles; ++t) {
-    const int f = tile_first[(size_t)t], l = tile_first[(size_t)t + 1];
-    const size_t k0 = sb_coef_first[(size_t)f], k1 = sb_coef_first[(size_t)l];
-    size_t n = (size_t)offs[k1] - offs[k0];
-    for (int sb = f; sb < l; ++sb) n += bs.sbs[(size_t)sb].size();
-    n -= k1 - k0;  // the placeholders
-    auto ts = std::make_unique<mth::TileStores>();
-    ts->st.resize(n);
-    ts->sb_end.assign((size_t)(l - f), 0);
-    ts->cdef_at.assign((size_t)(l - f), UINT32_MAX);
-    stores[(size_t)t] = std::move(ts);
-    nstores += n;
-  }
-  ThreadGroup tracers;  // joined on every return path
-  for (int t = 0; t < ntiles; ++t) {
-    const int f = tile_first[(size_t)t];
-    for (int part = 0; part < mth::kTracers; ++part)
-      tracers.v.emplace_back(mth::trace_tile_stores, j.plan.base_q_idx, cfg->updating_cdf, &bs.sbs[(size_t)f],
-                             tile_first[(size_t)t + 1] - f, bs.cdef_points.data() + f, toks.data(), offs.data(),
-                             sb_coef_first[(size_t)f], stores[(size_t)t].get(), part);
-  }
   mt_cdef_params cp = {};
   cp.w8 = pw;
   cp.h8 = ph;
@@ -1255,25 +1008,24 @@ int job_finish(Job& j, Buffers& buf, int i) {
   cp.base_q_idx = j.plan.base_q_idx;
   cp.bd = 8;
   cp.slow = cfg->speed <= MT_SPEED_SLOW;
-  const int unit_cols = (pw + 63) / 64, unit_rows = (ph + 63) / 64;
   uint8_t* d_skip8 = buf.get<uint8_t>(i, kSkip8, (size_t)nb);
   void* d_cs = buf.get<void>(i, kCdef, mt_cdef_scratch_bytes(&cp));
   if (!d_skip8 || !d_cs) return MT_ERR_DEVICE;
   if (cudaMemsetAsync(d_skip8, 0, (size_t)nb, st) != cudaSuccess) return MT_ERR_DEVICE;
   mt_cdef_decision dec = {};
-  std::vector<uint8_t> grid((size_t)unit_cols * unit_rows);
+  const int32_t* d_bits = nullptr;
+  const uint8_t* d_grid = nullptr;
   if (j.plan.cdef) {
-    if ((rc = mt_cdef_frame_device(flt[0], flt[1], flt[2], src[0], src[1], src[2], d_skip8, &cp, d_cs, &dec,
-                                   grid.data(), st)) != MT_OK)
+    if ((rc = mth::cdef_frame_enqueue(flt[0], flt[1], flt[2], src[0], src[1], src[2], d_skip8, &cp, d_cs, decided.e,
+                                      &d_bits, &d_grid, st)) != MT_OK)
       return rc;
-    size_t cd2h = 0, ch2d = 0;
-    mth::cdef_frame_transfer_bytes(&cp, &cd2h, &ch2d);
     cs.launches(mth::cdef_last_launches);
-    cs.d2h(cd2h);
-    if (mth::cdef_last_launches == 3) cs.h2d(ch2d);
+    // the coder needs the decision, not the filtered planes
+    if (cudaStreamWaitEvent(sc, decided.e, 0) != cudaSuccess) return MT_ERR_DEVICE;
   } else {
     dec.bits = -1;
   }
+  if ((rc = mth::stream_ranges(j.sg, j.d_plan, d_tok, tot.tokens, d_bits, d_grid, sc, &nl)) != MT_OK) return rc;
   if (j.recon_out) {  // the decoder's output: deblocked and CDEF-filtered
     if (cudaMemcpyAsync(j.recon_out[0], flt[0], ny * 2, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaMemcpyAsync(j.recon_out[1], flt[1], nc * 2, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
@@ -1282,36 +1034,34 @@ int job_finish(Job& j, Buffers& buf, int i) {
       return MT_ERR_DEVICE;
     cs.d2h((ny + 2 * nc) * 2);
   }
-  // phase 2: each tile's coder over its stores, following phase 1, with each
-  // superblock's cdef_idx (its 64x64 unit's) at its read_cdef() point; tiles
-  // are coded independently, on threads of their own when there are several
-  std::vector<uint8_t> sb_idx(sb_unit.size());
-  for (size_t k2 = 0; k2 < sb_unit.size(); ++k2) sb_idx[k2] = grid[(size_t)sb_unit[k2]];
-  std::vector<uint8_t*> tiles((size_t)ntiles, nullptr);
-  std::vector<size_t> tile_lens((size_t)ntiles, 0);
-  std::vector<int> tile_rc((size_t)ntiles, MT_OK);
-  auto code = [&](int t) {
-    const int f = tile_first[(size_t)t], n = tile_first[(size_t)t + 1] - f;
-    tile_rc[(size_t)t] = mth::code_tile_stores(stores[(size_t)t].get(), n, cfg->updating_cdf,
-                                               dec.bits > 0 ? sb_idx.data() + f : nullptr, dec.bits > 0 ? dec.bits : 0,
-                                               &tiles[(size_t)t], &tile_lens[(size_t)t]);
-  };
-  if (ntiles == 1) {
-    code(0);
-  } else {
-    ThreadGroup coders;
-    for (int t = 0; t < ntiles; ++t) coders.v.emplace_back(code, t);
-    coders.join();
+  if (cudaMemcpyAsync(&tot, mth::stream_totals(j.sg, j.d_plan), sizeof(tot), cudaMemcpyDeviceToHost, sc) !=
+          cudaSuccess ||
+      cudaMemcpyAsync(tile.data(), mth::stream_tiles(j.sg, j.d_plan), tile.size() * sizeof(tile[0]),
+                      cudaMemcpyDeviceToHost, sc) != cudaSuccess ||
+      cudaStreamSynchronize(sc) != cudaSuccess)
+    return MT_ERR_DEVICE;
+  uint32_t longest = 0;
+  size_t ntok = 0;
+  for (const mth::StreamTile& t : tile) {
+    longest = std::max(longest, t.nbytes);
+    ntok += t.ntok;
   }
-  tracers.join();
-  auto free_tiles = [&]() {
-    for (uint8_t* t : tiles) free(t);
-  };
-  for (int r2 : tile_rc)
-    if (r2 != MT_OK) {
-      free_tiles();
-      return r2;
-    }
+  void* d_dig = buf.get<void>(i, kDigits, mth::stream_digit_bytes(tot));
+  if (!d_dig) return MT_ERR_DEVICE;
+  const uint8_t* d_pay =
+      mth::stream_bytes(j.sg, j.d_plan, d_tok, tot.tokens, d_dig, tot, longest, sc, &nl);
+  std::vector<uint8_t> payload(tot.bytes);
+  if (!d_pay || cudaMemcpyAsync(payload.data(), d_pay, tot.bytes, cudaMemcpyDeviceToHost, sc) != cudaSuccess ||
+      cudaStreamSynchronize(sc) != cudaSuccess)
+    return MT_ERR_DEVICE;
+  cs.launches(nl);
+  cs.d2h(sizeof(tot) + tile.size() * sizeof(tile[0]) + tot.bytes);
+  if (j.plan.cdef) {
+    if ((rc = mth::cdef_frame_decision(&cp, d_cs, &dec, nullptr, st)) != MT_OK) return rc;
+    size_t cd2h = 0, ch2d = 0;
+    mth::cdef_frame_transfer_bytes(&cp, &cd2h, &ch2d);
+    cs.d2h(cd2h - (size_t)j.sg.sb_cols * j.sg.sb_rows);
+  }
   // headers and container
   mt_sequence_header_params sp = {};
   sp.width = width;
@@ -1342,11 +1092,15 @@ int job_finish(Job& j, Buffers& buf, int i) {
     for (int q = 0; q < 4; ++q) fp.cdef_strengths[e][q] = dec.strengths[e][q];
   fp.tile_cols_log2 = j.tcl;
   fp.tile_rows_log2 = j.trl;
-  std::vector<const uint8_t*> ctiles(tiles.begin(), tiles.end());
+  std::vector<const uint8_t*> ctiles;
+  std::vector<size_t> tile_lens;
+  for (const mth::StreamTile& t : tile) {
+    ctiles.push_back(payload.data() + t.byte);
+    tile_lens.push_back(t.nbytes);
+  }
   uint8_t* obu = nullptr;
   size_t obu_len = 0;
   rc = mt_av1_stream(&sp, &fp, ctiles.data(), tile_lens.data(), ntiles, &obu, &obu_len);
-  free_tiles();
   if (rc != MT_OK) return rc;
   mt_avif_item_params ip = {};
   ip.width = width;
@@ -1371,7 +1125,7 @@ int job_finish(Job& j, Buffers& buf, int i) {
   ip.max_pic_average_light_level = cfg->max_pic_average_light_level;
   rc = mt_wrap_av1_image(obu, obu_len, &ip, j.out, j.out_len);
   free(obu);
-  if (j.stats) j.stats->tokens = (uint32_t)nstores;
+  if (j.stats) j.stats->tokens = (uint32_t)(ntok - 3 * (size_t)j.sg.sb_cols * j.sg.sb_rows);
   cs.mark(3, st);
   cs.finish();
   return rc;
@@ -1487,7 +1241,8 @@ void mt_encode_release_buffers(void) {
         cudaFree(q);
         q = nullptr;
       }
-      if (b.st) cudaStreamDestroy(b.st);
+      for (cudaStream_t s : b.st)
+        if (s) cudaStreamDestroy(s);
     }
     ar.sets.clear();
   }

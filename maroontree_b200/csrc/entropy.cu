@@ -13,14 +13,11 @@
 #include <stdlib.h>
 #include <string.h>
 
-#include <atomic>
 #include <new>
-#include <thread>
 #include <vector>
 
 #include "../../include/maroontree_b200.h"
 #include "av1_cdfs.h"
-#include "pack.h"
 
 #if defined(__SSE2__)
 #include <emmintrin.h>
@@ -690,132 +687,3 @@ int mt_replay_tile_with_filters(const mt_tile_trace* t, int32_t tile_x0, int32_t
 void mt_free(void* p) { free(p); }
 
 }  // extern "C"
-
-// ---------------------------------------------------------------------------
-// The tile packer in two phases for the encoder.  Every token is one store of
-// the range coder, and which store it is depends only on the token and the
-// adapted CDFs, never on the coder's state or on the cdef_idx literals (raw
-// bits, no CDF).  Phase 1 turns the superblocks' tokens into their stores
-// (fl, fh, nms, as the tile trace holds them) with the CDF adaptation, reading
-// the syntax tokens and the coefficient blocks they point to in place; phase 2
-// runs the coder over the stores with each superblock's cdef_idx inserted at
-// its read_cdef() point.  Phase 1 can start as soon as the tokens exist, before
-// the CDEF decision is made, and phase 2 follows it superblock by superblock
-// on another thread.  The bytes are those of mt_pack_tile_filtered over the
-// spliced token stream.
-
-namespace mth {
-
-constexpr uint32_t kCoefMarker = 0xFFFFFFFFu;
-
-// The store of one token against the live CDFs, with the CDF update; false
-// for a malformed token.
-inline bool token_store(uint32_t t, uint16_t* data, const uint32_t* off, const uint16_t* lens, size_t nslots,
-                        bool updating, uint64_t& st) {
-  const uint32_t tag = t & kTagMask;
-  if (tag == 0 || tag == kTagNoUpdate) {
-    const uint32_t slot = (t >> 8) & 0xffff, s = t & 0xff;
-    if (slot >= nslots || s >= lens[slot]) return false;
-    uint16_t* cdf = data + off[slot];
-    const uint32_t fl = s > 0 ? cdf[s - 1] : 32768u;
-    st = ((uint64_t)fl << 24) | ((uint64_t)cdf[s] << 8) | (uint64_t)(lens[slot] - s);
-    if (tag == 0 && updating) update_cdf_padded(cdf, lens[slot], (int)s);
-  } else {
-    uint32_t b, p;
-    if (tag == kTagBool) {
-      b = t & 1;
-      p = (t >> 1) & 0xffff;
-    } else {  // gathered partition bool
-      const uint32_t slot = (t >> 2) & 0xffff;
-      if (slot >= nslots || lens[slot] != 10) return false;
-      b = (t >> 1) & 1;
-      p = gather_split_prob(data + off[slot], (t & 1) != 0);
-    }
-    st = b ? (((uint64_t)p << 24) | 1u) : (((uint64_t)32768u << 24) | ((uint64_t)p << 8) | 2u);
-  }
-  return true;
-}
-
-// Which phase-1 worker codes token t: symbols and gathered bools by their
-// CDF slot's parity, raw-bit bools on worker 0.
-inline int token_part(uint32_t t) {
-  const uint32_t tag = t & kTagMask;
-  if (tag == kTagBool) return 0;
-  const uint32_t slot = tag == 0 || tag == kTagNoUpdate ? (t >> 8) & 0xffff : (t >> 2) & 0xffff;
-  return (int)(slot % (uint32_t)kTracers);
-}
-
-void trace_tile_stores(uint8_t base_q_idx, int32_t updating_cdf, const std::vector<uint32_t>* sbs, int nsb,
-                       const int32_t* cdef_point, const uint32_t* toks, const uint32_t* offs, size_t first_coef,
-                       TileStores* out, int part) {
-  const int q = base_q_idx <= 20 ? 0 : base_q_idx <= 60 ? 1 : base_q_idx <= 120 ? 2 : 3;  // qcat
-  CdfSet c;
-  build_cdfs(q, c);
-  c.data.resize(c.data.size() + kCdfPad, 0);
-  uint16_t* const data = c.data.data();
-  const uint32_t* const off = c.off.data();
-  const uint16_t* const lens = c.len.data();
-  const size_t nslots = c.off.size(), cap = out->st.size();
-  const bool upd = updating_cdf != 0;
-  uint64_t* const w = out->st.data();
-  size_t n = 0, k = first_coef;
-  for (int i = 0; i < nsb; ++i) {
-    const std::vector<uint32_t>& syn = sbs[i];
-    uint32_t at = UINT32_MAX;
-    bool ok = true;
-    for (size_t t = 0; t < syn.size() && ok; ++t) {
-      if ((int32_t)t == cdef_point[i]) at = (uint32_t)n;
-      const uint32_t tok = syn[t];
-      if (tok == kCoefMarker) {
-        const uint32_t a = offs[k], b = offs[k + 1];
-        ++k;
-        if (n + (b - a) > cap) ok = false;
-        for (uint32_t e = a; e < b && ok; ++e, ++n)
-          if (token_part(toks[e]) == part) ok = token_store(toks[e], data, off, lens, nslots, upd, w[n]);
-      } else {
-        ok = n < cap;
-        if (ok && token_part(tok) == part) ok = token_store(tok, data, off, lens, nslots, upd, w[n]);
-        ++n;
-      }
-    }
-    if (cdef_point[i] >= 0 && (size_t)cdef_point[i] == syn.size()) at = (uint32_t)n;
-    if (!ok) {
-      out->failed.store(true, std::memory_order_release);
-      out->done[part].store(nsb, std::memory_order_release);
-      return;
-    }
-    if (part == 0) {
-      out->sb_end[(size_t)i] = (uint32_t)n;
-      out->cdef_at[(size_t)i] = at;
-    }
-    out->done[part].store(i + 1, std::memory_order_release);
-  }
-}
-
-int code_tile_stores(TileStores* in, int nsb, int32_t updating_cdf, const uint8_t* cdef_idx, int32_t cdef_bits,
-                     uint8_t** payload, size_t* payload_len) {
-  mt_range_encoder enc;
-  enc.updating_cdf = updating_cdf != 0;
-  enc.precarry.reserve(in->st.size() / 2 + 64);
-  const uint64_t* const st = in->st.data();
-  size_t a = 0;
-  for (int i = 0; i < nsb; ++i) {
-    // every phase-1 worker always reaches nsb (failure included): the wait ends
-    for (int p = 0; p < kTracers; ++p)
-      while (in->done[p].load(std::memory_order_acquire) <= i) std::this_thread::yield();
-    if (in->failed.load(std::memory_order_acquire)) return MT_ERR_INVALID_INPUT;
-    const size_t b = in->sb_end[(size_t)i], p = in->cdef_at[(size_t)i];
-    if (p == UINT32_MAX || cdef_bits <= 0) {
-      enc.replay(st + a, b - a);
-    } else {
-      enc.replay(st + a, p - a);
-      enc.encode_literal(cdef_idx[i], (uint32_t)cdef_bits);
-      enc.replay(st + p, b - p);
-    }
-    a = b;
-  }
-  return out_bytes(enc.done(), payload, payload_len);
-}
-
-}  // namespace mth
-
