@@ -19,11 +19,12 @@
 // Schedule: one persistent launch of 4-CTA clusters takes the frame's 8x8
 // blocks from a ticket counter in dependency-level order (a block after its
 // left, top, top-left and, where its edges use them, top-right and
-// bottom-left neighbours inside its tile) and waits on those neighbours'
-// done counts with bounded polls.  The 13 modes of a block are split over the
+// bottom-left neighbours inside its tile) and waits for those neighbours'
+// edge records with bounded polls.  The 13 modes of a block are split over the
 // cluster's CTAs and the seven transform types over a CTA's warps, each (mode,
-// type) candidate on eight lanes; the cluster minimum picks the winner.  Frames code in the spec-minimum uniform tiling
-// (one tile up to 64 superblocks wide and 2304 in area), tiles independent.
+// type) candidate on eight lanes; the cluster minimum picks the winner.  Frames
+// code in the spec-minimum uniform tiling (one tile up to 64 superblocks wide
+// and 2304 in area), tiles independent.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -67,14 +68,14 @@ struct EncArgs {
   int32_t* lv_v;
 };
 
-// One image of a launch: its arguments, its tables and its per-block done
-// counts.
+// One image of a launch: its arguments, its tables and its blocks' edge
+// records (zero at the launch).
 struct JobDesc {
   EncArgs a;
   const mt_coef_costs* cy;
   const uint8_t* qmy;
   const uint8_t* qmc;
-  uint32_t* done;
+  uint4* edges;
 };
 
 // The z-order position of the k-th 8x8 block of a superblock and its
@@ -130,12 +131,42 @@ constexpr int kGroupBufs = 4 * kTypes + 8;  // one per candidate, and eight grou
 __device__ __forceinline__ int mode_lo(int rank) { return rank ? 3 * rank + 1 : 0; }  // 0, 4, 7, 10
 __device__ __forceinline__ int mode_rank(int m) { return m < 4 ? 0 : (m - 1) / 3; }
 
-// The next block of a cluster: its ticket (kNoTicket past an abort) and its
-// list entry.
-constexpr uint32_t kNoTicket = 0xffffffffu;
-struct NextBlock {
-  uint32_t ticket, entry, image, pad;
-};
+// What the clusters tell each other about a finished block: per block and
+// plane two 16-byte records, the bottom row and the right column as bytes, then
+// a set word and, in luma, the mode.  A record is written and read whole, so
+// seeing the set word is seeing the samples: a reader polls the record itself
+// and needs no count, no fence and no second read.
+__device__ __forceinline__ uint4* edge_rec(uint4* base, int b, int plane, int right) {
+  return base + ((size_t)b * 3 + plane) * 2 + right;
+}
+__device__ __forceinline__ void put_rec(uint4* p, uint32_t lo, uint32_t hi, uint32_t mode) {
+  const unsigned __int128 v = ((unsigned __int128)(((unsigned long long)mode << 32) | 1u) << 64) |
+                              (((unsigned long long)hi << 32) | lo);
+  asm volatile("st.relaxed.gpu.global.b128 [%0], %1;" ::"l"(p), "q"(v) : "memory");
+}
+__device__ __forceinline__ uint4 get_rec(const uint4* p) {
+  unsigned __int128 v;
+  asm volatile("ld.relaxed.gpu.global.b128 %0, [%1];" : "=q"(v) : "l"(p) : "memory");
+  return make_uint4((uint32_t)v, (uint32_t)(v >> 32), (uint32_t)(v >> 64), (uint32_t)(v >> 96));
+}
+
+// What the CTAs of a cluster write into each other's shared memory.  A warp's
+// minimum key (cost, candidate) is stored with its bytes counted by the reading
+// CTA's barrier of the block: the barrier opens when all 28 keys are there, and
+// a waiting warp is suspended meanwhile (polling the keys instead took the
+// issue slots of the warps still at work: 1080p 8.8, 4096x4096 42.8 ms).  The
+// next block and the chroma warps' marks are words with the block's sequence
+// number in them, polled by a warp per CTA that has nothing else to do: sequence
+// (24 bits), end (1), image (7), list entry (32).
+constexpr uint32_t kSeqMask = 0xffffffu;
+__device__ __forceinline__ void put_word(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.relaxed.cluster.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ unsigned long long get_word(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.cluster.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
 
 // Everything one CTA keeps in shared memory beside the groups' buffers.
 struct StepShared {
@@ -150,50 +181,131 @@ struct StepShared {
   mtd::CoopScan scan;
   mt_coef_costs cy;
   float head[4][kTypes][64];                 // coop8_rate_head of this CTA's modes, by type and end of block
-  unsigned long long key[kTypes];            // the warps' minima
-  unsigned long long ckey[2][kClusterCtas];  // the CTAs' minima, by block parity
-  alignas(16) NextBlock next[2];             // by block parity
-  uint8_t nb_mode[2];                        // modes of the blocks above and to the left
-  int cur;                                   // the image whose tables are staged (-1: none)
-  JobDesc job;                               // its descriptor
+  alignas(8) unsigned long long key[2][32];  // by block parity: the cluster's luma warps' minima
+  unsigned long long key_bar[2];             // their barriers
+  unsigned long long mark[2][2];             // by block parity: the chroma warps' marks
+  unsigned long long next[2];                // by block parity
+  uint8_t nb_mode[2];             // modes of the blocks above and to the left
+  JobDesc job;                    // the descriptor of the image whose tables are staged
 };
 
 __device__ __forceinline__ void luma_bar() { asm volatile("bar.sync 1, %0;" ::"n"(kLumaThreads) : "memory"); }
 
-__device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
-  uint32_t v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+// A wait gives up after this many polls of a record in global memory, of a word
+// or of a barrier in shared memory (the last two longer: what they wait for may
+// be waiting for a record), and sets *err; a set *err ends all of them.
+constexpr int kMaxPolls = 1 << 20, kMaxWordPolls = 1 << 23, kMaxBarPolls = 1 << 20;
+
+__device__ __forceinline__ uint4 wait_rec(const uint4* p, uint32_t* err) {
+  uint4 v = get_rec(p);
+  for (int it = 1; v.z == 0; ++it) {
+    if ((it & 15) == 0 && *(volatile uint32_t*)err) break;
+    if (it > kMaxPolls) {
+      atomicExch(err, 1u);
+      break;
+    }
+    v = get_rec(p);
+  }
   return v;
 }
-__device__ __forceinline__ void add_release(uint32_t* p) {
-  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
+
+constexpr int kLumaKeys = kClusterCtas * kTypes;
+
+// The barriers of the luma keys: one arrival (arm) and 28 keys of 8 bytes each
+// a block, two barriers taken in turn.
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void key_bar_init(unsigned long long* bar) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
+}
+__device__ __forceinline__ void key_bar_arm(unsigned long long* bar) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "n"(kLumaKeys * 8)
+               : "memory");
+}
+__device__ __forceinline__ void put_key(const unsigned long long* slot, const unsigned long long* bar, int cta,
+                                        unsigned long long key) {
+  uint32_t rs, rb;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rs) : "r"(smem_addr(slot)), "r"(cta));
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rb) : "r"(smem_addr(bar)), "r"(cta));
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.u64 [%0], %1, [%2];" ::"r"(rs), "l"(key), "r"(rb)
+               : "memory");
+}
+__device__ __forceinline__ void wait_keys(const unsigned long long* bar, uint32_t phase, uint32_t* err) {
+  for (int it = 1;; ++it) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        " selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(smem_addr(bar)), "r"(phase)
+        : "memory");
+    if (__all_sync(0xffffffffu, ok != 0)) return;
+    uint32_t ab = 0;
+    if ((it & 15) == 0) ab = *(volatile uint32_t*)err;
+    if (__any_sync(0xffffffffu, ab != 0)) return;
+    if (it > kMaxBarPolls) {
+      if ((threadIdx.x & 31) == 0) atomicExch(err, 1u);
+      return;
+    }
+  }
 }
 
-constexpr uint32_t kDonePerBlock = kClusterCtas;  // each CTA of the coding cluster publishes once
-constexpr int kMaxPolls = 1 << 20;               // a dependency wait gives up after this many polls
+// The chroma warps' marks of a block (the fetching warp; lanes 0 and 1).
+__device__ __forceinline__ void wait_marks(const unsigned long long* mark, uint32_t seq, uint32_t* err) {
+  const int lane = threadIdx.x & 31;
+  for (int it = 1; !__all_sync(0xffffffffu, lane >= 2 || (uint32_t)get_word(mark + (lane & 1)) == seq); ++it) {
+    const uint32_t ab = lane == 0 ? *(volatile uint32_t*)err : 0;
+    if (__any_sync(0xffffffffu, ab != 0)) return;
+    if (it > kMaxWordPolls) {
+      if (lane == 0) atomicExch(err, 1u);
+      return;
+    }
+    __nanosleep(200);
+  }
+}
+
+// The block of sequence number seq.  Its word comes from the cluster's
+// fetching warp, whose own waits end, so that every warp of the cluster gets
+// the same blocks and leaves at the same one.
+constexpr unsigned long long kEnd = 1ull << 39;
+__device__ __forceinline__ unsigned long long wait_next(const unsigned long long* next, uint32_t seq, uint32_t* err) {
+  unsigned long long v = get_word(next);
+  for (int it = 1; (uint32_t)(v >> 40) != (seq & kSeqMask); ++it) {
+    if (it > 8 * kMaxWordPolls) {
+      atomicExch(err, 1u);
+      return kEnd;
+    }
+    if (it > 4) __nanosleep(100);
+    v = get_word(next);
+  }
+  return v;
+}
 
 // One chroma plane of a block on the last warp: UV_DC_PRED and DCT_DCT, 8x8 in
 // 4:4:4 and 4x4 in 4:2:0.  Only the levels and the reconstruction are wanted,
 // so the chain stops after the inverse.  Every group of lanes computes the
 // block; the first one writes it.
-__device__ __forceinline__ void code_chroma(StepShared& S, mtd::GroupBuf* bufs, const EncArgs& a, int pl, int b, int px,
-                                            int py, bool has_t, bool has_l) {
+__device__ __forceinline__ void code_chroma(StepShared& S, mtd::GroupBuf* bufs, const EncArgs& a, uint4* edges, int pl,
+                                            int b, int nbx, int px, int py, bool has_t, bool has_l, uint32_t* err) {
   const int lane = threadIdx.x & 31;
   const int n = a.sub ? 4 : 8, ln = a.sub ? 2 : 3;
   const int cx = a.sub ? px / 2 : px, cy = a.sub ? py / 2 : py, stride = a.pc.stride;
   uint16_t* rec = a.rec[1 + pl] + (size_t)cy * stride + cx;
   int32_t* lv = (pl == 0 ? a.lv_u : a.lv_v) + (size_t)b * n * n;
-  int32_t s = 0;  // dc_pred_sq_at; the neighbours are read past L1 (other SMs wrote them)
-  if (lane < n) {
-    if (has_t) s = __ldcg(rec - stride + lane);
-  } else if (lane < 2 * n) {
-    if (has_l) s = __ldcg(rec + (size_t)(lane - n) * stride - 1);
+  for (int i = lane; i < n * n; i += 32) {
+    const int y = i >> ln, x = i & (n - 1);
+    S.csrc[x * n + y] = (int16_t)a.src[1 + pl][(size_t)(cy + y) * stride + cx + x];
+  }
+  uint32_t s = 0;  // dc_pred_sq_at
+  if ((lane == 0 && has_t) || (lane == 1 && has_l)) {
+    const uint4 v = wait_rec(edge_rec(edges, lane == 0 ? b - nbx : b - 1, 1 + pl, lane), err);
+    s = __dp4a(v.x, 0x01010101u, __dp4a(v.y, 0x01010101u, 0u));  // 4:2:0 leaves the upper four bytes 0
   }
   s = __reduce_add_sync(0xffffffffu, s);
-  const int32_t dc = (has_t && has_l) ? (n + s) >> (ln + 1) : ((has_t || has_l) ? ((n >> 1) + s) >> ln : 128);
+  const int32_t dc = (has_t && has_l) ? (n + (int)s) >> (ln + 1) : ((has_t || has_l) ? ((n >> 1) + (int)s) >> ln : 128);
   int32_t c[8], v[8];
   float at[8];
   int e[8];
+  uint32_t row = 0, col[2] = {0, 0};  // this lane's byte of the bottom row in its word; its column
   if (n == 8) {
     const mtd::Coop<8> g;
     mtd::GroupBuf& o = bufs[lane >> 3];
@@ -204,16 +316,16 @@ __device__ __forceinline__ void code_chroma(StepShared& S, mtd::GroupBuf* bufs, 
     mtd::coop8_fwd(MT_TX_DCT_DCT, S.ccol, nullptr, S.pc, c, at, o, g);
     mtd::coop_trellis<8>(c, at, e, S.pc, o, g);
     mtd::coop8_inv(MT_TX_DCT_DCT, c, S.pc, v, o, g);
-    if (lane < 8) {
 #pragma unroll
-      for (int k = 0; k < 8; k++) {
-        lv[k * 8 + g.j] = c[k];
-        rec[(size_t)k * stride + g.j] = (uint16_t)min(max(dc + v[k], 0), 255);
-      }
+    for (int k = 0; k < 8; k++) {
+      v[k] = min(max(dc + v[k], 0), 255);
+      col[k >> 2] |= (uint32_t)v[k] << (8 * (k & 3));
     }
+    row = (uint32_t)v[7] << (8 * (lane & 3));
   } else {
     const mtd::Coop<4> g;
     mtd::GroupBuf& o = bufs[lane >> 2];
+    __syncwarp();
 #pragma unroll
     for (int x = 0; x < 4; x++) {
       e[x] = S.scan.row4[g.j][x];
@@ -222,41 +334,75 @@ __device__ __forceinline__ void code_chroma(StepShared& S, mtd::GroupBuf* bufs, 
     mtd::coop4_fwd(v, S.pc, c, at, o, g);
     mtd::coop_trellis<4>(c, at, e, S.pc, o, g);
     mtd::coop4_inv(c, S.pc, v, o, g);
-    if (lane < 4) {
 #pragma unroll
-      for (int k = 0; k < 4; k++) {
-        lv[k * 4 + g.j] = c[k];
-        rec[(size_t)k * stride + g.j] = (uint16_t)min(max(dc + v[k], 0), 255);
-      }
+    for (int k = 0; k < 4; k++) {
+      v[k] = min(max(dc + v[k], 0), 255);
+      col[0] |= (uint32_t)v[k] << (8 * k);
     }
+    row = (uint32_t)v[3] << (8 * (lane & 3));
   }
+  row |= __shfl_xor_sync(0xffffffffu, row, 1);
+  row |= __shfl_xor_sync(0xffffffffu, row, 2);
+  const uint32_t row_hi = __shfl_sync(0xffffffffu, row, 4);
+  if (lane == 0) put_rec(edge_rec(edges, b, 1 + pl, 0), row, n == 8 ? row_hi : 0, 0);
+  if (lane == n - 1) put_rec(edge_rec(edges, b, 1 + pl, 1), col[0], col[1], 0);
+  if (lane < n) {
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      if (k < n) {
+        lv[k * n + lane] = c[k];
+        rec[(size_t)k * stride + lane] = (uint16_t)v[k];
+      }
+  }
+  __syncwarp();
+}
+
+// Writes a record's samples to an edge (index 0 the first), repeating the last
+// one over the next eight when `fill`.
+__device__ __forceinline__ void put_edge(int16_t* e, const uint4& r, bool fill) {
+#pragma unroll
+  for (int k = 0; k < 8; ++k) e[k] = (int16_t)(((k < 4 ? r.x : r.y) >> (8 * (k & 3))) & 255);
+  if (fill)
+#pragma unroll
+    for (int k = 8; k < 16; ++k) e[k] = (int16_t)(r.y >> 24);
+}
+__device__ __forceinline__ void fill_edge(int16_t* e, int v) {
+#pragma unroll
+  for (int k = 0; k < 16; ++k) e[k] = (int16_t)v;
 }
 
 // The 8x8 blocks of the frame in dependency order, coded by persistent
-// clusters (one block per cluster at a time).  A cluster takes blocks from the
-// ticket counter (CTA 0 fetches the next one while the current block is
-// evaluated, and writes it to every CTA before the cluster meets), waits until
-// the block's left, top, top-left and, where its intra edges use them,
-// top-right and bottom-left neighbours are published (done[] ==
-// kDonePerBlock), builds the intra edges once, predicts its modes (a warp each)
-// and evaluates its candidates.  The CTAs exchange their minimum keys (cost,
-// candidate index) through distributed shared memory before the one cluster
-// barrier of the block; then the lanes that hold the cluster's minimum write
-// the block out and every CTA publishes.  Keys and next blocks alternate
-// between two slots, so nothing is overwritten before all have read it.
+// clusters (one block per cluster at a time).  CTA 0's last warp takes blocks
+// from the ticket counter, one ahead of the block being evaluated, and writes
+// them to every CTA.  A block's luma warps wait for the edge records of its
+// left, top, top-left and, where its intra edges use them, top-right and
+// bottom-left neighbours, which are its intra edges; predict the CTA's modes (a
+// warp each); evaluate the candidates; and write their minimum keys (cost,
+// candidate index) to every CTA.  Every warp takes the minimum of the cluster's
+// 28 keys, and the lanes that hold it write the block's records first and the
+// block itself behind them.  The chroma warps run beside, on their own records.
+//
+// What keeps the shared buffers apart: a key is written when its warp has read
+// all it reads of the block, so a warp that has waited for all the keys may
+// overwrite the block's source, edges and predictions.  The next block's words
+// and the keys alternate between two slots: the fetching warp writes block
+// n + 2 over block n's word after the luma keys and the chroma marks of block n,
+// and a key of block n + 2 needs that word.
+//
 // Tickets follow the dependency levels, so the lowest unfinished ticket's
 // cluster has nothing left to wait for: a cluster holds a later ticket only
 // while it works on an earlier one.  A wait that runs out of polls sets *err;
-// once *err is set the remaining waits stop and every cluster leaves at its
-// next ticket.
+// once *err is set the remaining waits stop and every cluster leaves at the
+// end its fetching warp writes.
 // list[i] = block index | have-top-right (bit 30) | left-has-bottom (bit 31).
 //
-// Bound by the dependency chain: a level's latency is the wait for the
-// neighbours, the edges, the prediction, one candidate chain and the exchange.
-// Measured against octets that mixed the types of a warp and three cluster
-// barriers a block: 512x512 4:4:4 (402 levels) 7.4 -> 3.4 ms, 1080p 4:2:0 (1,148
-// levels) 24.7 -> 10.1 ms, 4096x4096 4:4:4 (2,354 levels, 111 blocks each)
-// 136.9 -> 41.3 ms.
+// Bound by the dependency chain: a level's latency is the record's way between
+// two SMs, the prediction, one candidate chain and the keys' way in the
+// cluster; with more blocks per level than clusters, by instruction latency and
+// fetch (28 % of the issue slots at 16 warps per SM).  Measured against done
+// counts (a release per CTA, the edges read behind them) and a cluster barrier
+// per block: 512x512 4:4:4 (402 levels) 3.37 -> 2.80 ms, 1080p 4:2:0 (1,148)
+// 10.05 -> 8.68, 4096x4096 4:4:4 (2,354 levels of 111 blocks) 41.3 -> 41.4.
 __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThreads, MT_ENC_CTAS_PER_SM)
     encode_blocks_kernel(const JobDesc* __restrict__ jobs, const uint2* __restrict__ list, int nlist,
                          uint32_t* ticket_ctr, uint32_t* err) {
@@ -267,181 +413,217 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThre
   const int rank = (int)cluster.block_rank();
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   if (t < 64) S.scan.stage(t);
-  if (t == 64) S.cur = -1;
-  auto fetch = [&](int slot) {  // one thread of CTA 0
-    const uint32_t tk = atomicAdd(ticket_ctr, 1u);
-    const uint32_t ab = *(volatile uint32_t*)err;
-    uint2 ent = make_uint2(0, 0);
-    if (tk < (uint32_t)nlist) ent = list[tk];
-    const uint4 v = make_uint4(ab ? kNoTicket : tk, ent.x, ent.y, 0);
-    for (int q = 0; q < kClusterCtas; ++q) *reinterpret_cast<uint4*>(cluster.map_shared_rank(&S.next[slot], q)) = v;
-  };
-  cluster.sync();  // every CTA of the cluster has started
-  if (rank == 0 && t == 0) fetch(0);
-  cluster.sync();
+  if (t < 2) {  // sequence numbers start at 1
+    S.next[t] = 0;
+    S.mark[t][0] = S.mark[t][1] = 0;
+    key_bar_init(&S.key_bar[t]);
+    key_bar_arm(&S.key_bar[t]);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  cluster.sync();  // every CTA of the cluster has its slots set
+  if (warp == kSideWarp && rank < 2) {
+    if (rank == 0) {  // the fetching warp
+      for (uint32_t seq = 1;; ++seq) {
+        if (seq > 2) {
+          wait_keys(&S.key_bar[seq & 1], ((seq - 3) >> 1) & 1, err);
+          wait_marks(S.mark[seq & 1], (seq - 2) & kSeqMask, err);
+        }
+        uint32_t stop = 0;
+        if (lane == 0) {
+          const uint32_t tk = atomicAdd(ticket_ctr, 1u);
+          stop = *(volatile uint32_t*)err != 0 || tk >= (uint32_t)nlist;
+          unsigned long long v = kEnd;
+          if (!stop) {
+            const uint2 ent = list[tk];
+            v = ((unsigned long long)ent.y << 32) | ent.x;
+          }
+          v |= (unsigned long long)(seq & kSeqMask) << 40;
+          for (int q = 0; q < kClusterCtas; ++q) put_word(cluster.map_shared_rank(&S.next[seq & 1], q), v);
+        }
+        if (__any_sync(0xffffffffu, stop != 0)) break;
+      }
+    }
+    cluster.sync();
+    return;
+  }
+  const int nthr = rank < 2 ? kLumaThreads : kStepThreads;
+  auto cta_bar = [&]() { asm volatile("bar.sync 2, %0;" ::"r"(nthr) : "memory"); };
   const EncArgs& a = S.job.a;
   const int mlo = mode_lo(rank), nm = mode_lo(rank + 1) - mlo;  // this CTA's modes
-  for (int par = 0;; par ^= 1) {
-    const NextBlock nx = S.next[par];
-    if (nx.ticket >= (uint32_t)nlist) break;  // the same for every CTA of the cluster
-    const int img = (int)nx.image;
-    if (img != S.cur) {  // another image: its descriptor, then its tables
-      __syncthreads();
+  int cur = -1;                                                 // the image whose tables are staged
+  for (uint32_t seq = 1;; ++seq) {
+    const unsigned long long nx = wait_next(&S.next[seq & 1], seq, err);
+    if (nx & kEnd) break;  // the same for every warp of the cluster
+    const int img = (int)(nx >> 32) & 127;
+    if (img != cur) {  // another image: its descriptor, then its tables
+      cta_bar();
       const int* gj = reinterpret_cast<const int*>(jobs + img);
       int* sj = reinterpret_cast<int*>(&S.job);
-      for (int i = t; i < (int)(sizeof(JobDesc) / 4); i += blockDim.x) sj[i] = gj[i];
-      __syncthreads();
+      for (int i = t; i < (int)(sizeof(JobDesc) / 4); i += nthr) sj[i] = gj[i];
+      cta_bar();
       const float* gy = reinterpret_cast<const float*>(S.job.cy);
       float* sy = reinterpret_cast<float*>(&S.cy);
-      for (int i = t; i < (int)(sizeof(mt_coef_costs) / 4); i += blockDim.x) sy[i] = gy[i];
+      for (int i = t; i < (int)(sizeof(mt_coef_costs) / 4); i += nthr) sy[i] = gy[i];
       if (t < 64) S.py.stage(t, a.qy, a.tly, a.has_qm_y ? S.job.qmy : nullptr, 64);
       else if (t < 128) S.pc.stage(t - 64, a.qc, a.tlc, a.has_qm_c ? S.job.qmc : nullptr, a.sub ? 16 : 64);
-      __syncthreads();
-      for (int i = t; i < nm * kTypes * 64; i += blockDim.x) {
+      cta_bar();
+      for (int i = t; i < nm * kTypes * 64; i += nthr) {
         const int m = i / (kTypes * 64), x = i / 64 % kTypes;
         S.head[m][x][i & 63] = mtd::coop8_rate_head(S.cy, mlo + m, x, i & 63);
       }
-      __syncthreads();
-      if (t == 0) S.cur = img;
+      cta_bar();
+      cur = img;
     }
-    uint32_t* const done = S.job.done;
+    uint4* const edges = S.job.edges;
     const int nbx = a.w8 / 8;
-    const uint32_t e = nx.entry;
-    const int b = (int)(e & 0x3fffffffu);
-    const int bx = b % nbx, by = b / nbx;
+    const uint32_t e32 = (uint32_t)nx;
+    const int b = (int)(e32 & 0x3fffffffu);
+    const int by = b / nbx, bx = b - by * nbx;
     const int px = bx * 8, py = by * 8;
-    const bool thr = (e >> 30) & 1, lhb = (e >> 31) & 1;
+    const bool thr = (e32 >> 30) & 1, lhb = (e32 >> 31) & 1;
     // the block's tile: neighbours outside it are unavailable (AV1 intra edges
     // and contexts stop at tile edges)
     const int tx0 = bx - bx % a.tile_w8, ty0 = by - by % a.tile_h8;
     const int tx1 = min(tx0 + a.tile_w8, nbx), ty1 = min(ty0 + a.tile_h8, a.h8 / 8);
     const bool has_l = bx > tx0, has_t = by > ty0;
+    if (warp == kSideWarp) {
+      code_chroma(S, bufs + 4 * kTypes, a, edges, rank - 2, b, nbx, px, py, has_t, has_l, err);
+      if (lane == 0) put_word(cluster.map_shared_rank(&S.mark[seq & 1][rank - 2], 0), seq & kSeqMask);
+      continue;
+    }
     const bool have_tr = thr && has_t && bx + 1 < tx1;
     const bool have_bl = lhb && has_l && by + 1 < ty1;
-    if (t < 5) {  // one thread per dependency
-      int dep = -1;
-      if (t == 0 && has_l) dep = b - 1;
-      if (t == 1 && has_t) dep = b - nbx;
-      if (t == 2 && has_l && has_t) dep = b - nbx - 1;
-      if (t == 3 && have_tr) dep = b - nbx + 1;
-      if (t == 4 && have_bl) dep = b + nbx - 1;
-      if (dep >= 0) {
-        for (int it = 1; ld_acquire(done + dep) < kDonePerBlock; ++it) {
-          if ((it & 15) == 0 && *(volatile uint32_t*)err) break;
-          if (it > kMaxPolls) {
-            atomicExch(err, 1u);
-            break;
+    // the intra edges with their fills (predict_sq_at), a warp per neighbour,
+    // and the source block
+    if (warp < 5) {
+      if (lane == 0) {
+        int16_t* const A = S.edge.a + 2;
+        int16_t* const L = S.edge.l + 2;
+        if (warp == 0) {
+          if (has_l) {
+            const uint4 r = wait_rec(edge_rec(edges, b - 1, 0, 1), err);
+            put_edge(L, r, !have_bl);
+            if (!has_t) {
+              fill_edge(A, (int)(r.x & 255));
+              A[-1] = L[-1] = (int16_t)(r.x & 255);
+            }
+            S.nb_mode[1] = (uint8_t)r.w;
+          } else {
+            S.nb_mode[1] = MT_DC_PRED;
+            if (!has_t) {
+              fill_edge(A, 127);
+              fill_edge(L, 129);
+              A[-1] = L[-1] = 128;
+            }
           }
+        } else if (warp == 1) {
+          if (has_t) {
+            const uint4 r = wait_rec(edge_rec(edges, b - nbx, 0, 0), err);
+            put_edge(A, r, !have_tr);
+            if (!has_l) {
+              fill_edge(L, (int)(r.x & 255));
+              A[-1] = L[-1] = (int16_t)(r.x & 255);
+            }
+            S.nb_mode[0] = (uint8_t)r.w;
+          } else {
+            S.nb_mode[0] = MT_DC_PRED;
+          }
+        } else if (warp == 2) {
+          if (has_l && has_t) {
+            const uint4 r = wait_rec(edge_rec(edges, b - nbx - 1, 0, 0), err);
+            A[-1] = L[-1] = (int16_t)(r.y >> 24);
+          }
+        } else if (warp == 3) {
+          if (have_tr) put_edge(A + 8, wait_rec(edge_rec(edges, b - nbx + 1, 0, 0), err), false);
+        } else if (have_bl) {
+          put_edge(L + 8, wait_rec(edge_rec(edges, b + nbx - 1, 0, 1), err), false);
         }
       }
-    } else if (t >= 64 && t < 128) {  // the source block, which waits for nothing
-      const int i = t - 64, y = i >> 3, x = i & 7;
-      S.src[x * 8 + y] = (int16_t)a.src[0][(size_t)(py + y) * a.py.stride + px + x];
-    } else if (rank >= 2 && warp == kSideWarp) {
-      const int n = a.sub ? 4 : 8, sh = a.sub ? 2 : 3, cx = a.sub ? px / 2 : px, cy = a.sub ? py / 2 : py;
-      for (int i = lane; i < n * n; i += 32) {
-        const int y = i >> sh, x = i & (n - 1);
-        S.csrc[x * n + y] = (int16_t)a.src[rank - 1][(size_t)(cy + y) * a.pc.stride + cx + x];
-      }
-    }
-    __syncthreads();
-    int32_t c[8], rv[8];  // a lane's levels (row j) and reconstruction (column j)
-    if (warp == kSideWarp) {
-      if (rank >= 2) code_chroma(S, bufs + 4 * kTypes, a, rank - 2, b, px, py, has_t, has_l);
-      else if (rank == 0 && lane == 0) fetch(par ^ 1);
     } else {
-      // the intra edges with their fills (predict_sq_at), read past L1 (other
-      // SMs wrote them); an available far side lies inside the frame
-      if (t < 35) {
-        const uint16_t* r = a.rec[0] + (size_t)py * a.py.stride + px;
-        const int stride = a.py.stride;
-        auto px_at = [&](int x, int y) { return (int16_t)__ldcg(r + (ptrdiff_t)y * stride + x); };
-        if (t < 16) {
-          S.edge.a[2 + t] = has_t ? px_at(have_tr ? t : min(t, 7), -1) : (has_l ? px_at(-1, 0) : (int16_t)127);
-        } else if (t < 32) {
-          const int k = t - 16;
-          S.edge.l[2 + k] = has_l ? px_at(-1, have_bl ? k : min(k, 7)) : (has_t ? px_at(0, -1) : (int16_t)129);
-        } else if (t == 32) {
-          const int16_t cn = has_l ? px_at(-1, has_t ? -1 : 0) : (has_t ? px_at(0, -1) : (int16_t)128);
-          S.edge.a[1] = S.edge.l[1] = cn;
-        } else {  // the neighbours' modes: the filter type
-          const bool have = t == 33 ? has_t : has_l;
-          S.nb_mode[t - 33] = have ? __ldcg(a.mode + (t == 33 ? b - nbx : b - 1)) : (uint8_t)MT_DC_PRED;
-        }
-      }
-      luma_bar();
-      if (warp < nm)
-        mtd::coop8_predict(mlo + warp, S.edge, has_t, has_l, is_smooth(S.nb_mode[0]) || is_smooth(S.nb_mode[1]), S.src,
-                           S.pcol[warp], S.rcol[warp], S.rrow[warp], S.pb[warp]);
-      luma_bar();
-      const mtd::Coop<8> g;
-      const int slot = lane >> 3, ms = min(slot, nm - 1), TX = warp;
-      mtd::GroupBuf& o = bufs[4 * TX + slot];
-      int e[8];
-      {
-        const uint2 w = *reinterpret_cast<const uint2*>(S.scan.row8[g.j]);
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          e[k] = (w.x >> (8 * k)) & 255;
-          e[k + 4] = (w.y >> (8 * k)) & 255;
-        }
-      }
-      float at[8];
-      mtd::coop8_fwd(TX, S.rcol[ms], S.rrow[ms], S.py, c, at, o, g);
-      const int eob = mtd::coop_trellis<8>(c, at, e, S.py, o, g);
-      mtd::coop8_inv(TX, c, S.py, rv, o, g);
-      int32_t d[8], pr[8];
-      mtd::load8(S.pcol[ms] + g.j * 8, pr);
-      mtd::load8(S.src + g.j * 8, d);
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        rv[k] = min(max(pr[k] + rv[k], 0), 255);
-        d[k] -= rv[k];
-      }
-      const uint32_t satd = mtd::coop8_satd(d, g);
-      float price = __fmul_rn(__fmul_rn(__fmul_rn((float)satd, fmaxf((float)S.py.q.ac_q, 1.0f)), 0.25f), a.py.satd_scale);
-      if (a.py.satd_bridge != 0.0f) price = __fmul_rn(price, a.py.satd_bridge);
-      const float bits = mtd::coop8_rate(c, e, eob, S.cy, S.head[ms][TX], o, g);
-      const float cost = __fadd_rn(price, __fmul_rn(a.py.mode_lambda, bits));
-      unsigned long long k = ~0ull;
-      if (g.j == 0 && slot < nm)
-        k = ((unsigned long long)__float_as_uint(cost) << 32) | (unsigned)((mlo + ms) * kTypes + TX);
-#pragma unroll
-      for (int s = 8; s < 32; s <<= 1) {
-        const unsigned long long ok = __shfl_xor_sync(0xffffffffu, k, s);
-        k = ok < k ? ok : k;
-      }
-      if (lane == 0) S.key[warp] = k;
+      const int i = t - 160, y = i >> 3, x = i & 7;
+      S.src[x * 8 + y] = (int16_t)a.src[0][(size_t)(py + y) * a.py.stride + px + x];
     }
-    __syncthreads();
-    if (t < kClusterCtas) {  // this CTA's minimum to CTA t
-      unsigned long long k = S.key[0];
+    luma_bar();
+    if (warp < nm)
+      mtd::coop8_predict(mlo + warp, S.edge, has_t, has_l, is_smooth(S.nb_mode[0]) || is_smooth(S.nb_mode[1]), S.src,
+                         S.pcol[warp], S.rcol[warp], S.rrow[warp], S.pb[warp]);
+    luma_bar();
+    const mtd::Coop<8> g;
+    const int slot = lane >> 3, ms = min(slot, nm - 1), TX = warp;
+    mtd::GroupBuf& o = bufs[4 * TX + slot];
+    int32_t c[8], rv[8];  // this lane's levels (row j) and reconstruction (column j)
+    int e[8];
+    {
+      const uint2 w = *reinterpret_cast<const uint2*>(S.scan.row8[g.j]);
 #pragma unroll
-      for (int i = 1; i < kTypes; ++i) k = S.key[i] < k ? S.key[i] : k;
-      *cluster.map_shared_rank(&S.ckey[par][rank], t) = k;
+      for (int k = 0; k < 4; k++) {
+        e[k] = (w.x >> (8 * k)) & 255;
+        e[k + 4] = (w.y >> (8 * k)) & 255;
+      }
     }
-    cluster.sync();  // the keys and the next block are everywhere
-    unsigned long long w = S.ckey[par][0];
+    float at[8];
+    mtd::coop8_fwd(TX, S.rcol[ms], S.rrow[ms], S.py, c, at, o, g);
+    const int eob = mtd::coop_trellis<8>(c, at, e, S.py, o, g);
+    mtd::coop8_inv(TX, c, S.py, rv, o, g);
+    int32_t d[8], pr[8];
+    mtd::load8(S.pcol[ms] + g.j * 8, pr);
+    mtd::load8(S.src + g.j * 8, d);
 #pragma unroll
-    for (int q = 1; q < kClusterCtas; ++q) w = S.ckey[par][q] < w ? S.ckey[par][q] : w;
-    const int wi = (int)(w & 0xffffffffu), wm = wi / kTypes;
-    if (rank == mode_rank(wm) && warp == wi % kTypes && lane >> 3 == wm - mlo) {
-      const int j = lane & 7;
+    for (int k = 0; k < 8; k++) {
+      rv[k] = min(max(pr[k] + rv[k], 0), 255);
+      d[k] -= rv[k];
+    }
+    const uint32_t satd = mtd::coop8_satd(d, g);
+    float price = __fmul_rn(__fmul_rn(__fmul_rn((float)satd, fmaxf((float)S.py.q.ac_q, 1.0f)), 0.25f), a.py.satd_scale);
+    if (a.py.satd_bridge != 0.0f) price = __fmul_rn(price, a.py.satd_bridge);
+    const float bits = mtd::coop8_rate(c, e, eob, S.cy, S.head[ms][TX], o, g);
+    const float cost = __fadd_rn(price, __fmul_rn(a.py.mode_lambda, bits));
+    unsigned long long k = ~0ull;
+    if (g.j == 0 && slot < nm)
+      k = ((unsigned long long)__float_as_uint(cost) << 32) | (unsigned)((mlo + ms) * kTypes + TX);
+#pragma unroll
+    for (int s = 8; s < 32; s <<= 1) {
+      const unsigned long long ok = __shfl_xor_sync(0xffffffffu, k, s);
+      k = ok < k ? ok : k;
+    }
+    k = __shfl_sync(0xffffffffu, k, 0);
+    if (lane < kClusterCtas) put_key(&S.key[seq & 1][rank * kTypes + warp], &S.key_bar[seq & 1], lane, k);
+    wait_keys(&S.key_bar[seq & 1], ((seq - 1) >> 1) & 1, err);
+    if (t == 0) key_bar_arm(&S.key_bar[seq & 1]);  // for block seq + 2
+    const unsigned long long all = S.key[seq & 1][lane];
+    const uint32_t cst = lane < kLumaKeys ? (uint32_t)(all >> 32) : 0xffffffffu;
+    const uint32_t low = __reduce_min_sync(0xffffffffu, cst);
+    const int wi = (int)__reduce_min_sync(0xffffffffu, cst == low && lane < kLumaKeys ? (uint32_t)all : 255u);
+    const int wm = wi / kTypes;
+    if (rank == mode_rank(wm) && warp == wi - wm * kTypes && slot == wm - mlo) {
+      const unsigned gm = 0xffu << (lane & 24);
+      const int j = g.j;
+      uint32_t row = (uint32_t)rv[7] << (8 * (j & 3)), col[2] = {0, 0};
+      row |= __shfl_xor_sync(gm, row, 1, 8);
+      row |= __shfl_xor_sync(gm, row, 2, 8);
+      const uint32_t hi = __shfl_sync(gm, row, 4, 8);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) col[q >> 2] |= (uint32_t)rv[q] << (8 * (q & 3));
+      if (j == 0) put_rec(edge_rec(edges, b, 0, 0), row, hi, (uint32_t)wm);
+      if (j == 7) put_rec(edge_rec(edges, b, 0, 1), col[0], col[1], (uint32_t)wm);
       int32_t* lv = a.lv_y + (size_t)b * 64 + j;
       uint16_t* r = a.rec[0] + (size_t)py * a.py.stride + px + j;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) r[(size_t)k * a.py.stride] = (uint16_t)rv[k];
+      for (int q = 0; q < 8; ++q) r[(size_t)q * a.py.stride] = (uint16_t)rv[q];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) lv[k * 8] = c[k];
+      for (int q = 0; q < 8; ++q) lv[q * 8] = c[q];
       if (j == 0) {
         a.mode[b] = (uint8_t)wm;
         a.tx[b] = (uint8_t)warp;
       }
     }
-    __syncthreads();  // this CTA's writes of the block are issued
-    if (t == 0) add_release(done + b);
+    __syncwarp();
   }
-  // None may leave while another CTA can still write to its shared memory.
+  // None may leave while another CTA can still write to its shared memory: the
+  // keys of the last block have been waited for, unless the waits were cut
+  // short.
+  if (*(volatile uint32_t*)err)
+    for (int i = 0; i < 32; ++i) __nanosleep(1000);
   cluster.sync();
 }
 
@@ -678,10 +860,10 @@ int job_setup(Job& j, Buffers& buf, int i) {
   sg.tcols = (sb_cols + j.tile_sb_w - 1) / j.tile_sb_w;
   sg.trows = (sb_rows + j.tile_sb_h - 1) / j.tile_sb_h;
   j.d_plan = buf.get<void>(i, kPlan, mth::stream_plan_bytes(sg));
-  uint32_t* d_done = buf.get<uint32_t>(i, kSched, (size_t)nb * 4);
+  uint4* d_edges = buf.get<uint4>(i, kSched, (size_t)nb * 6 * sizeof(uint4));
   const cudaStream_t st = j.st = buf.stream(i, 0);
   j.st_code = buf.stream(i, 1);
-  if (!d_rgbbuf || !d_planes || !d_tabs || !d_decs || !d_levels || !j.d_plan || !d_done || !st || !j.st_code)
+  if (!d_rgbbuf || !d_planes || !d_tabs || !d_decs || !d_levels || !j.d_plan || !d_edges || !st || !j.st_code)
     return MT_ERR_DEVICE;
   uint16_t* const* src = j.src;
   for (int p = 0; p < 3; ++p) {
@@ -771,9 +953,9 @@ int job_setup(Job& j, Buffers& buf, int i) {
   j.desc.cy = d_cy;
   j.desc.qmy = d_qmy;
   j.desc.qmc = d_qmc;
-  j.desc.done = d_done;
+  j.desc.edges = d_edges;
   if (cudaMemsetAsync(a.mode, 0, (size_t)nb * 2, st) != cudaSuccess ||
-      cudaMemsetAsync(d_done, 0, (size_t)nb * 4, st) != cudaSuccess)
+      cudaMemsetAsync(d_edges, 0, (size_t)nb * 6 * sizeof(uint4), st) != cudaSuccess)
     return MT_ERR_DEVICE;
   // Dependency levels of the 8x8 blocks: a block needs its left, top,
   // top-left neighbours and, where the intra edge uses them, its top-right and
