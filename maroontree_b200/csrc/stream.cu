@@ -8,17 +8,18 @@
 //      to 8x8, src/coder/superblock.rs:950-990) and the coefficient symbols
 //      (src/coeffs.rs:109-420, :583) as 16-bit tokens; hist / part_scan /
 //      scatter put the tokens of each CDF in a list of their own, in order;
-//      trace_kernel adapts every CDF along its list (update_cdf) and writes
+//      trace and fix adapt every CDF along its list (update_cdf) and write
 //      the range coder's store (fl, fh, nms) of each token at its place.
 //   3. map / compose / walk / ranges: the coder's range before every piece of
-//      256 stores; shift_scan: the bit position of every piece.
-//   4. digits_kernel: every piece's share of the code value, added into
-//      16-bit digits; bytes_kernel: the carries resolved and the bytes written.
+//      256 stores and the piece's share of the code value; shift_scan: the bit
+//      position of every piece.
+//   4. digits_kernel: the shares added into 16-bit digits; bytes_kernel: the
+//      carries resolved and the bytes written.
 //
 // What makes each step parallel.  A token's contexts depend only on the levels
 // and modes of its block and its left and top neighbours, all final, so no
 // block waits for another.  A CDF depends only on the symbols coded with it:
-// the 246 CDFs this encoder uses adapt side by side, a warp each.  The coder's
+// the 246 CDFs this encoder uses adapt side by side.  The coder's
 // state (src/odec.rs:315-615) is its 16-bit range and the code value so far.
 // The code value is a sum (each symbol adds r - u at its bit position), so
 // pieces add up in any order.  The range is a serial chain, but a symbol other
@@ -95,6 +96,8 @@ constexpr uint32_t kGathered = 16;
 
 constexpr int kScanBlock = 4096;      // counts per scan block
 constexpr int kPart = 2048;           // tokens a warp partitions
+constexpr int kSeg = 1024;            // list entries a warp adapts a CDF along,
+constexpr int kWarm = 2048;           // after this many before them
 constexpr int kChunk = 256;           // stores per piece of the range chain
 constexpr int kGroup = 64;            // pieces per group
 constexpr int kGroupTokens = kChunk * kGroup;  // tiles start at multiples of this
@@ -454,12 +457,17 @@ struct Lists {
   uint8_t* sym;     // [padded] a list entry's symbol
   uint32_t* hist;   // [padded / kPart][256]
   uint2* list;      // [tiles][256] (first entry, entries)
+  uint32_t* seg0;   // [tiles][256] segments of the tile's lists before a list
+  uint16_t* seg_a;  // [segments][16] a CDF before a segment (entry 15: updates so far, 32 at most)
+  uint16_t* seg_b;  // [segments][16] and after it
   uint16_t* map;    // [padded / kChunk][128] the range after a piece, by class before it
   uint32_t* spos;   // [padded / kChunk] first store of a piece, or kNoStart
   uint16_t* gmap;   // [groups][128]
   uint16_t* gr;     // [groups] the range before a group
   uint16_t* cr;     // [padded / kChunk] the range before a piece
   uint32_t* cd;     // [padded / kChunk] bits shifted out before a piece, in its group
+  uint32_t* nd;     // [padded / kChunk] digits of a piece
+  uint32_t* loc;    // [padded + 4 pieces] every piece's digits, its first bit at the top of a digit
   uint32_t* gd;     // [groups] bits shifted out by a group, then before it
 };
 
@@ -484,7 +492,7 @@ __global__ void __launch_bounds__(128) hist_kernel(const Lists L, const StreamTi
 
 // A CTA per tile, four threads per CDF each over a quarter of the chunks.
 __global__ void __launch_bounds__(1024) part_scan_kernel(const Lists L, const StreamTile* __restrict__ tile) {
-  __shared__ uint32_t part[4][256], first[256];
+  __shared__ uint32_t part[4][256], first[256], segs[256];
   const StreamTile ti = tile[blockIdx.x];
   const int id = threadIdx.x & 255, q = threadIdx.x >> 8;
   const int c0 = (int)(ti.base / kPart), n = (int)((ti.ntok + kPart - 1) / kPart);
@@ -497,31 +505,34 @@ __global__ void __launch_bounds__(1024) part_scan_kernel(const Lists L, const St
   if (q == 0) {
     const uint32_t total = id < kIds ? part[0][id] + part[1][id] + part[2][id] + part[3][id] : 0;
     first[id] = total;
-    __syncwarp();
+    segs[id] = (total + kSeg - 1) / kSeg;
   }
   __syncthreads();
-  if (threadIdx.x < 32) {  // exclusive scan over the CDFs, eight per lane
+  if (threadIdx.x < 64) {  // exclusive scans over the CDFs, eight per lane: entries and segments
+    uint32_t* a = threadIdx.x < 32 ? first : segs;
+    const int l = threadIdx.x & 31;
     uint32_t v[8], sum = 0;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      v[k] = first[threadIdx.x * 8 + k];
+      v[k] = a[l * 8 + k];
       sum += v[k];
     }
     uint32_t ex = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const uint32_t w = __shfl_up_sync(~0u, ex, o);
-      if ((int)threadIdx.x >= o) ex += w;
+      if (l >= o) ex += w;
     }
     ex -= sum;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      first[threadIdx.x * 8 + k] = ex;
+      a[l * 8 + k] = ex;
       ex += v[k];
     }
   }
   __syncthreads();
   uint32_t run = ti.base + first[id];
+  if (q == 1) L.seg0[blockIdx.x * 256 + id] = segs[id];
   if (q == 0)
     L.list[blockIdx.x * 256 + id] = make_uint2(run, part[0][id] + part[1][id] + part[2][id] + part[3][id]);
   for (int k = 0; k < q; ++k) run += part[k][id];
@@ -561,76 +572,204 @@ __global__ void __launch_bounds__(128) scatter_kernel(const Lists L, const Strea
 }
 
 // ---------------------------------------------------------------------------
-// update_cdf along one CDF's list (a warp per CDF and tile; lane i holds entry
-// i): entries below the symbol move up by (32768 - c) >> rate, the others down
-// by c >> rate, as c - sg * ((k + sg * c) >> rate) with (sg, k) = (-1, 32768)
-// or (1, 0).  The values before each of 32 updates go to shared memory and
-// lane k takes the k-th symbol's.  Bound by the serial chain of the longest
-// list.
-__global__ void __launch_bounds__(32) trace_kernel(const Lists L, const uint16_t* __restrict__ cdfs, int updating) {
-  __shared__ uint32_t buf[32 * 17];
-  const int id = blockIdx.x, lane = threadIdx.x;
-  const uint2 li = L.list[blockIdx.y * 256 + id];
-  if (li.y == 0) return;
-  const int n = cdfs[id * 16 + 15];  // symbols
-  int c = lane < n - 1 ? cdfs[id * 16 + lane] : 0;
-  const int rate0 = 3 + min(n >> 1, 2);
-  uint32_t done = 0;
-  uint32_t nidx = 0, nsym = 0;
-  if ((uint32_t)lane < li.y) {
-    nidx = L.idx[li.x + lane];
-    nsym = L.sym[li.x + lane];
-  }
-  for (uint32_t b = 0; b < li.y; b += 32) {
-    const uint32_t i = nidx, sym = nsym;
-    const bool live = b + lane < li.y;
-    if (b + 32 + lane < li.y) {
-      nidx = L.idx[li.x + b + 32 + lane];
-      nsym = L.sym[li.x + b + 32 + lane];
+// update_cdf along a CDF's list.  Lanes i and 16 + i of a warp hold entry i:
+// entries below the symbol move up by (32768 - c) >> rate, the others down by
+// c >> rate.  With v the distance from where the entry is moving, 32768 - c or
+// c, both are v -= v >> rate, and only a change of direction costs a third
+// operation.  The distances before each of 32 updates go to shared memory and
+// lane k takes the k-th symbol's.
+//
+// The chain along a list is serial (16 cycles a symbol, 25 with the two
+// directions computed apart), but a CDF forgets: two states that see the same
+// symbols move together by 1/128 (1/64 for short CDFs) a symbol and, being whole
+// numbers, meet.  So a long list is cut into segments of 1024, each adapted by a
+// warp of its own from the initial CDF along the 2048 symbols before it;
+// fix_kernel then compares every segment's first state with the last one of the
+// segment before and adapts again, from the true state, those that differ (2-3 %
+// of them).
+
+// 32 updates of entry c; bit k of up: the k-th moves it up.
+template <int RATE, bool STORE>
+__device__ __forceinline__ int trace_batch(int c, uint32_t up, uint32_t* buf) {
+  const int lane = threadIdx.x & 15;
+  const uint32_t last = up >> 31;
+  uint32_t turn = up ^ (up >> 1) ^ (last << 31);
+  int v = (up & 1) ? 32768 - c : c;
+#pragma unroll 1
+  for (int g = 0; g < 4; ++g) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (STORE) buf[(g * 8 + k) * 17 + lane] = (uint32_t)v;  // twice the same
+      v -= v >> RATE;
+      if ((turn >> k) & 1) v = 32768 - v;
     }
+    turn >>= 8;
+  }
+  return last ? 32768 - v : v;
+}
+
+// Entries [from, to) of the list li from state c (updates so far: done).
+template <bool STORE>
+__device__ __forceinline__ void trace_span(const Lists& L, const uint2 li, uint32_t from, uint32_t to, int n,
+                                           bool updating, uint32_t* buf, int& c, uint32_t& done) {
+  const int lane = threadIdx.x & 31, rate0 = 3 + min(n >> 1, 2);
+  // four batches of 32 at a time, the next four loaded ahead: a batch is shorter
+  // than the way to L2
+  uint32_t nidx[4], nsym[4], idx[4], syms[4];
+  auto ahead = [&](uint32_t b) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t e = b + j * 32 + lane;
+      nidx[j] = STORE && e < to ? L.idx[li.x + e] : 0;
+      nsym[j] = e < to ? L.sym[li.x + e] : 0;
+    }
+  };
+  ahead(from);
+  for (uint32_t b = from; b < to; b += 32) {
+    const uint32_t q4 = ((b - from) >> 5) & 3;
+    if (q4 == 0) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        idx[j] = nidx[j];
+        syms[j] = nsym[j];
+      }
+      ahead(b + 128);
+    }
+    const uint32_t i = q4 < 2 ? (q4 ? idx[1] : idx[0]) : (q4 == 2 ? idx[2] : idx[3]);
+    const uint32_t sym = q4 < 2 ? (q4 ? syms[1] : syms[0]) : (q4 == 2 ? syms[2] : syms[3]);
+    const bool live = b + lane < to;
     const bool upd = live && updating && sym < kGathered;
     const uint32_t um = __ballot_sync(~0u, upd);
     uint32_t mask = 0;  // bit k: symbol k is above this lane's entry
     for (int e = 0; e < n - 1; ++e) {
       const uint32_t q = __ballot_sync(~0u, (int)sym > e);
-      if (lane == e) mask = q;
+      if ((lane & 15) == e) mask = q;
     }
     if (um == ~0u && done >= 32) {
-      const int rate = rate0 + 2;
-#pragma unroll
-      for (int k = 0; k < 32; ++k) {
-        if (lane < 16) buf[k * 17 + lane] = (uint32_t)c;
-        const int bit = (mask >> k) & 1, sg = 1 - 2 * bit;
-        c -= sg * (((bit << 15) + sg * c) >> rate);
-      }
-      done += 32;
+      if (rate0 == 5) c = trace_batch<7, STORE>(c, mask, buf);
+      else c = trace_batch<6, STORE>(c, mask, buf);
     } else {
       const uint32_t ord = done + __popc(um & ((1u << lane) - 1));
       const int myrate = rate0 + (int)(min(ord, 32u) >> 4);
+#pragma unroll 1
       for (int k = 0; k < 32; ++k) {
-        if (lane < 16) buf[k * 17 + lane] = (uint32_t)c;
         const int rate = __shfl_sync(~0u, myrate, k);
-        if ((um >> k) & 1) {
-          const int bit = (mask >> k) & 1, sg = 1 - 2 * bit;
-          c -= sg * (((bit << 15) + sg * c) >> rate);
-        }
+        const bool up = (mask >> k) & 1;
+        int v = up ? 32768 - c : c;
+        if (STORE) buf[k * 17 + (lane & 15)] = (uint32_t)v;
+        if ((um >> k) & 1) v -= v >> rate;
+        c = up ? 32768 - v : v;
       }
-      done += __popc(um);
     }
+    done = min(done + __popc(um), 32u);
+    if (!STORE) continue;
     __syncwarp();
     if (live) {
       const uint32_t* row = buf + lane * 17;
       uint32_t wd;
       if (sym < kGathered) {
-        wd = store_word(sym ? row[sym - 1] : 32768u, row[sym], (uint32_t)n - sym);
+        wd = store_word(sym ? 32768 - row[sym - 1] : 32768u, row[sym], (uint32_t)n - sym);
       } else {  // gather_split_prob_icdf (src/coeffs.rs:2927-2935), the split taken
-        auto r = [&](int s) { return (int)row[s]; };
+        auto r = [&](int s) { return 32768 - (int)row[s]; };
         const int out = (sym & 1) ? (r(1) - r(4)) + r(5) + (r(8) - r(7)) : (r(0) - r(1)) + (r(2) - r(6)) + (r(7) - r(8));
         wd = store_word((uint32_t)min(max(out, 1), 32767), 0, 1);
       }
       L.st[i] = wd;
     }
     __syncwarp();
+  }
+}
+
+constexpr int kCdfEntries = 16;
+__device__ __forceinline__ size_t seg_slot(const StreamTile* tile, int t, uint32_t k) {
+  return (size_t)tile[t].base / kSeg + 256 * t + k;
+}
+
+// A warp per segment.
+__global__ void __launch_bounds__(128) trace_kernel(const Lists L, const StreamTile* __restrict__ tile, int nt,
+                                                    const uint16_t* __restrict__ cdfs, int updating) {
+  __shared__ uint32_t bufs[4][32 * 17];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t slot = blockIdx.x * 4 + w;
+  int t = 0;
+  while (t + 1 < nt && seg_slot(tile, t + 1, 0) <= slot) ++t;
+  const uint32_t k = slot - (uint32_t)seg_slot(tile, t, 0);
+  // the list: the last one with its first segment at or before k (the ids past
+  // the CDFs hold the tile's number of segments)
+  const uint32_t* seg0 = L.seg0 + t * 256;
+  if (k >= seg0[255]) return;
+  const int hi = __popc(__ballot_sync(~0u, seg0[lane * 8] <= k)) - 1;
+  const int id = hi * 8 + __popc(__ballot_sync(~0u, lane < 8 && seg0[hi * 8 + (lane & 7)] <= k)) - 1;
+  const uint32_t seg = k - seg0[id];
+  const uint2 li = L.list[t * 256 + id];
+  const int n = cdfs[id * kCdfEntries + 15];  // symbols
+  int c = (lane & 15) < n - 1 ? cdfs[id * kCdfEntries + (lane & 15)] : 0;
+  uint32_t done = 0;
+  const uint32_t from = seg * kSeg, to = min(from + kSeg, li.y);
+  if (seg) trace_span<false>(L, li, from > kWarm ? from - kWarm : 0, from, n, updating, nullptr, c, done);
+  if (lane < 16) L.seg_a[(size_t)slot * 16 + lane] = (uint16_t)(lane == 15 ? done : (uint32_t)c);
+  trace_span<true>(L, li, from, to, n, updating, bufs[w], c, done);
+  if (lane < 16) L.seg_b[(size_t)slot * 16 + lane] = (uint16_t)(lane == 15 ? done : (uint32_t)c);
+}
+
+// A CTA per list of several segments, 256 of them at a time: the segments whose
+// first state is not the last one before them, eight at once (a warp each),
+// until there are none.  The first of them is right after one turn, most of the
+// others too: a wrong state spreads only through segments in which an entry
+// rests at its limit.
+__global__ void __launch_bounds__(256) fix_kernel(const Lists L, const StreamTile* __restrict__ tile,
+                                                  const uint16_t* __restrict__ cdfs, int updating) {
+  __shared__ uint32_t bufs[8][32 * 17], bad[8];
+  const int id = blockIdx.x, t = blockIdx.y, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint2 li = L.list[t * 256 + id];
+  const uint32_t nseg = (li.y + kSeg - 1) / kSeg;
+  if (nseg < 2) return;
+  const int n = cdfs[id * kCdfEntries + 15];
+  const size_t slot = seg_slot(tile, t, L.seg0[t * 256 + id]);
+  uint16_t* const A = L.seg_a + slot * 16;
+  uint16_t* const B = L.seg_b + slot * 16;
+  for (uint32_t s0 = 1; s0 < nseg; s0 += 256) {
+    for (;;) {
+      const uint32_t s = s0 + threadIdx.x;
+      bool differs = false;
+      if (s < nseg) {
+        const uint4* a = reinterpret_cast<const uint4*>(A + s * 16);
+        const uint4* b = reinterpret_cast<const uint4*>(B + s * 16 - 16);
+        const uint4 a0 = a[0], a1 = a[1], b0 = b[0], b1 = b[1];
+        differs = ((a0.x ^ b0.x) | (a0.y ^ b0.y) | (a0.z ^ b0.z) | (a0.w ^ b0.w) | (a1.x ^ b1.x) | (a1.y ^ b1.y) |
+                   (a1.z ^ b1.z) | (a1.w ^ b1.w)) != 0;
+      }
+      const uint32_t m = __ballot_sync(~0u, differs);
+      if (lane == 0) bad[w] = m;
+      __syncthreads();
+      // this warp's segment: the w-th differing one
+      int left = w, k = -1;
+      bool any = false;
+      for (int i = 0; i < 8; ++i) {
+        uint32_t q = bad[i];
+        any = any || q;
+        const int c = __popc(q);
+        if (k < 0 && left < c) {
+          for (; left; --left) q &= q - 1;
+          k = i * 32 + __ffs(q) - 1;
+        } else if (k < 0) {
+          left -= c;
+        }
+      }
+      if (!any) break;
+      const uint32_t seg = s0 + (uint32_t)k;
+      const uint32_t v = k >= 0 ? B[(seg - 1) * 16 + (lane & 15)] : 0;
+      __syncthreads();
+      if (k >= 0) {
+        if (lane < 16) A[seg * 16 + lane] = (uint16_t)v;
+        uint32_t done = __shfl_sync(~0u, v, 15);
+        int c = (lane & 15) < n - 1 ? (int)v : 0;
+        trace_span<true>(L, li, seg * kSeg, min((seg + 1) * kSeg, li.y), n, updating, bufs[w], c, done);
+        if (lane < 16) B[seg * 16 + lane] = (uint16_t)(lane == 15 ? done : (uint32_t)c);
+      }
+      __syncthreads();
+    }
+    __syncthreads();
   }
 }
 
@@ -657,17 +796,45 @@ __device__ __forceinline__ void sub_range(uint32_t w, uint32_t r, uint32_t& l, u
   nr = u - v;
 }
 
+// N states per lane over n stores, unpacked in shared memory: (fl, fh, 4 nms -
+// 4, set without a symbol below).  Ranges are kept with their top bit at bit 31.
+template <int N>
+__device__ __forceinline__ void map_batch(uint32_t* r, const uint4* w, int n) {
+#pragma unroll 2
+  for (int k = 0; k < n; ++k) {
+    const uint4 q = w[k];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const uint32_t R = r[j] >> 24;
+      const uint32_t top = q.w ? (r[j] >> 16) - q.z : ((R * q.x) >> 1) + 4;
+      const uint32_t nr = top - ((R * q.y) >> 1);
+      r[j] = nr << __clz(nr);
+    }
+  }
+}
+
 // A warp per piece: the range after it from each of the 128 classes before
-// it, four per lane.  A piece runs from its first start store (a tile's first
-// piece from the tile's first store) to the next piece's.
+// it, at first four per lane.  Ranges meet as the stores go by (50 to 60
+// different ones of the 128 are left after 32 stores, 35 after 64, under 30
+// after 128, mostly neighbours), so between batches of 32 equal neighbours are
+// merged whenever that halves the states per lane.  A piece runs from its first
+// start store (a tile's first piece from the tile's first store) to the next
+// piece's.
 __global__ void __launch_bounds__(128) map_kernel(const Lists L, const StreamTile* __restrict__ tile, int nt) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t c = blockIdx.x * 4 + (threadIdx.x >> 5), a = c * kChunk;
+  __shared__ uint32_t sh_r[4][kClasses];
+  __shared__ uint8_t sh_i[4][kClasses];
+  __shared__ uint4 sh_w[4][32];
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const uint32_t c = blockIdx.x * 4 + wp, a = c * kChunk;
   const StreamTile ti = tile[tile_of(tile, nt, a)];
   const uint32_t end = ti.base + ti.ntok;
-  uint32_t r[4];
+  uint32_t r[4], cls[4];  // the states of this lane; where its classes' states are
 #pragma unroll
-  for (int j = 0; j < 4; ++j) r[j] = (uint32_t)(kClasses + j * 32 + lane) << 8;
+  for (int j = 0; j < 4; ++j) {
+    r[j] = (uint32_t)(kClasses + j * 32 + lane) << 24;
+    cls[j] = j * 32 + lane;
+  }
+  int per = 4, cnt = kClasses;
   bool started = false;
   for (uint32_t b = a; b < end; b += 32) {
     const uint32_t w = b + lane < end ? L.st[b + lane] : 0;
@@ -684,25 +851,56 @@ __global__ void __launch_bounds__(128) map_kernel(const Lists L, const StreamTil
     } else if (b >= a + kChunk && starts) {  // the next piece starts here
       live &= (1u << (__ffs(starts) - 1)) - 1;
     }
-    while (live) {
-      const int k = __ffs(live) - 1;
-      live &= live - 1;
-      const uint32_t q = __shfl_sync(~0u, w, k);
-      const uint32_t fl = q & 1023, fh = (q >> 10) & 1023, nms = q >> 20;
+    if ((live >> lane) & 1) {
+      const uint32_t fl = w & 1023, nms = w >> 20;
+      sh_w[wp][__popc(live & ((1u << lane) - 1))] =
+          make_uint4(fl, (w >> 10) & 1023, 4 * (nms - 1), fl == 512);
+    }
+    __syncwarp();
+    const int nw = __popc(live);
+    if (per == 4) map_batch<4>(r, sh_w[wp], nw);
+    else if (per == 2) map_batch<2>(r, sh_w[wp], nw);
+    else map_batch<1>(r, sh_w[wp], nw);
+    __syncwarp();
+    if (b >= a + kChunk && starts) break;
+    if (per > 1) {
+      uint32_t at[4];  // a state's place after merging
+      int n = 0;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const uint32_t R = r[j] >> 8;
-        const uint32_t v = ((R * fh) >> 1) + 4 * (nms - 1);
-        const uint32_t u = fl == 512 ? r[j] : ((R * fl) >> 1) + 4 * nms;
-        const uint32_t nr = u - v;
-        r[j] = nr << (__clz(nr) - 16);
+        uint32_t before = __shfl_up_sync(~0u, r[j], 1);
+        const uint32_t last = __shfl_sync(~0u, r[j ? j - 1 : 0], 31);
+        if (lane == 0) before = j ? last : 0;
+        const uint32_t m = __ballot_sync(~0u, j * 32 + lane < cnt && r[j] != before);
+        at[j] = (uint32_t)(n + __popc(m & ((2u << lane) - 1)) - 1);
+        n += __popc(m);
+      }
+      if (n <= 16 * per) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (j * 32 + lane < cnt) {  // equal states write the same value
+            sh_r[wp][at[j]] = r[j];
+            sh_i[wp][j * 32 + lane] = (uint8_t)at[j];
+          }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          cls[j] = sh_i[wp][cls[j]];
+          r[j] = sh_r[wp][min(j * 32 + lane, n - 1)];
+        }
+        __syncwarp();
+        cnt = n;
+        per = n <= 32 ? 1 : 2;
       }
     }
-    if (b >= a + kChunk && starts) break;
   }
   if (!started && lane == 0) L.spos[c] = kNoStart;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) L.map[(size_t)c * kClasses + j * 32 + lane] = started ? (uint16_t)r[j] : 0;
+  for (int j = 0; j < 4; ++j)
+    if (j < per) sh_r[wp][j * 32 + lane] = r[j] >> 16;
+  __syncwarp();
+#pragma unroll
+  for (int j = 0; j < 4; ++j) L.map[(size_t)c * kClasses + j * 32 + lane] = started ? (uint16_t)sh_r[wp][cls[j]] : 0;
 }
 
 // A group's map from its pieces' (0: the range is unchanged).
@@ -743,9 +941,10 @@ __global__ void __launch_bounds__(256) walk_kernel(const Lists L, const StreamTi
   }
 }
 
-// Runs f(l, d, r after) over the stores of piece c from its range r: one
-// thread per piece, sixteen bytes of stores at a time, the next ones loaded
-// ahead.
+// Calls f(l, d) for the stores of a piece from its range r (l = d = 0 for a word
+// that is none): one thread per piece, sixteen bytes of stores at a time, the
+// next ones loaded ahead; straight-line code, as every lane of the warp is at
+// another store.
 template <class F>
 __device__ __forceinline__ void run_piece(const uint32_t* __restrict__ st, uint32_t from, uint32_t next,
                                           uint32_t end, uint32_t r, F&& f) {
@@ -759,21 +958,25 @@ __device__ __forceinline__ void run_piece(const uint32_t* __restrict__ st, uint3
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const uint32_t i = q * 4 + k;
-      if (i >= next && is_start(w[k])) run = false;
-      if (run && i >= from && i < end && w[k]) {
-        uint32_t l, nr;
-        sub_range(w[k], r, l, nr);
-        const int d = __clz(nr) - 16;
-        r = nr << d;
-        f(l, d);
-      }
+      run = run && !(i >= next && is_start(w[k]));
+      const bool on = run && i >= from && i < end && w[k] != 0;
+      uint32_t l, nr;
+      sub_range(w[k], r, l, nr);
+      const int d = on ? __clz(nr) - 16 : 0;
+      r = on ? nr << d : r;
+      f(on ? l : 0u, d);
     }
     cur = nx;
     ++q;
   }
 }
 
-// The range before every piece of a group and the bits each piece shifts out.
+// The range before every piece of a group, the bits each piece shifts out and
+// its share of the code value: the sum of its l, each at its bit position,
+// streamed through a window of two 16-bit digits.  A piece's first l ends at
+// bit 30 of its digits (the most significant first), so that it cannot overflow
+// the first digit; n stores shift at most 15 n bits and give n + 4 digits at
+// most.
 __global__ void __launch_bounds__(kGroup) ranges_kernel(const Lists L, const StreamTile* __restrict__ tile, int nt) {
   __shared__ uint16_t m[kGroup][kClasses];
   __shared__ uint16_t rs[kGroup];
@@ -797,8 +1000,25 @@ __global__ void __launch_bounds__(kGroup) ranges_kernel(const Lists L, const Str
   const uint32_t from = L.spos[c];
   L.cr[c] = rs[t];
   uint32_t bits = 0;
-  if (from != kNoStart)
-    run_piece(L.st, from, (c + 1) * kChunk, ti.base + ti.ntok, rs[t], [&](uint32_t, int d) { bits += d; });
+  if (from != kNoStart) {
+    uint32_t* dg = L.loc + from + 4 * c;
+    uint32_t q = 1;
+    int b = 15;  // bits of digit q in the window
+    unsigned long long acc = 0;
+    run_piece(L.st, from, (c + 1) * kChunk, ti.base + ti.ntok, rs[t], [&](uint32_t l, int d) {
+      bits += d;
+      acc = (acc + l) << d;
+      b += d;
+      const bool out = b > 16;
+      if (out) dg[q - 1] = (uint32_t)(acc >> b);
+      acc = out ? acc & ((1ull << b) - 1) : acc;
+      q += out;
+      b -= out ? 16 : 0;
+    });
+    dg[q - 1] = (uint32_t)(acc >> b);
+    dg[q] = (uint32_t)(acc & ((1ull << b) - 1)) << (16 - b);
+    L.nd[c] = q + 1;
+  }
   uint32_t s = bits;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -845,38 +1065,28 @@ __global__ void __launch_bounds__(1024) shift_scan_kernel(const Lists L, const S
 }
 
 // The code value after all stores, its units bit at digit bit 15 of digit 0
-// and the payload from digit 1 on (most significant first): a store's l sits
-// with its lowest bit at bit position 30 + (bits shifted out before it).  Each
-// piece streams its sum of l through a window of two digits and adds the
-// digits that leave it.
-__global__ void __launch_bounds__(kGroup) digits_kernel(const Lists L, const StreamTile* __restrict__ tile, int nt,
-                                                        uint32_t* __restrict__ digits) {
-  const uint32_t c = blockIdx.x * kGroup + threadIdx.x;
-  const StreamTile ti = tile[tile_of(tile, nt, blockIdx.x * kGroupTokens)];
+// and the payload from digit 1 on: a warp adds each piece's digits, shifted by
+// the bits shifted out before it.
+__global__ void __launch_bounds__(128) digits_kernel(const Lists L, const StreamTile* __restrict__ tile, int nt,
+                                                     uint32_t* __restrict__ digits) {
+  const uint32_t c = blockIdx.x * 4 + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  const StreamTile ti = tile[tile_of(tile, nt, c * kChunk)];
   uint32_t* dg = digits + ti.digit;
-  if (c * kChunk == ti.base) {  // done(): the sum is rounded up before its last bits are dropped
+  if (c * kChunk == ti.base && lane == 0) {  // done(): the sum is rounded up before its last bits are dropped
     const uint32_t at = ti.shift + 30, v = 0x3FFFu << (15 - (at & 15));
     atomicAdd(&dg[at >> 4], v & 0xffff);
     atomicAdd(&dg[(at >> 4) - 1], v >> 16);
   }
   const uint32_t from = L.spos[c];
   if (from == kNoStart) return;
-  const uint32_t at = L.gd[blockIdx.x] + L.cd[c] + 30;
-  uint32_t q = at >> 4;
-  int b = (int)(at & 15) + 1;  // bits of digit q in the window
-  unsigned long long acc = 0;
-  run_piece(L.st, from, (c + 1) * kChunk, ti.base + ti.ntok, L.cr[c], [&](uint32_t l, int d) {
-    acc = (acc + l) << d;
-    b += d;
-    if (b > 16) {
-      atomicAdd(&dg[q - 1], (uint32_t)(acc >> b));
-      acc &= (1ull << b) - 1;
-      ++q;
-      b -= 16;
-    }
-  });
-  atomicAdd(&dg[q - 1], (uint32_t)(acc >> b));
-  atomicAdd(&dg[q], (uint32_t)(acc & ((1ull << b) - 1)) << (16 - b));
+  const uint32_t* loc = L.loc + from + 4 * c;
+  const uint32_t n = L.nd[c], before = L.gd[c / kGroup] + L.cd[c], sh = before & 15;
+  dg += before >> 4;
+  for (uint32_t i = lane; i <= n; i += 32) {
+    const uint32_t v = (i < n ? loc[i] >> sh : 0) + (i ? (loc[i - 1] << (16 - sh)) & 0xffff : 0);
+    if (v) atomicAdd(&dg[i], v);
+  }
 }
 
 // Two payload bytes per thread: digit i with the overflow of the digit below
@@ -949,12 +1159,18 @@ size_t carve_lists(const StreamGeom& g, uint32_t padded, void* mem, Lists* L) {
   L->sym = c.take<uint8_t>(n);
   L->hist = c.take<uint32_t>(n / kPart * 256);
   L->list = c.take<uint2>(nt * 256);
+  L->seg0 = c.take<uint32_t>(nt * 256);
+  const size_t ns = n / kSeg + 256 * nt;
+  L->seg_a = c.take<uint16_t>(ns * 16);
+  L->seg_b = c.take<uint16_t>(ns * 16);
   L->map = c.take<uint16_t>(nc * kClasses);
   L->spos = c.take<uint32_t>(nc);
   L->gmap = c.take<uint16_t>(ng * kClasses);
   L->gr = c.take<uint16_t>(ng);
   L->cr = c.take<uint16_t>(nc);
   L->cd = c.take<uint32_t>(nc);
+  L->nd = c.take<uint32_t>(nc);
+  L->loc = c.take<uint32_t>(n + 4 * nc);
   L->gd = c.take<uint32_t>(ng);
   return c.at;
 }
@@ -972,7 +1188,6 @@ void launch_units(const StreamGeom& g, const StreamInput& in, const StreamPlan& 
     units_kernel<8, false, WRITE><<<dim3(n, 2), 128, 0, st>>>(g, in, p, tokens);
 }
 
-constexpr int kCdfEntries = 16;
 uint16_t g_cdfs[8][256 * kCdfEntries];  // by quantiser context and chroma transform size
 std::once_flag g_cdfs_once;
 
@@ -1037,8 +1252,10 @@ int stream_trace(const StreamGeom& g, const StreamInput& in, void* plan, void* t
   hist_kernel<<<padded / kPart / 4, 128, 0, st>>>(L, p.tile, nt);
   part_scan_kernel<<<nt, 1024, 0, st>>>(L, p.tile);
   scatter_kernel<<<padded / kPart / 4, 128, 0, st>>>(L, p.tile, nt);
-  trace_kernel<<<dim3(kIds, nt), 32, 0, st>>>(L, static_cast<const uint16_t*>(d_cdfs), updating);
-  *launches += 6;
+  const uint16_t* cdfs = static_cast<const uint16_t*>(d_cdfs);
+  trace_kernel<<<(padded / kSeg + 256 * nt) / 4, 128, 0, st>>>(L, p.tile, nt, cdfs, updating);
+  fix_kernel<<<dim3(kIds, nt), 256, 0, st>>>(L, p.tile, cdfs, updating);
+  *launches += 7;
   return status();
 }
 
@@ -1072,7 +1289,7 @@ const uint8_t* stream_bytes(const StreamGeom& g, void* plan, void* tokens, uint3
   uint32_t* dg = static_cast<uint32_t*>(digits);
   uint8_t* out = static_cast<uint8_t*>(digits) + up256((size_t)t.digits * 4);
   if (cudaMemsetAsync(dg, 0, (size_t)t.digits * 4, st) != cudaSuccess) return nullptr;
-  digits_kernel<<<padded / kGroupTokens, kGroup, 0, st>>>(L, p.tile, nt, dg);
+  digits_kernel<<<padded / kChunk / 4, 128, 0, st>>>(L, p.tile, nt, dg);
   bytes_kernel<<<dim3((max_bytes + 511) / 512, nt), 256, 0, st>>>(p.tile, dg, out);
   *launches += 2;
   return status() == MT_OK ? out : nullptr;
