@@ -22,6 +22,7 @@
 //                        kernels, so that tables, search and apply run back to
 //                        back on the stream and the host reads the decision
 //                        once at the end.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <limits.h>
 #include <math.h>
@@ -698,7 +699,7 @@ float frame_lambda_d(int qidx, int bd, int sub_x, int sub_y, float dc_q) {
 
 // ---------------------------------------------------------------------------
 // The staged strength search (src/coder/frame_cdef.rs:116-520) on the device,
-// as a chain of small kernels on the stream (no host round trip): the unit
+// as one cluster or a chain of small kernels on the stream (no host round trip): the unit
 // statistics, the candidate list, the single-entry pass, seven greedy entry
 // passes, the assignment of the 2-, 4- and 8-entry sets to the units, the rate
 // decision and the per-unit strengths the apply kernel reads.  Integer sums
@@ -814,8 +815,7 @@ __global__ void __launch_bounds__(kSearchThreads) cdef_unit_stats_kernel(SearchA
 
 // The candidate list (one thread): Slow ranks pri 1 / 2 / 4 by their gains
 // and pairs the useful ones with sec 1 and 2; otherwise all 12.
-__global__ void cdef_plan_kernel(SearchArgs a) {
-  SearchState& S = *a.S;
+__device__ __forceinline__ void search_plan(const SearchArgs& a, SearchState& S) {
   int n = 0;
   auto push = [&](int pri, int sec) {
     S.cand[n][0] = (uint8_t)pri;
@@ -852,6 +852,7 @@ __global__ void cdef_plan_kernel(SearchArgs a) {
   S.entries[0] = 0;
   S.nentries = 1;
 }
+__global__ void cdef_plan_kernel(SearchArgs a) { search_plan(a, *a.S); }
 
 // Per (pair, chunk of units): the pair's total over the signalling units.
 // Pass 0 (the single-entry pass): its distortion.  Greedy passes: the set
@@ -876,28 +877,41 @@ __global__ void __launch_bounds__(kSearchThreads) cdef_pair_sum_kernel(SearchArg
   block_add<1>(v, dst);
 }
 
-// First minimum over the pairs of unsig_off + tot[buf][pair].
+// First minimum over the pairs of unsig_off + tot[buf][pair], by a whole warp
+// (by one thread it was most of a greedy step's 9.4 us).
 __device__ __forceinline__ int first_min(const SearchState& S, int buf, long long* best) {
   int bp = 0;
   long long bt = LLONG_MAX;
-  for (int pp = 0; pp < S.np; pp++) {
+  for (int pp = threadIdx.x & 31; pp < S.np; pp += 32) {
     const long long t = (long long)(S.unsig_off + S.tot[buf][pp]);
     if (t < bt) {
       bt = t;
       bp = pp;
     }
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const long long t = __shfl_xor_sync(0xffffffffu, bt, o);
+    const int p = __shfl_xor_sync(0xffffffffu, bp, o);
+    if (t < bt || (t == bt && p < bp)) {
+      bt = t;
+      bp = p;
+    }
+  }
   *best = bt;
   return bp;
 }
 
-// The single-entry pass's best pair (one thread).
+// The single-entry pass's best pair (one warp).
 __global__ void cdef_global_entry_kernel(SearchArgs a) {
   SearchState& S = *a.S;
   if (S.n_sig == 0) return;
   long long bt;
-  S.global_entry = first_min(S, 0, &bt);
-  S.prefix[0] = bt;
+  const int bp = first_min(S, 0, &bt);
+  if (threadIdx.x == 0) {
+    S.global_entry = bp;
+    S.prefix[0] = bt;
+  }
 }
 
 // One greedy step: every CTA finds the pass's best pair (the same one) and
@@ -908,10 +922,13 @@ __global__ void __launch_bounds__(kSearchThreads) cdef_greedy_step_kernel(Search
   if (S.n_sig == 0) return;
   __shared__ int s_best;
   __shared__ long long s_tot;
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
     long long bt;
-    s_best = first_min(S, buf, &bt);
-    s_tot = bt;
+    const int bp = first_min(S, buf, &bt);
+    if (threadIdx.x == 0) {
+      s_best = bp;
+      s_tot = bt;
+    }
   }
   __syncthreads();
   const int bp = s_best;
@@ -932,72 +949,76 @@ __global__ void __launch_bounds__(kSearchThreads) cdef_greedy_step_kernel(Search
   }
 }
 
-// The 2-, 4- and 8-entry sets' per-unit entries and totals: a unit takes the
-// smallest-magnitude entry within its margin (ties by distortion, then list
-// order), else the zero entry at CDEF off, else its best entry.
+// The 2-, 4- and 8-entry sets' entries of unit u and their distortions (dist:
+// the unit's distortion of a pair): a unit takes the smallest-magnitude entry
+// within its margin (ties by distortion, then list order), else the zero entry
+// at CDEF off, else its best entry.
+template <typename F>
+__device__ __forceinline__ void assign_unit(const SearchArgs& a, const SearchState& S, int u, bool sig, long long off,
+                                            long long thr, unsigned long long (&v)[3], F&& dist) {
+  for (int b = 1; b <= 3; b++) {
+    const int nset = 1 << b;
+    uint8_t g = 0;
+    if (!sig) {
+      v[b - 1] += (unsigned long long)off;
+    } else {
+      int z = -1;
+      for (int e = 0; e < nset; e++)
+        if (S.entries[e] == 0) {
+          z = e;
+          break;
+        }
+      bool have = false;
+      int pm = 0, pe = 0, rb_e = 0;
+      long long pd = 0, rb_d = LLONG_MAX;
+      for (int e = 0; e < nset; e++) {
+        const long long d = dist(S.entries[e]);
+        if (d < rb_d) {
+          rb_d = d;
+          rb_e = e;
+        }
+        if (d < thr) {
+          int s[4];
+          pair_strengths(S, a.mono, S.entries[e], s);
+          const int mag = s[0] + s[1] + s[2] + s[3];
+          if (!have || mag < pm || (mag == pm && d < pd)) {
+            have = true;
+            pm = mag;
+            pd = d;
+            pe = e;
+          }
+        }
+      }
+      long long t;
+      if (have) {
+        t = pd;
+        g = (uint8_t)pe;
+      } else if (z >= 0) {
+        t = off;
+        g = (uint8_t)z;
+      } else {
+        t = rb_d;
+        g = (uint8_t)rb_e;
+      }
+      v[b - 1] += (unsigned long long)t;
+    }
+    a.grids[(size_t)(b - 1) * a.nu + u] = g;
+  }
+}
+
 __global__ void __launch_bounds__(kSearchThreads) cdef_assign_kernel(SearchArgs a) {
   const SearchState& S = *a.S;
   if (S.n_sig == 0) return;
   const int u = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long v[3] = {0, 0, 0};
-  if (u < a.nu) {
-    for (int b = 1; b <= 3; b++) {
-      const int nset = 1 << b;
-      uint8_t g = 0;
-      if (!a.sig[u]) {
-        v[b - 1] = (unsigned long long)a.d_off[u];
-      } else {
-        int z = -1;
-        for (int e = 0; e < nset; e++)
-          if (S.entries[e] == 0) {
-            z = e;
-            break;
-          }
-        bool have = false;
-        int pm = 0, pe = 0, rb_e = 0;
-        long long pd = 0, rb_d = LLONG_MAX;
-        for (int e = 0; e < nset; e++) {
-          const long long d = d_pair(a, S, S.entries[e], u);
-          if (d < rb_d) {
-            rb_d = d;
-            rb_e = e;
-          }
-          if (d < a.thr[u]) {
-            int s[4];
-            pair_strengths(S, a.mono, S.entries[e], s);
-            const int mag = s[0] + s[1] + s[2] + s[3];
-            if (!have || mag < pm || (mag == pm && d < pd)) {
-              have = true;
-              pm = mag;
-              pd = d;
-              pe = e;
-            }
-          }
-        }
-        long long t;
-        if (have) {
-          t = pd;
-          g = (uint8_t)pe;
-        } else if (z >= 0) {
-          t = a.d_off[u];
-          g = (uint8_t)z;
-        } else {
-          t = rb_d;
-          g = (uint8_t)rb_e;
-        }
-        v[b - 1] = (unsigned long long)t;
-      }
-      a.grids[(size_t)(b - 1) * a.nu + u] = g;
-    }
-  }
+  if (u < a.nu) assign_unit(a, S, u, a.sig[u], a.d_off[u], a.thr[u], v, [&](int pp) { return d_pair(a, S, pp, u); });
   unsigned long long* const dst[3] = {&a.S->assign_total[1], &a.S->assign_total[2], &a.S->assign_total[3]};
   block_add<3>(v, dst);
 }
 
 // The rate decision (one thread): CDEF off, the single entry, or 2 / 4 / 8
 // entries, each priced as distortion + lambda_d x (entry bits + index bits).
-__global__ void cdef_decide_kernel(SearchArgs a) {
-  SearchState& S = *a.S;
+__device__ __forceinline__ void search_decide(const SearchArgs& a, SearchState& S) {
   S.bits = -1;
   S.n_strengths = 0;
   for (int e = 0; e < 8; e++)
@@ -1034,29 +1055,190 @@ __global__ void cdef_decide_kernel(SearchArgs a) {
   }
 }
 
+__global__ void cdef_decide_kernel(SearchArgs a) { search_decide(a, *a.S); }
+
 // Each unit's entry and strengths under the decision (all zero when CDEF is
 // off: the apply kernel then leaves the planes as they are).
-__global__ void __launch_bounds__(kSearchThreads) cdef_unit_strengths_kernel(SearchArgs a) {
-  const SearchState& S = *a.S;
-  const int u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= a.nu) return;
+__device__ __forceinline__ void unit_strengths(const SearchArgs& a, const SearchState& S, int u) {
   const int g = S.bits > 0 ? a.grids[(size_t)(S.bits - 1) * a.nu + u] : 0;
   a.grid[u] = (uint8_t)g;
 #pragma unroll
   for (int k = 0; k < 4; k++) a.ustr[(size_t)u * 4 + k] = S.bits >= 0 ? S.strengths[g][k] : 0;
 }
+__global__ void __launch_bounds__(kSearchThreads) cdef_unit_strengths_kernel(SearchArgs a) {
+  const int u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u < a.nu) unit_strengths(a, *a.S, u);
+}
 
-// The search's launches on the stream, after the tables.
+// The whole search in one launch of one cluster, for frames whose tables fit
+// in a CTA's shared memory: every CTA holds all units' distortions (by
+// candidate, the chroma planes' sums taken once), its own copy of the greedy
+// set's best and of the search state, and sums every eighth pair, a warp per
+// pair; the totals go to every CTA's memory and one cluster barrier ends a
+// pass.  CTA 0 assigns and decides.  The chain of launches is bound by its
+// launches (1080p, 510 units, 21 launches: 172 us; 150x101: 118 us).
+constexpr int kSearchCtas = 8, kClusterThreads = 512;
+constexpr size_t search_smem(int nu) { return (size_t)nu * (2 * kNCand + 3) * 8 + (size_t)nu; }
+constexpr size_t kSearchSmemMax = 200 * 1024;
+
+__global__ void __cluster_dims__(kSearchCtas, 1, 1) __launch_bounds__(kClusterThreads)
+    cdef_search_cluster_kernel(SearchArgs a) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  extern __shared__ __align__(16) unsigned char search_dyn[];
+  __shared__ SearchState S;
+  __shared__ unsigned long long sums[7];
+  __shared__ int s_best;
+  const int nu = a.nu, t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int rank = (int)cluster.block_rank();
+  long long* const lt = reinterpret_cast<long long*>(search_dyn);  // [candidate][unit]
+  long long* const uv = lt + (size_t)kNCand * nu;
+  long long* const off = uv + (size_t)kNCand * nu;
+  long long* const thr = off + nu;
+  long long* const cm = thr + nu;
+  uint8_t* const sig = reinterpret_cast<uint8_t*>(cm + nu);
+  for (int i = t; i < nu * kNCand; i += kClusterThreads) {
+    const int u = i / kNCand, k = i - u * kNCand;
+    lt[(size_t)k * nu + u] = a.ltab[i];
+    uv[(size_t)k * nu + u] = a.mono ? 0 : a.utab[i] + a.vtab[i];
+  }
+  if (t < 7) sums[t] = 0;
+  __syncthreads();
+  {
+    unsigned long long v[7] = {0, 0, 0, 0, 0, 0, 0};
+    for (int u = t; u < nu; u += kClusterThreads) {
+      const bool sg = a.dv_cnt[u] > 0;
+      const long long cnt = a.dv_cnt[u] > 1 ? a.dv_cnt[u] : 1;
+      const long long lo = lt[u], o = lo + uv[u], lim = off_of(lo);
+      off[u] = cm[u] = o;
+      thr[u] = off_of(o);
+      sig[u] = sg;
+      v[0] += sg;
+      v[1] += (long long)a.dv_sum[u] / cnt >= kGate;
+      v[2] += (unsigned long long)o;
+      v[3] += sg ? 0ull : (unsigned long long)o;
+#pragma unroll
+      for (int i = 0; i < 3; i++) {
+        const long long on = lt[(size_t)(1 + i) * nu + u];
+        v[4 + i] += on < lim ? (unsigned long long)(lo - on) : 0ull;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 7; k++) {
+      const unsigned long long s = warp_sum(v[k]);
+      if (lane == 0 && s) atomicAdd(&sums[k], s);
+    }
+  }
+  __syncthreads();
+  if (t == 0) {
+    S.n_sig = sums[0];
+    S.n_trusted = sums[1];
+    S.total_off = sums[2];
+    S.unsig_off = sums[3];
+    for (int k = 0; k < 3; k++) S.gsum[k] = sums[4 + k];
+    search_plan(a, S);
+  }
+  // every CTA has started, and its state is set
+  cluster.sync();
+  const bool any = S.n_sig != 0;  // the same in every CTA
+  for (int pass = 0; any && pass <= kGreedySteps; pass++) {
+    const int buf = pass & 1;
+    for (int pp = rank + kSearchCtas * w; pp < S.np; pp += kSearchCtas * (kClusterThreads / 32)) {
+      const long long* l = lt + (size_t)S.col[pp / S.nc] * nu;
+      const long long* c = uv + (size_t)S.col[pp % S.nc] * nu;
+      unsigned long long v = 0;
+      for (int u = lane; u < nu; u += 32) {
+        if (!sig[u]) continue;
+        const long long r = l[u] + (a.mono ? 0 : c[u]);
+        if (pass == 0) {
+          v += (unsigned long long)r;
+        } else {
+          const long long b = cm[u] < r ? cm[u] : r;
+          v += (unsigned long long)(b >= thr[u] ? off[u] : b);
+        }
+      }
+      v = __shfl_sync(0xffffffffu, warp_sum(v), 0);
+      if (lane < kSearchCtas) *cluster.map_shared_rank(&S.tot[buf][pp], lane) = v;
+    }
+    cluster.sync();
+    if (w == 0) {
+      long long bt;
+      const int bp = first_min(S, buf, &bt);
+      if (lane == 0) {
+        s_best = bp;
+        if (pass == 0) {
+          S.global_entry = bp;
+          S.prefix[0] = bt;
+        } else {
+          const int n = S.nentries + 1;
+          S.entries[n - 1] = bp;
+          S.nentries = n;
+          if ((n & (n - 1)) == 0) S.prefix[__ffs(n) - 1] = bt;
+        }
+      }
+    }
+    __syncthreads();
+    if (pass) {
+      const long long* l = lt + (size_t)S.col[s_best / S.nc] * nu;
+      const long long* c = uv + (size_t)S.col[s_best % S.nc] * nu;
+      for (int u = t; u < nu; u += kClusterThreads) {
+        const long long r = l[u] + (a.mono ? 0 : c[u]);
+        if (sig[u] && r < cm[u]) cm[u] = r;
+      }
+    }
+    __syncthreads();
+  }
+  if (rank) return;  // nobody writes to this CTA's memory any more
+  if (t < 3) sums[t] = 0;
+  __syncthreads();
+  if (any) {
+    unsigned long long v[3] = {0, 0, 0};
+    for (int u = t; u < nu; u += kClusterThreads)
+      assign_unit(a, S, u, sig[u], off[u], thr[u], v, [&](int pp) {
+        return lt[(size_t)S.col[pp / S.nc] * nu + u] + (a.mono ? 0 : uv[(size_t)S.col[pp % S.nc] * nu + u]);
+      });
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const unsigned long long s = warp_sum(v[k]);
+      if (lane == 0 && s) atomicAdd(&sums[k], s);
+    }
+  }
+  __syncthreads();
+  if (t == 0) {
+    for (int k = 0; k < 3; k++) S.assign_total[1 + k] = sums[k];
+    search_decide(a, S);
+    SearchState& out = *a.S;
+    out.bits = S.bits;
+    out.n_strengths = S.n_strengths;
+    for (int e = 0; e < 8; e++)
+      for (int k = 0; k < 4; k++) out.strengths[e][k] = S.strengths[e][k];
+  }
+  __syncthreads();
+  for (int u = t; u < nu; u += kClusterThreads) unit_strengths(a, S, u);
+}
+
+// The search's launches on the stream, after the tables: one cluster where the
+// units' tables fit in shared memory (up to 943 units), else the chain, which
+// spreads the units over the SMs.
 constexpr int kSearchLaunches = 7 + 2 * kGreedySteps;
 
-int launch_search(const SearchArgs& a, cudaStream_t st) {
+int launch_search(const SearchArgs& a, cudaStream_t st, int* launches) {
+  if (search_smem(a.nu) <= kSearchSmemMax) {
+    if (cudaFuncSetAttribute(cdef_search_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kSearchSmemMax) != cudaSuccess)
+      return MT_ERR_DEVICE;
+    cdef_search_cluster_kernel<<<kSearchCtas, kClusterThreads, search_smem(a.nu), st>>>(a);
+    *launches = 1;
+    return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_DEVICE;
+  }
+  *launches = kSearchLaunches;
   if (cudaMemsetAsync(a.S, 0, sizeof(SearchState), st) != cudaSuccess) return MT_ERR_DEVICE;
   const int ublocks = (a.nu + kSearchThreads - 1) / kSearchThreads;
   const int chunks = std::min(ublocks, 16);  // unit chunks per pair in the pass sums
   cdef_unit_stats_kernel<<<ublocks, kSearchThreads, 0, st>>>(a);
   cdef_plan_kernel<<<1, 1, 0, st>>>(a);
   cdef_pair_sum_kernel<<<dim3(chunks, kMaxPairs), kSearchThreads, 0, st>>>(a, 0);
-  cdef_global_entry_kernel<<<1, 1, 0, st>>>(a);
+  cdef_global_entry_kernel<<<1, 32, 0, st>>>(a);
   for (int k = 0; k < kGreedySteps; k++) {
     const int buf = 1 + (k & 1);
     cdef_pair_sum_kernel<<<dim3(chunks, kMaxPairs), kSearchThreads, 0, st>>>(a, buf);
@@ -1143,8 +1325,9 @@ int cdef_frame_enqueue(uint16_t* d_y, uint16_t* d_u, uint16_t* d_v, const uint16
   sa.grids = s + L.grids;
   sa.grid = s + L.grid;
   sa.ustr = s + L.ustr;
-  if ((rc = launch_search(sa, st)) != MT_OK) return rc;
-  mth::cdef_last_launches += kSearchLaunches;
+  int search_launches = 0;
+  if ((rc = launch_search(sa, st, &search_launches)) != MT_OK) return rc;
+  mth::cdef_last_launches += search_launches;
   if (d_bits) *d_bits = &sa.S->bits;
   if (d_grid) *d_grid = sa.grid;
   if (decided && cudaEventRecord(decided, st) != cudaSuccess) return MT_ERR_DEVICE;
