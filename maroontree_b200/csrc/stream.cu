@@ -97,7 +97,7 @@ constexpr uint32_t kGathered = 16;
 constexpr int kScanBlock = 4096;      // counts per scan block
 constexpr int kPart = 2048;           // tokens a warp partitions
 constexpr int kSeg = 1024;            // list entries a warp adapts a CDF along,
-constexpr int kWarm = 2048;           // after this many before them
+constexpr int kWarm = 2 * kSeg;       // after this many before them
 constexpr int kChunk = 256;           // stores per piece of the range chain
 constexpr int kGroup = 64;            // pieces per group
 constexpr int kGroupTokens = kChunk * kGroup;  // tiles start at multiples of this
@@ -460,6 +460,7 @@ struct Lists {
   uint32_t* seg0;   // [tiles][256] segments of the tile's lists before a list
   uint16_t* seg_a;  // [segments][16] a CDF before a segment (entry 15: updates so far, 32 at most)
   uint16_t* seg_b;  // [segments][16] and after it
+  uint16_t* seg_m;  // [segments] its largest symbol, and the smallest << 8
   uint16_t* map;    // [padded / kChunk][128] the range after a piece, by class before it
   uint32_t* spos;   // [padded / kChunk] first store of a piece, or kNoStart
   uint16_t* gmap;   // [groups][128]
@@ -582,11 +583,16 @@ __global__ void __launch_bounds__(128) scatter_kernel(const Lists L, const Strea
 // The chain along a list is serial (16 cycles a symbol, 25 with the two
 // directions computed apart), but a CDF forgets: two states that see the same
 // symbols move together by 1/128 (1/64 for short CDFs) a symbol and, being whole
-// numbers, meet.  So a long list is cut into segments of 1024, each adapted by a
-// warp of its own from the initial CDF along the 2048 symbols before it;
-// fix_kernel then compares every segment's first state with the last one of the
-// segment before and adapts again, from the true state, those that differ (2-3 %
-// of them).
+// numbers, meet; only an entry within 1 << rate of its end of the range rests
+// where it is until a symbol moves it away, and then comes back to just that
+// distance.  So a long list is cut into segments of 1024.  The first of each list
+// is adapted by itself; the others by a warp each, along the 2048 symbols before
+// the segment from the state after the first one, its entries at rest put at
+// that distance if a symbol has moved them since.  fix_kernel then compares every
+// segment's first state with the last one of the segment before and adapts
+// again, from the true state, those that differ (none of 659 segments at
+// 1920x1080, 1 of 2,960 in a tile of 4096x4096; from the initial CDF 16 and 66,
+// most of them in a row).
 
 // 32 updates of entry c; bit k of up: the k-th moves it up.
 template <int RATE, bool STORE>
@@ -685,28 +691,85 @@ __device__ __forceinline__ size_t seg_slot(const StreamTile* tile, int t, uint32
   return (size_t)tile[t].base / kSeg + 256 * t + k;
 }
 
-// A warp per segment.
-__global__ void __launch_bounds__(128) trace_kernel(const Lists L, const StreamTile* __restrict__ tile, int nt,
-                                                    const uint16_t* __restrict__ cdfs, int updating) {
-  __shared__ uint32_t bufs[4][32 * 17];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t slot = blockIdx.x * 4 + w;
-  int t = 0;
+// The list and segment of a warp's slot; false past the tile's segments.
+__device__ __forceinline__ bool find_segment(const Lists& L, const StreamTile* __restrict__ tile, int nt,
+                                             uint32_t slot, int& t, int& id, uint32_t& seg) {
+  const int lane = threadIdx.x & 31;
+  t = 0;
   while (t + 1 < nt && seg_slot(tile, t + 1, 0) <= slot) ++t;
   const uint32_t k = slot - (uint32_t)seg_slot(tile, t, 0);
   // the list: the last one with its first segment at or before k (the ids past
   // the CDFs hold the tile's number of segments)
   const uint32_t* seg0 = L.seg0 + t * 256;
-  if (k >= seg0[255]) return;
+  if (k >= seg0[255]) return false;
   const int hi = __popc(__ballot_sync(~0u, seg0[lane * 8] <= k)) - 1;
-  const int id = hi * 8 + __popc(__ballot_sync(~0u, lane < 8 && seg0[hi * 8 + (lane & 7)] <= k)) - 1;
-  const uint32_t seg = k - seg0[id];
+  id = hi * 8 + __popc(__ballot_sync(~0u, lane < 8 && seg0[hi * 8 + (lane & 7)] <= k)) - 1;
+  seg = k - seg0[id];
+  return true;
+}
+
+// The first segment of every list, and the symbols' extremes of the others.
+__global__ void __launch_bounds__(128) first_kernel(const Lists L, const StreamTile* __restrict__ tile, int nt,
+                                                    const uint16_t* __restrict__ cdfs, int updating) {
+  __shared__ uint32_t bufs[4][32 * 17];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t slot = blockIdx.x * 4 + w;
+  int t, id;
+  uint32_t seg;
+  if (!find_segment(L, tile, nt, slot, t, id, seg)) return;
   const uint2 li = L.list[t * 256 + id];
-  const int n = cdfs[id * kCdfEntries + 15];  // symbols
-  int c = (lane & 15) < n - 1 ? cdfs[id * kCdfEntries + (lane & 15)] : 0;
-  uint32_t done = 0;
   const uint32_t from = seg * kSeg, to = min(from + kSeg, li.y);
-  if (seg) trace_span<false>(L, li, from > kWarm ? from - kWarm : 0, from, n, updating, nullptr, c, done);
+  if (seg == 0) {
+    const int n = cdfs[id * kCdfEntries + 15];  // symbols
+    int c = (lane & 15) < n - 1 ? cdfs[id * kCdfEntries + (lane & 15)] : 0;
+    uint32_t done = 0;
+    trace_span<true>(L, li, from, to, n, updating, bufs[w], c, done);
+    if (lane < 16) L.seg_b[(size_t)slot * 16 + lane] = (uint16_t)(lane == 15 ? done : (uint32_t)c);
+  } else {
+    uint32_t hi = 0, lo = 255;
+#pragma unroll 8
+    for (uint32_t i = from + lane; i < to; i += 32) {
+      const uint32_t s = L.sym[li.x + i];
+      hi = max(hi, s < kGathered ? s : 0);
+      lo = min(lo, s);
+    }
+    hi = __reduce_max_sync(~0u, hi);
+    lo = __reduce_min_sync(~0u, lo);
+    if (lane == 0) L.seg_m[slot] = (uint16_t)(hi | (lo << 8));
+  }
+}
+
+// A warp per later segment.
+__global__ void __launch_bounds__(128) trace_kernel(const Lists L, const StreamTile* __restrict__ tile, int nt,
+                                                    const uint16_t* __restrict__ cdfs, int updating) {
+  __shared__ uint32_t bufs[4][32 * 17];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t slot = blockIdx.x * 4 + w;
+  int t, id;
+  uint32_t seg;
+  if (!find_segment(L, tile, nt, slot, t, id, seg) || seg == 0) return;
+  const uint2 li = L.list[t * 256 + id];
+  const int n = cdfs[id * kCdfEntries + 15], e = lane & 15;
+  const uint32_t start = seg > kWarm / kSeg ? seg - kWarm / kSeg : 1;  // the warm-up's first segment
+  const uint32_t first = slot - seg;
+  uint32_t hi = 0, lo = 255;
+  for (uint32_t k = 1 + lane; k < start; k += 32) {
+    const uint32_t m = L.seg_m[first + k];
+    hi = max(hi, m & 255);
+    lo = min(lo, m >> 8);
+  }
+  hi = __reduce_max_sync(~0u, hi);
+  lo = __reduce_min_sync(~0u, lo);
+  const uint32_t v = L.seg_b[(size_t)first * 16 + e];
+  uint32_t done = __shfl_sync(~0u, v, 15);
+  int c = e < n - 1 ? (int)v : 0;
+  const int rest = (1 << (5 + min(n >> 1, 2))) - 1;
+  if (e < n - 1 && updating) {
+    if (hi > (uint32_t)e && c < rest) c = rest;
+    if (lo <= (uint32_t)e && c > 32768 - rest) c = 32768 - rest;
+  }
+  const uint32_t from = seg * kSeg, to = min(from + kSeg, li.y);
+  trace_span<false>(L, li, start * kSeg, from, n, updating, nullptr, c, done);
   if (lane < 16) L.seg_a[(size_t)slot * 16 + lane] = (uint16_t)(lane == 15 ? done : (uint32_t)c);
   trace_span<true>(L, li, from, to, n, updating, bufs[w], c, done);
   if (lane < 16) L.seg_b[(size_t)slot * 16 + lane] = (uint16_t)(lane == 15 ? done : (uint32_t)c);
@@ -714,9 +777,7 @@ __global__ void __launch_bounds__(128) trace_kernel(const Lists L, const StreamT
 
 // A CTA per list of several segments, 256 of them at a time: the segments whose
 // first state is not the last one before them, eight at once (a warp each),
-// until there are none.  The first of them is right after one turn, most of the
-// others too: a wrong state spreads only through segments in which an entry
-// rests at its limit.
+// until there are none; the first of them is right after one turn.
 __global__ void __launch_bounds__(256) fix_kernel(const Lists L, const StreamTile* __restrict__ tile,
                                                   const uint16_t* __restrict__ cdfs, int updating) {
   __shared__ uint32_t bufs[8][32 * 17], bad[8];
@@ -1163,6 +1224,7 @@ size_t carve_lists(const StreamGeom& g, uint32_t padded, void* mem, Lists* L) {
   const size_t ns = n / kSeg + 256 * nt;
   L->seg_a = c.take<uint16_t>(ns * 16);
   L->seg_b = c.take<uint16_t>(ns * 16);
+  L->seg_m = c.take<uint16_t>(ns);
   L->map = c.take<uint16_t>(nc * kClasses);
   L->spos = c.take<uint32_t>(nc);
   L->gmap = c.take<uint16_t>(ng * kClasses);
@@ -1253,9 +1315,11 @@ int stream_trace(const StreamGeom& g, const StreamInput& in, void* plan, void* t
   part_scan_kernel<<<nt, 1024, 0, st>>>(L, p.tile);
   scatter_kernel<<<padded / kPart / 4, 128, 0, st>>>(L, p.tile, nt);
   const uint16_t* cdfs = static_cast<const uint16_t*>(d_cdfs);
-  trace_kernel<<<(padded / kSeg + 256 * nt) / 4, 128, 0, st>>>(L, p.tile, nt, cdfs, updating);
+  const unsigned ns = padded / kSeg + 256 * nt;
+  first_kernel<<<ns / 4, 128, 0, st>>>(L, p.tile, nt, cdfs, updating);
+  trace_kernel<<<ns / 4, 128, 0, st>>>(L, p.tile, nt, cdfs, updating);
   fix_kernel<<<dim3(kIds, nt), 256, 0, st>>>(L, p.tile, cdfs, updating);
-  *launches += 7;
+  *launches += 8;
   return status();
 }
 
