@@ -63,6 +63,7 @@ struct CoopPlane {
   int has_qm;
   mt_quant q;
   alignas(16) float zero[64];  // the suffix chain's empty second terms
+  float idt[2][256];           // IDTX targets 8 m / ac_q and 8 m / dc_q of a residual of magnitude m
 
   // Thread t of 64: qm the plane's inverse QM row (NULL: flat), n its samples.
   __device__ __forceinline__ void stage(int t, const mt_quant& quant, float lam, const uint8_t* qm, int n) {
@@ -74,6 +75,10 @@ struct CoopPlane {
     lrate[t] = __fmul_rn(lam, kCoefRateLut[t]);
     const int bin = t < 2 ? t : 32 - __clz(t), extra = bin > 1 ? bin - 2 : 0;
     lsig[t] = __fmul_rn(lam, __fadd_rn(__fmul_rn((float)bin, 0.9f), __fadd_rn((float)extra, 2.0f)));
+    for (int m = t; m < 256; m += 64) {
+      idt[0][m] = __fdiv_rn((float)(m * 8), (float)quant.ac_q);
+      idt[1][m] = __fdiv_rn((float)(m * 8), (float)quant.dc_q);
+    }
     if (t == 0) {
       lambda = lam;
       dq2 = __fmul_rn((float)quant.dc_q, (float)quant.dc_q);
@@ -188,35 +193,36 @@ __device__ __forceinline__ void coop_quant(const int32_t* v, const CoopPlane& P,
 }
 
 // Forward transform and quantisation of type TX from the residual (col / row:
-// columns and rows of eight int16).
+// columns and rows of eight int16, magnitudes below 256).  The two passes are
+// one loop, so that a warp runs the second from the instructions it has just
+// fetched: the kernel's code is larger than the instruction caches.
 __device__ __forceinline__ void coop8_fwd(int TX, const int16_t* col, const int16_t* row, const CoopPlane& P, int32_t* c,
                                           float* at, GroupBuf& o, const Coop<8>& g) {
   const int j = g.j;
   int32_t v[8];
+  load8((TX == MT_TX_IDTX || TX == MT_TX_H_DCT ? row : col) + j * 8, v);
   if (TX == MT_TX_IDTX) {
-    load8(row + j * 8, v);
 #pragma unroll
     for (int k = 0; k < 8; k++) {
       const bool dc = k == 0 && j == 0;
-      const int32_t qd = dc ? P.q.dc_q : P.q.ac_q, num = v[k] * 8;
-      at[k] = fabsf(__fdiv_rn((float)num, (float)qd));
-      const uint32_t am = (uint32_t)abs(num);
+      const int32_t qd = dc ? P.q.dc_q : P.q.ac_q;
+      const uint32_t m = (uint32_t)abs(v[k]), am = m * 8;
+      at[k] = P.idt[dc][m];
       // (am + qd / 2) / qd: exact for am + qd / 2 < 2^16 and qd < 2^12
       const int32_t level = (int32_t)__umulhi(am + (uint32_t)(qd >> 1), dc ? P.idiv[0] : P.idiv[1]);
-      c[k] = (int32_t)am < qd ? 0 : (num < 0 ? -level : level);
+      c[k] = (int32_t)am < qd ? 0 : (v[k] < 0 ? -level : level);
     }
     return;
   }
-  if (TX == MT_TX_H_DCT) {
-    load8(row + j * 8, v);
-  } else {
-    load8(col + j * 8, v);
-    if (TX == MT_TX_ADST_ADST || TX == MT_TX_ADST_DCT) fadst8(v); else fdct8(v);
-    coop_transpose<8>(v, o.t, j);
+  const bool one = TX == MT_TX_V_DCT || TX == MT_TX_H_DCT;  // one pass, quant_fullstep
+#pragma unroll 1
+  for (int pass = TX == MT_TX_H_DCT; pass < 2; pass++) {
+    const bool adst = TX == MT_TX_ADST_ADST || TX == (pass ? MT_TX_DCT_ADST : MT_TX_ADST_DCT);
+    if (adst) fadst8(v);
+    else if (!(pass && TX == MT_TX_V_DCT)) fdct8(v);
+    if (!pass) coop_transpose<8>(v, o.t, j);
   }
-  if (TX == MT_TX_ADST_ADST || TX == MT_TX_DCT_ADST) fadst8(v);
-  else if (TX != MT_TX_V_DCT) fdct8(v);
-  if (TX == MT_TX_V_DCT || TX == MT_TX_H_DCT) {  // quant_fullstep
+  if (one) {
 #pragma unroll
     for (int k = 0; k < 8; k++) {
       const int32_t p = v[k] * 2 * (k == 0 && j == 0 ? P.q.q_mult_dc : P.q.q_mult_ac), l = (abs(p) + 32768) >> 16;
@@ -361,29 +367,27 @@ __device__ __forceinline__ void coop_dequant(const int32_t* c, bool flat, const 
 }
 
 // Dequantisation + inverse transform of type TX: lane j gets column j of the
-// inverse residual.
+// inverse residual.  Both passes in one loop, as in the forward transform.
 __device__ __forceinline__ void coop8_inv(int TX, const int32_t* c, const CoopPlane& P, int32_t* v, GroupBuf& o,
                                           const Coop<8>& g) {
   const mt_quant& q = P.q;
   coop_dequant<8>(c, TX == MT_TX_IDTX || TX == MT_TX_V_DCT || TX == MT_TX_H_DCT, P, v, g.j);
-  if (TX == MT_TX_IDTX || TX == MT_TX_V_DCT) {
+#pragma unroll 1
+  for (int pass = 0; pass < 2; pass++) {  // rows, columns
+    const int32_t lo = pass ? q.cmin : q.rmin, hi = pass ? q.cmax : q.rmax;
+    if (TX == MT_TX_IDTX || TX == (pass ? MT_TX_H_DCT : MT_TX_V_DCT)) {
 #pragma unroll
-    for (int x = 0; x < 8; x++) v[x] *= 2;
-  } else if (TX == MT_TX_ADST_ADST || TX == MT_TX_DCT_ADST) {
-    iadst8s(v, 1, q.rmin, q.rmax);
-  } else {
-    idct8s(v, 1, q.rmin, q.rmax);
-  }
+      for (int x = 0; x < 8; x++) v[x] *= 2;
+    } else if (TX == MT_TX_ADST_ADST || TX == (pass ? MT_TX_ADST_DCT : MT_TX_DCT_ADST)) {
+      iadst8s(v, 1, lo, hi);
+    } else {
+      idct8s(v, 1, lo, hi);
+    }
+    if (!pass) {
 #pragma unroll
-  for (int x = 0; x < 8; x++) v[x] = clampi((v[x] + 1) >> 1, q.cmin, q.cmax);
-  coop_transpose<8>(v, o.t, g.j);
-  if (TX == MT_TX_IDTX || TX == MT_TX_H_DCT) {
-#pragma unroll
-    for (int y = 0; y < 8; y++) v[y] *= 2;
-  } else if (TX == MT_TX_ADST_ADST || TX == MT_TX_ADST_DCT) {
-    iadst8s(v, 1, q.cmin, q.cmax);
-  } else {
-    idct8s(v, 1, q.cmin, q.cmax);
+      for (int x = 0; x < 8; x++) v[x] = clampi((v[x] + 1) >> 1, q.cmin, q.cmax);
+      coop_transpose<8>(v, o.t, g.j);
+    }
   }
 #pragma unroll
   for (int y = 0; y < 8; y++) v[y] = (v[y] + 8) >> 4;

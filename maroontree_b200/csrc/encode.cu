@@ -353,13 +353,19 @@ __device__ __forceinline__ unsigned long long wait_next(const unsigned long long
 // 4:4:4 and 4x4 in 4:2:0.  Only the levels and the reconstruction are wanted,
 // so the chain stops after the inverse.  Every group of lanes computes the
 // block; the first one writes it.
-__device__ __forceinline__ void code_chroma(StepShared& S, mtd::GroupBuf* bufs, const EncArgs& a, uint4* edges, int pl,
-                                            int b, int nbx, int px, int py, bool has_t, bool has_l, uint32_t* err) {
+struct ChromaBlock {
+  uint16_t* rec;
+  int32_t* lv;
+  int stride, n;
+  int32_t dc;
+};
+
+// The source and the DC prediction.
+__device__ __forceinline__ ChromaBlock chroma_start(StepShared& S, const EncArgs& a, uint4* edges, int pl, int b,
+                                                    int nbx, int px, int py, bool has_t, bool has_l, uint32_t* err) {
   const int lane = threadIdx.x & 31;
   const int n = a.sub ? 4 : 8, ln = a.sub ? 2 : 3;
   const int cx = a.sub ? px / 2 : px, cy = a.sub ? py / 2 : py, stride = a.pc.stride;
-  uint16_t* rec = a.rec[1 + pl] + (size_t)cy * stride + cx;
-  int32_t* lv = (pl == 0 ? a.lv_u : a.lv_v) + (size_t)b * n * n;
   for (int i = lane; i < n * n; i += 32) {
     const int y = i >> ln, x = i & (n - 1);
     S.csrc[x * n + y] = (int16_t)a.src[1 + pl][(size_t)(cy + y) * stride + cx + x];
@@ -370,74 +376,40 @@ __device__ __forceinline__ void code_chroma(StepShared& S, mtd::GroupBuf* bufs, 
     s = __dp4a(v.x, 0x01010101u, __dp4a(v.y, 0x01010101u, 0u));  // 4:2:0 leaves the upper four bytes 0
   }
   s = __reduce_add_sync(0xffffffffu, s);
-  const int32_t dc = (has_t && has_l) ? (n + (int)s) >> (ln + 1) : ((has_t || has_l) ? ((n >> 1) + (int)s) >> ln : 128);
-  int32_t c[8], v[8];
-  float at[8];
-  int e[8];
-  uint32_t row = 0, col[2] = {0, 0};  // this lane's byte of the bottom row in its word; its column
-  if (n == 8) {
-    const mtd::Coop<8> g;
-    mtd::GroupBuf& o = bufs[lane >> 3];
-    for (int i = lane; i < 64; i += 32) S.ccol[i] = (int16_t)(S.csrc[i] - dc);
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < 8; k++) e[k] = S.scan.row8[g.j][k];
-    mtd::coop8_fwd(MT_TX_DCT_DCT, S.ccol, nullptr, S.pc, c, at, o, g);
-    mtd::coop_trellis<8>(c, at, e, S.pc, o, g);
-    mtd::coop8_inv(MT_TX_DCT_DCT, c, S.pc, v, o, g);
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      v[k] = min(max(dc + v[k], 0), 255);
-      col[k >> 2] |= (uint32_t)v[k] << (8 * (k & 3));
-    }
-    row = (uint32_t)v[7] << (8 * (lane & 3));
-  } else {
-    const mtd::Coop<4> g;
-    mtd::GroupBuf& o = bufs[lane >> 2];
-    __syncwarp();
-#pragma unroll
-    for (int x = 0; x < 4; x++) {
-      e[x] = S.scan.row4[g.j][x];
-      v[x] = S.csrc[g.j * 4 + x] - dc;
-    }
-    mtd::coop4_fwd(v, S.pc, c, at, o, g);
-    mtd::coop_trellis<4>(c, at, e, S.pc, o, g);
-    mtd::coop4_inv(c, S.pc, v, o, g);
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      v[k] = min(max(dc + v[k], 0), 255);
-      col[0] |= (uint32_t)v[k] << (8 * k);
-    }
-    row = (uint32_t)v[3] << (8 * (lane & 3));
-  }
-  row |= __shfl_xor_sync(0xffffffffu, row, 1);
-  row |= __shfl_xor_sync(0xffffffffu, row, 2);
-  const uint32_t row_hi = __shfl_sync(0xffffffffu, row, 4);
-  if (lane == 0) put_rec(edge_rec(edges, b, 1 + pl, 0), row, n == 8 ? row_hi : 0, 0);
-  if (lane == n - 1) put_rec(edge_rec(edges, b, 1 + pl, 1), col[0], col[1], 0);
-  if (lane < n) {
-#pragma unroll
-    for (int k = 0; k < 8; k++)
-      if (k < n) {
-        lv[k * n + lane] = c[k];
-        rec[(size_t)k * stride + lane] = (uint16_t)v[k];
-      }
-  }
-  __syncwarp();
+  ChromaBlock k;
+  k.rec = a.rec[1 + pl] + (size_t)cy * stride + cx;
+  k.lv = (pl == 0 ? a.lv_u : a.lv_v) + (size_t)b * n * n;
+  k.stride = stride;
+  k.n = n;
+  k.dc = (has_t && has_l) ? (n + (int)s) >> (ln + 1) : ((has_t || has_l) ? ((n >> 1) + (int)s) >> ln : 128);
+  return k;
 }
 
-// Writes a record's samples to an edge (index 0 the first), repeating the last
-// one over the next eight when `fill`.
-__device__ __forceinline__ void put_edge(int16_t* e, const uint4& r, bool fill) {
+// The reconstruction from the inverse's columns v, the records, the block.
+template <int N>
+__device__ __forceinline__ void chroma_finish(const ChromaBlock& k, uint4* edges, int pl, int b, const int32_t* c,
+                                              int32_t* v) {
+  const int lane = threadIdx.x & 31;
+  uint32_t col[2] = {0, 0};
 #pragma unroll
-  for (int k = 0; k < 8; ++k) e[k] = (int16_t)(((k < 4 ? r.x : r.y) >> (8 * (k & 3))) & 255);
-  if (fill)
+  for (int y = 0; y < N; y++) {
+    v[y] = min(max(k.dc + v[y], 0), 255);
+    col[y >> 2] |= (uint32_t)v[y] << (8 * (y & 3));
+  }
+  uint32_t row = (uint32_t)v[N - 1] << (8 * (lane & 3));
+  row |= __shfl_xor_sync(0xffffffffu, row, 1);
+  row |= __shfl_xor_sync(0xffffffffu, row, 2);
+  const uint32_t hi = N == 8 ? __shfl_sync(0xffffffffu, row, 4) : 0;
+  if (lane == 0) put_rec(edge_rec(edges, b, 1 + pl, 0), row, hi, 0);
+  if (lane == N - 1) put_rec(edge_rec(edges, b, 1 + pl, 1), col[0], col[1], 0);
+  if (lane < N) {
 #pragma unroll
-    for (int k = 8; k < 16; ++k) e[k] = (int16_t)(r.y >> 24);
-}
-__device__ __forceinline__ void fill_edge(int16_t* e, int v) {
-#pragma unroll
-  for (int k = 0; k < 16; ++k) e[k] = (int16_t)v;
+    for (int y = 0; y < N; y++) {
+      k.lv[y * N + lane] = c[y];
+      k.rec[(size_t)y * k.stride + lane] = (uint16_t)v[y];
+    }
+  }
+  __syncwarp();
 }
 
 // The 8x8 blocks of the frame in dependency order, coded by persistent
@@ -468,10 +440,13 @@ __device__ __forceinline__ void fill_edge(int16_t* e, int v) {
 // Bound by the dependency chain: a level's latency is the record's way between
 // two SMs, the prediction, one candidate chain and the keys' way in the
 // cluster; with more blocks per level than clusters, by instruction latency and
-// fetch (28 % of the issue slots at 16 warps per SM).  Measured against done
-// counts (a release per CTA, the edges read behind them) and a cluster barrier
-// per block: 512x512 4:4:4 (402 levels) 3.37 -> 2.80 ms, 1080p 4:2:0 (1,148)
-// 10.05 -> 8.68, 4096x4096 4:4:4 (2,354 levels of 111 blocks) 41.3 -> 41.4.
+// fetch.  Measured against done counts (a release per CTA, the edges read behind
+// them) and a cluster barrier per block: 512x512 4:4:4 (402 levels) 3.37 -> 2.80
+// ms, 1080p 4:2:0 (1,148) 10.05 -> 8.68; with late tickets 2.70 and 8.53.  The
+// kernel's code is kept small (118 KB; 153 KB with chroma's own copy of the chain,
+// both passes of the transforms written out and a poll and an edge writer per
+// neighbour): 4096x4096 4:4:4 (2,354 levels of 111 blocks) 41.4 -> 31.7 ms, 1080p
+// 8.53 -> 8.04.  Three CTAs per SM (80 registers) were slower at 153 KB: 44.3 ms.
 __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThreads, MT_ENC_CTAS_PER_SM)
     encode_blocks_kernel(const JobDesc* __restrict__ jobs, const uint2* __restrict__ list, int nlist,
                          uint32_t* ticket_ctr, uint32_t* err, int late) {
@@ -553,70 +528,81 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThre
     // neighbours outside the block's tile are unavailable (AV1 intra edges and
     // contexts stop at tile edges)
     const bool has_l = ent & kHasL, has_t = ent & kHasT, have_tr = ent & kHasTr, have_bl = ent & kHasBl;
-    if (warp == kSideWarp) {
-      code_chroma(S, bufs + 4 * kTypes, a, edges, rank - 2, b, nbx, px, py, has_t, has_l, err);
+    const bool chroma = warp == kSideWarp;
+    auto chroma_done = [&]() {
       if (lane == 0) put_word(cluster.map_shared_rank(&S.mark[seq & 1][rank - 2], 0), seq & kSeqMask);
-      continue;
+    };
+    ChromaBlock cb;
+    if (chroma) {
+      cb = chroma_start(S, a, edges, rank - 2, b, nbx, px, py, has_t, has_l, err);
+      __syncwarp();
+      if (a.sub) {
+        const mtd::Coop<4> g;
+        mtd::GroupBuf& o = bufs[4 * kTypes + (lane >> 2)];
+        int32_t c[4], v[4];
+        float at[4];
+        int e[4];
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+          e[x] = S.scan.row4[g.j][x];
+          v[x] = S.csrc[g.j * 4 + x] - cb.dc;
+        }
+        mtd::coop4_fwd(v, S.pc, c, at, o, g);
+        mtd::coop_trellis<4>(c, at, e, S.pc, o, g);
+        mtd::coop4_inv(c, S.pc, v, o, g);
+        chroma_finish<4>(cb, edges, rank - 2, b, c, v);
+        chroma_done();
+        continue;
+      }
+      for (int i = lane; i < 64; i += 32) S.ccol[i] = (int16_t)(S.csrc[i] - cb.dc);
+      __syncwarp();
     }
-    // the intra edges with their fills (predict_sq_at), a warp per neighbour,
-    // and the source block
-    if (warp < 5) {
-      if (lane == 0) {
+    if (!chroma) {
+      // the intra edges with their fills (predict_sq_at), a warp per neighbour
+      // (left, top, top-left, top-right, bottom-left), a lane per sample, and the
+      // source block
+      if (warp < 5) {
         int16_t* const A = S.edge.a + 2;
         int16_t* const L = S.edge.l + 2;
-        if (warp == 0) {
-          if (has_l) {
-            const uint4 r = wait_rec(edge_rec(edges, b - 1, 0, 1), err);
-            put_edge(L, r, !have_bl);
-            if (!has_t) {
-              fill_edge(A, (int)(r.x & 255));
-              A[-1] = L[-1] = (int16_t)(r.x & 255);
-            }
-            S.nb_mode[1] = (uint8_t)r.w;
+        const bool up = warp == 1 || warp == 3;  // a row of the above edge, else a column of the left one
+        int16_t* const e = (up ? A : L) + (warp > 2 ? 8 : 0);
+        const bool have = warp == 0 ? has_l : (warp == 1 ? has_t : (warp == 2 ? has_l && has_t : (up ? have_tr : have_bl)));
+        const int from = b + (warp == 1 ? -nbx : (warp == 2 ? -nbx - 1 : (warp == 3 ? 1 - nbx : (warp == 4 ? nbx - 1 : -1))));
+        if (have) {
+          const uint4 r = wait_rec(edge_rec(edges, from, 0, !(up || warp == 2)), err);
+          const int k = min(lane, 7);  // an unavailable far side repeats the last sample
+          const int16_t v = (int16_t)(((k < 4 ? r.x : r.y) >> (8 * (k & 3))) & 255);
+          if (warp == 2) {
+            if (lane == 7) A[-1] = L[-1] = v;
           } else {
-            S.nb_mode[1] = MT_DC_PRED;
-            if (!has_t) {
-              fill_edge(A, 127);
-              fill_edge(L, 129);
-              A[-1] = L[-1] = 128;
+            if (lane < (warp < 2 && !(up ? have_tr : have_bl) ? 16 : 8)) e[lane] = v;
+            if (warp < 2) {
+              if (!(up ? has_l : has_t)) {  // the other side repeats this one's first sample
+                if (lane < 17) (up ? L : A)[lane - 1] = (int16_t)(r.x & 255);
+                if (lane == 0) e[-1] = v;
+              }
+              if (lane == 0) S.nb_mode[1 - warp] = (uint8_t)r.w;
             }
           }
-        } else if (warp == 1) {
-          if (has_t) {
-            const uint4 r = wait_rec(edge_rec(edges, b - nbx, 0, 0), err);
-            put_edge(A, r, !have_tr);
-            if (!has_l) {
-              fill_edge(L, (int)(r.x & 255));
-              A[-1] = L[-1] = (int16_t)(r.x & 255);
-            }
-            S.nb_mode[0] = (uint8_t)r.w;
-          } else {
-            S.nb_mode[0] = MT_DC_PRED;
-          }
-        } else if (warp == 2) {
-          if (has_l && has_t) {
-            const uint4 r = wait_rec(edge_rec(edges, b - nbx - 1, 0, 0), err);
-            A[-1] = L[-1] = (int16_t)(r.y >> 24);
-          }
-        } else if (warp == 3) {
-          if (have_tr) put_edge(A + 8, wait_rec(edge_rec(edges, b - nbx + 1, 0, 0), err), false);
-        } else if (have_bl) {
-          put_edge(L + 8, wait_rec(edge_rec(edges, b + nbx - 1, 0, 1), err), false);
+        } else if (warp < 2) {
+          if (lane == 0) S.nb_mode[1 - warp] = MT_DC_PRED;
+          if (!has_l && !has_t && lane < 17) e[lane - 1] = (int16_t)(lane == 0 ? 128 : (up ? 127 : 129));
         }
+      } else {
+        const int i = t - 160, y = i >> 3, x = i & 7;
+        S.src[x * 8 + y] = (int16_t)a.src[0][(size_t)(py + y) * a.py.stride + px + x];
       }
-    } else {
-      const int i = t - 160, y = i >> 3, x = i & 7;
-      S.src[x * 8 + y] = (int16_t)a.src[0][(size_t)(py + y) * a.py.stride + px + x];
+      luma_bar();
+      if (t == 0) *(volatile uint32_t*)&S.begun = seq;
+      if (warp < nm)
+        mtd::coop8_predict(mlo + warp, S.edge, has_t, has_l, is_smooth(S.nb_mode[0]) || is_smooth(S.nb_mode[1]), S.src,
+                           S.pcol[warp], S.rcol[warp], S.rrow[warp], S.pb[warp]);
+      luma_bar();
     }
-    luma_bar();
-    if (t == 0) *(volatile uint32_t*)&S.begun = seq;
-    if (warp < nm)
-      mtd::coop8_predict(mlo + warp, S.edge, has_t, has_l, is_smooth(S.nb_mode[0]) || is_smooth(S.nb_mode[1]), S.src,
-                         S.pcol[warp], S.rcol[warp], S.rrow[warp], S.pb[warp]);
-    luma_bar();
     const mtd::Coop<8> g;
-    const int slot = lane >> 3, ms = min(slot, nm - 1), TX = warp;
-    mtd::GroupBuf& o = bufs[4 * TX + slot];
+    const int slot = lane >> 3, ms = min(slot, nm - 1), TX = chroma ? MT_TX_DCT_DCT : warp;
+    mtd::GroupBuf& o = bufs[4 * warp + slot];
+    const mtd::CoopPlane& P = chroma ? S.pc : S.py;
     int32_t c[8], rv[8];  // this lane's levels (row j) and reconstruction (column j)
     int e[8];
     {
@@ -628,9 +614,14 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThre
       }
     }
     float at[8];
-    mtd::coop8_fwd(TX, S.rcol[ms], S.rrow[ms], S.py, c, at, o, g);
-    const int eob = mtd::coop_trellis<8>(c, at, e, S.py, o, g);
-    mtd::coop8_inv(TX, c, S.py, rv, o, g);
+    mtd::coop8_fwd(TX, chroma ? S.ccol : S.rcol[ms], S.rrow[ms], P, c, at, o, g);
+    const int eob = mtd::coop_trellis<8>(c, at, e, P, o, g);
+    mtd::coop8_inv(TX, c, P, rv, o, g);
+    if (chroma) {
+      chroma_finish<8>(cb, edges, rank - 2, b, c, rv);
+      chroma_done();
+      continue;
+    }
     int32_t d[8], pr[8];
     mtd::load8(S.pcol[ms] + g.j * 8, pr);
     mtd::load8(S.src + g.j * 8, d);
