@@ -339,13 +339,19 @@ __device__ __forceinline__ int32_t lane_fwd(const uint16_t* __restrict__ src, in
 #pragma unroll
     for (int r = 0; r < N; r++) v[r] *= 64;
   }
-  pass(col_adst);
+  // one copy of the transform for both passes: the chain's code is larger than
+  // the instruction caches
+#pragma unroll 1
+  for (int ps = 0; ps < 2; ps++) {
+    pass(ps ? row_adst : col_adst);
+    if (ps == 0) {
 #pragma unroll
-  for (int r = 0; r < N; r++) w.t[r * (N + 1) + j] = v[r];
-  g.sync();
+      for (int r = 0; r < N; r++) w.t[r * (N + 1) + j] = v[r];
+      g.sync();
 #pragma unroll
-  for (int u = 0; u < N; u++) v[u] = w.t[j * (N + 1) + u];
-  pass(row_adst);
+      for (int u = 0; u < N; u++) v[u] = w.t[j * (N + 1) + u];
+    }
+  }
 #pragma unroll
   for (int u = 0; u < N; u++) {
     const int idx = u * N + j;
@@ -833,23 +839,22 @@ __device__ __forceinline__ void lane_inv_err(const uint16_t* __restrict__ src, i
     }
   };
   auto ident = [](int32_t x) { return 2 * x + ((x * 1697 + 1024) >> 11); };
-  if (idtx) {
+#pragma unroll 1
+  for (int ps = 0; ps < 2; ps++) {  // rows, columns
+    if (idtx) {
 #pragma unroll
-    for (int u = 0; u < N; u++) v[u] = ident(v[u]);
-  } else {
-    pass(row_adst, q.rmin, q.rmax);
-  }
+      for (int u = 0; u < N; u++) v[u] = ident(v[u]);
+    } else {
+      pass(ps ? col_adst : row_adst, ps ? q.cmin : q.rmin, ps ? q.cmax : q.rmax);
+    }
+    if (ps == 0) {
 #pragma unroll
-  for (int u = 0; u < N; u++)
-    w.t[j * (N + 1) + u] = clampi(N == 8 ? (v[u] + 1) >> 1 : (v[u] + 2) >> 2, q.cmin, q.cmax);
-  g.sync();
+      for (int u = 0; u < N; u++)
+        w.t[j * (N + 1) + u] = clampi(N == 8 ? (v[u] + 1) >> 1 : (v[u] + 2) >> 2, q.cmin, q.cmax);
+      g.sync();
 #pragma unroll
-  for (int y = 0; y < N; y++) v[y] = w.t[y * (N + 1) + j];
-  if (idtx) {
-#pragma unroll
-    for (int y = 0; y < N; y++) v[y] = ident(v[y]);
-  } else {
-    pass(col_adst, q.cmin, q.cmax);
+      for (int y = 0; y < N; y++) v[y] = w.t[y * (N + 1) + j];
+    }
   }
   int32_t* err = reinterpret_cast<int32_t*>(w.tf);
   int16_t* rec = w.rec();

@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(lane_threads<N>()) leaf64_kernel(
   long long sse_sum = 0;
 #pragma unroll 1
   for (int ty = 0; ty < G; ty++)
-#pragma unroll
+#pragma unroll 1
     for (int tx = 0; tx < G; tx++) {
       const int t = ty * G + tx;
       const int sx = tx * N, sy = ty * N, bx = jb.px + sx, by = jb.py + sy;
@@ -433,7 +433,8 @@ __global__ void __launch_bounds__(lane_threads<N>()) leaf64_kernel(
                       reinterpret_cast<int32_t*>(&w), g);
       int ds, sk = 0;
       if constexpr (kGrid) {
-        const uint32_t la4 = actx[tx], ll4 = ty == 0 ? lctx[0] : (ty == 1 ? lctx[1] : (ty == 2 ? lctx[2] : lctx[3]));
+        const uint32_t la4 = tx == 0 ? actx[0] : (tx == 1 ? actx[1] : (tx == 2 ? actx[2] : actx[3]));
+        const uint32_t ll4 = ty == 0 ? lctx[0] : (ty == 1 ? lctx[1] : (ty == 2 ? lctx[2] : lctx[3]));
         uint32_t la = 0, ll = 0;
         int s = -8;
 #pragma unroll
@@ -476,10 +477,11 @@ __global__ void __launch_bounds__(lane_threads<N>()) leaf64_kernel(
         const int32_t c0 = w.cf[0];
         const uint32_t rc = eob < 0 ? 0x40u : (min(cul, 63u) | (c0 == 0 ? 0x40u : (c0 < 0 ? 0u : 0x80u)));
         const uint32_t rc4 = rc * 0x01010101u;
-        actx[tx] = rc4;
 #pragma unroll
-        for (int i = 0; i < G; i++)
+        for (int i = 0; i < G; i++) {
+          if (i == tx) actx[i] = rc4;
           if (i == ty) lctx[i] = rc4;
+        }
         if (ok && cf_out)
           for (int i = g.j; i < NN; i += N) cf_out[(size_t)job * 4096 + t * NN + i] = w.cf[i];
       } else {
