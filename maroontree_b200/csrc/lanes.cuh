@@ -237,7 +237,7 @@ __device__ __forceinline__ void lane_predict(const R& rd, int fw, int fh, int ox
       const int dx = kDrDeriv[angle >> 1];
       const int max_base_x = (edge_len - 1) << up_a, frac_bits = 6 - up_a;
       const int32_t last = a[max_base_x];
-#pragma unroll 4
+#pragma unroll 2
       for (int y = 0; y < N; y++) {
         const int xpos = dx * (y + 1), shift = ((xpos << up_a) & 0x3f) >> 1;
         const int b = (xpos >> frac_bits) + (x << up_a);
@@ -248,14 +248,14 @@ __device__ __forceinline__ void lane_predict(const R& rd, int fw, int fh, int ox
       const int max_base_y = (edge_len - 1) << up_l, frac_bits = 6 - up_l;
       const int ypos = dy * (x + 1), shift = ((ypos << up_l) & 0x3f) >> 1, b0 = ypos >> frac_bits;
       const int32_t last = l[max_base_y];
-#pragma unroll 4
+#pragma unroll 2
       for (int y = 0; y < N; y++) {
         const int b = b0 + (y << up_l);
         out[y * N] = (int16_t)(b >= max_base_y ? last : (l[b] * (32 - shift) + l[b + 1] * shift + 16) >> 5);
       }
     } else {
       const int dy = kDrDeriv[(angle - 90) >> 1], dx = kDrDeriv[(180 - angle) >> 1];
-#pragma unroll 4
+#pragma unroll 2
       for (int y = 0; y < N; y++) {
         const int t = (y + 1) * dx - 64;
         const int x0 = t <= 0 ? 0 : ::min((t + 63) >> 6, N);
@@ -270,7 +270,7 @@ __device__ __forceinline__ void lane_predict(const R& rd, int fw, int fh, int ox
     }
   } else if (mode == MT_PAETH_PRED) {
     const int32_t tv = a0, cn = A[-1];
-#pragma unroll 4
+#pragma unroll 2
     for (int y = 0; y < N; y++) {
       const int32_t lv = Lf[y], b = lv + tv - cn;
       const int32_t ld = abs(lv - b), td = abs(tv - b), cd = abs(cn - b);
@@ -278,7 +278,7 @@ __device__ __forceinline__ void lane_predict(const R& rd, int fw, int fh, int ox
     }
   } else {
     const int32_t right = A[N - 1], bottom = Lf[N - 1], wh = sm_weight<N>(x);
-#pragma unroll 4
+#pragma unroll 2
     for (int y = 0; y < N; y++) {
       const int32_t wv = sm_weight<N>(y);
       const int32_t v = wv * a0 + (256 - wv) * bottom, h = wh * Lf[y] + (256 - wh) * right;
@@ -353,10 +353,12 @@ __device__ __forceinline__ int32_t lane_fwd(const uint16_t* __restrict__ src, in
     }
   }
 #pragma unroll
+  for (int u = 0; u < N; u++) w.t[j * (N + 1) + u] = v[u];  // the lane's own row: a loop over it stays short
+#pragma unroll 4
   for (int u = 0; u < N; u++) {
     const int idx = u * N + j;
     const int32_t m = idx == 0 ? q.q_mult_dc : q.q_mult_ac;
-    int32_t c = v[u];
+    int32_t c = w.t[j * (N + 1) + u];
     if constexpr (N == 16) c = mul_q16(c, 32768);
     if constexpr (N == 32) c = (int32_t)(((long long)c * 16384 + (1ll << 21)) >> 22);
     float x = __fmul_rn(__fmul_rn((float)c, (float)m), 1.0f / 65536.0f);
@@ -817,8 +819,7 @@ __device__ __forceinline__ void lane_inv_err(const uint16_t* __restrict__ src, i
   const uint8_t* wq = idtx ? nullptr : qm;
   const bool col_adst = N != 32 && (tx == MT_TX_ADST_ADST || tx == MT_TX_ADST_DCT);
   const bool row_adst = N != 32 && (tx == MT_TX_ADST_ADST || tx == MT_TX_DCT_ADST);
-  int32_t v[N];
-#pragma unroll
+#pragma unroll 4
   for (int u = 0; u < N; u++) {
     const int rc = u * N + j;
     const int32_t l = w.cf[rc];
@@ -827,8 +828,11 @@ __device__ __forceinline__ void lane_inv_err(const uint16_t* __restrict__ src, i
     int32_t mag = (int32_t)((uabs(l) * (uint32_t)step) & 0xffffffu);
     if constexpr (N == 32) mag >>= 1;
     mag = ::min(mag, q.cf_max + (l < 0 ? 1 : 0));
-    v[u] = l == 0 ? 0 : (l < 0 ? -mag : mag);
+    w.t[j * (N + 1) + u] = l == 0 ? 0 : (l < 0 ? -mag : mag);
   }
+  int32_t v[N];
+#pragma unroll
+  for (int u = 0; u < N; u++) v[u] = w.t[j * (N + 1) + u];
   auto pass = [&](bool adst, int32_t mn, int32_t mx) {
     if constexpr (N == 32) {
       idct32s(v, 1, mn, mx);
@@ -859,8 +863,10 @@ __device__ __forceinline__ void lane_inv_err(const uint16_t* __restrict__ src, i
   int32_t* err = reinterpret_cast<int32_t*>(w.tf);
   int16_t* rec = w.rec();
 #pragma unroll
+  for (int y = 0; y < N; y++) w.t[y * (N + 1) + j] = v[y];  // the lane's own column
+#pragma unroll 4
   for (int y = 0; y < N; y++) {
-    const int32_t r = clampi((int32_t)w.pred[y * N + j] + (int16_t)((v[y] + 8) >> 4), 0, maxv);
+    const int32_t r = clampi((int32_t)w.pred[y * N + j] + (int16_t)((w.t[y * (N + 1) + j] + 8) >> 4), 0, maxv);
     rec[y * N + j] = (int16_t)r;
     err[y * N + j] = j < vw && y < vh ? (int32_t)src[(size_t)y * stride + j] - r : 0;
   }
