@@ -192,22 +192,23 @@ __device__ __forceinline__ void coop_quant(const int32_t* v, const CoopPlane& P,
   }
 }
 
-// Forward transform and quantisation of type TX from the residual (col / row:
-// columns and rows of eight int16, magnitudes below 256).  The two passes are
-// one loop, so that a warp runs the second from the instructions it has just
-// fetched: the kernel's code is larger than the instruction caches.
-__device__ __forceinline__ void coop8_fwd(int TX, const int16_t* col, const int16_t* row, const CoopPlane& P, int32_t* c,
-                                          float* at, GroupBuf& o, const Coop<8>& g) {
+// Whether a type's forward transform starts from the rows of the residual.
+__device__ __forceinline__ bool coop8_by_rows(int TX) { return TX == MT_TX_IDTX || TX == MT_TX_H_DCT; }
+
+// Forward transform and quantisation of type TX from column j (or row j:
+// coop8_by_rows) of the residual, magnitudes below 256.  The two passes are one
+// loop, so that a warp runs the second from the instructions it has just
+// fetched: the kernels' code is larger than the instruction caches.
+__device__ __forceinline__ void coop8_fwd(int TX, int32_t* v, const CoopPlane& P, int32_t* c, float* at, GroupBuf& o,
+                                          const Coop<8>& g) {
   const int j = g.j;
-  int32_t v[8];
-  load8((TX == MT_TX_IDTX || TX == MT_TX_H_DCT ? row : col) + j * 8, v);
   if (TX == MT_TX_IDTX) {
 #pragma unroll
     for (int k = 0; k < 8; k++) {
       const bool dc = k == 0 && j == 0;
       const int32_t qd = dc ? P.q.dc_q : P.q.ac_q;
       const uint32_t m = (uint32_t)abs(v[k]), am = m * 8;
-      at[k] = P.idt[dc][m];
+      at[k] = P.idt[dc][::min(m, 255u)];
       // (am + qd / 2) / qd: exact for am + qd / 2 < 2^16 and qd < 2^12
       const int32_t level = (int32_t)__umulhi(am + (uint32_t)(qd >> 1), dc ? P.idiv[0] : P.idiv[1]);
       c[k] = (int32_t)am < qd ? 0 : (v[k] < 0 ? -level : level);
@@ -244,11 +245,11 @@ __device__ __forceinline__ void coop4_fwd(int32_t* v, const CoopPlane& P, int32_
 }
 
 // trellis_optimize (trellis8 / trellis4) over row j's levels c and target
-// magnitudes at, e their scan indexes.  Returns the final end of block (-1: all
-// zero).
+// magnitudes at, e their scan indexes; without `run` the levels stay.  Returns
+// the final end of block (-1: all zero).
 template <int W>
 __device__ __forceinline__ int coop_trellis(int32_t* c, const float* at, const int* e, const CoopPlane& P, GroupBuf& o,
-                                            const Coop<W>& g) {
+                                            const Coop<W>& g, bool run = true) {
   constexpr unsigned kAll = 0xffffffffu;
   int e1 = 0;
   bool big = false;
@@ -258,7 +259,7 @@ __device__ __forceinline__ int coop_trellis(int32_t* c, const float* at, const i
     big |= abs(c[k]) > 63;
   }
   const int m = (int)g.max((unsigned)e1);
-  if (!(P.lambda > 0.0f) || !__any_sync(kAll, m != 0)) return m - 1;
+  if (!run || !(P.lambda > 0.0f) || !__any_sync(kAll, m != 0)) return m - 1;
   const int full8 = m & ~7, chunked = full8 + ((m - full8) >= 4 ? 4 : 0);
   // step A.  The reference decides each position of a chunk (of eight, then one
   // of four) from the chunk's starting values, in the AVX2 FMA form unless the
@@ -450,9 +451,10 @@ __device__ __forceinline__ float add_ones(float b, int n) {
 }
 
 // The first terms of a coded block's rate, in the walk's order: txb_skip, the
-// tx-type symbol, the end-of-block position (rate8, contexts 0, no skip price).
-__device__ __forceinline__ float coop8_rate_head(const mt_coef_costs& T, int mode, int tx, int eob) {
-  float bits = __fadd_rn(T.txb_skip[0][0], T.txtp[mode][tx]);
+// tx-type symbol, the end-of-block position (rate8); coded: the price of the
+// first.
+__device__ __forceinline__ float coop8_rate_head(const mt_coef_costs& T, float coded, int mode, int tx, int eob) {
+  float bits = __fadd_rn(coded, T.txtp[mode][tx]);
   const int bin = eob < 2 ? eob : 32 - __clz(eob);
   bits = __fadd_rn(bits, T.eob_bin[bin]);
   if (bin > 1) {
@@ -463,8 +465,9 @@ __device__ __forceinline__ float coop8_rate_head(const mt_coef_costs& T, int mod
   return bits;
 }
 
-// rate8 (txb_skip and dc_sign context 0, no skip price) over the group; head:
-// coop8_rate_head of the candidate's (mode, type) by end of block.  The
+// rate8 over the group; none: the bits of a block without levels; head(eob): the
+// first terms of one with levels (coop8_rate_head); sign: the dc_sign context's
+// row.  The
 // reference's reverse walk has entered exactly the later scan positions when it
 // reads a context, and the five neighbours of a position inside the block are
 // later ones (past a column's end its map holds nothing yet), so contexts come
@@ -475,8 +478,10 @@ __device__ __forceinline__ float coop8_rate_head(const mt_coef_costs& T, int mod
 // DC add to the br cost first) in shared memory in the walk's order, an absent
 // one as +0, and lane 0 adds them, DC's sign and the sign bits behind them, and
 // returns the bits.
+template <typename Head>
 __device__ __forceinline__ float coop8_rate(const int32_t* c, const int* e, int eob, const mt_coef_costs& T,
-                                            const float* head, GroupBuf& o, const Coop<8>& g) {
+                                            float none, Head&& head, const float* sign, GroupBuf& o,
+                                            const Coop<8>& g) {
   constexpr unsigned kAll = 0xffffffffu;
   const int j = g.j;
   uint32_t m[8], w[2] = {0, 0}, nz = 0, top = 0;
@@ -547,7 +552,7 @@ __device__ __forceinline__ float coop8_rate(const int32_t* c, const int* e, int 
   __syncwarp();
   float bits = 0.0f;
   if (j == 0) {
-    bits = eob < 0 ? T.txb_skip[0][1] : head[eob];
+    bits = eob < 0 ? none : head(eob);
     if (eob >= 0) {
       const int first = (63 - eob) & ~3;
       if (!any3) {
@@ -569,7 +574,7 @@ __device__ __forceinline__ float coop8_rate(const int32_t* c, const int* e, int 
         for (int k = first; k < 64; k++)
           bits = __fadd_rn(__fadd_rn(__fadd_rn(bits, o.b[2 * k]), o.b[2 * k + 1]), T3[k]);
       }
-      if (c[0] != 0) bits = __fadd_rn(bits, T.dc_sign[0][c[0] < 0]);
+      if (c[0] != 0) bits = __fadd_rn(bits, sign[c[0] < 0]);
       if (eob > 0) bits = add_ones(bits, (int)nz - (c[0] != 0));
     }
   }

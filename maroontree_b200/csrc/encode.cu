@@ -515,7 +515,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThre
       cta_bar();
       for (int i = t; i < nm * kTypes * 64; i += nthr) {
         const int m = i / (kTypes * 64), x = i / 64 % kTypes;
-        S.head[m][x][i & 63] = mtd::coop8_rate_head(S.cy, mlo + m, x, i & 63);
+        S.head[m][x][i & 63] = mtd::coop8_rate_head(S.cy, S.cy.txb_skip[0][0], mlo + m, x, i & 63);
       }
       cta_bar();
       cur = img;
@@ -614,7 +614,11 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThre
       }
     }
     float at[8];
-    mtd::coop8_fwd(TX, chroma ? S.ccol : S.rcol[ms], S.rrow[ms], P, c, at, o, g);
+    {
+      int32_t v[8];
+      mtd::load8((chroma ? S.ccol : (mtd::coop8_by_rows(TX) ? S.rrow[ms] : S.rcol[ms])) + g.j * 8, v);
+      mtd::coop8_fwd(TX, v, P, c, at, o, g);
+    }
     const int eob = mtd::coop_trellis<8>(c, at, e, P, o, g);
     mtd::coop8_inv(TX, c, P, rv, o, g);
     if (chroma) {
@@ -633,7 +637,9 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThre
     const uint32_t satd = mtd::coop8_satd(d, g);
     float price = __fmul_rn(__fmul_rn(__fmul_rn((float)satd, fmaxf((float)S.py.q.ac_q, 1.0f)), 0.25f), a.py.satd_scale);
     if (a.py.satd_bridge != 0.0f) price = __fmul_rn(price, a.py.satd_bridge);
-    const float bits = mtd::coop8_rate(c, e, eob, S.cy, S.head[ms][TX], o, g);
+    const float* const head = S.head[ms][TX];
+    const float bits = mtd::coop8_rate(c, e, eob, S.cy, S.cy.txb_skip[0][1], [head](int k) { return head[k]; },
+                                       S.cy.dc_sign[0], o, g);
     const float cost = __fadd_rn(price, __fmul_rn(a.py.mode_lambda, bits));
     unsigned long long k = ~0ull;
     if (g.j == 0 && slot < nm)
