@@ -155,9 +155,12 @@ __device__ __forceinline__ int lane_cfl(const uint16_t* __restrict__ l, int ls, 
                                         int32_t maxv, LaneBuf<N>& w, const Lanes<N>& g) {
   constexpr int L = log2w<N>();
   const int x = g.j;
-  int16_t ac[N];
+  // the lane's column of the AC, over the scratch that the transform takes next:
+  // loops a few rows at a time instead of the column in registers (at 32x32 the
+  // seven alphas written out were 40 KB of code)
+  int32_t* const ac = reinterpret_cast<int32_t*>(w.a) + x;
   int32_t sum = 0;
-#pragma unroll
+#pragma unroll 4
   for (int y = 0; y < N; y++) {
     int32_t v;
     if constexpr (SUB) {
@@ -166,17 +169,18 @@ __device__ __forceinline__ int lane_cfl(const uint16_t* __restrict__ l, int ls, 
     } else {
       v = (int32_t)l[(size_t)y * ls + x] << 3;
     }
-    ac[y] = (int16_t)v;
+    ac[y * N] = (int16_t)v;
     sum += v;
   }
   const int32_t mean = (g.sum(sum) + N * N / 2) >> (2 * L);
   const bool vis_x = x < P.vw;
   long long num = 0, den = 0;
-#pragma unroll
+#pragma unroll 4
   for (int y = 0; y < N; y++) {
-    ac[y] = (int16_t)(ac[y] - mean);
+    const int16_t a = (int16_t)(ac[y * N] - mean);
+    ac[y * N] = a;
     if (vis_x && y < P.vh) {
-      const long long v = ac[y];
+      const long long v = a;
       num += (long long)((int32_t)P.src[(size_t)y * stride + x] - dc) * v;
       den += v * v;
     }
@@ -190,13 +194,14 @@ __device__ __forceinline__ int lane_cfl(const uint16_t* __restrict__ l, int ls, 
   long long e[7];
 #pragma unroll
   for (int k = 0; k < 7; k++) e[k] = 0;
-#pragma unroll
+#pragma unroll 1
   for (int y = 0; y < N; y++) {
     if (vis_x && y < P.vh) {
+      const int32_t a = ac[y * N];
       const int32_t s = P.src[(size_t)y * stride + x];
 #pragma unroll
       for (int k = 0; k < 7; k++) {
-        const long long d = s - cfl_pred_pixel(dc, ac[y], (int)a0 - 3 + k, maxv);
+        const long long d = s - cfl_pred_pixel(dc, a, (int)a0 - 3 + k, maxv);
         e[k] += d * d;
       }
     }
@@ -212,8 +217,8 @@ __device__ __forceinline__ int lane_cfl(const uint16_t* __restrict__ l, int ls, 
     }
   }
   if (den == 0) alpha = 0;
-#pragma unroll
-  for (int y = 0; y < N; y++) w.pred[y * N + x] = (int16_t)cfl_pred_pixel(dc, ac[y], alpha, maxv);
+#pragma unroll 4
+  for (int y = 0; y < N; y++) w.pred[y * N + x] = (int16_t)cfl_pred_pixel(dc, ac[y * N], alpha, maxv);
   g.sync();
   return alpha;
 }
@@ -271,10 +276,13 @@ __device__ __noinline__ void plane_predict(const uint16_t* __restrict__ rec, int
 // trellis, DC's total without mode bits, no deltas after CfL.  k16_420 is
 // pick_uv16_420 (block16.rs:980-1381): the joint (mode, delta) shortlist of the
 // SATD ranking in place of the top-3 and the deltas.
-// Bound by issue and the chains' latency, HBM is idle.  Measured at 1080p against
-// a thread per leaf with its working set in shared memory (3, 10 or 50 KB, so
-// 55, 21 or 4 leaves per SM): k16_420 2.83 -> 1.09 ms, k16_444 25.2 -> 2.27 ms,
-// k32_420 24.2 -> 0.78 ms, k32_444 56 -> 2.15 ms.
+// Bound by issue, instruction fetch and the chains' latency, HBM is idle.
+// Measured at 1080p against a thread per leaf with its working set in shared
+// memory (3, 10 or 50 KB, so 55, 21 or 4 leaves per SM): k16_420 2.83 -> 0.94 ms,
+// k16_444 25.2 -> 2.1, k32_420 24.2 -> 0.7, k32_444 56 -> 1.72 ms; of that, code
+// kept short (one transform for both passes, rows four at a time, CfL's column in
+// shared memory; 185 to 350 KB -> 158 to 173) k16_420 1.09 -> 0.94 and k32_444
+// 2.18 -> 1.72.
 template <UvForm F, typename J>
 __global__ void __launch_bounds__(UvShape<F>::kThreads) uv_kernel(
     const uint16_t* __restrict__ src_u, const uint16_t* __restrict__ src_v, const uint16_t* __restrict__ rec_u,
