@@ -462,12 +462,14 @@ __device__ __forceinline__ int lane_trellis_ctx(W& w, float dc_q, float ac_q, fl
         return __fadd_rn(__fadd_rn(bt[3], hi_cost(T, k, bc)), 1.0f);
       };
       uint32_t best_k = l;
-      float best_c = __fadd_rn(distw(i, rc, l), __fmul_rn(lambda, rate_k(l)));
-      for (int32_t k = (int32_t)l - 1; k >= 0; k--) {
+      float best_c = 0.0f;
+#pragma unroll 1
+      for (int32_t k = (int32_t)l; k >= 0; k--) {  // the level itself, then the lower ones
+        const bool first = k == (int32_t)l;
         const float dk = distw(i, rc, (uint32_t)k);
-        if (dk >= best_c) break;
+        if (!first && dk >= best_c) break;
         const float c = __fadd_rn(dk, __fmul_rn(lambda, rate_k((uint32_t)k)));
-        if (c < best_c) {
+        if (first || c < best_c) {
           best_c = c;
           best_k = (uint32_t)k;
         }
@@ -491,12 +493,14 @@ __device__ __forceinline__ int lane_trellis_ctx(W& w, float dc_q, float ac_q, fl
         return __fadd_rn(b, sgn_bits);
       };
       uint32_t best_k = l;
-      float best_c = __fadd_rn(distw(0, 0, l), __fmul_rn(lambda, dc_rate(l)));
-      for (int32_t k = (int32_t)l - 1; k >= 0; k--) {
+      float best_c = 0.0f;
+#pragma unroll 1
+      for (int32_t k = (int32_t)l; k >= 0; k--) {
+        const bool first = k == (int32_t)l;
         const float dk = distw(0, 0, (uint32_t)k);
-        if (dk >= best_c) break;
+        if (!first && dk >= best_c) break;
         const float c = __fadd_rn(dk, __fmul_rn(lambda, dc_rate((uint32_t)k)));
-        if (c < best_c) {
+        if (first || c < best_c) {
           best_c = c;
           best_k = (uint32_t)k;
         }
@@ -613,13 +617,14 @@ __device__ __forceinline__ int lane_trellis_ctx(W& w, float dc_q, float ac_q, fl
     if (k != 0) {
       const float base = __fadd_rn(__fadd_rn(__fadd_rn(dc_cost, A[e]), __fmul_rn(lambda, eob_pt_cost(e))), S[e + 1]);
       uint32_t m_best = k;
-      float c = __fadd_rn(base, __fadd_rn(__fmul_rn(lambda, eob_coeff_cost(e, rc, k)), distw(e, rc, k)));
-      if (k >= 2) {
-        const float c_low =
-            __fadd_rn(base, __fadd_rn(__fmul_rn(lambda, eob_coeff_cost(e, rc, k - 1)), distw(e, rc, k - 1)));
-        if (c_low < c) {
-          c = c_low;
-          m_best = k - 1;
+      float c = 0.0f;
+#pragma unroll 1
+      for (uint32_t lv1 = k; lv1 >= ::max(k - 1, 1u); lv1--) {  // the level, and the one below where it is not zero
+        const float cl =
+            __fadd_rn(base, __fadd_rn(__fmul_rn(lambda, eob_coeff_cost(e, rc, lv1)), distw(e, rc, lv1)));
+        if (lv1 == k || cl < c) {
+          c = cl;
+          m_best = lv1;
         }
       }
       if (c < best_cost || (c == best_cost && e < best_e)) {
@@ -905,6 +910,7 @@ __device__ __forceinline__ long long lane_sse(const W& w, int vw, int vh, float 
 #pragma unroll
     for (int r = 0; r < 4; r++) D[i][r] = kWsseD[k][r];
   }
+#pragma unroll 1
   for (int r0 = 0; r0 < N; r0 += 4)
 #pragma unroll 2
     for (int c0 = 0; c0 < N; c0 += 8) {
@@ -940,6 +946,7 @@ __device__ __forceinline__ long long lane_sse(const W& w, int vw, int vh, float 
   }
   const bool tail = pairs < pw;
   if (__any_sync(kFull, tail)) {  // the 4-wide tail tiles, into the four sums
+#pragma unroll 1
     for (int r0 = 0; r0 < N; r0 += 4) {
       float e[4];
 #pragma unroll
