@@ -497,8 +497,10 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThre
   const EncArgs& a = S.job.a;
   const int mlo = mode_lo(rank), nm = mode_lo(rank + 1) - mlo;  // this CTA's modes
   int cur = -1;                                                 // the image whose tables are staged
+  unsigned long long ahead = 0;                                 // the next block's word, if it was there early
   for (uint32_t seq = 1;; ++seq) {
-    const unsigned long long nx = wait_next(&S.next[seq & 1], seq, err);
+    const unsigned long long nx =
+        (uint32_t)(ahead >> 40) == (seq & kSeqMask) ? ahead : wait_next(&S.next[seq & 1], seq, err);
     if (nx & kEnd) break;  // the same for every warp of the cluster
     const int img = (int)(nx >> 32) & 127;
     if (img != cur) {  // another image: its descriptor, then its tables
@@ -651,6 +653,14 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThre
     }
     k = __shfl_sync(0xffffffffu, k, 0);
     if (lane < kClusterCtas) put_key(&S.key[seq & 1][rank * kTypes + warp], &S.key_bar[seq & 1], lane, k);
+    // every group's records, while the keys are on their way
+    uint32_t row = (uint32_t)rv[7] << (8 * (g.j & 3)), col[2] = {0, 0};
+    row |= __shfl_xor_sync(0xffffffffu, row, 1);
+    row |= __shfl_xor_sync(0xffffffffu, row, 2);
+    const uint32_t row_hi = __shfl_sync(0xffffffffu, row, 4, 8);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) col[q >> 2] |= (uint32_t)rv[q] << (8 * (q & 3));
+    ahead = get_word(&S.next[(seq + 1) & 1]);
     wait_keys(&S.key_bar[seq & 1], ((seq - 1) >> 1) & 1, err);
     if (t == 0) key_bar_arm(&S.key_bar[seq & 1]);  // for block seq + 2
     const unsigned long long all = S.key[seq & 1][lane];
@@ -659,15 +669,8 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThre
     const int wi = (int)__reduce_min_sync(0xffffffffu, cst == low && lane < kLumaKeys ? (uint32_t)all : 255u);
     const int wm = wi / kTypes;
     if (rank == mode_rank(wm) && warp == wi - wm * kTypes && slot == wm - mlo) {
-      const unsigned gm = 0xffu << (lane & 24);
       const int j = g.j;
-      uint32_t row = (uint32_t)rv[7] << (8 * (j & 3)), col[2] = {0, 0};
-      row |= __shfl_xor_sync(gm, row, 1, 8);
-      row |= __shfl_xor_sync(gm, row, 2, 8);
-      const uint32_t hi = __shfl_sync(gm, row, 4, 8);
-#pragma unroll
-      for (int q = 0; q < 8; ++q) col[q >> 2] |= (uint32_t)rv[q] << (8 * (q & 3));
-      if (j == 0) put_rec(edge_rec(edges, b, 0, 0), row, hi, (uint32_t)wm);
+      if (j == 0) put_rec(edge_rec(edges, b, 0, 0), row, row_hi, (uint32_t)wm);
       if (j == 7) put_rec(edge_rec(edges, b, 0, 1), col[0], col[1], (uint32_t)wm);
       int32_t* lv = a.lv_y + (size_t)b * 64 + j;
       uint16_t* r = a.rec[0] + (size_t)py * a.py.stride + px + j;
@@ -812,11 +815,14 @@ class Buffers {
         if (s) cudaStreamDestroy(s);
     }
   }
+  // slack: what a buffer whose size follows the picture's content gets beside,
+  // so that the next picture seldom has to grow it (a free waits for the device).
   template <class T>
-  T* get(int i, Slot s, size_t n) {
+  T* get(int i, Slot s, size_t n, bool slack = false) {
     BufSet& b = set(i);
     n = n ? n : 1;
     if (b.cap[s] < n) {
+      if (slack) n += n / 4;
       cudaFree(b.p[s]);
       b.p[s] = nullptr;
       b.cap[s] = 0;
@@ -1265,7 +1271,7 @@ int job_finish(Job& j, Buffers& buf, int i) {
       cudaStreamWaitEvent(sc, counted.e, 0) != cudaSuccess)
     return MT_ERR_DEVICE;
   cs.d2h(sizeof(tot));
-  void* d_tok = buf.get<void>(i, kTokens, mth::stream_token_bytes(j.sg, tot.tokens));
+  void* d_tok = buf.get<void>(i, kTokens, mth::stream_token_bytes(j.sg, tot.tokens), true);
   if (!d_tok) return MT_ERR_DEVICE;
   if ((rc = mth::stream_trace(j.sg, j.si, j.d_plan, d_tok, tot.tokens, j.d_cdfs, cfg->updating_cdf != 0, sc, &nl)) !=
       MT_OK)
@@ -1344,7 +1350,7 @@ int job_finish(Job& j, Buffers& buf, int i) {
     longest = std::max(longest, t.nbytes);
     ntok += t.ntok;
   }
-  void* d_dig = buf.get<void>(i, kDigits, mth::stream_digit_bytes(tot));
+  void* d_dig = buf.get<void>(i, kDigits, mth::stream_digit_bytes(tot), true);
   if (!d_dig) return MT_ERR_DEVICE;
   const uint8_t* d_pay =
       mth::stream_bytes(j.sg, j.d_plan, d_tok, tot.tokens, d_dig, tot, longest, sc, &nl);
