@@ -293,8 +293,8 @@ __device__ __forceinline__ void lane_predict(const R& rd, int fw, int fh, int ox
 // into w.cf / w.tf: fwd8x8 / fwd16x16 and apply_qm; at 32x32 the residual gets
 // 6 bits of headroom and each output the 64-bit rounding (x * 16384 + 2^21) >>
 // 22 of dct32x32_quant_t_direct (src/dct.rs:705-736).  qs: the forward scale of
-// each QM weight value.  8x8 and 32x32 take the 2-D types only (32x32:
-// DCT_DCT).  Returns the sum of the residual.
+// each QM weight value.  32x32 takes DCT_DCT only, 16x16 no V_DCT / H_DCT.
+// Returns the sum of the residual.
 template <int N, typename W>
 __device__ __forceinline__ int32_t lane_fwd(const uint16_t* __restrict__ src, int stride, int tx, const mt_quant& q,
                                             const uint8_t* qm, const float* qs, W& w, const Lanes<N>& g) {
@@ -310,7 +310,7 @@ __device__ __forceinline__ int32_t lane_fwd(const uint16_t* __restrict__ src, in
   }
   sum = g.sum(sum);
   g.sync();  // the edges of the prediction are done with
-  if (N == 16 && tx == MT_TX_IDTX) {
+  if (N != 32 && tx == MT_TX_IDTX) {
 #pragma unroll
     for (int y = 0; y < N; y++) {
       const int rc = y + j * N;
@@ -326,6 +326,7 @@ __device__ __forceinline__ int32_t lane_fwd(const uint16_t* __restrict__ src, in
   }
   const bool col_adst = N != 32 && (tx == MT_TX_ADST_ADST || tx == MT_TX_ADST_DCT);
   const bool row_adst = N != 32 && (tx == MT_TX_ADST_ADST || tx == MT_TX_DCT_ADST);
+  const bool one = N == 8 && (tx == MT_TX_V_DCT || tx == MT_TX_H_DCT);  // one pass, quant_fullstep
   auto pass = [&](bool adst) {
     if constexpr (N == 32) {
       fdct32(v);
@@ -343,7 +344,7 @@ __device__ __forceinline__ int32_t lane_fwd(const uint16_t* __restrict__ src, in
   // the instruction caches
 #pragma unroll 1
   for (int ps = 0; ps < 2; ps++) {
-    pass(ps ? row_adst : col_adst);
+    if (!one || tx == (ps ? MT_TX_H_DCT : MT_TX_V_DCT)) pass(ps ? row_adst : col_adst);
     if (ps == 0) {
 #pragma unroll
       for (int r = 0; r < N; r++) w.t[r * (N + 1) + j] = v[r];
@@ -361,9 +362,17 @@ __device__ __forceinline__ int32_t lane_fwd(const uint16_t* __restrict__ src, in
     int32_t c = w.t[j * (N + 1) + u];
     if constexpr (N == 16) c = mul_q16(c, 32768);
     if constexpr (N == 32) c = (int32_t)(((long long)c * 16384 + (1ll << 21)) >> 22);
-    float x = __fmul_rn(__fmul_rn((float)c, (float)m), 1.0f / 65536.0f);
-    Coef l = (Coef)quant_q16(c, m);
-    if (qm) {
+    float x;
+    Coef l;
+    if (one) {
+      const int32_t p = c * 2 * m, lv = (abs(p) + 32768) >> 16;
+      x = __fmul_rn((float)p, 1.0f / 65536.0f);
+      l = (Coef)(abs(p) < 65536 ? 0 : (p < 0 ? -lv : lv));
+    } else {
+      x = __fmul_rn(__fmul_rn((float)c, (float)m), 1.0f / 65536.0f);
+      l = (Coef)quant_q16(c, m);
+    }
+    if (qm && !one) {
       x = __fmul_rn(x, qs[qm[idx]]);
       const float tr = truncf(x);
       const float step = fabsf(__fsub_rn(x, tr)) >= 0.5f ? copysignf(1.0f, x) : 0.0f;
@@ -820,8 +829,9 @@ __device__ __forceinline__ void lane_inv_err(const uint16_t* __restrict__ src, i
                                              const uint8_t* qm, int vw, int vh, int32_t maxv, W& w,
                                              const Lanes<N>& g) {
   const int j = g.j;
-  const bool idtx = N == 16 && tx == MT_TX_IDTX;
-  const uint8_t* wq = idtx ? nullptr : qm;
+  const bool idtx = N != 32 && tx == MT_TX_IDTX;
+  const bool one = N == 8 && (tx == MT_TX_V_DCT || tx == MT_TX_H_DCT);
+  const uint8_t* wq = idtx || one ? nullptr : qm;
   const bool col_adst = N != 32 && (tx == MT_TX_ADST_ADST || tx == MT_TX_ADST_DCT);
   const bool row_adst = N != 32 && (tx == MT_TX_ADST_ADST || tx == MT_TX_DCT_ADST);
 #pragma unroll 4
@@ -847,10 +857,10 @@ __device__ __forceinline__ void lane_inv_err(const uint16_t* __restrict__ src, i
       if (adst) iadst8s(v, 1, mn, mx); else idct8s(v, 1, mn, mx);
     }
   };
-  auto ident = [](int32_t x) { return 2 * x + ((x * 1697 + 1024) >> 11); };
+  auto ident = [](int32_t x) { return N == 8 ? 2 * x : 2 * x + ((x * 1697 + 1024) >> 11); };
 #pragma unroll 1
   for (int ps = 0; ps < 2; ps++) {  // rows, columns
-    if (idtx) {
+    if (idtx || (one && tx == (ps ? MT_TX_H_DCT : MT_TX_V_DCT))) {
 #pragma unroll
       for (int u = 0; u < N; u++) v[u] = ident(v[u]);
     } else {

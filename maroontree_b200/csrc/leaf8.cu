@@ -1,8 +1,7 @@
-// The leaf luma searches, batched: pick_block8's (src/coder/block8.rs:689-1420)
-// Slow mode-loop candidates and winner transform-type refinement
-// (leaf8_kernel, one thread per job), pick_luma16's and pick_luma32's
-// (leaf_lanes_kernel, N lanes per job), and the 64x64 leaf's two legs
-// (leaf64_kernel).
+// The leaf luma searches, batched: pick_block8's (src/coder/block8.rs:689-1420),
+// pick_luma16's and pick_luma32's Slow mode-loop candidates and winner
+// transform-type refinements (leaf_lanes_kernel, N lanes per job), and the 64x64
+// leaf's two legs (leaf64_kernel).
 // The stages are the split trial's (leaf8.cuh, over lanes in lanes.cuh):
 // DCT_DCT + QM with trellis_optimize_ctx, the dav1d inverse, sse_recon, the
 // bounded 2-D and the 1-D rate walks; every type runs through one loop body.
@@ -24,8 +23,6 @@ namespace {
 
 using namespace mtd;
 
-constexpr int kLeafThreads = 128;
-
 struct LeafArgs {
   mt_split16_params p;
   mt_quant q;
@@ -33,189 +30,45 @@ struct LeafArgs {
   int has_qm;
 };
 
-// Per-thread working set of one 8x8 job.  u: the prediction edges, then the
-// targets [0, 64) and the transform temporary [64, 128).
-struct Leaf8Work {
-  int32_t u[128];
-  int16_t pred[64], resid[64];
-  int16_t cfs[2][64];  // levels of the candidate and of the winner
-  int16_t rrs[2][64];  // their inverses
-  TrellisCtxScratch tr;
-  uint8_t lv[160];  // rate walks' level maps
-};
-
 __device__ __forceinline__ float rd_cost_i64(long long d, float lam, float rate) {
   return __fadd_rn((float)d, __fmul_rn(lam, rate));
 }
 
-// pick_block8's mode-loop candidates (REFINE = false) and winner refinement
-// (REFINE = true), one thread per job.
-template <bool REFINE>
-__global__ void __launch_bounds__(kLeafThreads) leaf8_kernel(
-    const uint16_t* __restrict__ src, const uint16_t* __restrict__ rec, LeafArgs a,
-    const uint8_t* __restrict__ qm_row, const mt_coef_costs* __restrict__ costs,
-    const mt_leaf8_job* __restrict__ jobs, int n, mt_leaf8_result* __restrict__ res, int32_t* __restrict__ cf_out,
-    uint16_t* __restrict__ rec_out) {
-  __shared__ mt_coef_costs sT;
-  constexpr int N = 8, NN = 64, L = 3;
-  __shared__ uint8_t sQm[NN];
-  __shared__ float sQs[NN];
-  {
-    const float* g = reinterpret_cast<const float*>(costs);
-    float* s = reinterpret_cast<float*>(&sT);
-    for (int i = threadIdx.x; i < (int)(sizeof(mt_coef_costs) / 4); i += blockDim.x) s[i] = g[i];
-    for (int i = threadIdx.x; i < NN; i += blockDim.x) {
-      const int w = a.has_qm ? qm_row[i] : 32;
-      sQm[i] = (uint8_t)w;
-      sQs[i] = fwd_qm_scale(w);
-    }
-    __syncthreads();
-  }
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const mt_split16_params& p = a.p;
-  const mt_quant& q = a.q;
-  const mt_coef_costs& T = sT;
-  const uint8_t* qm = a.has_qm ? sQm : nullptr;
-  const mt_leaf8_job jb = jobs[j];
-  mt_leaf8_result& r = res[j];
-  const bool ok = jb.px + N <= p.frame_w && jb.py + N <= p.frame_h && jb.mode <= MT_PAETH_PRED &&
-                  jb.angle_delta >= -3 && jb.angle_delta <= 3 &&
-                  (jb.angle_delta == 0 || (jb.mode >= MT_V_PRED && jb.mode <= MT_D67_PRED)) && jb.dcs_ctx < 3;
-  if (!ok) {
-    r.sse = 0;
-    r.bits = r.cost = __int_as_float(0x7f800000);
-    r.tx_type = 255;
-    for (int i = 0; i < 7; i++) r.reserved[i] = 0;
-    if (cf_out)
-      for (int i = 0; i < NN; i++) cf_out[(size_t)j * NN + i] = 0;
-    if (rec_out)
-      for (int i = 0; i < NN; i++) rec_out[(size_t)j * NN + i] = 0;
-    return;
-  }
-  Leaf8Work w;
-  const int32_t maxv = (1 << p.bd) - 1;
-  const float dcq = (float)q.dc_q, acq = (float)q.ac_q, rd_lam = p.rd_lambda;
-  const bool qm_full = q.qm_level >= 5;
-  const int vis_w = p.vis_w > 0 ? p.vis_w : p.frame_w, vis_h = p.vis_h > 0 ? p.vis_h : p.frame_h;
-  predict_sq<N>(rec, p.stride, p.frame_w, p.frame_h, jb.px, jb.py, jb.mode, jb.angle_delta, jb.flags & 1,
-                (jb.flags >> 1) & 1, (jb.flags >> 2) & 1, p.bd, w.pred, w.u);
-#pragma unroll 8
-  for (int i = 0; i < NN; i++)
-    w.resid[i] = (int16_t)((int32_t)src[(size_t)(jb.py + (i >> L)) * p.stride + jb.px + (i & (N - 1))] - w.pred[i]);
-  const int ds = jb.dcs_ctx;
-  ErrBlock<int16_t, int16_t> eb;
-  eb.src = src + (size_t)jb.py * p.stride + jb.px;
-  eb.stride = p.stride;
-  eb.pred = w.pred;
-  eb.w = N;
-  eb.vw = min(max(vis_w - jb.px, 0), N);
-  eb.vh = min(max(vis_h - jb.py, 0), N);
-  eb.maxv = maxv;
-  const float skip1 = p.use_skip_bits ? p.skip_bits[0][0] : 0.0f;
-  const float skip0 = p.use_skip_bits ? p.skip_bits[0][1] : 0.0f;
-  float* tf = reinterpret_cast<float*>(w.u);
-  int32_t* tmp = w.u + NN;
-  // DCT_DCT, then (refinement) ADST_ADST, ADST_DCT, DCT_ADST, IDTX[, V_DCT,
-  // H_DCT]; nibble k: the k-th type.
-  constexpr uint32_t kTypeOrder = 0x3206541u;
-  const int ntypes = REFINE ? (p.tx_search ? 7 : 5) : 1;
-  int best = 0, btx = MT_TX_DCT_DCT;
-  long long bsse = 0, dct_sse = 0, dct_guard = 0;
-  float bbits = 0.0f;
-#pragma unroll 1
-  for (int k = 0; k < ntypes; k++) {
-    const int t = (int)((kTypeOrder >> (4 * k)) & 15u);
-    const int cur = k == 0 ? 0 : 1 - best;
-    int16_t* cf = w.cfs[cur];
-    int16_t* rr = w.rrs[cur];
-    fwd8x8(w.resid, t, q, cf, tf, tmp);
-    if (t == MT_TX_DCT_DCT || t >= MT_TX_ADST_ADST) {
-      if (qm) apply_qm(cf, tf, sQs, NN);
-      if (a.lambda > 0.0f) trellis_ctx8(cf, tf, dcq, acq, a.lambda, T, ds, qm, qm_full, p.band_tilt, w.tr);
-    }
-    inv8x8(cf, t, q, qm, rr, tmp);
-    eb.resid = rr;
-    const long long asse = sse_recon_block(eb, p.wsse_scale);
-    if (k > 0) {
-      // the gates of block8.rs:1214-1396: the ADST family within tx_guard of
-      // the DCT's SSE, IDTX within tx_guard of the current best's, V / H at
-      // most the current best's
-      bool gate;
-      if (t >= MT_TX_ADST_ADST) gate = asse <= dct_sse + dct_guard;
-      else if (t == MT_TX_IDTX) gate = asse <= bsse + (p.tx_guard_shift >= 63 ? 0 : (bsse >> p.tx_guard_shift));
-      else gate = asse <= bsse;
-      if (!gate) continue;
-    }
-    const float base_rd = k == 0 ? 0.0f : rd_cost_i64(bsse, rd_lam, bbits);
-    float abits;
-    if (t == MT_TX_V_DCT || t == MT_TX_H_DCT) {
-      abits = rate_1d<8>(cf, t == MT_TX_V_DCT, T, ds, jb.mode, w.lv);
-    } else {
-      // unbounded: the DCT and IDTX
-      const float bound = k == 0 || t == MT_TX_IDTX ? __int_as_float(0x7f800000)
-                                                    : __fdiv_rn(__fsub_rn(base_rd, (float)asse), rd_lam);
-      abits = rate_bounded<8>(cf, T, 0, ds, jb.mode, t, p.use_skip_bits != 0, skip1, skip0, bound, w.lv);
-    }
-    if (k == 0 || rd_cost_i64(asse, rd_lam, abits) < base_rd) {
-      best = cur;
-      bsse = asse;
-      bbits = abits;
-      btx = t;
-    }
-    if (k == 0) {
-      dct_sse = asse;
-      dct_guard = p.tx_guard_shift >= 63 ? 0 : (asse >> p.tx_guard_shift);
-    }
-  }
-  r.sse = bsse;
-  r.bits = bbits;
-  r.cost = REFINE ? rd_cost_i64(bsse, rd_lam, bbits) : rd_cost_i64(bsse, rd_lam, __fadd_rn(bbits, jb.syntax_bits));
-  r.tx_type = (uint8_t)btx;
-  for (int i = 0; i < 7; i++) r.reserved[i] = 0;
-  const int16_t* bcf = w.cfs[best];
-  const int16_t* brr = w.rrs[best];
-  if (cf_out) {
-    int4* o = reinterpret_cast<int4*>(cf_out + (size_t)j * NN);
-#pragma unroll 4
-    for (int i = 0; i < NN / 4; i++) o[i] = make_int4(bcf[4 * i], bcf[4 * i + 1], bcf[4 * i + 2], bcf[4 * i + 3]);
-  }
-  if (rec_out) {
-    uint16_t* o = rec_out + (size_t)j * NN;
-#pragma unroll 8
-    for (int i = 0; i < NN; i++) o[i] = (uint16_t)clampi((int32_t)w.pred[i] + brr[i], 0, maxv);
-  }
-}
-
-// Blocks per CTA of the lane kernels: 8 of 16x16 (4 warps) or 5 of 32x32 (5
-// warps), two CTAs of the latter filling an SM's shared memory.
+// Blocks per CTA of the lane kernels: 32 of 8x8 (8 warps: the tables that a CTA
+// stages are a tenth of its work), 8 of 16x16 (4 warps) or 5 of 32x32 (5 warps),
+// two CTAs of the latter filling an SM's shared memory.
 template <int N>
 __host__ __device__ constexpr int lane_blocks() {
-  return N == 32 ? 5 : 8;
+  return N == 32 ? 5 : (N == 16 ? 8 : 32);
 }
 template <int N>
 __host__ __device__ constexpr int lane_threads() {
   return lane_blocks<N>() * N;
 }
 
-// pick_luma16's mode-loop candidates (src/coder/partition_search.rs:4802-4880)
-// and winner refinement (:5252-5474: ADST_ADST, ADST_DCT, DCT_ADST, IDTX with
-// the 8x8 leaf's gates, REFINE), and pick_luma32's mode-loop candidates
+// The leaves' mode-loop candidates -- pick_block8's
+// (src/coder/block8.rs:738-808), pick_luma16's
+// (src/coder/partition_search.rs:4802-4880) and pick_luma32's
 // (src/coder/block32.rs:776-836: TX_32X32 DCT_DCT, the only intra type of that
-// size, trellis_optimize_ctx of class 3, no tx-type symbol in the rate).  N
-// lanes per job.  A rejected job of a warp that holds a good one runs along on
-// the block at the origin and writes its rejection.
-// Bound by instruction issue and the diagonals' latency; HBM is idle.  Measured
-// on the 1080p mode loops, against a thread per job with its working set in
-// local memory: 16x16 (104,520 jobs) 7.7 -> 1.23 ms, 32x32 (25,740 jobs) 33.0
-// -> 1.50 ms.
+// size, trellis_optimize_ctx of class 3, no tx-type symbol in the rate) -- and
+// their winner refinements (REFINE; block8.rs:1183-1404: ADST_ADST, ADST_DCT,
+// DCT_ADST, IDTX and, with tx_search, V_DCT and H_DCT;
+// partition_search.rs:5252-5474: the first five).  N lanes per job.  A rejected
+// job of a warp that holds a good one runs along on the block at the origin and
+// writes its rejection.
+// Bound by instruction issue and fetch and the diagonals' latency; HBM is idle.
+// Measured on the 1080p mode loops, against a thread per job with its working
+// set in local memory: 8x8 (421,200 jobs) 1.38 -> 0.98 ms (300x200: 239 -> 60
+// us), 16x16 (104,520 jobs) 7.7 -> 1.08 ms, 32x32 (25,740 jobs) 33.0 -> 1.40 ms;
+// refinements: 8x8 (32,400 jobs, 7 types) 0.97 -> 0.64 ms (300x200: 796 -> 145
+// us), 16x16 (8,040) 3.84 -> 0.72 ms.
 template <int N, bool REFINE>
 __global__ void __launch_bounds__(lane_threads<N>()) leaf_lanes_kernel(
     const uint16_t* __restrict__ src, const uint16_t* __restrict__ rec, LeafArgs a,
     const uint8_t* __restrict__ qm_row, const mt_coef_costs* __restrict__ costs,
     const mt_leaf8_job* __restrict__ jobs, int n, mt_leaf8_result* __restrict__ res, int32_t* __restrict__ cf_out,
     uint16_t* __restrict__ rec_out) {
-  static_assert(N == 16 || (N == 32 && !REFINE), "16x16, and the 32x32 mode loop");
+  static_assert(N != 32 || !REFINE, "32x32 has one transform type");
   constexpr int NN = N * N;
   using Buf = LaneBuf<N, REFINE>;
   __shared__ LaneTables<NN> S;
@@ -257,18 +110,20 @@ __global__ void __launch_bounds__(lane_threads<N>()) leaf_lanes_kernel(
   const int ds = jb.dcs_ctx;
   lane_predict<N>(PlaneRead{rec, p.stride}, p.frame_w, p.frame_h, jb.px, jb.py, jb.mode, jb.angle_delta, jb.flags & 1,
                   (jb.flags >> 1) & 1, (jb.flags >> 2) & 1, p.bd, w.pred, reinterpret_cast<int32_t*>(&w), g);
-  // DCT_DCT, then (refinement) ADST_ADST, ADST_DCT, DCT_ADST, IDTX (the 16x16
-  // intra set has no V / H); nibble k: the k-th type
-  constexpr uint32_t kTypeOrder = 0x06541u;
+  // DCT_DCT, then (refinement) ADST_ADST, ADST_DCT, DCT_ADST, IDTX and at 8x8
+  // V_DCT, H_DCT (the 16x16 intra set has none); nibble k: the k-th type
+  constexpr uint32_t kTypeOrder = 0x3206541u;
+  const int ntypes = !REFINE ? 1 : (N == 8 && p.tx_search ? 7 : 5);
   int btx = MT_TX_DCT_DCT;
   long long bsse = 0, dct_sse = 0, dct_guard = 0;
   float bbits = 0.0f;
 #pragma unroll 1
-  for (int k = 0; k < (REFINE ? 5 : 1); k++) {
+  for (int k = 0; k < ntypes; k++) {
     const int t = REFINE ? (int)((kTypeOrder >> (4 * k)) & 15u) : MT_TX_DCT_DCT;
     lane_fwd<N>(s0, p.stride, t, q, qm, S.qs, w, g);
+    const bool one = REFINE && N == 8 && (t == MT_TX_V_DCT || t == MT_TX_H_DCT);
     int eob;
-    if (t != MT_TX_IDTX && a.lambda > 0.0f)
+    if (t != MT_TX_IDTX && !one && a.lambda > 0.0f)
       eob = lane_trellis_ctx<N>(w, (float)q.dc_q, (float)q.ac_q, a.lambda, S.T, ds, qm, q.qm_level >= 5, p.band_tilt,
                                 g);
     else
@@ -278,20 +133,29 @@ __global__ void __launch_bounds__(lane_threads<N>()) leaf_lanes_kernel(
     bool gate = true;
     if (REFINE && k > 0) {
       // the ADST family within tx_guard of the DCT's SSE, IDTX within tx_guard
-      // of the current best's (partition_search.rs:5320-5470)
-      gate = t == MT_TX_IDTX ? asse <= bsse + (p.tx_guard_shift >= 63 ? 0 : (bsse >> p.tx_guard_shift))
-                             : asse <= dct_sse + dct_guard;
+      // of the current best's (partition_search.rs:5320-5470,
+      // block8.rs:1214-1396), V / H at most the current best's
+      gate = one ? asse <= bsse
+                 : (t == MT_TX_IDTX ? asse <= bsse + (p.tx_guard_shift >= 63 ? 0 : (bsse >> p.tx_guard_shift))
+                                    : asse <= dct_sse + dct_guard);
       if (!__any_sync(kFull, gate)) continue;
     }
     const float base_rd = k == 0 ? 0.0f : rd_cost_i64(bsse, rd_lam, bbits);
-    // bounded: ADST_ADST (ADST_DCT / DCT_ADST are priced with luma_bits,
-    // partition_search.rs:5396-5404).  tx-type symbol: the 5-type TX_16X16
-    // set drops V_DCT / H_DCT; TX_32X32 codes none.
-    const float bound = !REFINE || t != MT_TX_ADST_ADST ? __int_as_float(0x7f800000)
-                                                        : __fdiv_rn(__fsub_rn(base_rd, (float)asse), rd_lam);
-    const int sym = N == 32 ? -1 : (t >= MT_TX_ADST_ADST ? t - 2 : t);
-    const float abits = lane_rate<N, REFINE>(w, eob, S.T, 0, ds, jb.mode, sym, p.use_skip_bits != 0, skip1, skip0,
-                                             bound, g);
+    // bounded: the ADST family at 8x8, ADST_ADST at 16x16 (ADST_DCT / DCT_ADST
+    // are priced with luma_bits there, partition_search.rs:5396-5404).  tx-type
+    // symbol: the 5-type TX_16X16 set drops V_DCT / H_DCT; TX_32X32 codes none.
+    const bool bounded = REFINE && (N == 8 ? t >= MT_TX_ADST_ADST : t == MT_TX_ADST_ADST);
+    const float bound = bounded ? __fdiv_rn(__fsub_rn(base_rd, (float)asse), rd_lam) : __int_as_float(0x7f800000);
+    const int sym = N == 32 ? -1 : (N == 16 && t >= MT_TX_ADST_ADST ? t - 2 : t);
+    float abits = 0.0f;
+    if (one) {  // the 1-D walk, few of them past their gate, on one lane
+      if (g.j == 0 && gate)
+        abits = rate_1d<N>(w.cf, t == MT_TX_V_DCT, S.T, ds, jb.mode, reinterpret_cast<uint8_t*>(w.t));
+      abits = g.from(abits, 0);
+      g.sync();
+    } else {
+      abits = lane_rate<N, REFINE>(w, eob, S.T, 0, ds, jb.mode, sym, p.use_skip_bits != 0, skip1, skip0, bound, g);
+    }
     if (k == 0 || (gate && rd_cost_i64(asse, rd_lam, abits) < base_rd)) {
       bsse = asse;
       bbits = abits;
@@ -541,16 +405,11 @@ int leaf_device(const uint16_t* d_src, const uint16_t* d_recon, const mt_split16
                                          : 0.0f;
   a.has_qm = quant->qm_level < 15 && d_qm_row != nullptr;
   const cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if constexpr (N == 8) {
-    leaf8_kernel<REFINE><<<(unsigned)((n + kLeafThreads - 1) / kLeafThreads), kLeafThreads, 0, st>>>(
-        d_src, d_recon, a, d_qm_row, d_costs, d_jobs, n, d_results, d_cf, d_rec);
-  } else {
-    constexpr int B = lane_blocks<N>();
-    size_t dyn = 0;
-    if (!lane_smem_bytes<LaneBuf<N, REFINE>>(leaf_lanes_kernel<N, REFINE>, B, &dyn)) return MT_ERR_DEVICE;
-    leaf_lanes_kernel<N, REFINE><<<(unsigned)((n + B - 1) / B), lane_threads<N>(), dyn, st>>>(
-        d_src, d_recon, a, d_qm_row, d_costs, d_jobs, n, d_results, d_cf, d_rec);
-  }
+  constexpr int B = lane_blocks<N>();
+  size_t dyn = 0;
+  if (!lane_smem_bytes<LaneBuf<N, REFINE>>(leaf_lanes_kernel<N, REFINE>, B, &dyn)) return MT_ERR_DEVICE;
+  leaf_lanes_kernel<N, REFINE><<<(unsigned)((n + B - 1) / B), lane_threads<N>(), dyn, st>>>(
+      d_src, d_recon, a, d_qm_row, d_costs, d_jobs, n, d_results, d_cf, d_rec);
   return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_DEVICE;
 }
 
