@@ -101,6 +101,11 @@ struct UvShape {
   static constexpr bool kCtx = k420;
   static constexpr int kSlots = N == 8 ? 8 : (N == 16 ? 6 : 4);
   static constexpr int kThreads = kSlots * N;
+  // CTAs per SM that ptxas keeps registers for.  Shared memory decides it for
+  // the wider blocks; the 8x8 form would take 117 registers (8 CTAs).  At 1080p
+  // 8, 10, 11, 12, 14, 16 CTAs: 939, 907, 870, 872, 891, 917 us (80 registers
+  // hold the chain, below that it spills).
+  static constexpr int kMinCtas = F == UvForm::k16_420 ? 11 : 1;
 };
 
 // One N x N plane of a candidate after its prediction (w.pred): the transform
@@ -278,13 +283,13 @@ __device__ __noinline__ void plane_predict(const uint16_t* __restrict__ rec, int
 // SATD ranking in place of the top-3 and the deltas.
 // Bound by issue, instruction fetch and the chains' latency, HBM is idle.
 // Measured at 1080p against a thread per leaf with its working set in shared
-// memory (3, 10 or 50 KB, so 55, 21 or 4 leaves per SM): k16_420 2.83 -> 0.94 ms,
+// memory (3, 10 or 50 KB, so 55, 21 or 4 leaves per SM): k16_420 2.83 -> 0.87 ms,
 // k16_444 25.2 -> 2.1, k32_420 24.2 -> 0.7, k32_444 56 -> 1.72 ms; of that, code
 // kept short (one transform for both passes, rows four at a time, CfL's column in
-// shared memory; 185 to 350 KB -> 158 to 173) k16_420 1.09 -> 0.94 and k32_444
+// shared memory; 185 to 350 KB -> 158 to 173) k16_420 1.09 -> 0.94 ms and k32_444
 // 2.18 -> 1.72.
 template <UvForm F, typename J>
-__global__ void __launch_bounds__(UvShape<F>::kThreads) uv_kernel(
+__global__ void __launch_bounds__(UvShape<F>::kThreads, UvShape<F>::kMinCtas) uv_kernel(
     const uint16_t* __restrict__ src_u, const uint16_t* __restrict__ src_v, const uint16_t* __restrict__ rec_u,
     const uint16_t* __restrict__ rec_v, const uint16_t* __restrict__ luma, const __grid_constant__ UvArgs a,
     const uint8_t* __restrict__ qm_row, const mt_coef_costs* __restrict__ costs,
