@@ -45,6 +45,16 @@ template <int N>
 __host__ __device__ constexpr int lane_threads() {
   return lane_blocks<N>() * N;
 }
+// The 16x16 mode loop in large CTAs: two of 24 jobs (12 warps) fill an SM's
+// shared memory with 48 jobs, where five of 8 hold 40, and stage a third of the
+// tables: 104,520 jobs 1.08 -> 0.86 ms (14 jobs: 1.01), 22,568 jobs 262 -> 244
+// us.  Where they would fill the device less than twice, small CTAs spread
+// better: 11,440 jobs 146 us in CTAs of 8, 151 of 24; 468 jobs 69 and 76.
+constexpr int kModes16 = 24;
+template <int N, bool REFINE>
+__host__ __device__ constexpr int leaf_max_blocks() {
+  return N == 16 && !REFINE ? kModes16 : lane_blocks<N>();
+}
 
 // The leaves' mode-loop candidates -- pick_block8's
 // (src/coder/block8.rs:738-808), pick_luma16's
@@ -59,11 +69,11 @@ __host__ __device__ constexpr int lane_threads() {
 // Bound by instruction issue and fetch and the diagonals' latency; HBM is idle.
 // Measured on the 1080p mode loops, against a thread per job with its working
 // set in local memory: 8x8 (421,200 jobs) 1.38 -> 0.98 ms (300x200: 239 -> 60
-// us), 16x16 (104,520 jobs) 7.7 -> 1.08 ms, 32x32 (25,740 jobs) 33.0 -> 1.40 ms;
+// us), 16x16 (104,520 jobs) 7.7 -> 0.86 ms, 32x32 (25,740 jobs) 33.0 -> 1.40 ms;
 // refinements: 8x8 (32,400 jobs, 7 types) 0.97 -> 0.64 ms (300x200: 796 -> 145
 // us), 16x16 (8,040) 3.84 -> 0.72 ms.
 template <int N, bool REFINE>
-__global__ void __launch_bounds__(lane_threads<N>()) leaf_lanes_kernel(
+__global__ void __launch_bounds__(leaf_max_blocks<N, REFINE>() * N) leaf_lanes_kernel(
     const uint16_t* __restrict__ src, const uint16_t* __restrict__ rec, LeafArgs a,
     const uint8_t* __restrict__ qm_row, const mt_coef_costs* __restrict__ costs,
     const mt_leaf8_job* __restrict__ jobs, int n, mt_leaf8_result* __restrict__ res, int32_t* __restrict__ cf_out,
@@ -76,7 +86,7 @@ __global__ void __launch_bounds__(lane_threads<N>()) leaf_lanes_kernel(
   S.load(costs, qm_row, a.has_qm);
   const Lanes<N> g;
   Buf& w = reinterpret_cast<Buf*>(lane_smem)[threadIdx.x / N];
-  const int job = blockIdx.x * lane_blocks<N>() + threadIdx.x / N;
+  const int job = blockIdx.x * (blockDim.x / N) + threadIdx.x / N;
   const bool live = job < n;
   const mt_split16_params& p = a.p;
   const mt_quant& q = a.q;
@@ -372,11 +382,13 @@ __global__ void __launch_bounds__(lane_threads<N>()) leaf64_kernel(
   }
 }
 
-// Shared memory of a lane kernel's blocks, opted in for.
+// Shared memory of a CTA of `blocks`, opted in for: always for the kernel's
+// largest CTA, since another thread may be about to launch one.
 template <typename B, typename K>
-bool lane_smem_bytes(K kernel, int blocks, size_t* dyn) {
+bool lane_smem_bytes(K kernel, int blocks, int max_blocks, size_t* dyn) {
   *dyn = sizeof(B) * (size_t)blocks;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*dyn) == cudaSuccess;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(B) * max_blocks)) ==
+         cudaSuccess;
 }
 
 int check(const mt_split16_params* p, const mt_quant* q, int32_t n) {
@@ -405,10 +417,18 @@ int leaf_device(const uint16_t* d_src, const uint16_t* d_recon, const mt_split16
                                          : 0.0f;
   a.has_qm = quant->qm_level < 15 && d_qm_row != nullptr;
   const cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  constexpr int B = lane_blocks<N>();
+  int B = lane_blocks<N>();
+  if constexpr (leaf_max_blocks<N, REFINE>() > lane_blocks<N>()) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      return MT_ERR_DEVICE;
+    if (n >= 2 * 2 * leaf_max_blocks<N, REFINE>() * sms) B = leaf_max_blocks<N, REFINE>();
+  }
   size_t dyn = 0;
-  if (!lane_smem_bytes<LaneBuf<N, REFINE>>(leaf_lanes_kernel<N, REFINE>, B, &dyn)) return MT_ERR_DEVICE;
-  leaf_lanes_kernel<N, REFINE><<<(unsigned)((n + B - 1) / B), lane_threads<N>(), dyn, st>>>(
+  if (!lane_smem_bytes<LaneBuf<N, REFINE>>(leaf_lanes_kernel<N, REFINE>, B, leaf_max_blocks<N, REFINE>(), &dyn))
+    return MT_ERR_DEVICE;
+  leaf_lanes_kernel<N, REFINE><<<(unsigned)((n + (int64_t)B - 1) / B), (unsigned)(B * N), dyn, st>>>(
       d_src, d_recon, a, d_qm_row, d_costs, d_jobs, n, d_results, d_cf, d_rec);
   return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_DEVICE;
 }
@@ -434,7 +454,7 @@ int leaf64_device(const uint16_t* d_src, const uint16_t* d_recon, const mt_split
   a.has_qm = quant->qm_level < 15 && d_qm_row != nullptr;
   constexpr int B = lane_blocks<N>();
   size_t dyn = 0;
-  if (!lane_smem_bytes<LaneBuf<N>>(leaf64_kernel<N, J, R>, B, &dyn)) return MT_ERR_DEVICE;
+  if (!lane_smem_bytes<LaneBuf<N>>(leaf64_kernel<N, J, R>, B, B, &dyn)) return MT_ERR_DEVICE;
   leaf64_kernel<N, J, R><<<(unsigned)((n + B - 1) / B), lane_threads<N>(), dyn,
                            reinterpret_cast<cudaStream_t>(stream)>>>(d_src, d_recon, a, d_qm_row, d_costs, d_jobs, n,
                                                                      d_results, d_cf);

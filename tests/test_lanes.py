@@ -79,6 +79,27 @@ def test_lane_leaves_match_oracle(mt_lib, oracle_lib, cuda, family, n, kind, qid
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("over", [-1, 0, 25])
+def test_leaf16_cta_sizes_match_oracle(mt_lib, oracle_lib, cuda, over):
+    """Job counts around the one from which the 16x16 mode loop runs in CTAs of
+    24 jobs (96 per SM), the last CTA full, with one job, or with all but one."""
+    import torch
+
+    n = 96 * torch.cuda.get_device_properties(0).multi_processor_count + over
+    src, rec = _case("photo", 9)
+    q, qm = oracle_lib.quant_new(90, 8, 6), oracle_lib.qm_row(6, 0, 16)
+    c = oracle_lib.default_cdfs(oracle_lib.qcat(90), 16)
+    jobs = _jobs("leaf16", 9)
+    jobs = jobs[np.random.default_rng(n).integers(0, len(jobs), n)]
+    jobs["mode"][n - 1:] = 13  # rejected
+    prm = mt_lib.split16_params(W, H, trellis_lambda0=0.05, rd_lambda=40.0, band_tilt=1.9, wsse_scale=0.5)
+    got = mt_lib.leaf16(src, rec, prm, q, qm, mt_lib.coef_costs(c), jobs, want_cf=True, want_rec=True)
+    want = oracle_lib.leaf16(src, rec, prm, q, qm, c, jobs, threads=os.cpu_count() or 1)
+    for a, b in zip(got, want):
+        assert np.asarray(a).tobytes() == np.asarray(b).tobytes()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("form", ["16_420", "32_420", "16_444", "32_444"])
 @pytest.mark.parametrize("kind,qidx,cut,wsse,lam0,joint_k,ad", [
     ("photo", 70, (0, 0), 0.0, 0.05, 1, True),
