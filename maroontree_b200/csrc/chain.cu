@@ -260,10 +260,13 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) level8_kernel(const uint
 // instead of a thread with 0.9 KB of local memory that overflows L1 at 12 warps
 // an SM.  Persistent CTAs, a warp per item, so that the tables are staged once a
 // CTA and the warps of the device run one combo at any moment.  For quantisers
-// and lambdas inside the range of 8-bit video (coop_range); 1080p, 13 modes x 4
-// types: 3.31 -> 1.79 ms.
+// and lambdas inside the range of 8-bit video (coop_range); 1080p, 13 modes x 5
+// types: 3.36 -> 1.79 ms.  Seven CTAs an SM: shared memory (28 KB) holds no
+// eighth, and their 71 registers do not spill; 1080p with 4, 5, 6, 7 CTAs: 1.86,
+// 1.84, 1.80, 1.79 ms.
+constexpr int kLanesCtas = 7;
 template <bool VIS>
-__global__ void __launch_bounds__(kThreads, 5) level8_lanes_kernel(
+__global__ void __launch_bounds__(kThreads, kLanesCtas) level8_lanes_kernel(
     const uint16_t* __restrict__ src, ChainArgs a, const uint8_t* __restrict__ qm_row,
     const mt_coef_costs* __restrict__ costs, const mt_block8* __restrict__ blocks, int nblocks,
     const mt_combo* __restrict__ combos, int ncombos, const LevelRuns* __restrict__ runs,
@@ -658,7 +661,8 @@ cudaError_t launch_level8(const uint16_t* src, const uint16_t* rec, const mt_cha
   if (mtd::coop_range(args) && cudaGetDevice(&dev) == cudaSuccess &&
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) {
     const long long items = (long long)((nblocks + 3) / 4) * ncombos, ctas = (items + 3) / 4;
-    const unsigned n = (unsigned)(ctas < 5ll * sms ? ctas : 5ll * sms);
+    const long long most = (long long)mtd::kLanesCtas * sms;
+    const unsigned n = (unsigned)(ctas < most ? ctas : most);
     if (clipped(p))
       mtd::level8_lanes_kernel<true><<<n, mtd::kThreads, 0, st>>>(src, args, qm_row, costs, blocks, nblocks, combos,
                                                                   ncombos, runs, preds, res, keys);
