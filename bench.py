@@ -53,9 +53,9 @@ MPIX = W * H / 1e6
 METRIC = "MPix/s (AVIF encode, mt_encode_rgb8 1920x1080 4:2:0 quality 60)"
 LEVEL_METRIC = "MPix/s (8x8 RDO level, 1080p luma)"
 SMS, LANES_PER_SM = 148, 128  # B200: SMs x INT32/FP32 lanes per SM
-# DRAM bytes of one level8_kernel launch on this workload, dram__bytes_read.sum
-# + dram__bytes_write.sum of the ncu capture in profiles/level8_kernel_1080p_q60.md
-NCU_DRAM_BYTES_PER_LAUNCH = 198_752_000 + 1_367_270_000
+# DRAM bytes of one level8_lanes_kernel launch on this workload, dram__bytes_read.sum
+# + dram__bytes_write.sum of the ncu capture in profiles/level8_lanes_kernel_1080p_q60.md
+NCU_DRAM_BYTES_PER_LAUNCH = 33_382_144 + 18_815_488
 
 # Algorithmic integer / FP32 operations of one 8x8 candidate chain, counted on
 # the oracle's scalar restatement (oracle/oracle_chain.cpp; one add, sub, mul,
@@ -1226,14 +1226,14 @@ def run_ours(args):
 
 # The single measurements of --only: name -> (what it runs).
 ONLY = {
-    "uv16": "pick_uv16_420 over the 8,040 16x16 leaves of the 1080p frame (uv16_420_kernel)",
-    "quad32": "the 64x64 leaf's four-TX_32X32 leg, 480 blocks x 13 modes (quad32_kernel)",
-    "grid16": "the 64x64 leaf's sixteen-TX_16X16 leg, 480 blocks (grid16_kernel)",
-    "leaf32": "the 32x32 leaf's mode-loop candidates, 1,980 blocks x 13 modes (leaf_kernel<32>)",
+    "uv16": "pick_uv16_420 over the 8,040 16x16 leaves of the 1080p frame (uv_kernel)",
+    "quad32": "the 64x64 leaf's four-TX_32X32 leg, 480 blocks x 13 modes (leaf64_kernel)",
+    "grid16": "the 64x64 leaf's sixteen-TX_16X16 leg, 480 blocks (leaf64_kernel)",
+    "leaf32": "the 32x32 leaf's mode-loop candidates, 1,980 blocks x 13 modes (leaf_lanes_kernel<32>)",
     "c3_filters": "the 4096x4096 4:4:4 frame filters: deblocking and CDEF (lf_fused_kernel, the CDEF search)",
-    "uv444": "pick_uv16_444 over the 8,040 16x16 leaves of the 1080p frame at 4:4:4 (uv444_kernel<16>)",
-    "uv32_420": "pick_uv32_420 over the 1,980 32x32 leaves of the 1080p frame (uv32_420_kernel)",
-    "uv32_444": "pick_uv32_444 over the 1,980 32x32 leaves of the 1080p frame at 4:4:4 (uv444_kernel<32>)",
+    "uv444": "pick_uv16_444 over the 8,040 16x16 leaves of the 1080p frame at 4:4:4 (uv_kernel)",
+    "uv32_420": "pick_uv32_420 over the 1,980 32x32 leaves of the 1080p frame (uv_kernel)",
+    "uv32_444": "pick_uv32_444 over the 1,980 32x32 leaves of the 1080p frame at 4:4:4 (uv_kernel)",
 }
 
 
