@@ -55,7 +55,7 @@ LEVEL_METRIC = "MPix/s (8x8 RDO level, 1080p luma)"
 SMS, LANES_PER_SM = 148, 128  # B200: SMs x INT32/FP32 lanes per SM
 # DRAM bytes of one level8_lanes_kernel launch on this workload, dram__bytes_read.sum
 # + dram__bytes_write.sum of the ncu capture in profiles/level8_lanes_kernel_1080p_q60.md
-NCU_DRAM_BYTES_PER_LAUNCH = 33_382_144 + 18_815_488
+NCU_DRAM_BYTES_PER_LAUNCH = 33_389_056 + 18_811_392
 
 # Algorithmic integer / FP32 operations of one 8x8 candidate chain, counted on
 # the oracle's scalar restatement (oracle/oracle_chain.cpp; one add, sub, mul,
