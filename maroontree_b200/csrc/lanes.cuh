@@ -636,7 +636,7 @@ __device__ __forceinline__ int lane_trellis_ctx(W& w, float dc_q, float ac_q, fl
           m_best = lv1;
         }
       }
-      if (c < best_cost || (c == best_cost && e < best_e)) {
+      if (c < best_cost) {  // rising e: the first one on ties; never an infinite cost
         best_cost = c;
         best_e = e;
         best_m = m_best;
@@ -795,7 +795,7 @@ __device__ __forceinline__ int lane_trellis_plain(W& w, float dc_q, float ac_q, 
       const int extra = bin > 1 ? bin - 2 : 0;
       const float sig = __fadd_rn(__fmul_rn((float)bin, 0.9f), __fadd_rn((float)extra, 2.0f));
       const float c = __fadd_rn(__fadd_rn(B[e], __fmul_rn(lambda, sig)), S[e + 1]);
-      if (c < best || (c == best && e < best_e)) {
+      if (c < best) {  // rising e: the first one on ties; never an infinite cost
         best = c;
         best_e = e;
       }
