@@ -1271,10 +1271,22 @@ int job_finish(Job& j, Buffers& buf, int i) {
       cudaStreamWaitEvent(sc, counted.e, 0) != cudaSuccess)
     return MT_ERR_DEVICE;
   cs.d2h(sizeof(tot));
+  // the tiles that go through the entropy coding together: all, but for a frame
+  // of very many tokens
+  mth::StreamGroup grp;
+  grp.ntiles = ntiles;
+  grp.tokens = tot.tokens;
+  if (tot.groups > 1) {
+    if (cudaMemcpyAsync(tile.data(), mth::stream_tiles(j.sg, j.d_plan), tile.size() * sizeof(tile[0]),
+                        cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess)
+      return MT_ERR_DEVICE;
+    cs.d2h(tile.size() * sizeof(tile[0]));
+    grp = mth::stream_group(tile.data(), ntiles, 0);
+  }
   void* d_tok = buf.get<void>(i, kTokens, mth::stream_token_bytes(j.sg, tot.tokens), true);
   if (!d_tok) return MT_ERR_DEVICE;
-  if ((rc = mth::stream_trace(j.sg, j.si, j.d_plan, d_tok, tot.tokens, j.d_cdfs, cfg->updating_cdf != 0, sc, &nl)) !=
-      MT_OK)
+  if ((rc = mth::stream_trace(j.sg, j.si, j.d_plan, d_tok, grp, j.d_cdfs, cfg->updating_cdf != 0, sc, &nl)) != MT_OK)
     return rc;
   // deblocking (uniform 8x8 blocks and transforms) and the CDEF decision
   int32_t ly, luv, sharp;
@@ -1329,7 +1341,7 @@ int job_finish(Job& j, Buffers& buf, int i) {
   } else {
     dec.bits = -1;
   }
-  if ((rc = mth::stream_ranges(j.sg, j.d_plan, d_tok, tot.tokens, d_bits, d_grid, sc, &nl)) != MT_OK) return rc;
+  if ((rc = mth::stream_ranges(j.sg, j.d_plan, d_tok, grp, d_bits, d_grid, sc, &nl)) != MT_OK) return rc;
   if (j.recon_out) {  // the decoder's output: deblocked and CDEF-filtered
     if (cudaMemcpyAsync(j.recon_out[0], flt[0], ny * 2, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaMemcpyAsync(j.recon_out[1], flt[1], nc * 2, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
@@ -1338,28 +1350,41 @@ int job_finish(Job& j, Buffers& buf, int i) {
       return MT_ERR_DEVICE;
     cs.d2h((ny + 2 * nc) * 2);
   }
-  if (cudaMemcpyAsync(&tot, mth::stream_totals(j.sg, j.d_plan), sizeof(tot), cudaMemcpyDeviceToHost, sc) !=
-          cudaSuccess ||
-      cudaMemcpyAsync(tile.data(), mth::stream_tiles(j.sg, j.d_plan), tile.size() * sizeof(tile[0]),
-                      cudaMemcpyDeviceToHost, sc) != cudaSuccess ||
-      cudaStreamSynchronize(sc) != cudaSuccess)
-    return MT_ERR_DEVICE;
-  uint32_t longest = 0;
   size_t ntok = 0;
-  for (const mth::StreamTile& t : tile) {
-    longest = std::max(longest, t.nbytes);
-    ntok += t.ntok;
+  std::vector<uint8_t> payload;
+  std::vector<size_t> tile_at;  // a tile's payload
+  for (;;) {
+    mth::StreamTile* const gt = tile.data() + grp.tile0;
+    const size_t gt_bytes = (size_t)grp.ntiles * sizeof(tile[0]), before = payload.size();
+    if (cudaMemcpyAsync(&tot, mth::stream_totals(j.sg, j.d_plan), sizeof(tot), cudaMemcpyDeviceToHost, sc) !=
+            cudaSuccess ||
+        cudaMemcpyAsync(gt, mth::stream_tiles(j.sg, j.d_plan) + grp.tile0, gt_bytes, cudaMemcpyDeviceToHost, sc) !=
+            cudaSuccess ||
+        cudaStreamSynchronize(sc) != cudaSuccess)
+      return MT_ERR_DEVICE;
+    uint32_t longest = 0;
+    for (int k = 0; k < grp.ntiles; ++k) {
+      longest = std::max(longest, gt[k].nbytes);
+      ntok += gt[k].ntok;
+      tile_at.push_back(before + gt[k].byte);
+    }
+    void* d_dig = buf.get<void>(i, kDigits, mth::stream_digit_bytes(tot), true);
+    if (!d_dig) return MT_ERR_DEVICE;
+    const uint8_t* d_pay = mth::stream_bytes(j.sg, j.d_plan, d_tok, grp, d_dig, tot, longest, sc, &nl);
+    payload.resize(before + tot.bytes);
+    if (!d_pay ||
+        cudaMemcpyAsync(payload.data() + before, d_pay, tot.bytes, cudaMemcpyDeviceToHost, sc) != cudaSuccess ||
+        cudaStreamSynchronize(sc) != cudaSuccess)
+      return MT_ERR_DEVICE;
+    cs.d2h(sizeof(tot) + gt_bytes + tot.bytes);
+    if (grp.tile0 + grp.ntiles == ntiles) break;
+    grp = mth::stream_group(tile.data(), ntiles, grp.tile0 + grp.ntiles);
+    if ((rc = mth::stream_trace(j.sg, j.si, j.d_plan, d_tok, grp, j.d_cdfs, cfg->updating_cdf != 0, sc, &nl)) !=
+            MT_OK ||
+        (rc = mth::stream_ranges(j.sg, j.d_plan, d_tok, grp, d_bits, d_grid, sc, &nl)) != MT_OK)
+      return rc;
   }
-  void* d_dig = buf.get<void>(i, kDigits, mth::stream_digit_bytes(tot), true);
-  if (!d_dig) return MT_ERR_DEVICE;
-  const uint8_t* d_pay =
-      mth::stream_bytes(j.sg, j.d_plan, d_tok, tot.tokens, d_dig, tot, longest, sc, &nl);
-  std::vector<uint8_t> payload(tot.bytes);
-  if (!d_pay || cudaMemcpyAsync(payload.data(), d_pay, tot.bytes, cudaMemcpyDeviceToHost, sc) != cudaSuccess ||
-      cudaStreamSynchronize(sc) != cudaSuccess)
-    return MT_ERR_DEVICE;
   cs.launches(nl);
-  cs.d2h(sizeof(tot) + tile.size() * sizeof(tile[0]) + tot.bytes);
   if (j.plan.cdef) {
     if ((rc = mth::cdef_frame_decision(&cp, d_cs, &dec, nullptr, st)) != MT_OK) return rc;
     size_t cd2h = 0, ch2d = 0;
@@ -1398,9 +1423,9 @@ int job_finish(Job& j, Buffers& buf, int i) {
   fp.tile_rows_log2 = j.trl;
   std::vector<const uint8_t*> ctiles;
   std::vector<size_t> tile_lens;
-  for (const mth::StreamTile& t : tile) {
-    ctiles.push_back(payload.data() + t.byte);
-    tile_lens.push_back(t.nbytes);
+  for (int t = 0; t < ntiles; ++t) {
+    ctiles.push_back(payload.data() + tile_at[(size_t)t]);
+    tile_lens.push_back(tile[(size_t)t].nbytes);
   }
   uint8_t* obu = nullptr;
   size_t obu_len = 0;

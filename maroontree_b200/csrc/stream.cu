@@ -62,6 +62,7 @@ struct StreamPlan {
 namespace {
 
 using mth::StreamGeom;
+using mth::StreamGroup;
 using mth::StreamInput;
 using mth::StreamPlan;
 using mth::StreamTile;
@@ -167,7 +168,7 @@ constexpr int kLevStride = 12, kLevRows = 10;
 // token writes.
 template <int N, bool LUMA, bool WRITE>
 __global__ void __launch_bounds__(128) units_kernel(const StreamGeom g, const StreamInput in, const StreamPlan p,
-                                                    uint16_t* __restrict__ tokens) {
+                                                    const StreamGroup grp, uint16_t* __restrict__ tokens) {
   constexpr int PER = N * N / 8, LG = N == 8 ? 3 : 2;
   __shared__ __align__(16) int32_t cfs[16][64];
   __shared__ uint8_t lev[16][kLevStride * kLevRows];
@@ -252,7 +253,7 @@ __global__ void __launch_bounds__(128) units_kernel(const StreamGeom g, const St
     return;
   }
   __syncwarp();
-  if (!live) return;
+  if (!live || (uint32_t)(pl.tile - grp.tile0) >= (uint32_t)grp.ntiles) return;
   uint32_t o = p.off[slot] + p.bpre[slot / kScanBlock] + p.delta[pl.tile];
   auto tok = [&](uint32_t at, int id, uint32_t s) { tokens[at] = (uint16_t)(id | (s << 8)); };
   const bool has_t = y > pl.ty0, has_l = x > pl.tx0;
@@ -369,7 +370,12 @@ __global__ void __launch_bounds__(128) units_kernel(const StreamGeom g, const St
 
 // ---------------------------------------------------------------------------
 // Placement: an exclusive scan of the 3 nb counts, 4096 per CTA, then of the
-// CTAs' sums, which also lays the tiles out.
+// CTAs' sums, which also lays the tiles out, in groups of whole tiles that the
+// following steps take one after the other in the same buffers.  A frame's total
+// may pass 32 bits (from some 75 Mpx of 4:4:4 noise at quality 99 on), and the
+// running sums here wrap; a tile's extent and its place in its group do not:
+// at most 31 tokens per coefficient (levels below 2^13 at the finest steps) and
+// 2,376 superblocks make under 2^30, and differences of wrapped sums are exact.
 
 __device__ __forceinline__ uint32_t block_scan_1024(uint32_t v, uint32_t* warp_sum, uint32_t* total) {
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
@@ -434,15 +440,22 @@ __global__ void __launch_bounds__(1024) scan_blocks_kernel(const StreamGeom g, c
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    uint32_t base = 0;
+    uint32_t base = 0, most = 0, groups = 1;
     for (int k = 0; k < nt; ++k) {
       const uint32_t start = p.delta[k], end = k + 1 < nt ? p.delta[k + 1] : carry;
+      const uint32_t n = (end - start + kGroupTokens - 1) / kGroupTokens * kGroupTokens;
+      if (base && (base >= g.max_tokens || n > g.max_tokens - base)) {  // the next group
+        base = 0;
+        ++groups;
+      }
       p.tile[k].base = base;
       p.tile[k].ntok = end - start;
       p.delta[k] = base - start;
-      base += (end - start + kGroupTokens - 1) / kGroupTokens * kGroupTokens;
+      base += n;
+      most = max(most, base);
     }
-    p.total->tokens = base;
+    p.total->tokens = most;
+    p.total->groups = groups;
   }
 }
 
@@ -837,11 +850,14 @@ __global__ void __launch_bounds__(256) fix_kernel(const Lists L, const StreamTil
 // ---------------------------------------------------------------------------
 // The range coder.
 
-__global__ void cdef_fill_kernel(const StreamPlan p, uint32_t* __restrict__ st, const int32_t* __restrict__ bits,
+__global__ void cdef_fill_kernel(const StreamGeom g, const StreamPlan p, const StreamGroup grp,
+                                 uint32_t* __restrict__ st, const int32_t* __restrict__ bits,
                                  const uint8_t* __restrict__ grid, int nsb) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int n = *bits;
   if (i >= nsb || n <= 0 || n > 3) return;
+  const int tile = i / g.sb_cols * 8 / g.tile_h8 * g.tcols + i % g.sb_cols * 8 / g.tile_w8;
+  if ((uint32_t)(tile - grp.tile0) >= (uint32_t)grp.ntiles) return;
   for (int k = 0; k < n; ++k) st[p.cdef_at[i] + k] = bool_word((grid[i] >> (n - 1 - k)) & 1);
 }
 
@@ -1095,10 +1111,10 @@ __global__ void __launch_bounds__(kGroup) ranges_kernel(const Lists L, const Str
 
 // The bits before every group of its tile, and where the tiles' digits and
 // bytes go.
-__global__ void __launch_bounds__(1024) shift_scan_kernel(const Lists L, const StreamPlan p, int nt) {
+__global__ void __launch_bounds__(1024) shift_scan_kernel(const Lists L, const StreamPlan p, const StreamGroup grp) {
   __shared__ uint32_t ws[32];
   uint32_t digit = 0, byte = 0;
-  for (int k = 0; k < nt; ++k) {
+  for (int k = grp.tile0; k < grp.tile0 + grp.ntiles; ++k) {
     const StreamTile ti = p.tile[k];
     const int g0 = (int)(ti.base / kGroupTokens), n = (int)((ti.ntok + kGroupTokens - 1) / kGroupTokens);
     uint32_t carry = 0;
@@ -1240,14 +1256,14 @@ size_t carve_lists(const StreamGeom& g, uint32_t padded, void* mem, Lists* L) {
 int status() { return cudaGetLastError() == cudaSuccess ? MT_OK : MT_ERR_DEVICE; }
 
 template <bool WRITE>
-void launch_units(const StreamGeom& g, const StreamInput& in, const StreamPlan& p, uint16_t* tokens,
-                  cudaStream_t st) {
+void launch_units(const StreamGeom& g, const StreamInput& in, const StreamPlan& p, const StreamGroup& grp,
+                  uint16_t* tokens, cudaStream_t st) {
   const unsigned n = (unsigned)(((size_t)g.nbx * g.nby + 15) / 16);
-  units_kernel<8, true, WRITE><<<n, 128, 0, st>>>(g, in, p, tokens);
+  units_kernel<8, true, WRITE><<<n, 128, 0, st>>>(g, in, p, grp, tokens);
   if (g.sub)
-    units_kernel<4, false, WRITE><<<dim3(n, 2), 128, 0, st>>>(g, in, p, tokens);
+    units_kernel<4, false, WRITE><<<dim3(n, 2), 128, 0, st>>>(g, in, p, grp, tokens);
   else
-    units_kernel<8, false, WRITE><<<dim3(n, 2), 128, 0, st>>>(g, in, p, tokens);
+    units_kernel<8, false, WRITE><<<dim3(n, 2), 128, 0, st>>>(g, in, p, grp, tokens);
 }
 
 uint16_t g_cdfs[8][256 * kCdfEntries];  // by quantiser context and chroma transform size
@@ -1284,14 +1300,26 @@ const void* stream_cdf_table(int qctx, int sub) {
 int stream_count(const StreamGeom& g, const StreamInput& in, void* plan, cudaStream_t st, int* launches) {
   StreamPlan p;
   carve_plan(g, plan, &p);
-  launch_units<false>(g, in, p, nullptr, st);
+  launch_units<false>(g, in, p, StreamGroup{}, nullptr, st);
+  *launches += 2;
+  return stream_place(g, plan, st, launches);
+}
+
+int stream_place(const StreamGeom& g, void* plan, cudaStream_t st, int* launches) {
+  StreamPlan p;
+  carve_plan(g, plan, &p);
   const int n = 3 * g.nbx * g.nby, nblk = (n + kScanBlock - 1) / kScanBlock;
   scan_local_kernel<<<nblk, 1024, 0, st>>>(p.off, n, p.bpre);
   scan_blocks_kernel<<<1, 1024, 0, st>>>(g, p, nblk);
-  *launches += 4;
+  *launches += 2;
   return status();
 }
 
+uint32_t* stream_counts(const StreamGeom& g, void* plan) {
+  StreamPlan p;
+  carve_plan(g, plan, &p);
+  return p.off;
+}
 const StreamTotals* stream_totals(const StreamGeom& g, void* plan) {
   StreamPlan p;
   carve_plan(g, plan, &p);
@@ -1303,58 +1331,70 @@ const StreamTile* stream_tiles(const StreamGeom& g, void* plan) {
   return p.tile;
 }
 
-int stream_trace(const StreamGeom& g, const StreamInput& in, void* plan, void* tokens, uint32_t padded,
+StreamGroup stream_group(const StreamTile* tiles, int ntiles, int tile0) {
+  StreamGroup grp;
+  grp.tile0 = tile0;
+  for (int k = tile0; k < ntiles && (k == tile0 || tiles[k].base != 0); ++k) {
+    grp.ntiles += 1;
+    grp.tokens = tiles[k].base + (tiles[k].ntok + kGroupTokens - 1) / kGroupTokens * kGroupTokens;
+  }
+  return grp;
+}
+
+int stream_trace(const StreamGeom& g, const StreamInput& in, void* plan, void* tokens, const StreamGroup& grp,
                  const void* d_cdfs, bool updating, cudaStream_t st, int* launches) {
   StreamPlan p;
   Lists L;
   carve_plan(g, plan, &p);
-  carve_lists(g, padded, tokens, &L);
-  const int nt = g.tcols * g.trows;
-  launch_units<true>(g, in, p, L.tok, st);
-  hist_kernel<<<padded / kPart / 4, 128, 0, st>>>(L, p.tile, nt);
-  part_scan_kernel<<<nt, 1024, 0, st>>>(L, p.tile);
-  scatter_kernel<<<padded / kPart / 4, 128, 0, st>>>(L, p.tile, nt);
+  carve_lists(g, grp.tokens, tokens, &L);
+  const StreamTile* tile = p.tile + grp.tile0;
+  const int nt = grp.ntiles;
+  launch_units<true>(g, in, p, grp, L.tok, st);
+  hist_kernel<<<grp.tokens / kPart / 4, 128, 0, st>>>(L, tile, nt);
+  part_scan_kernel<<<nt, 1024, 0, st>>>(L, tile);
+  scatter_kernel<<<grp.tokens / kPart / 4, 128, 0, st>>>(L, tile, nt);
   const uint16_t* cdfs = static_cast<const uint16_t*>(d_cdfs);
-  const unsigned ns = padded / kSeg + 256 * nt;
-  first_kernel<<<ns / 4, 128, 0, st>>>(L, p.tile, nt, cdfs, updating);
-  trace_kernel<<<ns / 4, 128, 0, st>>>(L, p.tile, nt, cdfs, updating);
-  fix_kernel<<<dim3(kIds, nt), 256, 0, st>>>(L, p.tile, cdfs, updating);
+  const unsigned ns = grp.tokens / kSeg + 256 * nt;
+  first_kernel<<<ns / 4, 128, 0, st>>>(L, tile, nt, cdfs, updating);
+  trace_kernel<<<ns / 4, 128, 0, st>>>(L, tile, nt, cdfs, updating);
+  fix_kernel<<<dim3(kIds, nt), 256, 0, st>>>(L, tile, cdfs, updating);
   *launches += 8;
   return status();
 }
 
-int stream_ranges(const StreamGeom& g, void* plan, void* tokens, uint32_t padded, const int32_t* bits,
+int stream_ranges(const StreamGeom& g, void* plan, void* tokens, const StreamGroup& grp, const int32_t* bits,
                   const uint8_t* grid, cudaStream_t st, int* launches) {
   StreamPlan p;
   Lists L;
   carve_plan(g, plan, &p);
-  carve_lists(g, padded, tokens, &L);
-  const int nt = g.tcols * g.trows, nsb = g.sb_cols * g.sb_rows;
+  carve_lists(g, grp.tokens, tokens, &L);
+  const StreamTile* tile = p.tile + grp.tile0;
+  const int nt = grp.ntiles, nsb = g.sb_cols * g.sb_rows;
   if (bits) {
-    cdef_fill_kernel<<<(nsb + 127) / 128, 128, 0, st>>>(p, L.st, bits, grid, nsb);
+    cdef_fill_kernel<<<(nsb + 127) / 128, 128, 0, st>>>(g, p, grp, L.st, bits, grid, nsb);
     *launches += 1;
   }
-  map_kernel<<<padded / kChunk / 4, 128, 0, st>>>(L, p.tile, nt);
-  compose_kernel<<<padded / kGroupTokens, kClasses, 0, st>>>(L);
-  walk_kernel<<<nt, 256, 0, st>>>(L, p.tile);
-  ranges_kernel<<<padded / kGroupTokens, kGroup, 0, st>>>(L, p.tile, nt);
-  shift_scan_kernel<<<1, 1024, 0, st>>>(L, p, nt);
+  map_kernel<<<grp.tokens / kChunk / 4, 128, 0, st>>>(L, tile, nt);
+  compose_kernel<<<grp.tokens / kGroupTokens, kClasses, 0, st>>>(L);
+  walk_kernel<<<nt, 256, 0, st>>>(L, tile);
+  ranges_kernel<<<grp.tokens / kGroupTokens, kGroup, 0, st>>>(L, tile, nt);
+  shift_scan_kernel<<<1, 1024, 0, st>>>(L, p, grp);
   *launches += 5;
   return status();
 }
 
-const uint8_t* stream_bytes(const StreamGeom& g, void* plan, void* tokens, uint32_t padded, void* digits,
+const uint8_t* stream_bytes(const StreamGeom& g, void* plan, void* tokens, const StreamGroup& grp, void* digits,
                             const StreamTotals& t, uint32_t max_bytes, cudaStream_t st, int* launches) {
   StreamPlan p;
   Lists L;
   carve_plan(g, plan, &p);
-  carve_lists(g, padded, tokens, &L);
-  const int nt = g.tcols * g.trows;
+  carve_lists(g, grp.tokens, tokens, &L);
+  const StreamTile* tile = p.tile + grp.tile0;
   uint32_t* dg = static_cast<uint32_t*>(digits);
   uint8_t* out = static_cast<uint8_t*>(digits) + up256((size_t)t.digits * 4);
   if (cudaMemsetAsync(dg, 0, (size_t)t.digits * 4, st) != cudaSuccess) return nullptr;
-  digits_kernel<<<padded / kChunk / 4, 128, 0, st>>>(L, p.tile, nt, dg);
-  bytes_kernel<<<dim3((max_bytes + 511) / 512, nt), 256, 0, st>>>(p.tile, dg, out);
+  digits_kernel<<<grp.tokens / kChunk / 4, 128, 0, st>>>(L, tile, grp.ntiles, dg);
+  bytes_kernel<<<dim3((max_bytes + 511) / 512, grp.ntiles), 256, 0, st>>>(tile, dg, out);
   *launches += 2;
   return status() == MT_OK ? out : nullptr;
 }
