@@ -1475,10 +1475,15 @@ void encode_jobs(std::vector<Job>& jobs) {
     if (jobs[0].rc == MT_OK) jobs[0].rc = job_finish(jobs[0], buf, 0);
     return;
   }
+  int dev = 0;  // a new thread starts on device 0; the streams and buffers are the caller's device's
+  const bool have_dev = cudaGetDevice(&dev) == cudaSuccess;
   std::vector<std::thread> pool;
   for (int i = 0; i < n; ++i)
     if (jobs[(size_t)i].rc == MT_OK)
-      pool.emplace_back([&jobs, &buf, i]() { jobs[(size_t)i].rc = job_finish(jobs[(size_t)i], buf, i); });
+      pool.emplace_back([&jobs, &buf, i, dev, have_dev]() {
+        jobs[(size_t)i].rc =
+            have_dev && cudaSetDevice(dev) == cudaSuccess ? job_finish(jobs[(size_t)i], buf, i) : MT_ERR_DEVICE;
+      });
   for (std::thread& t : pool) t.join();
 }
 
