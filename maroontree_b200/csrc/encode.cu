@@ -246,10 +246,15 @@ struct StepShared {
 
 __device__ __forceinline__ void luma_bar() { asm volatile("bar.sync 1, %0;" ::"n"(kLumaThreads) : "memory"); }
 
-// A wait gives up after this many polls of a record in global memory, of a word
-// or of a barrier in shared memory (the last two longer: what they wait for may
-// be waiting for a record), and sets *err; a set *err ends all of them.
-constexpr int kMaxPolls = 1 << 20, kMaxWordPolls = 1 << 23, kMaxBarPolls = 1 << 20;
+// Every wait gives up after a number of polls and sets *err.  Of them only the
+// waits for records, which depend on other clusters, end early on a set *err:
+// what a cluster's CTAs tell each other (keys, marks, words) still comes, late
+// by one such wait at most, since every warp goes on to its key or mark, and
+// cutting those waits short would let a word be overwritten, or a barrier armed
+// twice, before all have seen it.  Their limits are there for what cannot
+// happen, each several times what it waits for: a record's wait lasts some
+// 0.2 s, the fetching warp's waits 3 to 4 s each, the one for its word 27 s.
+constexpr int kMaxPolls = 1 << 20, kMaxWordPolls = 1 << 24, kMaxBarPolls = 1 << 23;
 
 __device__ __forceinline__ uint4 wait_rec(const uint4* p, uint32_t* err) {
   uint4 v = get_rec(p);
@@ -284,7 +289,8 @@ __device__ __forceinline__ void put_key(const unsigned long long* slot, const un
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.u64 [%0], %1, [%2];" ::"r"(rs), "l"(key), "r"(rb)
                : "memory");
 }
-__device__ __forceinline__ void wait_keys(const unsigned long long* bar, uint32_t phase, uint32_t* err) {
+// False when the limit has passed.
+__device__ __forceinline__ bool wait_keys(const unsigned long long* bar, uint32_t phase, uint32_t* err) {
   for (int it = 1;; ++it) {
     uint32_t ok;
     asm volatile(
@@ -293,57 +299,55 @@ __device__ __forceinline__ void wait_keys(const unsigned long long* bar, uint32_
         : "=r"(ok)
         : "r"(smem_addr(bar)), "r"(phase)
         : "memory");
-    if (__all_sync(0xffffffffu, ok != 0)) return;
-    uint32_t ab = 0;
-    if ((it & 15) == 0) ab = *(volatile uint32_t*)err;
-    if (__any_sync(0xffffffffu, ab != 0)) return;
+    if (__all_sync(0xffffffffu, ok != 0)) return true;
     if (it > kMaxBarPolls) {
       if ((threadIdx.x & 31) == 0) atomicExch(err, 1u);
-      return;
+      return false;
     }
+    if (it > 1024) __nanosleep(500);
   }
 }
 
 // The chroma warps' marks of a block (the fetching warp; lanes 0 and 1).
-__device__ __forceinline__ void wait_marks(const unsigned long long* mark, uint32_t seq, uint32_t* err) {
+__device__ __forceinline__ bool wait_marks(const unsigned long long* mark, uint32_t seq, uint32_t* err) {
   const int lane = threadIdx.x & 31;
   for (int it = 1; !__all_sync(0xffffffffu, lane >= 2 || (uint32_t)get_word(mark + (lane & 1)) == seq); ++it) {
-    const uint32_t ab = lane == 0 ? *(volatile uint32_t*)err : 0;
-    if (__any_sync(0xffffffffu, ab != 0)) return;
     if (it > kMaxWordPolls) {
       if (lane == 0) atomicExch(err, 1u);
-      return;
+      return false;
     }
     __nanosleep(200);
   }
+  return true;
 }
 
 // Until the CTA's luma warps have block seq's edges: a ticket taken earlier
 // would sit behind a block that is still waiting, while another cluster may be
 // free to code it.
-__device__ __forceinline__ void wait_begun(const uint32_t* begun, uint32_t seq, uint32_t* err) {
-  for (int it = 1; *(volatile const uint32_t*)begun != seq; ++it) {
-    if ((it & 15) == 0 && *(volatile uint32_t*)err) return;
-    if (it > kMaxWordPolls) {
-      atomicExch(err, 1u);
-      return;
+__device__ __forceinline__ bool wait_begun(const uint32_t* begun, uint32_t seq, uint32_t* err) {
+  for (int it = 1; !__all_sync(0xffffffffu, *(volatile const uint32_t*)begun == seq); ++it) {
+    if (it > 2 * kMaxWordPolls) {
+      if ((threadIdx.x & 31) == 0) atomicExch(err, 1u);
+      return false;
     }
     __nanosleep(100);
   }
+  return true;
 }
 
-// The block of sequence number seq.  Its word comes from the cluster's
-// fetching warp, whose own waits end, so that every warp of the cluster gets
-// the same blocks and leaves at the same one.
+// The block of sequence number seq (a warp, all lanes the same).  Its word comes
+// from the cluster's fetching warp, which writes it to every CTA or, when one of
+// its own waits has run out, to none: every warp of the cluster gets the same
+// blocks and leaves at the same one.
 constexpr unsigned long long kEnd = 1ull << 39;
 __device__ __forceinline__ unsigned long long wait_next(const unsigned long long* next, uint32_t seq, uint32_t* err) {
   unsigned long long v = get_word(next);
-  for (int it = 1; (uint32_t)(v >> 40) != (seq & kSeqMask); ++it) {
-    if (it > 8 * kMaxWordPolls) {
-      atomicExch(err, 1u);
+  for (int it = 1; !__all_sync(0xffffffffu, (uint32_t)(v >> 40) == (seq & kSeqMask)); ++it) {
+    if (it > 4 * kMaxWordPolls) {
+      if ((threadIdx.x & 31) == 0) atomicExch(err, 1u);
       return kEnd;
     }
-    if (it > 4) __nanosleep(100);
+    if (it > 4) __nanosleep(it > 4096 ? 400 : 100);
     v = get_word(next);
   }
   return v;
@@ -432,9 +436,10 @@ __device__ __forceinline__ void chroma_finish(const ChromaBlock& k, uint4* edges
 //
 // Tickets follow the dependency levels, so the lowest unfinished ticket's
 // cluster has nothing left to wait for: a cluster holds a later ticket only
-// while it works on an earlier one.  A wait that runs out of polls sets *err;
-// once *err is set the remaining waits stop and every cluster leaves at the
-// end its fetching warp writes.
+// while it works on an earlier one.  A wait for a record that runs out of polls
+// sets *err; once it is set the other waits for records stop, the blocks in hand
+// are coded from what there is, and every cluster leaves at the end that its
+// fetching warp writes.
 // list[i] = (entry, image).
 //
 // Bound by the dependency chain: a level's latency is the record's way between
@@ -469,11 +474,10 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThre
   if (warp == kSideWarp && rank < 2) {
     if (rank == 0) {  // the fetching warp
       for (uint32_t seq = 1;; ++seq) {
-        if (seq > 2) {
-          wait_keys(&S.key_bar[seq & 1], ((seq - 3) >> 1) & 1, err);
-          wait_marks(S.mark[seq & 1], (seq - 2) & kSeqMask, err);
-        }
-        if (late && seq > 1) wait_begun(&S.begun, seq - 1, err);
+        if (seq > 2 && (!wait_keys(&S.key_bar[seq & 1], ((seq - 3) >> 1) & 1, err) ||
+                        !wait_marks(S.mark[seq & 1], (seq - 2) & kSeqMask, err)))
+          break;
+        if (late && seq > 1 && !wait_begun(&S.begun, seq - 1, err)) break;
         uint32_t stop = 0;
         if (lane == 0) {
           const uint32_t tk = atomicAdd(ticket_ctr, 1u);
@@ -499,8 +503,9 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThre
   int cur = -1;                                                 // the image whose tables are staged
   unsigned long long ahead = 0;                                 // the next block's word, if it was there early
   for (uint32_t seq = 1;; ++seq) {
-    const unsigned long long nx =
-        (uint32_t)(ahead >> 40) == (seq & kSeqMask) ? ahead : wait_next(&S.next[seq & 1], seq, err);
+    unsigned long long nx = ahead;
+    if (!__all_sync(0xffffffffu, (uint32_t)(ahead >> 40) == (seq & kSeqMask)))
+      nx = wait_next(&S.next[seq & 1], seq, err);
     if (nx & kEnd) break;  // the same for every warp of the cluster
     const int img = (int)(nx >> 32) & 127;
     if (img != cur) {  // another image: its descriptor, then its tables
@@ -661,8 +666,8 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThre
 #pragma unroll
     for (int q = 0; q < 8; ++q) col[q >> 2] |= (uint32_t)rv[q] << (8 * (q & 3));
     ahead = get_word(&S.next[(seq + 1) & 1]);
-    wait_keys(&S.key_bar[seq & 1], ((seq - 1) >> 1) & 1, err);
-    if (t == 0) key_bar_arm(&S.key_bar[seq & 1]);  // for block seq + 2
+    const bool complete = wait_keys(&S.key_bar[seq & 1], ((seq - 1) >> 1) & 1, err);
+    if (t == 0 && complete) key_bar_arm(&S.key_bar[seq & 1]);  // for block seq + 2
     const unsigned long long all = S.key[seq & 1][lane];
     const uint32_t cst = lane < kLumaKeys ? (uint32_t)(all >> 32) : 0xffffffffu;
     const uint32_t low = __reduce_min_sync(0xffffffffu, cst);
@@ -686,8 +691,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThre
     __syncwarp();
   }
   // None may leave while another CTA can still write to its shared memory: the
-  // keys of the last block have been waited for, unless the waits were cut
-  // short.
+  // keys of the last block have been waited for, unless that wait has run out.
   if (*(volatile uint32_t*)err)
     for (int i = 0; i < 32; ++i) __nanosleep(1000);
   cluster.sync();
@@ -1144,7 +1148,8 @@ int job_setup(Job& j, Buffers& buf, int i) {
 // blocks merged wave by wave into one ticket list (each image's order is
 // still a dependency order), the persistent clusters taking tickets across
 // images.
-int decide_all(std::vector<Job>& jobs, Buffers& buf) {
+// skip: tickets left out at the list's start (none but to test the waits' end).
+int decide_all(std::vector<Job>& jobs, Buffers& buf, int skip) {
   std::vector<JobDesc> descs;
   std::vector<int> slot;  // job index per descriptor
   size_t total = 0;
@@ -1205,8 +1210,8 @@ int decide_all(std::vector<Job>& jobs, Buffers& buf) {
   constexpr int dyn = kGroupBufs * (int)sizeof(mtd::GroupBuf);
   if (cudaFuncSetAttribute(encode_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) != cudaSuccess)
     return MT_ERR_DEVICE;
-  encode_blocks_kernel<<<nclusters * kClusterCtas, kStepThreads, dyn, ks>>>(d_jobs, d_list, (int)total, d_ctl,
-                                                                            d_ctl + 1, late);
+  encode_blocks_kernel<<<nclusters * kClusterCtas, kStepThreads, dyn, ks>>>(d_jobs, d_list + skip, (int)total - skip,
+                                                                            d_ctl, d_ctl + 1, late);
   for (int d : slot) {
     jobs[(size_t)d].cs->mark(2, ks);
     jobs[(size_t)d].cs->launches(4);
@@ -1464,11 +1469,11 @@ int job_finish(Job& j, Buffers& buf, int i) {
 // their decisions, then each image's finishing work on a host thread of its
 // own (the calling thread for one image).  Every image's bytes are those of
 // encoding it alone.
-void encode_jobs(std::vector<Job>& jobs) {
+void encode_jobs(std::vector<Job>& jobs, int skip = 0) {
   const int n = (int)jobs.size();
   Buffers buf(n);
   for (int i = 0; i < n; ++i) jobs[(size_t)i].rc = job_setup(jobs[(size_t)i], buf, i);
-  const int rc = decide_all(jobs, buf);
+  const int rc = decide_all(jobs, buf, skip);
   for (Job& j : jobs)
     if (j.rc == MT_OK && rc != MT_OK) j.rc = rc;
   if (n == 1) {
@@ -1489,7 +1494,7 @@ void encode_jobs(std::vector<Job>& jobs) {
 
 int encode_one(const uint8_t* rgb, bool rgb_on_device, const uint8_t* const* yuv, uint32_t width, uint32_t height,
                const mt_encode_config* cfg, uint8_t** out, size_t* out_len, uint16_t* recon_out[3],
-               mt_encode_stats* stats) {
+               mt_encode_stats* stats, int skip = 0) {
   std::vector<Job> jobs(1);
   Job& j = jobs[0];
   j.rgb = rgb;
@@ -1502,11 +1507,23 @@ int encode_one(const uint8_t* rgb, bool rgb_on_device, const uint8_t* const* yuv
   j.out_len = out_len;
   j.recon_out = recon_out;
   j.stats = stats;
-  encode_jobs(jobs);
+  encode_jobs(jobs, skip);
   return j.rc;
 }
 
 }  // namespace
+
+namespace mth {
+// mt_encode_rgb8 of a frame whose first block nobody codes: the waits for its
+// records run out, and the call returns MT_ERR_DEVICE.
+int encode_without_first_block(const uint8_t* rgb, uint32_t width, uint32_t height, const mt_encode_config* cfg) {
+  uint8_t* out = nullptr;
+  size_t len = 0;
+  const int rc = encode_one(rgb, false, nullptr, width, height, cfg, &out, &len, nullptr, nullptr, 1);
+  free(out);
+  return rc;
+}
+}  // namespace mth
 
 extern "C" {
 
