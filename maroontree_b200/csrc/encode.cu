@@ -967,6 +967,31 @@ int tile_levels(int w, int h) {
   return n + (more_c ? more_c * (n - count(w - 8, h)) : 0) + (more_r ? more_r * (n - count(w, h - 8)) : 0);
 }
 
+}  // namespace
+
+namespace mth {
+// The most blocks that a tile of cols x rows superblocks has in one wave (a
+// tile's partial superblocks have fewer): a superblock's blocks by their wave,
+// then along a row and over the rows as running sums at the waves' strides.
+int widest_wave(int cols, int rows) {
+  const int n = kWaveCol * (cols - 1) + kWaveRow * (rows - 1) + kWave.last + 1;
+  std::vector<int> sum((size_t)n), at((size_t)n, 0);
+  for (const auto& row : kWave.t)
+    for (uint8_t t : row) at[t] += 1;
+  auto along = [&](int stride, int count) {
+    for (int i = 0; i < n; ++i)
+      sum[(size_t)i] = at[(size_t)i] + (i >= stride ? sum[(size_t)(i - stride)] : 0) -
+                       (i >= stride * count ? at[(size_t)(i - stride * count)] : 0);
+    at.swap(sum);
+  };
+  along(kWaveCol, cols);
+  along(kWaveRow, rows);
+  return *std::max_element(at.begin(), at.end());
+}
+}  // namespace mth
+
+namespace {
+
 int frame_levels(int nbx, int nby, int tile_w8, int tile_h8) {
   int n = 0;  // the full tiles and the last ones of the rows and columns
   for (int w : {std::min(tile_w8, nbx), nbx - (nbx - 1) / tile_w8 * tile_w8})
@@ -1163,8 +1188,7 @@ int decide_all(std::vector<Job>& jobs, Buffers& buf, int skip) {
       nb_max = std::max(nb_max, j.nb);
       const int tc = std::min(j.tile_sb_w, j.sb_cols), tr = std::min(j.tile_sb_h, j.sb_rows);
       waves = std::max(waves, kWaveCol * (tc - 1) + kWaveRow * (tr - 1) + kWave.last + 1);
-      // blocks of a wave: under three (64 over kWaveCol) per superblock row that it crosses
-      width_max += j.sg.tcols * j.sg.trows * (3 * std::min(tr, kWaveCol * tc / kWaveRow + 2) + 2);
+      width_max += j.sg.tcols * j.sg.trows * mth::widest_wave(tc, tr);
     }
   if (slot.empty()) return MT_OK;
   const int i0 = slot[0];
@@ -1191,14 +1215,16 @@ int decide_all(std::vector<Job>& jobs, Buffers& buf, int skip) {
   list_kernel<false><<<lg, 256, 0, ks>>>(d_jobs, d_wave, nullptr);
   wave_scan_kernel<<<1, 1024, 0, ks>>>(d_wave, waves);
   list_kernel<true><<<lg, 256, 0, ks>>>(d_jobs, d_wave, d_list);
-  // one cluster per block that can run at once (the widest merged wave), at
-  // most as many as the SMs hold
+  // one cluster per block that can run at once (no merged wave is wider than the
+  // tiles' widest together) and a quarter more, since a cluster that writes its
+  // block is not free yet (512x512 4:4:4, 20 blocks: 2.84 ms with 20 clusters, 2.82
+  // with 25), at most as many as the SMs hold
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
     return MT_ERR_DEVICE;
   const int most = std::max(1, sms * MT_ENC_CTAS_PER_SM / kClusterCtas);
-  const int nclusters = std::min(width_max, most);
+  const int nclusters = std::min(width_max + width_max / 4, most);
   // With a cluster for every block that can run, a ticket is better left to the
   // cluster that can start it (1080p 9.05 -> 8.59 ms, 512x512 4:4:4 2.88 -> 2.71);
   // with fewer, the next ticket is wanted at once (4096x4096 42.1 -> 41.0 ms).
