@@ -170,3 +170,73 @@ def test_groups_of_tiles_give_the_bytes_of_one(mt_lib, cuda, sub, max_tokens, ng
             assert len(groups) == 1
     assert len(groups) > 1 and ngroups in (None, len(groups))
     assert len(got[0]) == 15 and got[0] == got[1]
+
+
+SEG, WARM, TXTP = 1024, 2, 66  # entries of a segment, warm-up segments, the tx-type CDF of DC_PRED
+
+
+class Cdf:
+    """update_cdf on an inverse CDF of n symbols, one symbol at a time."""
+
+    def __init__(self, entries, n, done=0):
+        self.c, self.n, self.done = [int(v) for v in entries[:n - 1]], n, done
+
+    def copy(self):
+        return Cdf(self.c, self.n, self.done)
+
+    def code(self, s):
+        """The store of symbol s (fl >> 6, fh >> 6 << 10, n - s << 20), then the update."""
+        c = self.c
+        word = ((c[s - 1] if s else 32768) >> 6) | ((c[s] if s < self.n - 1 else 0) >> 6) << 10 | (self.n - s) << 20
+        rate = 3 + min(self.n >> 1, 2) + (self.done >> 4)
+        for e in range(self.n - 1):
+            c[e] += ((32768 - c[e]) >> rate) if s > e else -(c[e] >> rate)
+        self.done = min(self.done + 1, 32)
+        return word
+
+
+def test_segments_that_started_wrong_are_redone(mt_lib, cuda):
+    """A list of 260 segments (two turns of 256) of a repeated pattern, on which
+    two states need not meet: most segments are adapted from a wrong state at
+    first, many in a row, and every store still is the one of the serial
+    adaptation."""
+    nbx, nby = 512, 520
+    nb = nbx * nby
+    y, x = np.mgrid[0:nby, 0:nbx]
+    z = sum(((x >> i) & 1) << (2 * i) | ((y >> i) & 1) << (2 * i + 1) for i in range(3))
+    pos = ((y >> 3) * (nbx // 8) + (x >> 3)) * 64 + z
+    seq = np.arange(nb) % 3 * 3  # the types' symbols, in coding order
+    luma = np.zeros((nb, 64), np.int32)
+    luma[:, 0] = 1
+    none = np.zeros((nb, 16), np.int32)
+    s = Steps(mt_lib.load(), cuda, nbx, nby, 2, (nbx, nby), 1 << 30)
+    (grp,) = s.load(np.zeros(nb, np.uint8), seq[pos].astype(np.uint8).ravel(), [luma, none, none])
+    s.trace(grp)
+    n = grp.tokens  # the buffer starts with the stores, an index and the tokens (4, 4 and 2 bytes each)
+    raw = s.tokens[:10 * n].cpu().numpy()
+    stores, tok = raw[:4 * n].view(np.uint32), raw[8 * n:].view(np.uint16)[:s.tiles()["ntok"][0]]
+    at = np.flatnonzero((tok & 255) == TXTP)
+    assert np.array_equal(tok[at] >> 8, seq) and len(seq) > 256 * SEG
+    cdf = Cdf(s.cdfs[TXTP], int(s.cdfs[TXTP][15]))
+    want, before = np.zeros(nb, np.uint32), []
+    symbols = seq.tolist()
+    for i, sym in enumerate(symbols):
+        if i % SEG == 0:
+            before.append(cdf.copy())
+        want[i] = cdf.code(sym)
+    # the segments of the first 24 whose warmed-up state is not the true one
+    wrong = []
+    rest = (1 << (5 + min(cdf.n >> 1, 2))) - 1
+    for k in range(WARM + 2, 24):
+        first = symbols[SEG:(k - WARM) * SEG]
+        guess = before[1].copy()
+        for e in range(cdf.n - 1):
+            if max(first) > e and guess.c[e] < rest:
+                guess.c[e] = rest
+            if min(first) <= e and guess.c[e] > 32768 - rest:
+                guess.c[e] = 32768 - rest
+        for sym in symbols[(k - WARM) * SEG:k * SEG]:
+            guess.code(sym)
+        wrong.append(guess.c != before[k].c)
+    assert sum(wrong) > 8 and any(a and b for a, b in zip(wrong, wrong[1:]))
+    assert np.array_equal(stores[at], want)
