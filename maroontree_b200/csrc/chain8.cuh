@@ -59,15 +59,8 @@ __device__ __forceinline__ uint32_t level_byte(uint32_t m) {
   return m == 0 ? 0u : (m <= 2 ? m * 0x41u : min(m, 15u) + 0xC0u);
 }
 
-// Round-down decision of one coefficient: the AVX2 FMA lane form
-// (src/avx/trellis.rs:79-118) or the scalar form (src/avx/trellis.rs:139-161).
-__device__ __forceinline__ bool round_down_fma(float at, int32_t li, float q2, float lambda) {
-  const int32_t ldi = max(li - 1, 0);
-  const float el = __fsub_rn(at, (float)li), ed = __fsub_rn(at, (float)ldi);
-  const float cl = __fmaf_rn(q2, __fmul_rn(el, el), __fmul_rn(lambda, kCoefRateLut[li]));
-  const float cd = __fmaf_rn(q2, __fmul_rn(ed, ed), __fmul_rn(lambda, kCoefRateLut[ldi]));
-  return cd < cl;
-}
+// Round-down decision of one coefficient, the scalar form
+// (src/avx/trellis.rs:139-161).
 __device__ __forceinline__ bool round_down_plain(float at, uint32_t l, float q2, float lambda) {
   const float el = __fsub_rn(at, (float)l), ed = __fsub_rn(at, (float)(l - 1));
   const float cl = __fadd_rn(__fmul_rn(q2, __fmul_rn(el, el)), __fmul_rn(lambda, coef_rate_bits(l)));

@@ -58,7 +58,6 @@ struct EncArgs {
   float tly, tlc;          // scaled trellis lambdas
   int has_qm_y, has_qm_c;  // a QM row for luma / chroma (level < 15)
   int sub;                 // 0 4:4:4, 2 4:2:0
-  int sb_cols;
   int w8, h8;
   int tile_w8, tile_h8;    // the uniform tile size in 8x8 blocks (the last tile may be smaller)
   uint8_t* mode;           // per 8x8 block (frame raster of 8x8 blocks)
@@ -1053,8 +1052,6 @@ int job_setup(Job& j, Buffers& buf, int i) {
   uint8_t* d_decs = buf.get<uint8_t>(i, kDecisions, (size_t)nb * 2);
   int32_t* d_levels = buf.get<int32_t>(i, kLevels, (size_t)nb * (64 + 2 * cl) * 4);
   mth::StreamGeom& sg = j.sg;
-  sg.w8 = pw;
-  sg.h8 = ph;
   sg.nbx = nbx;
   sg.nby = nby;
   sg.sub = sub;
@@ -1139,7 +1136,6 @@ int job_setup(Job& j, Buffers& buf, int i) {
   a.has_qm_y = qmy != nullptr;
   a.has_qm_c = qmc != nullptr;
   a.sub = sub;
-  a.sb_cols = sb_cols;
   a.w8 = pw;
   a.h8 = ph;
   a.tile_w8 = j.tile_sb_w * 8;

@@ -105,10 +105,6 @@ __device__ __forceinline__ int32_t dc_pred_sq_at(const R& rd, int ox, int oy, in
   if (top || left) return ((n >> 1) + sum) >> log2n;
   return 1 << (bd - 1);
 }
-__device__ __forceinline__ int32_t dc_pred_sq(const uint16_t* __restrict__ rec, int stride, int ox, int oy, int n,
-                                              int log2n, int bd) {
-  return dc_pred_sq_at(PlaneRead{rec, stride}, ox, oy, n, log2n, bd);
-}
 
 // Prediction of an N x N block (N = 4, 8, 16 or 32) into out[N*N] (row-major),
 // neighbours read through `rd`.  `scratch` holds 3 * edge_cap<N>() words: the

@@ -405,7 +405,7 @@ __device__ __forceinline__ void lane_level_map(W& w, const Lanes<N>& g) {
   w.lv[N * N + N + g.j] = 0;
 }
 
-// trellis_ctx<N> over the block's lanes (same parameters).  Returns the final
+// trellis_ctx8 at side N over the block's lanes (same parameters).  Returns the final
 // end of block (-1: all zero).
 template <int N, typename W>
 __device__ __forceinline__ int lane_trellis_ctx(W& w, float dc_q, float ac_q, float lambda, const mt_coef_costs& T,

@@ -660,7 +660,3 @@ int leaf_host(const uint16_t* src, const uint16_t* recon, const mt_split16_param
 }
 
 }  // namespace
-
-extern "C" {
-
-}  // extern "C"

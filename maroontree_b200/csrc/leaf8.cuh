@@ -43,27 +43,24 @@ __host__ __device__ constexpr int log2w() {
   return W == 4 ? 2 : (W == 8 ? 3 : (W == 16 ? 4 : 5));
 }
 
-// Scratch of trellis_ctx<W>: the zero-distortion suffix sums and the level map
-// (stride W with the reference's two zero columns of padding).
-template <int W>
-struct TrellisCtxScratchW {
-  float suf0[W * W + 1];
-  uint8_t lv[(W + 2) * W];
+// Scratch of trellis_ctx8: the zero-distortion suffix sums and the level map
+// (stride 8 with the reference's two zero columns of padding).
+struct TrellisCtxScratch {
+  float suf0[65];
+  uint8_t lv[80];
 };
-using TrellisCtxScratch = TrellisCtxScratchW<8>;
 
-// trellis_optimize_ctx of one TX_WxW luma block (W = 8: class 1, 16: class 2,
-// 32: class 3; plane 0; the cost slice of that class) under the
+// trellis_optimize_ctx of one TX_8X8 luma block (plane 0, class 1) under the
 // shipped tuning: trellis_aom / eob_reprice / eob_zero_term / pad_stride off,
 // dead zone 0, the DC-only terminal in eob_base context 0 with br context 0,
 // skip priced at trellis_zero_bits = 1, tilt magnitude cap 2.  `lambda` is
 // scaled_trellis_lambda (src/trellis.rs:50-53); qm (NULL = flat) the inverse
 // QM row, weighted w/32 and squared from QM level 5 (qm_full).
-template <int W, typename C>
-__device__ void trellis_ctx(C* __restrict__ cf, const float* __restrict__ tf, float dc_q, float ac_q, float lambda,
-                            const mt_coef_costs& T, int dcs, const uint8_t* __restrict__ qm, bool qm_full,
-                            float band_t, TrellisCtxScratchW<W>& s) {
-  constexpr int N = W * W, L = log2w<W>();
+template <typename C>
+__device__ void trellis_ctx8(C* __restrict__ cf, const float* __restrict__ tf, float dc_q, float ac_q, float lambda,
+                             const mt_coef_costs& T, int dcs, const uint8_t* __restrict__ qm, bool qm_full,
+                             float band_t, TrellisCtxScratch& s) {
+  constexpr int W = 8, N = W * W, L = log2w<W>();
   constexpr float kCap = 2.0f, kNInv = 1.0f / (float)N;
   int eob = -1;
   for (int i = N - 1; i >= 0; i--)
@@ -301,14 +298,6 @@ __device__ void trellis_ctx(C* __restrict__ cf, const float* __restrict__ tf, fl
     }
     for (int i = best_e + 1; i < m; i++) cf[scan_rc<W>(i)] = 0;
   }
-}
-
-template <typename C>
-__device__ __forceinline__ void trellis_ctx8(C* __restrict__ cf, const float* __restrict__ tf, float dc_q, float ac_q,
-                                             float lambda, const mt_coef_costs& T, int dcs,
-                                             const uint8_t* __restrict__ qm, bool qm_full, float band_t,
-                                             TrellisCtxScratch& s) {
-  trellis_ctx<8>(cf, tf, dc_q, ac_q, lambda, T, dcs, qm, qm_full, band_t, s);
 }
 
 // real_block_bits_bounded of a TX_WxW luma block (W = 4, 8, 16, 32: classes

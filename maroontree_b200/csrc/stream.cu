@@ -478,7 +478,6 @@ struct Lists {
   uint32_t* spos;   // [padded / kChunk] first store of a piece, or kNoStart
   uint16_t* gmap;   // [groups][128]
   uint16_t* gr;     // [groups] the range before a group
-  uint16_t* cr;     // [padded / kChunk] the range before a piece
   uint32_t* cd;     // [padded / kChunk] bits shifted out before a piece, in its group
   uint32_t* nd;     // [padded / kChunk] digits of a piece
   uint32_t* loc;    // [padded + 4 pieces] every piece's digits, its first bit at the top of a digit
@@ -1075,7 +1074,6 @@ __global__ void __launch_bounds__(kGroup) ranges_kernel(const Lists L, const Str
   __syncthreads();
   const StreamTile ti = tile[tile_of(tile, nt, blockIdx.x * kGroupTokens)];
   const uint32_t from = L.spos[c];
-  L.cr[c] = rs[t];
   uint32_t bits = 0;
   if (from != kNoStart) {
     uint32_t* dg = L.loc + from + 4 * c;
@@ -1245,7 +1243,6 @@ size_t carve_lists(const StreamGeom& g, uint32_t padded, void* mem, Lists* L) {
   L->spos = c.take<uint32_t>(nc);
   L->gmap = c.take<uint16_t>(ng * kClasses);
   L->gr = c.take<uint16_t>(ng);
-  L->cr = c.take<uint16_t>(nc);
   L->cd = c.take<uint32_t>(nc);
   L->nd = c.take<uint32_t>(nc);
   L->loc = c.take<uint32_t>(n + 4 * nc);

@@ -10,7 +10,6 @@ namespace mth {
 // The frame: 8x8 blocks in raster order, uniform tiles of tile_w8 x tile_h8
 // blocks (the last of a row or column smaller).
 struct StreamGeom {
-  int w8 = 0, h8 = 0;    // frame size in samples (multiples of 8)
   int nbx = 0, nby = 0;  // in 8x8 blocks
   int sub = 0;           // 2: 4:2:0, 0: 4:4:4
   int sb_cols = 0, sb_rows = 0;

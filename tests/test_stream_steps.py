@@ -13,8 +13,8 @@ GROUP_TOKENS = 256 * 64  # what a tile's tokens are padded to
 
 
 class Geom(C.Structure):
-    _fields_ = [(n, I32) for n in ("w8", "h8", "nbx", "nby", "sub", "sb_cols", "sb_rows", "tile_w8", "tile_h8",
-                                   "tcols", "trows")] + [("max_tokens", U32)]
+    _fields_ = [(n, I32) for n in ("nbx", "nby", "sub", "sb_cols", "sb_rows", "tile_w8", "tile_h8", "tcols",
+                                   "trows")] + [("max_tokens", U32)]
 
 
 class Input(C.Structure):
@@ -38,7 +38,7 @@ class Steps:
     def __init__(self, lib, torch, nbx, nby, sub, tile8, max_tokens):
         self.torch, self.n = torch, I32(0)
         up = lambda a, b: (a + b - 1) // b  # noqa: E731
-        self.g = Geom(nbx * 8, nby * 8, nbx, nby, sub, up(nbx, 8), up(nby, 8), tile8[0], tile8[1],
+        self.g = Geom(nbx, nby, sub, up(nbx, 8), up(nby, 8), tile8[0], tile8[1],
                       up(nbx, tile8[0]), up(nby, tile8[1]), max_tokens)
         self.nt = self.g.tcols * self.g.trows
 
