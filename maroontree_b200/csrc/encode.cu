@@ -825,12 +825,17 @@ class Buffers {
     BufSet& b = set(i);
     n = n ? n : 1;
     if (b.cap[s] < n) {
-      if (slack) n += n / 4;
       cudaFree(b.p[s]);
       b.p[s] = nullptr;
       b.cap[s] = 0;
-      if (cudaMalloc(&b.p[s], n) != cudaSuccess) return nullptr;
-      b.cap[s] = n;
+      const size_t more = slack ? n + n / 4 : n;
+      if (cudaMalloc(&b.p[s], more) == cudaSuccess) {
+        b.cap[s] = more;
+      } else {  // where the slack does not fit, without it
+        cudaGetLastError();
+        if (more == n || cudaMalloc(&b.p[s], n) != cudaSuccess) return nullptr;
+        b.cap[s] = n;
+      }
     }
     return reinterpret_cast<T*>(b.p[s]);
   }
