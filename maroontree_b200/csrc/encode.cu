@@ -1385,11 +1385,12 @@ int job_finish(Job& j, Buffers& buf, int i) {
     cs.d2h((ny + 2 * nc) * 2);
   }
   size_t ntok = 0;
-  std::vector<uint8_t> payload;
-  std::vector<size_t> tile_at;  // a tile's payload
+  std::vector<std::vector<uint8_t>> payloads;  // by group
+  std::vector<const uint8_t*> ctiles;
+  std::vector<size_t> tile_lens;
   for (;;) {
     mth::StreamTile* const gt = tile.data() + grp.tile0;
-    const size_t gt_bytes = (size_t)grp.ntiles * sizeof(tile[0]), before = payload.size();
+    const size_t gt_bytes = (size_t)grp.ntiles * sizeof(tile[0]);
     if (cudaMemcpyAsync(&tot, mth::stream_totals(j.sg, j.d_plan), sizeof(tot), cudaMemcpyDeviceToHost, sc) !=
             cudaSuccess ||
         cudaMemcpyAsync(gt, mth::stream_tiles(j.sg, j.d_plan) + grp.tile0, gt_bytes, cudaMemcpyDeviceToHost, sc) !=
@@ -1400,16 +1401,19 @@ int job_finish(Job& j, Buffers& buf, int i) {
     for (int k = 0; k < grp.ntiles; ++k) {
       longest = std::max(longest, gt[k].nbytes);
       ntok += gt[k].ntok;
-      tile_at.push_back(before + gt[k].byte);
     }
     void* d_dig = buf.get<void>(i, kDigits, mth::stream_digit_bytes(tot), true);
     if (!d_dig) return MT_ERR_DEVICE;
     const uint8_t* d_pay = mth::stream_bytes(j.sg, j.d_plan, d_tok, grp, d_dig, tot, longest, sc, &nl);
-    payload.resize(before + tot.bytes);
-    if (!d_pay ||
-        cudaMemcpyAsync(payload.data() + before, d_pay, tot.bytes, cudaMemcpyDeviceToHost, sc) != cudaSuccess ||
+    payloads.emplace_back(tot.bytes);
+    uint8_t* const payload = payloads.back().data();
+    if (!d_pay || cudaMemcpyAsync(payload, d_pay, tot.bytes, cudaMemcpyDeviceToHost, sc) != cudaSuccess ||
         cudaStreamSynchronize(sc) != cudaSuccess)
       return MT_ERR_DEVICE;
+    for (int k = 0; k < grp.ntiles; ++k) {
+      ctiles.push_back(payload + gt[k].byte);
+      tile_lens.push_back(gt[k].nbytes);
+    }
     cs.d2h(sizeof(tot) + gt_bytes + tot.bytes);
     if (grp.tile0 + grp.ntiles == ntiles) break;
     grp = mth::stream_group(tile.data(), ntiles, grp.tile0 + grp.ntiles);
@@ -1455,12 +1459,6 @@ int job_finish(Job& j, Buffers& buf, int i) {
     for (int q = 0; q < 4; ++q) fp.cdef_strengths[e][q] = dec.strengths[e][q];
   fp.tile_cols_log2 = j.tcl;
   fp.tile_rows_log2 = j.trl;
-  std::vector<const uint8_t*> ctiles;
-  std::vector<size_t> tile_lens;
-  for (int t = 0; t < ntiles; ++t) {
-    ctiles.push_back(payload.data() + tile_at[(size_t)t]);
-    tile_lens.push_back(tile[(size_t)t].nbytes);
-  }
   uint8_t* obu = nullptr;
   size_t obu_len = 0;
   rc = mt_av1_stream(&sp, &fp, ctiles.data(), tile_lens.data(), ntiles, &obu, &obu_len);
